@@ -20,6 +20,7 @@
 
 #include "driver_api.h"
 #include "nn_kernels.h"
+#include "pdl_launch.h"
 #include "ptx.cuh"
 #include "per_device.h"
 
@@ -53,7 +54,7 @@ struct AttSmem {
 template <int SEQ, bool VMN>
 __global__ void __launch_bounds__(ATT_THREADS)
 attention_tc(const __grid_constant__ CUtensorMap tmap_qk, const __grid_constant__ CUtensorMap tmap_vt,
-             __nv_bfloat16* __restrict__ out, int ld_out, const float* __restrict__ v_bias, int hidden, float scale_log2e,
+             __nv_bfloat16* out, int ld_out, const float* v_bias, int hidden, float scale_log2e,
              uint32_t* status) {
   using L = AttSmem<SEQ>;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -85,9 +86,11 @@ attention_tc(const __grid_constant__ CUtensorMap tmap_qk, const __grid_constant_
   if (warp == 4) {
     ptx::tmem_alloc(&tmem_base_smem, L::TMEM_COLS);
     ptx::tmem_relinquish();
+    ptx::grid_dep_launch();  // after the allocation, see pdl_launch.h
   }
   ptx::tc_fence_before();
   __syncthreads();
+  ptx::grid_dep_wait();
   ptx::tc_fence_after();
   const uint32_t tmem_s = tmem_base_smem;          // scores: columns [0, SEQ)
   const uint32_t tmem_o = tmem_base_smem + (L::ALIAS ? 0 : SEQ);  // output: columns [SEQ, SEQ+64), or over the scores
@@ -205,8 +208,8 @@ attention_tc(const __grid_constant__ CUtensorMap tmap_qk, const __grid_constant_
 #pragma unroll
           for (int t = 0; t < 4; t++) {
             const int d = c + j * 8 + 2 * t;
-            const float b0 = v_bias ? __ldg(v_bias + head * HD + d) : 0.f;
-            const float b1 = v_bias ? __ldg(v_bias + head * HD + d + 1) : 0.f;
+            const float b0 = v_bias ? *(v_bias + head * HD + d) : 0.f;
+            const float b1 = v_bias ? *(v_bias + head * HD + d + 1) : 0.f;
             h[t] = __floats2bfloat162_rn(__uint_as_float(r[j * 8 + 2 * t]) * inv + b0,
                                          __uint_as_float(r[j * 8 + 2 * t + 1]) * inv + b1);
           }
@@ -255,9 +258,8 @@ cudaError_t launch(const CUtensorMap& tqk, const CUtensorMap& tvt, void* out, in
     attr.set(dev);
   }
   const float scale_log2e = 0.125f * 1.4426950408889634f;
-  attention_tc<SEQ, VMN><<<dim3(heads, batch), ATT_THREADS, smem, s>>>(tqk, tvt, (__nv_bfloat16*)out, ld_out, v_bias, hidden,
-                                                                  scale_log2e, status);
-  return cudaGetLastError();
+  return launch_pdl(attention_tc<SEQ, VMN>, dim3(heads, batch), dim3(ATT_THREADS), smem, s, tqk, tvt, (__nv_bfloat16*)out, ld_out, v_bias,
+                    hidden, scale_log2e, status);
 }
 
 }  // namespace

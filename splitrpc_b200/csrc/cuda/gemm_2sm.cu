@@ -33,6 +33,7 @@
 #include <cstdlib>
 
 #include "gemm_tcgen05.h"
+#include "pdl_launch.h"
 #include "per_device.h"
 #include "ptx.cuh"
 #include "tp_device.cuh"
@@ -175,10 +176,12 @@ gemm_2sm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
   if (warp == 1) {
     ptx::tmem_alloc_2sm(&tmem_base_smem, TMEM_COLS);
     ptx::tmem_relinquish_2sm();
+    ptx::grid_dep_launch();  // after the allocation, see pdl_launch.h
   }
   ptx::tc_fence_before();
   __syncthreads();
   ptx::cluster_sync_all();  // the peer's barriers exist before anything signals them
+  ptx::grid_dep_wait();     // set-up above overlaps the kernel before; its results are read below
   ptx::tc_fence_after();
   const uint32_t tmem_base = tmem_base_smem;
   if (threadIdx.x == 0) GEMM2_TRACE(1);
@@ -282,7 +285,7 @@ gemm_2sm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
       const bool row_ok = m < M;
       const int n0 = t.n * BN;
       float* bias_s = s_bias;
-      if (ep.bias && et < BN) bias_s[et] = (n0 + et < N) ? __ldg(ep.bias + n0 + et) : 0.f;
+      if (ep.bias && et < BN) bias_s[et] = (n0 + et < N) ? *(ep.bias + n0 + et) : 0.f;
       const bool mine = (*(volatile uint32_t*)&s_error == 0) && ptx::mbar_wait(&tmem_full_bar[acc], (local >> 1) & 1u);
       if (!named_bar_all(2, EPI_THREADS, mine)) {  // uniform outcome; also orders the bias writes before their reads
         if (lane == 0) atomicExch(&s_error, GEMM_ERR_EPILOGUE_WAIT);
@@ -326,7 +329,7 @@ gemm_2sm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
             if (vec_res && col0 + 32 <= N) {
 #pragma unroll
               for (int q = 0; q < 4; q++) {
-                const uint4 rq = __ldg(reinterpret_cast<const uint4*>(rp) + q);
+                const uint4 rq = *(reinterpret_cast<const uint4*>(rp) + q);
                 const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&rq);
 #pragma unroll
                 for (int u = 0; u < 4; u++) {
@@ -485,8 +488,8 @@ cudaError_t launch_2sm(const void* A, int lda, const void* B, int ldb, int M, in
   o.clusters = std::min(o.tiles_m2 * o.tiles_n, std::min(max_clusters, srpc_gemm_grid_sms() / 2));
   o.group_m = 4;
   o.m_rot2 = 0;
-  gemm_2sm_kernel<BN, false><<<2 * o.clusters, C::THREADS, C::SMEM_BYTES, stream>>>(ta, tb, to, M, N, K, o, ep, status, TpParams{});
-  return cudaGetLastError();
+  return launch_pdl(gemm_2sm_kernel<BN, false>, dim3(2 * o.clusters), dim3(C::THREADS), C::SMEM_BYTES, stream, ta, tb, to, M, N, K,
+                    o, ep, status, TpParams{});
 }
 
 // Tensor-parallel launch: `tp` arrives with mblocks_per_rank / mblock_bytes filled in and an even n_copy.

@@ -32,6 +32,7 @@
 #include <unordered_map>
 
 #include "gemm_tcgen05.h"
+#include "pdl_launch.h"
 #include "ptx.cuh"
 #include "per_device.h"
 
@@ -277,6 +278,7 @@ gemm_conv_persistent(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
   uint32_t pr_ph = 0;
   bool pr_more = true;
   int img_off = 0;
+  if (threadIdx.x == 0) ptx::grid_dep_wait();  // set-up above overlaps the kernel before; its results are read below
   if (threadIdx.x == 0 && p.in_stub)
     img_off = (int)((*reinterpret_cast<const unsigned long long*>(p.in_stub) - p.in_ring_base) / p.in_slot_bytes);
   auto produce = [&](int budget) {
@@ -344,9 +346,11 @@ gemm_conv_persistent(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
   if (warp == 1) {
     ptx::tmem_alloc(&tmem_base_smem, ACC * ACC_STRIDE);
     ptx::tmem_relinquish();
+    ptx::grid_dep_launch();  // after the allocation, see pdl_launch.h
   }
   ptx::tc_fence_before();
   __syncthreads();
+  ptx::grid_dep_wait();
   ptx::tc_fence_after();
   const uint32_t tmem_base = tmem_base_smem;
   if (threadIdx.x == 0) GEMM_TRACE(1);
@@ -459,11 +463,11 @@ gemm_conv_persistent(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
       if (!LEAN && res_vec_tile) {
         const __nv_bfloat16* rp = ep.residual + row_off * ep.ldr + n0 + cbase;
 #pragma unroll
-        for (int j = 0; j < CPW / 8; j++) resq[j] = __ldg(reinterpret_cast<const uint4*>(rp) + j);
+        for (int j = 0; j < CPW / 8; j++) resq[j] = *(reinterpret_cast<const uint4*>(rp) + j);
       }
       if (j == 5 && et == 0) GEMM_TRACE(10);
       float* bias_s = s_bias[local & 1u];
-      if (ep.bias && et < BN) bias_s[et] = (n0 + et < p.N) ? __ldg(ep.bias + n0 + et) : 0.f;
+      if (ep.bias && et < BN) bias_s[et] = (n0 + et < p.N) ? *(ep.bias + n0 + et) : 0.f;
       // Each thread's wait is bounded; the vote makes the outcome uniform so that no
       // thread is left alone at a later barrier.  (It also orders the bias writes before their reads.)
       bool mine = (*(volatile uint32_t*)&s_error == 0) && ptx::mbar_wait(&tmem_full_bar[acc], (local >> ACC_LOG2) & 1u);
@@ -535,7 +539,7 @@ gemm_conv_persistent(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
           if (res_vec_tile) {
 #pragma unroll
             for (int j = 0; j < 4; j++) {
-              if (LEAN) resq[0] = __ldg(reinterpret_cast<const uint4*>(ep.residual + row_off * ep.ldr + col0) + j);
+              if (LEAN) resq[0] = *(reinterpret_cast<const uint4*>(ep.residual + row_off * ep.ldr + col0) + j);
               const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&resq[LEAN ? 0 : ch * 4 + j]);
 #pragma unroll
               for (int t = 0; t < 4; t++) {
@@ -785,8 +789,8 @@ cudaError_t launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorM
       grid = per_n * p.tiles_n;
     }
   }
-  gemm_conv_persistent<BN, STAGES, OB><<<grid, Threads<BN>::TOTAL, smem, st>>>(ta, tb, to, tr, p, ep, use_tma_store, status);
-  return cudaGetLastError();
+  return launch_pdl(gemm_conv_persistent<BN, STAGES, OB>, dim3(grid), dim3(Threads<BN>::TOTAL), smem, st, ta, tb, to, tr, p, ep,
+                    use_tma_store, status);
 }
 
 cudaError_t dispatch(int bn, const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& to, const CUtensorMap& tr,

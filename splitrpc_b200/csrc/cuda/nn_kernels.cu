@@ -11,6 +11,7 @@
 
 #include "../host/p2p_rpc_app.h"
 #include "nn_kernels.h"
+#include "pdl_launch.h"
 #include "per_device.h"
 #include "ptx.cuh"
 #include "resp_push.cuh"
@@ -47,8 +48,10 @@ __device__ __forceinline__ float block_sum(float v, float* sh) {
 // (x - mean[c]) * inv_std[c].  With this order one 16-byte chunk of a row is 7
 // consecutive input pixels of one image row and channel, so a thread reads 28
 // contiguous bytes and writes one 16-byte store.
-__global__ void __launch_bounds__(256) stem_im2col(const g_params* stub, const float* __restrict__ direct_in, int batch,
-                                                   __nv_bfloat16* __restrict__ out, float3 mean, float3 inv_std) {
+__global__ void __launch_bounds__(256) stem_im2col(const g_params* stub, const float* direct_in, int batch,
+                                                   __nv_bfloat16* out, float3 mean, float3 inv_std) {
+  ptx::grid_dep_launch();
+  ptx::grid_dep_wait();
   const float* in = direct_in ? direct_in : reinterpret_cast<const float*>(stub->req);
   const size_t total = (size_t)batch * 112 * 112 * 24;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
@@ -67,7 +70,7 @@ __global__ void __launch_bounds__(256) stem_im2col(const g_params* stub, const f
 #pragma unroll
         for (int j = 0; j < 7; j++) {
           const int ix = ix0 + j;
-          v[j] = (ix >= 0 && ix < 224) ? (__ldg(row + ix) - m) * s : 0.f;
+          v[j] = (ix >= 0 && ix < 224) ? (*(row + ix) - m) * s : 0.f;
         }
         v[7] = 0.f;
         __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&o);
@@ -85,8 +88,10 @@ __global__ void __launch_bounds__(256) stem_im2col(const g_params* stub, const f
 // channel c (zero outside the image; channels 6, 7, 14, 15 are zero).  Four horizontally adjacent pixels are 64
 // contiguous channels, so the convolution reads its rows straight from this array through a tensor map whose pixel
 // stride is 16 elements: no im2col matrix is ever written (27 MB per 64 images instead of 308 MB).
-__global__ void __launch_bounds__(256) stem_s2d(const g_params* stub, const float* __restrict__ direct_in, int batch,
-                                                __nv_bfloat16* __restrict__ out, float3 mean, float3 inv_std) {
+__global__ void __launch_bounds__(256) stem_s2d(const g_params* stub, const float* direct_in, int batch,
+                                                __nv_bfloat16* out, float3 mean, float3 inv_std) {
+  ptx::grid_dep_launch();
+  ptx::grid_dep_wait();
   const float* in = direct_in ? direct_in : reinterpret_cast<const float*>(stub->req);
   const size_t total = (size_t)batch * 115 * 115 * 2;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
@@ -106,7 +111,7 @@ __global__ void __launch_bounds__(256) stem_s2d(const g_params* stub, const floa
 #pragma unroll
         for (int dx = 0; dx < 2; dx++) {
           const int ix = ix0 + dx;
-          if (ix >= 0 && ix < 224) v[dx * 3 + c] = (__ldg(row + ix) - m) * s;
+          if (ix >= 0 && ix < 224) v[dx * 3 + c] = (*(row + ix) - m) * s;
         }
       }
     }
@@ -121,8 +126,10 @@ __global__ void __launch_bounds__(256) stem_s2d(const g_params* stub, const floa
 // 3x3 stride-2 pad-1 max pooling, NHWC bf16, 8 channels per thread.  Window positions outside the image are clamped
 // to the nearest pixel inside (a duplicate does not change a maximum), so the nine 16-byte loads of a thread carry no
 // branches and are all in flight together.
-__global__ void __launch_bounds__(256) maxpool3x3s2(const __nv_bfloat16* __restrict__ in, __nv_bfloat16* __restrict__ out,
+__global__ void __launch_bounds__(256) maxpool3x3s2(const __nv_bfloat16* in, __nv_bfloat16* out,
                                                     int n, int h, int w, int c) {
+  ptx::grid_dep_launch();
+  ptx::grid_dep_wait();
   const int oh = (h + 2 - 3) / 2 + 1, ow = (w + 2 - 3) / 2 + 1, cv = c / 8;
   const size_t total = (size_t)n * oh * ow * cv;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
@@ -138,7 +145,7 @@ __global__ void __launch_bounds__(256) maxpool3x3s2(const __nv_bfloat16* __restr
 #pragma unroll
       for (int dx = 0; dx < 3; dx++) {
         const int ix = min(max(ox * 2 - 1 + dx, 0), w - 1);
-        q[dy * 3 + dx] = __ldg(reinterpret_cast<const uint4*>(in + (((size_t)b * h + iy) * w + ix) * c + cc * 8));
+        q[dy * 3 + dx] = *(reinterpret_cast<const uint4*>(in + (((size_t)b * h + iy) * w + ix) * c + cc * 8));
       }
     }
     __nv_bfloat162 m[4];
@@ -163,8 +170,10 @@ __global__ void __launch_bounds__(256) maxpool3x3s2(const __nv_bfloat16* __restr
 
 // Global average pooling NHWC -> [n, c]; block (x = channel chunk of 512, y = image), two channels per thread, the
 // pixel loop unrolled so that several loads are in flight.
-__global__ void __launch_bounds__(256) global_avgpool(const __nv_bfloat16* __restrict__ in, __nv_bfloat16* __restrict__ out,
+__global__ void __launch_bounds__(256) global_avgpool(const __nv_bfloat16* in, __nv_bfloat16* out,
                                                       int hw, int c) {
+  ptx::grid_dep_launch();
+  ptx::grid_dep_wait();
   const int b = blockIdx.y, ch = (blockIdx.x * 256 + threadIdx.x) * 2;
   if (ch >= c) return;
   const __nv_bfloat16* src = in + (size_t)b * hw * c + ch;
@@ -196,9 +205,11 @@ __global__ void __launch_bounds__(256) global_avgpool(const __nv_bfloat16* __res
 // (row pair, kq) walks every sixteenth 8-element slice of its two rows of `a` with the next slice's loads in flight, and
 // the sixteen partial sums of a row meet through shuffles.
 constexpr int FC_NB = 8, FC_ROWS = 32;
-__global__ void __launch_bounds__(256, 2) fc_skinny(const __nv_bfloat16* __restrict__ a, int lda, const __nv_bfloat16* __restrict__ w,
-                                                 int ldw, const float* __restrict__ bias, float* __restrict__ out, int ldo, int M,
+__global__ void __launch_bounds__(256, 2) fc_skinny(const __nv_bfloat16* a, int lda, const __nv_bfloat16* w,
+                                                 int ldw, const float* bias, float* out, int ldo, int M,
                                                  int N, int K) {
+  ptx::grid_dep_launch();
+  ptx::grid_dep_wait();
   extern __shared__ __align__(16) float4 s_w[];  // [FC_NB][2][K/8]
   const int n0 = blockIdx.x * FC_NB, kvn = K / 8;
   for (int base = 0; base < FC_NB * kvn; base += 256 * 8) {
@@ -207,7 +218,7 @@ __global__ void __launch_bounds__(256, 2) fc_skinny(const __nv_bfloat16* __restr
     for (int u = 0; u < 8; u++) {
       const int i = base + u * 256 + threadIdx.x, col = i / kvn, kv = i - col * kvn;
       q[u] = make_uint4(0, 0, 0, 0);
-      if (i < FC_NB * kvn && n0 + col < N) q[u] = __ldg(reinterpret_cast<const uint4*>(w + (size_t)(n0 + col) * ldw + kv * 8));
+      if (i < FC_NB * kvn && n0 + col < N) q[u] = *(reinterpret_cast<const uint4*>(w + (size_t)(n0 + col) * ldw + kv * 8));
     }
 #pragma unroll
     for (int u = 0; u < 8; u++) {
@@ -256,7 +267,7 @@ __global__ void __launch_bounds__(256, 2) fc_skinny(const __nv_bfloat16* __restr
     }
   };
   auto load = [&](const __nv_bfloat16* r, int kv) {
-    return kv < kvn ? __ldg(reinterpret_cast<const uint4*>(r + kv * 8)) : make_uint4(0, 0, 0, 0);
+    return kv < kvn ? *(reinterpret_cast<const uint4*>(r + kv * 8)) : make_uint4(0, 0, 0, 0);
   };
   // two slices per trip, the next trip's four loads issued before this trip's arithmetic
   uint4 qa0 = load(ar0, kq), qa1 = load(ar1, kq), qb0 = load(ar0, kq + 16), qb1 = load(ar1, kq + 16);
@@ -299,10 +310,12 @@ __global__ void __launch_bounds__(256, 2) fc_skinny(const __nv_bfloat16* __restr
 // With a response-push block (`push`, see resp_push.cuh) each row goes straight to
 // the place the producer named for its slot (the ingress transmit arena, in another
 // process's pinned memory or on a peer GPU) and the row's block completes the slot.
-__global__ void __launch_bounds__(256) softmax_response(const float* __restrict__ logits, int n, int ld, const g_params* stub,
+__global__ void __launch_bounds__(256) softmax_response(const float* logits, int n, int ld, const g_params* stub,
                                                         uint8_t* direct_out, size_t resp_stride, int write_argmax,
                                                         uint32_t* counter, volatile uint32_t* flag, uint32_t flag_value,
                                                         const RespPushCtx* push) {
+  ptx::grid_dep_launch();
+  ptx::grid_dep_wait();
   __shared__ float sh[32];
   __shared__ float s_max, s_sum;
   __shared__ int s_arg;
@@ -378,10 +391,12 @@ __global__ void __launch_bounds__(256) softmax_response(const float* __restrict_
 
 // ------------------------------------------------------------------ LayerNorm (+ residual)
 // y = LN(x + residual) * gamma + beta, one row per block; hidden <= 8 * blockDim.x.
-__global__ void __launch_bounds__(256) layernorm_rows(const __nv_bfloat16* __restrict__ x,
-                                                      const __nv_bfloat16* __restrict__ residual,
-                                                      const float* __restrict__ gamma, const float* __restrict__ beta,
-                                                      __nv_bfloat16* __restrict__ y, int hidden, float eps) {
+__global__ void __launch_bounds__(256) layernorm_rows(const __nv_bfloat16* x,
+                                                      const __nv_bfloat16* residual,
+                                                      const float* gamma, const float* beta,
+                                                      __nv_bfloat16* y, int hidden, float eps) {
+  ptx::grid_dep_launch();
+  ptx::grid_dep_wait();
   __shared__ float sh[32];
   const size_t row = blockIdx.x;
   const __nv_bfloat16* xr = x + row * hidden;
@@ -408,10 +423,12 @@ __global__ void __launch_bounds__(256) layernorm_rows(const __nv_bfloat16* __res
 // Warp-per-row LayerNorm for hidden sizes that are multiples of 256 (up to 2048): each lane owns hidden/32 values as
 // 16-byte vectors, the row never leaves registers, and both reductions are warp shuffles.
 template <int VPL>  // uint4 vectors per lane: hidden = VPL * 256
-__global__ void __launch_bounds__(256) layernorm_rows_warp(const __nv_bfloat16* __restrict__ x,
-                                                           const __nv_bfloat16* __restrict__ residual,
-                                                           const float* __restrict__ gamma, const float* __restrict__ beta,
-                                                           __nv_bfloat16* __restrict__ y, int rows, float eps) {
+__global__ void __launch_bounds__(256) layernorm_rows_warp(const __nv_bfloat16* x,
+                                                           const __nv_bfloat16* residual,
+                                                           const float* gamma, const float* beta,
+                                                           __nv_bfloat16* y, int rows, float eps) {
+  ptx::grid_dep_launch();
+  ptx::grid_dep_wait();
   constexpr int HIDDEN = VPL * 256;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int row = blockIdx.x * 8 + warp;
@@ -443,8 +460,8 @@ __global__ void __launch_bounds__(256) layernorm_rows_warp(const __nv_bfloat16* 
 #pragma unroll
   for (int i = 0; i < VPL; i++) {
     const int c0 = (i * 32 + lane) * 8;
-    const float4 g0 = __ldg(reinterpret_cast<const float4*>(gamma + c0)), g1 = __ldg(reinterpret_cast<const float4*>(gamma + c0 + 4));
-    const float4 b0 = __ldg(reinterpret_cast<const float4*>(beta + c0)), b1 = __ldg(reinterpret_cast<const float4*>(beta + c0 + 4));
+    const float4 g0 = *(reinterpret_cast<const float4*>(gamma + c0)), g1 = *(reinterpret_cast<const float4*>(gamma + c0 + 4));
+    const float4 b0 = *(reinterpret_cast<const float4*>(beta + c0)), b1 = *(reinterpret_cast<const float4*>(beta + c0 + 4));
     const float gg[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
     const float bb[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
     uint4 o;
@@ -460,12 +477,14 @@ __global__ void __launch_bounds__(256) layernorm_rows_warp(const __nv_bfloat16* 
 // ------------------------------------------------------------------ BERT embedding
 // Request = seq int32 token ids per sequence.  y[token] = LN(word[id] + pos[t] + type[0]).
 // Reads ids through the stub (ring window) or from `direct_ids`.
-__global__ void __launch_bounds__(256) bert_embed_ln(const g_params* stub, const int* __restrict__ direct_ids, size_t req_stride,
-                                                     int seq, const __nv_bfloat16* __restrict__ word,
-                                                     const __nv_bfloat16* __restrict__ pos,
-                                                     const __nv_bfloat16* __restrict__ type, const float* __restrict__ gamma,
-                                                     const float* __restrict__ beta, __nv_bfloat16* __restrict__ y, int hidden,
+__global__ void __launch_bounds__(256) bert_embed_ln(const g_params* stub, const int* direct_ids, size_t req_stride,
+                                                     int seq, const __nv_bfloat16* word,
+                                                     const __nv_bfloat16* pos,
+                                                     const __nv_bfloat16* type, const float* gamma,
+                                                     const float* beta, __nv_bfloat16* y, int hidden,
                                                      int vocab, float eps) {
+  ptx::grid_dep_launch();
+  ptx::grid_dep_wait();
   __shared__ float sh[32];
   const int tok = blockIdx.x, b = tok / seq, t = tok - b * seq;
   const int* ids = direct_ids ? direct_ids + (size_t)b * seq
@@ -568,30 +587,27 @@ int grid_for(size_t total, int threads) {
 cudaError_t nn_stem_im2col(const void* d_stub, const float* direct_in, int batch, void* out, const float mean[3],
                            const float inv_std[3], cudaStream_t s) {
   size_t total = (size_t)batch * 112 * 112 * 24;
-  stem_im2col<<<grid_for(total, 256), 256, 0, s>>>((const g_params*)d_stub, direct_in, batch, (__nv_bfloat16*)out,
-                                                   make_float3(mean[0], mean[1], mean[2]),
-                                                   make_float3(inv_std[0], inv_std[1], inv_std[2]));
-  return cudaGetLastError();
+  return launch_pdl(stem_im2col, dim3(grid_for(total, 256)), dim3(256), 0, s, (const g_params*)d_stub, direct_in, batch,
+                    (__nv_bfloat16*)out, make_float3(mean[0], mean[1], mean[2]), make_float3(inv_std[0], inv_std[1],
+                    inv_std[2]));
 }
 cudaError_t nn_stem_s2d(const void* d_stub, const float* direct_in, int batch, void* out, const float mean[3],
                         const float inv_std[3], cudaStream_t s) {
   size_t total = (size_t)batch * 115 * 115 * 2;
-  stem_s2d<<<grid_for(total, 256), 256, 0, s>>>((const g_params*)d_stub, direct_in, batch, (__nv_bfloat16*)out,
-                                                make_float3(mean[0], mean[1], mean[2]),
-                                                make_float3(inv_std[0], inv_std[1], inv_std[2]));
-  return cudaGetLastError();
+  return launch_pdl(stem_s2d, dim3(grid_for(total, 256)), dim3(256), 0, s, (const g_params*)d_stub, direct_in, batch,
+                    (__nv_bfloat16*)out, make_float3(mean[0], mean[1], mean[2]), make_float3(inv_std[0], inv_std[1],
+                    inv_std[2]));
 }
 cudaError_t nn_maxpool3x3s2(const void* in, void* out, int n, int h, int w, int c, cudaStream_t s) {
   if (c % 8) return cudaErrorInvalidValue;
   int oh = (h - 1) / 2 + 1, ow = (w - 1) / 2 + 1;
-  maxpool3x3s2<<<grid_for((size_t)n * oh * ow * (c / 8), 256), 256, 0, s>>>((const __nv_bfloat16*)in, (__nv_bfloat16*)out, n,
-                                                                          h, w, c);
-  return cudaGetLastError();
+  return launch_pdl(maxpool3x3s2, dim3(grid_for((size_t)n * oh * ow * (c / 8), 256)), dim3(256), 0, s, (const __nv_bfloat16*)in,
+                    (__nv_bfloat16*)out, n, h, w, c);
 }
 cudaError_t nn_global_avgpool(const void* in, void* out, int n, int hw, int c, cudaStream_t s) {
   if (c % 2) return cudaErrorInvalidValue;
-  global_avgpool<<<dim3((c + 511) / 512, n), 256, 0, s>>>((const __nv_bfloat16*)in, (__nv_bfloat16*)out, hw, c);
-  return cudaGetLastError();
+  return launch_pdl(global_avgpool, dim3((c + 511) / 512, n), dim3(256), 0, s, (const __nv_bfloat16*)in, (__nv_bfloat16*)out,
+                    hw, c);
 }
 cudaError_t nn_fc_skinny(const void* a, int lda, const void* w, int ldw, const float* bias, float* out, int ldo, int M, int N, int K,
                          cudaStream_t s) {
@@ -604,17 +620,15 @@ cudaError_t nn_fc_skinny(const void* a, int lda, const void* w, int ldw, const f
     if (e != cudaSuccess) return e;
     attr_set.set(dev);
   }
-  fc_skinny<<<dim3((N + FC_NB - 1) / FC_NB, (M + FC_ROWS - 1) / FC_ROWS), 256, smem, s>>>((const __nv_bfloat16*)a, lda, (const __nv_bfloat16*)w,
-                                                                          ldw, bias, out, ldo, M, N, K);
-  return cudaGetLastError();
+  return launch_pdl(fc_skinny, dim3((N + FC_NB - 1) / FC_NB, (M + FC_ROWS - 1) / FC_ROWS), dim3(256), smem, s, (const
+                    __nv_bfloat16*)a, lda, (const __nv_bfloat16*)w, ldw, bias, out, ldo, M, N, K);
 }
 cudaError_t nn_softmax_response(const float* logits, int rows, int n, int ld, const void* d_stub, void* direct_out,
                                 size_t resp_stride, int write_argmax, uint32_t* counter, uint32_t* flag, uint32_t flag_value,
                                 cudaStream_t s, const void* d_push) {
   if (rows <= 0) return cudaSuccess;
-  softmax_response<<<rows, 256, 0, s>>>(logits, n, ld, (const g_params*)d_stub, (uint8_t*)direct_out, resp_stride,
-                                        write_argmax, counter, flag, flag_value, (const RespPushCtx*)d_push);
-  return cudaGetLastError();
+  return launch_pdl(softmax_response, dim3(rows), dim3(256), 0, s, logits, n, ld, (const g_params*)d_stub, (uint8_t*)direct_out,
+                    resp_stride, write_argmax, counter, flag, flag_value, (const RespPushCtx*)d_push);
 }
 cudaError_t nn_layernorm(const void* x, const void* residual, const float* gamma, const float* beta, void* y, int rows,
                          int hidden, float eps, cudaStream_t s) {
@@ -623,21 +637,23 @@ cudaError_t nn_layernorm(const void* x, const void* residual, const float* gamma
   const int grid = (rows + 7) / 8;
   const __nv_bfloat16 *xp = (const __nv_bfloat16*)x, *rp = (const __nv_bfloat16*)residual;
   __nv_bfloat16* yp = (__nv_bfloat16*)y;
-  if (aligned && hidden == 768) layernorm_rows_warp<3><<<grid, 256, 0, s>>>(xp, rp, gamma, beta, yp, rows, eps);
-  else if (aligned && hidden == 1024) layernorm_rows_warp<4><<<grid, 256, 0, s>>>(xp, rp, gamma, beta, yp, rows, eps);
-  else if (aligned && hidden == 512) layernorm_rows_warp<2><<<grid, 256, 0, s>>>(xp, rp, gamma, beta, yp, rows, eps);
-  else if (aligned && hidden == 256) layernorm_rows_warp<1><<<grid, 256, 0, s>>>(xp, rp, gamma, beta, yp, rows, eps);
-  else layernorm_rows<<<rows, 256, 0, s>>>(xp, rp, gamma, beta, yp, hidden, eps);
-  return cudaGetLastError();
+  if (aligned && hidden == 768) return launch_pdl(layernorm_rows_warp<3>, dim3(grid), dim3(256), 0, s, xp, rp, gamma, beta, yp,
+                                                  rows, eps);
+  if (aligned && hidden == 1024) return launch_pdl(layernorm_rows_warp<4>, dim3(grid), dim3(256), 0, s, xp, rp, gamma, beta, yp,
+                                                   rows, eps);
+  if (aligned && hidden == 512) return launch_pdl(layernorm_rows_warp<2>, dim3(grid), dim3(256), 0, s, xp, rp, gamma, beta, yp,
+                                                  rows, eps);
+  if (aligned && hidden == 256) return launch_pdl(layernorm_rows_warp<1>, dim3(grid), dim3(256), 0, s, xp, rp, gamma, beta, yp,
+                                                  rows, eps);
+  return launch_pdl(layernorm_rows, dim3(rows), dim3(256), 0, s, xp, rp, gamma, beta, yp, hidden, eps);
 }
 cudaError_t nn_bert_embed_ln(const void* d_stub, const int* direct_ids, size_t req_stride, int batch, int seq, const void* word,
                              const void* pos, const void* type, const float* gamma, const float* beta, void* y, int hidden,
                              int vocab, float eps, cudaStream_t s) {
   if (hidden > 2048) return cudaErrorInvalidValue;
-  bert_embed_ln<<<batch * seq, 256, 0, s>>>((const g_params*)d_stub, direct_ids, req_stride, seq, (const __nv_bfloat16*)word,
-                                            (const __nv_bfloat16*)pos, (const __nv_bfloat16*)type, gamma, beta,
-                                            (__nv_bfloat16*)y, hidden, vocab, eps);
-  return cudaGetLastError();
+  return launch_pdl(bert_embed_ln, dim3(batch * seq), dim3(256), 0, s, (const g_params*)d_stub, direct_ids, req_stride, seq,
+                    (const __nv_bfloat16*)word, (const __nv_bfloat16*)pos, (const __nv_bfloat16*)type, gamma, beta,
+                    (__nv_bfloat16*)y, hidden, vocab, eps);
 }
 cudaError_t nn_attention_d64(const void* qkv, void* out, int batch, int seq, int heads, int ld_qkv, int q_off, int k_off,
                              int v_off, int ld_out, cudaStream_t s) {

@@ -59,6 +59,13 @@ __device__ __forceinline__ uint64_t ld_relaxed_sys_u64(const uint64_t* p) {
   return v;
 }
 
+// ---------------------------------------------------------------- programmatic dependent launch (see pdl_launch.h)
+// Waits until the kernel before this one in the stream has finished and its writes are visible (returns at once in a
+// kernel that was launched the ordinary way).
+__device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Lets the next kernel's blocks be scheduled once every block of this grid has called it or left.
+__device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ---------------------------------------------------------------- mbarrier
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
