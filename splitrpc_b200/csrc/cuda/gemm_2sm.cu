@@ -8,7 +8,7 @@
 // and writes 128 accumulator rows into each CTA's tensor memory.
 //
 // Protocol (both CTAs run the same code; rank 0 of the pair is the leader):
-//   producer   thread 0 of each CTA loads its A rows and its half of B for every k-block through a 5-stage ring.  The
+//   producer   two threads of each CTA, in turn, load its A rows and its half of B for every k-block into a stage ring.  The
 //              "full" barrier of a stage is the LEADER's: the leader's producer posts the expected byte count of both
 //              CTAs, and both CTAs' TMA loads (cp.async.bulk.tensor ... cta_group::2, no multicast) count on it.
 //   MMA        one thread of the leader waits for a full stage, issues four 256 x 256 x 16 MMAs and commits them to
@@ -61,7 +61,7 @@ struct Cfg {
   static constexpr int STAGES = BN == 256 ? 6 : (BN == 192 ? 6 : 7);
   static constexpr int OUT_BYTES = (PASS_COLS / 64) * OUT_HALF_BYTES;
   static constexpr int EPI_THREADS = 2 * BN;
-  static constexpr int THREADS = 64 + EPI_THREADS;
+  static constexpr int THREADS = 64 + EPI_THREADS + 32;  // TMA, MMA, epilogue, second TMA warp
   static constexpr int ACC_STRIDE = BN == 192 ? 256 : BN;  // TMEM columns between the two accumulators
   static constexpr int TMEM_COLS = 2 * ACC_STRIDE;
   static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + OUT_BYTES;
@@ -186,12 +186,16 @@ gemm_2sm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
   const uint32_t tmem_base = tmem_base_smem;
   if (threadIdx.x == 0) GEMM2_TRACE(1);
 
-  if (threadIdx.x == 0) {
-    // ---------------- producer (one per CTA)
-    int s = 0;
+  if (warp == 0 || warp == Cfg<BN>::THREADS / 32 - 1) {
+    // ---------------- producers: one lane each of two warps per CTA take the k-blocks in turn (see gemm_persistent.cu)
+    constexpr int PRODUCERS = 2;
+    int kb = warp == 0 ? 0 : 1, s = kb, j = 0;
     uint32_t ph = 0;
     PairTile t;
-    for (int j = 0; layout_ok && pair_tile(j, order, &t) && *(volatile uint32_t*)&s_error == 0; j++) {
+    bool ok = layout_ok && lane == 0;
+    while (ok) {
+      for (; kb >= num_kb; kb -= num_kb) j++;
+      if (!pair_tile(j, order, &t) || *(volatile uint32_t*)&s_error != 0) break;
       const int row0 = (t.m2 * 2 + (int)rank) * BM;
       const int brow0 = t.n * BN + (int)rank * (BN / 2);
       if constexpr (TP) {
@@ -207,9 +211,10 @@ gemm_2sm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
           }
         }
       }
-      for (int kb = 0; kb < num_kb; kb++) {
+      for (; kb < num_kb; kb += PRODUCERS) {
         if (!ptx::mbar_wait(&empty_bar[s], ph ^ 1u)) {
           atomicExch(&s_error, GEMM_ERR_PRODUCER_WAIT);
+          ok = false;
           break;
         }
         const uint32_t full_leader = ptx::mapa_shared(ptx::smem_u32(&full_bar[s]), 0);
@@ -218,56 +223,59 @@ gemm_2sm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
         ptx::tma_load_2d_2sm(sa, &tmap_a, full_leader, kb * BK, row0);
         ptx::tma_load_2d_2sm(sa + A_BYTES, &tmap_b, full_leader, kb * BK, brow0);
         if (j == 0 && kb == 0) GEMM2_TRACE(2);
-        if (++s == STAGES) {
-          s = 0;
+        s += PRODUCERS;
+        if (s >= STAGES) {
+          s -= STAGES;
           ph ^= 1u;
         }
       }
     }
-  } else if (threadIdx.x == 32) {
-    // ---------------- MMA issue (leader only)
+  } else if (warp == 1) {
+    // ---------------- MMA issue (leader only): the warp walks the schedule together, one elected lane issues, so that
+    // descriptors and addresses stay in uniform registers (see gemm_persistent.cu)
     if (leader) {
+      const bool elected = ptx::elect_one();
       const uint32_t idesc = ptx::umma_idesc_bf16(2 * BM, BN);
+      const uint32_t ring_lo = ptx::umma_desc_lo(ptx::smem_u32(smem));
+      constexpr uint32_t K_LO = UMMA_K * 2 / 16;
       int s = 0;
       uint32_t ph = 0, local = 0;
       PairTile t;
-      for (int j = 0; layout_ok && pair_tile(j, order, &t) && *(volatile uint32_t*)&s_error == 0; j++, local++) {
+      bool ok = layout_ok;
+      for (int j = 0; ok && pair_tile(j, order, &t); j++, local++) {
         const uint32_t acc = local & 1u;
-        if (!ptx::mbar_wait(&tmem_empty_bar[acc], ((local >> 1) & 1u) ^ 1u)) {
-          atomicExch(&s_error, GEMM_ERR_MMA_WAIT);
-          break;
-        }
+        ok = ptx::mbar_wait_warp(&tmem_empty_bar[acc], ((local >> 1) & 1u) ^ 1u);
+        if (!ok) break;
         ptx::tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * ACC_STRIDE;
-        bool ok = true;
         for (int kb = 0; kb < num_kb; kb++) {
-          if (!ptx::mbar_wait(&full_bar[s], ph)) {
-            atomicExch(&s_error, GEMM_ERR_MMA_WAIT);
-            ok = false;
-            break;
-          }
-          ptx::tc_fence_after();
-          if (j == 0 && kb == 0) GEMM2_TRACE(3);
-          if (j == 0 && kb == 8) GEMM2_TRACE(10);
-          if (j == 0 && kb == 24) GEMM2_TRACE(11);
-          const uint32_t sa = ptx::smem_u32(smem + (size_t)s * STAGE_BYTES);
-          const uint32_t sb = sa + A_BYTES;
+          ok = ptx::mbar_wait_warp(&full_bar[s], ph);
+          if (!ok) break;
+          if (j == 0 && kb == 0 && lane == 0) GEMM2_TRACE(3);
+          if (j == 0 && kb == 8 && lane == 0) GEMM2_TRACE(10);
+          if (j == 0 && kb == 24 && lane == 0) GEMM2_TRACE(11);
+          const uint32_t sa = ring_lo + (uint32_t)s * (STAGE_BYTES / 16), sb = sa + A_BYTES / 16;
+          if (elected) {
 #pragma unroll
-          for (int k = 0; k < BK / UMMA_K; k++)
-            ptx::umma_bf16_2sm(d_tmem, ptx::umma_desc_sw128(sa + k * UMMA_K * 2), ptx::umma_desc_sw128(sb + k * UMMA_K * 2), idesc,
-                               (kb | k) != 0 ? 1u : 0u);
-          ptx::umma_commit_2sm(&empty_bar[s], 3);  // frees the stage in both CTAs
+            for (int k = 0; k < BK / UMMA_K; k++)
+              ptx::umma_bf16_2sm(d_tmem, ptx::umma_desc_join(sa + k * K_LO), ptx::umma_desc_join(sb + k * K_LO), idesc,
+                                 (kb | k) != 0 ? 1u : 0u);
+            ptx::umma_commit_2sm(&empty_bar[s], 3);  // frees the stage in both CTAs
+          }
           if (++s == STAGES) {
             s = 0;
             ph ^= 1u;
           }
         }
         if (!ok) break;
-        ptx::umma_commit_2sm(&tmem_full_bar[acc], 3);
-        if (j == 0) GEMM2_TRACE(4);
+        if (elected) ptx::umma_commit_2sm(&tmem_full_bar[acc], 3);
+        if (j == 0 && lane == 0) GEMM2_TRACE(4);
+        ok = *(volatile uint32_t*)&s_error == 0;
+        ok = __all_sync(0xffffffffu, ok);
       }
+      if (!ok && elected) atomicCAS(&s_error, 0u, (uint32_t)GEMM_ERR_MMA_WAIT);
     }
-  } else if (warp >= 2) {
+  } else {
     // ---------------- epilogue: the warps of a TMEM lane quarter (w, w+4, ...) split the columns of a pass
     const int warp_q = warp & 3;
     const int cgroup = (warp - 2) >> 2;      // 0 .. EPI_THREADS/128 - 1
@@ -286,7 +294,8 @@ gemm_2sm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
       const int n0 = t.n * BN;
       float* bias_s = s_bias;
       if (ep.bias && et < BN) bias_s[et] = (n0 + et < N) ? *(ep.bias + n0 + et) : 0.f;
-      const bool mine = (*(volatile uint32_t*)&s_error == 0) && ptx::mbar_wait(&tmem_full_bar[acc], (local >> 1) & 1u);
+      // one warp polls, the others wait for it at the hardware barrier (see gemm_persistent.cu)
+      const bool mine = warp != 2 || ((*(volatile uint32_t*)&s_error == 0) && ptx::mbar_wait(&tmem_full_bar[acc], (local >> 1) & 1u));
       if (!named_bar_all(2, EPI_THREADS, mine)) {  // uniform outcome; also orders the bias writes before their reads
         if (lane == 0) atomicExch(&s_error, GEMM_ERR_EPILOGUE_WAIT);
         break;

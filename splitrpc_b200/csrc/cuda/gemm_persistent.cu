@@ -4,9 +4,9 @@
 //   out = act(conv(in NHWC, filter [Cout][R][S][Cin]) + bias + residual)   (convolution mode)
 //
 // One CTA per SM loops over output tiles (128 x BN).  Warp roles:
-//   warp 0   one elected thread issues TMA loads for every k-block of every tile
-//            of this CTA, running ahead through a STAGES-deep shared-memory ring
-//            that is not drained at tile boundaries;
+//   warp 0 and the last warp   one thread each issues the TMA loads of every second
+//            k-block of this CTA's tiles, running ahead through a STAGES-deep
+//            shared-memory ring that is not drained at tile boundaries;
 //   warp 1   one elected thread issues tcgen05.mma into one of two TMEM
 //            accumulators (2 x BN columns), so tile i+1 accumulates while tile i
 //            is being written out;
@@ -58,7 +58,7 @@ template <int BN>
 struct Threads {
   // BN = 256 / 192: four / three warps per quarter, 64 columns each
   static constexpr int EPI = BN == 256 ? 512 : (BN == 192 ? 384 : (BN == 128 ? SRPC_EPI128 : 256));
-  static constexpr int TOTAL = 64 + EPI + 32;  // + the store warp
+  static constexpr int TOTAL = 64 + EPI + 64;  // + the store warp, the second producer warp
 };
 
 // Division by a launch-time constant as multiply-high + shift (dividends below 2^24): every thread of every role
@@ -104,7 +104,7 @@ struct TileParams {
   // short-tile k loop) for a 3 x 3 filter.  num_kb then counts load groups (s * cblocks); panel_kb counts all k-blocks.
   int reuse;
   int panel_kb;
-  FastDiv fd_tiles_n, fd_group, fd_tiles_w, fd_tiles_h;  // filled in by launch()
+  FastDiv fd_tiles_n, fd_group, fd_tiles_w, fd_tiles_h, fd_cblocks, fd_s;  // filled in by launch()
   // Input that lives in a request ring (convolution mode): the tensor map covers the whole ring, one "image" per slot,
   // and the batch starts at the slot that the app stub's request pointer names when the kernel runs, so one captured
   // graph serves every ring position.  in_stub == nullptr: the input starts at image 0.
@@ -271,77 +271,83 @@ gemm_conv_persistent(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
     if (use_tma_store) ptx::prefetch_tmap(&tmap_out);
     if (p.res_tma) ptx::prefetch_tmap(&tmap_res);
   }
-  // TMA producer = thread 0.  Its state lives across two calls: the first fills the (initially free) ring right after
-  // the barriers exist, before the block-wide set-up barrier, so that the first operands are already in flight while
-  // tensor memory is being allocated; the second runs the rest of the schedule.
-  int pr_s = 0, pr_j = 0, pr_kb = 0;
+  // TMA producers: the elected lanes of warp 0 and of the last warp take the k-blocks of this CTA's schedule in turn (even
+  // ones, odd ones).  One of them needs about 250 ns per k-block (wait for the stage, post the byte count, issue two
+  // loads), as long as the tensor pipe takes for the widest tile and twice as long as for a 128-wide one.  Measured with
+  // two producers and the uniform MMA loop below: 258 -> 211 ns per k-block of a single 128 x 128 tile; 3x3 convolutions of
+  // 64 images: 56x56x64 44.0 -> 30.3 us, 14x14x256 25.7 -> 22.3 us, 7x7x512 39.9 -> 22.9 us.
+  // The state lives across two calls: the first fills one (initially free) stage each right after the barriers exist,
+  // before the block-wide set-up barrier, so that the first operands are already in flight while tensor memory is being
+  // allocated; the second runs the rest of the schedule.
+  constexpr int PRODUCERS = 2;
+  const int producer = warp == 0 ? 0 : (warp == Threads<BN>::TOTAL / 32 - 1 ? 1 : -1);
+  int pr_s = producer, pr_kb = producer, pr_j = 0;
   uint32_t pr_ph = 0;
-  bool pr_more = true;
   int img_off = 0;
-  if (threadIdx.x == 0) ptx::grid_dep_wait();  // set-up above overlaps the kernel before; its results are read below
-  if (threadIdx.x == 0 && p.in_stub)
-    img_off = (int)((*reinterpret_cast<const unsigned long long*>(p.in_stub) - p.in_ring_base) / p.in_slot_bytes);
-  auto produce = [&](int budget) {
-    const uint32_t b_tx = (uint32_t)(b_per_stage * B_BYTES);
-    TileCoord tc;
-    while (pr_more && budget > 0) {
-      if (!get_tile(p, pr_j, &tc) || *(volatile uint32_t*)&s_error != 0) {
-        pr_more = false;
-        break;
-      }
-      for (; pr_kb < p.num_kb && budget > 0; pr_kb++, budget--) {
-        if (!ptx::mbar_wait(&empty_bar[pr_s], pr_ph ^ 1u)) {
-          atomicExch(&s_error, GEMM_ERR_PRODUCER_WAIT);
-          pr_more = false;
-          return;
-        }
-        uint8_t* sa = a_ring + (size_t)pr_s * a_stride;
-        if (p.mode == 0) {
-          ptx::mbar_expect_tx(&full_bar[pr_s], (uint32_t)A_BYTES + b_tx);
-          ptx::tma_load_2d(sa, &tmap_a, &full_bar[pr_s], pr_kb * BK, tc.m_idx * BM);
-        } else if (p.reuse) {
-          // load group (fs, cb): the box covers filter rows 0 .. r-1 at once
-          ptx::mbar_expect_tx(&full_bar[pr_s], p.a_box_bytes + b_tx);
-          const int fs = pr_kb / p.cblocks, cb = pr_kb - fs * p.cblocks;
-          tma_load_4d_box(sa, &tmap_a, &full_bar[pr_s], cb * BK, tc.w0 + fs - p.pad, tc.h0 - p.pad, tc.img0 + img_off);
-          if (!p.b_stationary)
-            for (int fr = 0; fr < p.r; fr++)
-              ptx::tma_load_2d(sa + A_BYTES + fr * B_BYTES, &tmap_b, &full_bar[pr_s], ((fr * p.s + fs) * p.cblocks + cb) * BK,
-                               tc.n_idx * BN);
-        } else {
-          ptx::mbar_expect_tx(&full_bar[pr_s], p.a_box_bytes + b_tx);
-          if (pr_kb >= p.kb_split) {
-            // second input of a two-input 1x1 convolution (its map travels in the residual map's place)
-            tma_load_4d_box(sa, &tmap_res, &full_bar[pr_s], (pr_kb - p.kb_split) * BK, tc.w0 * p.stride2, tc.h0 * p.stride2,
-                            tc.img0);
-          } else {
-            const int tap = pr_kb / p.cblocks, cb = pr_kb - tap * p.cblocks;
-            const int fr = tap / p.s, fs = tap - fr * p.s;
-            tma_load_4d_box(sa, &tmap_a, &full_bar[pr_s], cb * BK, tc.w0 * p.stride + fs - p.pad,
-                            tc.h0 * p.stride + fr - p.pad, tc.img0 + img_off);
-          }
-        }
-        if (!p.b_stationary && !p.reuse) ptx::tma_load_2d(sa + A_BYTES, &tmap_b, &full_bar[pr_s], pr_kb * BK, tc.n_idx * BN);
-        if (pr_j == 0 && pr_kb == 0) GEMM_TRACE(2);
-        if (++pr_s == nst) {
-          pr_s = 0;
-          pr_ph ^= 1u;
-        }
-      }
-      if (pr_kb == p.num_kb) {
-        pr_kb = 0;
-        pr_j++;
+  TileCoord pr_tc;
+  bool pr_more = false;
+  // Moves to the tile that holds k-block pr_kb; false when the schedule is through.
+  auto producer_tile = [&]() {
+    while (pr_kb >= p.num_kb) {
+      pr_kb -= p.num_kb;
+      pr_j++;
+    }
+    return get_tile(p, pr_j, &pr_tc) && *(volatile uint32_t*)&s_error == 0;
+  };
+  const uint32_t b_tx = (uint32_t)(b_per_stage * B_BYTES);
+  auto produce_one = [&]() {
+    if (!ptx::mbar_wait(&empty_bar[pr_s], pr_ph ^ 1u)) {
+      atomicExch(&s_error, GEMM_ERR_PRODUCER_WAIT);
+      pr_more = false;
+      return;
+    }
+    uint8_t* sa = a_ring + (size_t)pr_s * a_stride;
+    if (p.mode == 0) {
+      ptx::mbar_expect_tx(&full_bar[pr_s], (uint32_t)A_BYTES + b_tx);
+      ptx::tma_load_2d(sa, &tmap_a, &full_bar[pr_s], pr_kb * BK, pr_tc.m_idx * BM);
+    } else {
+      ptx::mbar_expect_tx(&full_bar[pr_s], p.a_box_bytes + b_tx);
+      const int tap = (int)fdiv(p.fd_cblocks, (uint32_t)pr_kb), cb = pr_kb - tap * p.cblocks;
+      if (p.reuse) {
+        // load group (fs, cb): the box covers filter rows 0 .. r-1 at once
+        const int fs = tap;
+        tma_load_4d_box(sa, &tmap_a, &full_bar[pr_s], cb * BK, pr_tc.w0 + fs - p.pad, pr_tc.h0 - p.pad, pr_tc.img0 + img_off);
+        if (!p.b_stationary)
+          for (int fr = 0; fr < p.r; fr++)
+            ptx::tma_load_2d(sa + A_BYTES + fr * B_BYTES, &tmap_b, &full_bar[pr_s], ((fr * p.s + fs) * p.cblocks + cb) * BK,
+                             pr_tc.n_idx * BN);
+      } else if (pr_kb >= p.kb_split) {
+        // second input of a two-input 1x1 convolution (its map travels in the residual map's place)
+        tma_load_4d_box(sa, &tmap_res, &full_bar[pr_s], (pr_kb - p.kb_split) * BK, pr_tc.w0 * p.stride2, pr_tc.h0 * p.stride2,
+                        pr_tc.img0);
+      } else {
+        const int fr = (int)fdiv(p.fd_s, (uint32_t)tap), fs = tap - fr * p.s;
+        tma_load_4d_box(sa, &tmap_a, &full_bar[pr_s], cb * BK, pr_tc.w0 * p.stride + fs - p.pad, pr_tc.h0 * p.stride + fr - p.pad,
+                        pr_tc.img0 + img_off);
       }
     }
+    if (!p.b_stationary && !p.reuse) ptx::tma_load_2d(sa + A_BYTES, &tmap_b, &full_bar[pr_s], pr_kb * BK, pr_tc.n_idx * BN);
+    if (pr_j == 0 && pr_kb == 0) GEMM_TRACE(2);
+    pr_kb += PRODUCERS;
+    pr_s += PRODUCERS;
+    if (pr_s >= nst) {
+      pr_s -= nst;
+      pr_ph ^= 1u;
+    }
   };
-  if (threadIdx.x == 0 && layout_ok) {
+  if (warp == 0) __syncwarp();
+  const bool produces = producer >= 0 && layout_ok && lane == 0;
+  if (producer == 0 && lane == 0) {
+    ptx::grid_dep_wait();  // set-up above overlaps the kernel before; its results are read below
+    if (p.in_stub)
+      img_off = (int)((*reinterpret_cast<const unsigned long long*>(p.in_stub) - p.in_ring_base) / p.in_slot_bytes);
     TileCoord tc;
-    if (p.b_stationary && get_tile(p, 0, &tc)) {
+    if (layout_ok && p.b_stationary && get_tile(p, 0, &tc)) {
       ptx::mbar_expect_tx(&bpanel_bar, (uint32_t)panel_bytes);
       for (int kb = 0; kb < p.panel_kb; kb++)
         ptx::tma_load_2d(smem + (size_t)kb * B_BYTES, &tmap_b, &bpanel_bar, kb * BK, tc.n_idx * BN);
     }
-    produce(nst < 2 ? nst : 2);  // more would hold thread 0 (and with it the set-up barrier) behind a full TMA queue
+    if (layout_ok && (pr_more = producer_tile())) produce_one();
   }
   if (warp == 1) {
     ptx::tmem_alloc(&tmem_base_smem, ACC * ACC_STRIDE);
@@ -355,70 +361,82 @@ gemm_conv_persistent(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
   const uint32_t tmem_base = tmem_base_smem;
   if (threadIdx.x == 0) GEMM_TRACE(1);
 
-  if (threadIdx.x == 0) {
-    produce(1 << 30);  // the rest of the k-blocks, paced by the MMA warp through the empty barriers
-  } else if (warp == 0) {
-    // lanes 1-31 of the producer warp have nothing to do
-  } else if (warp == 1) {
-    if (ptx::elect_one()) {
-      const uint32_t idesc = ptx::umma_idesc_bf16(BM, BN);
-      uint32_t local = 0;
-      int s = 0;
-      uint32_t ph = 0;
-      TileCoord tc;
-      bool panel_ok = true;
-      if (p.b_stationary && get_tile(p, 0, &tc)) {
-        panel_ok = ptx::mbar_wait(&bpanel_bar, 0);
-        if (!panel_ok) atomicExch(&s_error, GEMM_ERR_MMA_WAIT);
+  if (producer >= 0) {
+    if (producer == 1) {
+      if (p.in_stub)
+        img_off = (int)((*reinterpret_cast<const unsigned long long*>(p.in_stub) - p.in_ring_base) / p.in_slot_bytes);
+      pr_more = true;
+    }
+    // the rest of this producer's k-blocks, paced by the MMA warp through the empty barriers
+    if (produces && pr_more)
+      while (producer_tile()) {
+        const int j = pr_j;
+        while (pr_more && pr_j == j && pr_kb < p.num_kb) produce_one();
+        if (!pr_more) break;
       }
-      for (int j = 0; panel_ok && get_tile(p, j, &tc) && *(volatile uint32_t*)&s_error == 0; j++, local++) {
-        const uint32_t acc = local & (ACC - 1);
-        if (!ptx::mbar_wait(&tmem_empty_bar[acc], ((local >> ACC_LOG2) & 1u) ^ 1u)) {
-          atomicExch(&s_error, GEMM_ERR_MMA_WAIT);
-          break;
-        }
-        ptx::tc_fence_after();
-        const uint32_t d_tmem = tmem_base + acc * ACC_STRIDE;
-        bool ok = true;
-        for (int kb = 0; kb < p.num_kb; kb++) {
-          if (!ptx::mbar_wait(&full_bar[s], ph)) {
-            atomicExch(&s_error, GEMM_ERR_MMA_WAIT);
-            ok = false;
-            break;
-          }
-          ptx::tc_fence_after();
-          if (j == 0 && kb == 0) GEMM_TRACE(3);
-          const uint32_t sa = ptx::smem_u32(a_ring + (size_t)s * a_stride);
-          if (p.reuse) {
-            const int fs = kb / p.cblocks, cb = kb - fs * p.cblocks;
-            for (int fr = 0; fr < p.r; fr++) {
-              const uint32_t sa_fr = sa + (uint32_t)(fr * p.pw * 128);  // fr image rows further into the box
-              const uint32_t sb = p.b_stationary
-                                      ? ptx::smem_u32(smem + (size_t)((fr * p.s + fs) * p.cblocks + cb) * B_BYTES)
-                                      : sa + A_BYTES + fr * B_BYTES;
+  } else if (warp == 1) {
+    // The whole warp walks the schedule and waits together; one elected lane issues.  Every value that a tcgen05
+    // instruction takes lives in uniform registers then; with the loop inside the elected lane's branch each of them was
+    // moved there one by one, and issuing a k-block (four MMAs) took 260 ns whatever the tile's width, up to three times
+    // the tensor pipe's own time.  No tcgen05 fence per k-block: the operands arrive through TMA and an mbarrier, no
+    // tcgen05 instruction of another thread has to be ordered before the MMAs here.
+    const bool elected = ptx::elect_one();
+    const uint32_t idesc = ptx::umma_idesc_bf16(BM, BN);
+    const uint32_t ring_lo = ptx::umma_desc_lo(ptx::smem_u32(a_ring)), stride_lo = (uint32_t)a_stride >> 4;
+    const uint32_t panel_lo = ptx::umma_desc_lo(ptx::smem_u32(smem));
+    constexpr uint32_t K_LO = UMMA_K * 2 / 16;  // descriptor step from one 16-deep slice to the next
+    uint32_t local = 0;
+    int s = 0;
+    uint32_t ph = 0;
+    TileCoord tc;
+    bool ok = true;
+    if (p.b_stationary && get_tile(p, 0, &tc)) ok = ptx::mbar_wait_warp(&bpanel_bar, 0);
+    for (int j = 0; ok && get_tile(p, j, &tc); j++, local++) {
+      const uint32_t acc = local & (ACC - 1);
+      ok = ptx::mbar_wait_warp(&tmem_empty_bar[acc], ((local >> ACC_LOG2) & 1u) ^ 1u);
+      if (!ok) break;
+      ptx::tc_fence_after();
+      const uint32_t d_tmem = tmem_base + acc * ACC_STRIDE;
+      for (int kb = 0; kb < p.num_kb; kb++) {
+        ok = ptx::mbar_wait_warp(&full_bar[s], ph);
+        if (!ok) break;
+        if (j == 0 && kb == 0 && lane == 0) GEMM_TRACE(3);
+        const uint32_t sa = ring_lo + (uint32_t)s * stride_lo;
+        if (p.reuse) {
+          const int fs = kb / p.cblocks, cb = kb - fs * p.cblocks;
+          for (int fr = 0; fr < p.r; fr++) {
+            const uint32_t sa_fr = sa + (uint32_t)(fr * p.pw * 128 / 16);  // fr image rows further into the box
+            const uint32_t sb = p.b_stationary ? panel_lo + (uint32_t)((fr * p.s + fs) * p.cblocks + cb) * (B_BYTES / 16)
+                                               : sa + (uint32_t)(A_BYTES + fr * B_BYTES) / 16;
+            if (elected) {
 #pragma unroll
               for (int k = 0; k < BK / UMMA_K; k++)
-                ptx::umma_bf16(d_tmem, ptx::umma_desc_sw128(sa_fr + k * UMMA_K * 2), ptx::umma_desc_sw128(sb + k * UMMA_K * 2),
-                               idesc, (kb | fr | k) != 0 ? 1u : 0u);
+                ptx::umma_bf16(d_tmem, ptx::umma_desc_join(sa_fr + k * K_LO), ptx::umma_desc_join(sb + k * K_LO), idesc,
+                               (kb | fr | k) != 0 ? 1u : 0u);
             }
-          } else {
-            const uint32_t sb = p.b_stationary ? ptx::smem_u32(smem + (size_t)kb * B_BYTES) : sa + A_BYTES;
+          }
+        } else {
+          const uint32_t sb = p.b_stationary ? panel_lo + (uint32_t)kb * (B_BYTES / 16) : sa + A_BYTES / 16;
+          if (elected) {
 #pragma unroll
             for (int k = 0; k < BK / UMMA_K; k++)
-              ptx::umma_bf16(d_tmem, ptx::umma_desc_sw128(sa + k * UMMA_K * 2), ptx::umma_desc_sw128(sb + k * UMMA_K * 2), idesc,
+              ptx::umma_bf16(d_tmem, ptx::umma_desc_join(sa + k * K_LO), ptx::umma_desc_join(sb + k * K_LO), idesc,
                              (kb | k) != 0 ? 1u : 0u);
           }
-          ptx::umma_commit(&empty_bar[s]);
-          if (++s == nst) {
-            s = 0;
-            ph ^= 1u;
-          }
         }
-        if (!ok) break;
-        ptx::umma_commit(&tmem_full_bar[acc]);
-        if (j == 0) GEMM_TRACE(4);
+        if (elected) ptx::umma_commit(&empty_bar[s]);
+        if (++s == nst) {
+          s = 0;
+          ph ^= 1u;
+        }
       }
+      if (!ok) break;
+      if (elected) ptx::umma_commit(&tmem_full_bar[acc]);
+      if (j == 0 && lane == 0) GEMM_TRACE(4);
+      ok = *(volatile uint32_t*)&s_error == 0;
+      ok = __all_sync(0xffffffffu, ok);
     }
+    if (!ok && elected) atomicCAS(&s_error, 0u, (uint32_t)GEMM_ERR_MMA_WAIT);
   } else if (warp < 2 + Threads<BN>::EPI / 32) {
     // ---------------- epilogue warps (8): warp pair (w, w+4) shares a TMEM lane quarter and splits the columns
     constexpr int CPW = BN / (Threads<BN>::EPI / 128);  // columns per warp
@@ -468,13 +486,18 @@ gemm_conv_persistent(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
       if (j == 5 && et == 0) GEMM_TRACE(10);
       float* bias_s = s_bias[local & 1u];
       if (ep.bias && et < BN) bias_s[et] = (n0 + et < p.N) ? *(ep.bias + n0 + et) : 0.f;
-      // Each thread's wait is bounded; the vote makes the outcome uniform so that no
-      // thread is left alone at a later barrier.  (It also orders the bias writes before their reads.)
-      bool mine = (*(volatile uint32_t*)&s_error == 0) && ptx::mbar_wait(&tmem_full_bar[acc], (local >> ACC_LOG2) & 1u);
-      // The staging buffer: with a prefetched residual it is ready when the residual has landed (the store warp loads
-      // it only into a buffer whose last store has been read); otherwise when the store warp has handed it back.
-      if (res_tma && mine) mine = ptx::mbar_wait(&res_full_bar[local % OB], (local / OB) & 1u);
-      else if (use_tma_store && mine) mine = ptx::mbar_wait(&out_empty_bar[local % OB], ((local / OB) & 1u) ^ 1u);
+      // One warp waits for the accumulator and the staging buffer, the others for that warp at a hardware barrier: a
+      // dozen warps polling the same barrier words keep the shared-memory pipe busy that the producer's and the MMA
+      // warp's hand-offs go through.  Its wait is bounded; the vote makes the outcome uniform so that no thread is left
+      // alone at a later barrier, and orders the wait and the bias writes before what follows.
+      bool mine = true;
+      if (warp == 2) {
+        mine = (*(volatile uint32_t*)&s_error == 0) && ptx::mbar_wait(&tmem_full_bar[acc], (local >> ACC_LOG2) & 1u);
+        // The staging buffer: with a prefetched residual it is ready when the residual has landed (the store warp loads
+        // it only into a buffer whose last store has been read); otherwise when the store warp has handed it back.
+        if (res_tma && mine) mine = ptx::mbar_wait(&res_full_bar[local % OB], (local / OB) & 1u);
+        else if (use_tma_store && mine) mine = ptx::mbar_wait(&out_empty_bar[local % OB], ((local / OB) & 1u) ^ 1u);
+      }
       if (!named_bar_all(2, EPI_THREADS, mine)) {
         if (lane == 0) atomicExch(&s_error, GEMM_ERR_EPILOGUE_WAIT);
         break;
@@ -597,7 +620,7 @@ gemm_conv_persistent(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
         if (lane == 0) ptx::mbar_arrive(&out_full_bar[local % OB]);
       }
     }
-  } else if (lane == 0 && use_tma_store) {
+  } else if (warp == 2 + Threads<BN>::EPI / 32 && lane == 0 && use_tma_store) {
     // ---------------- store warp (one thread): TMA stores of finished tiles, residual prefetch, buffer hand-back
     const bool res_tma = OB > RES_DIST && p.res_tma != 0;
     // Loads the residual tile of this CTA's jj-th tile into staging buffer jj % OB (one elected thread).
@@ -776,6 +799,8 @@ cudaError_t launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorM
   p.fd_group = make_fastdiv((uint32_t)(8 * p.tiles_n));  // GROUP_M row blocks x all column blocks (see get_tile)
   p.fd_tiles_w = make_fastdiv((uint32_t)(p.tiles_w > 0 ? p.tiles_w : 1));
   p.fd_tiles_h = make_fastdiv((uint32_t)(p.tiles_h > 0 ? p.tiles_h : 1));
+  p.fd_cblocks = make_fastdiv((uint32_t)(p.cblocks > 0 ? p.cblocks : 1));
+  p.fd_s = make_fastdiv((uint32_t)(p.s > 0 ? p.s : 1));
   static const int allow_bs = [] { const char* e = getenv("SPLITRPC_GEMM_BSTAT"); return e ? atoi(e) : 1; }();
   // The panel may take the ring's memory as long as three A stages remain (a 3x3 convolution over 64 channels keeps its
   // nine 8 KB filter taps resident: otherwise every CTA re-reads the same few L2 lines for every tile).

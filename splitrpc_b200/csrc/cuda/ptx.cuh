@@ -110,6 +110,11 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
   }
 }
 
+// Bounded wait of a whole (converged) warp.  The vote makes the outcome, and with it the control flow behind it, uniform.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity));
+}
+
 // ---------------------------------------------------------------- math
 // GELU with the exact (erf) definition, x * Phi(x), from the rational approximation of erfc by Abramowitz & Stegun
 // 7.1.26 (absolute error of erf below 1.5e-7, far under bf16 resolution): 7 FMA/MUL, one rcp.approx and one ex2.approx
@@ -220,6 +225,12 @@ __device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t smem_addr) {
   d |= (uint64_t)2 << 61;                             // layout: SWIZZLE_128B
   return d;
 }
+
+// The same descriptor from its two words: the high word is a constant, the low word (start address / 16) advances by
+// bytes / 16 from one operand tile to the next, so that a loop over tiles costs one addition per operand.
+constexpr uint32_t UMMA_DESC_SW128_HI = (1024u >> 4) | (1u << 14) | (2u << 29);
+__device__ __forceinline__ uint32_t umma_desc_lo(uint32_t smem_addr) { return ((smem_addr & 0x3FFFF) >> 4) | (1u << 16); }
+__device__ __forceinline__ uint64_t umma_desc_join(uint32_t lo) { return ((uint64_t)UMMA_DESC_SW128_HI << 32) | lo; }
 
 // Instruction descriptor for kind::f16 with bf16 A/B (both K-major) and fp32 D.
 __device__ __host__ constexpr uint32_t umma_idesc_bf16(int M, int N) {
