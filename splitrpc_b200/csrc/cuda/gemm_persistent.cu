@@ -861,42 +861,45 @@ int srpc_gemm_trace_read(unsigned long long* out, int n) {
 }
 
 // Tile shape.  Narrow outputs take 64 columns.  Otherwise the shape with the lowest estimated time wins: rounds of
-// tiles over the SMs (or SM pairs) x (k-blocks x time per k-block + hand-over).  The per-k-block times are what the
-// kernels measure on large problems: the one-SM 128-wide tile is bound by the issue rate of its four MMAs per
-// k-block, the wider one-SM tiles by operand delivery, the two-SM tiles (256 rows per SM pair, gemm_2sm.cu) by the
-// tensor pipe.  Returns the width; *two_sm says which kernel.
-static int pick_tile(int M, int N, int num_kb, bool bf16_out, bool allow_two_sm, bool* two_sm) {
+// tiles over the SMs (or SM pairs) x (k-blocks x time per k-block + hand-over).  The per-k-block times are measured with
+// every SM busy (rounds x k-blocks of 4096 .. 6144 x 768 .. 4096 products with K = 768 .. 4096): the one-SM tiles are bound by
+// operand delivery (32 - 48 KB per k-block and SM), the two-SM tiles (256 rows per SM pair, gemm_2sm.cu) take a third less
+// of it.  With these figures 6144 x 1024 x 4096 takes pairs of 256 x 192 tiles (50.3 -> 42.6 us), 6144 x 1024 x 1024 too
+// (22.3 -> 17.9 us), 1024 x 768 x 3072 takes 64 columns (16.4 -> 15.1 us).  Below eight k-blocks memory and the epilogue
+// decide; the older figures pick the right shapes there.  Returns the width; *two_sm says which kernel, *cost_us the estimate.
+static int pick_tile(int M, int N, int num_kb, bool bf16_out, bool allow_two_sm, bool* two_sm, double* cost_us = nullptr) {
   static const int allow256 = [] { const char* e = getenv("SPLITRPC_GEMM_BN256"); return e ? atoi(e) : 1; }();
   static const int allow192 = [] { const char* e = getenv("SPLITRPC_GEMM_BN192"); return e ? atoi(e) : 1; }();
   *two_sm = false;
-  if (N <= 64) return 64;
   struct Cand {
     int bn, rows, units;
-    double t_kb;  // microseconds per 64-deep k-block
+    double t_kb, t_short;  // microseconds per 64-deep k-block; the same for the choice among short k loops
     bool pair;
   };
   const int sms = num_sms();
-  // (the pair kernels run at about 0.4 us per k-block whatever their width: the stage ring covers one round trip
-  //  MMA done -> stage free -> TMA -> stage full, not more)
-  const Cand cands[6] = {{256, 256, sms / 2, 0.40, true},  {192, 256, sms / 2, 0.40, true}, {128, 256, sms / 2, 0.40, true},
-                         {256, 128, sms, 0.49, false},     {192, 128, sms, 0.37, false},    {128, 128, sms, 0.27, false}};
-  int best = 128;
+  const Cand cands[7] = {{256, 256, sms / 2, 0.35, 0.40, true},  {192, 256, sms / 2, 0.29, 0.40, true}, {128, 256, sms / 2, 0.23, 0.40, true},
+                         {256, 128, sms, 0.43, 0.49, false},     {192, 128, sms, 0.335, 0.37, false},   {128, 128, sms, 0.25, 0.27, false},
+                         {64, 128, sms, 0.21, 0.27, false}};
+  int best = N <= 64 ? 64 : 128;
   double best_cost = 1e30;
   for (const Cand& c : cands) {
+    if (N <= 64 && c.bn != 64) continue;
+    if (N > 64 && c.bn == 64 && num_kb < 8) continue;
     // pairs only where the k loop dominates: short-K shapes are bound by memory and keep the B-stationary schedule
     if (c.pair && !(allow_two_sm && M >= 256 && num_kb >= 8)) continue;
     if (c.bn == 256 && !(allow256 && bf16_out && N >= 256 && ((N % 256) == 0 || N >= 1024))) continue;
-    if (c.bn == 192 && !(allow192 && bf16_out && N >= 192 && ((N % 192) == 0 || N >= 1536))) continue;
+    if (c.bn == 192 && !(allow192 && bf16_out && N >= 192 && ((N % 192) == 0 || N >= 1024))) continue;
     if (c.pair && c.bn == 128 && (N % 128) != 0 && N < 1024) continue;
     const long tiles = (long)((M + c.rows - 1) / c.rows) * ((N + c.bn - 1) / c.bn);
     const long rounds = (tiles + c.units - 1) / c.units;
-    const double cost = (double)rounds * (num_kb * c.t_kb + 0.25) + (c.pair ? 0.3 : 0.0);  // pairs: cluster set-up
+    const double cost = (double)rounds * (num_kb * (num_kb >= 8 ? c.t_kb : c.t_short) + 0.25) + (c.pair ? 0.8 : 0.0);  // pairs: cluster set-up
     if (cost < best_cost * 0.98) {  // near-ties go to the candidate listed first
       best_cost = cost;
       best = c.bn;
       *two_sm = c.pair;
     }
   }
+  if (cost_us) *cost_us = best_cost;
   return best;
 }
 
