@@ -47,6 +47,25 @@ def test_sg_copy_matches_reference(C, torch_cuda, impl, align):
     assert torch.equal(dst, ref)
 
 
+@pytest.mark.parametrize("lens", [[1] * 300, [16384] * 40, [5] * 20 + [900000] + [7] * 20, [900000] + [3] * 200, [16385, 1, 40000, 16384] * 9])
+@pytest.mark.parametrize("n_blocks", [0, 7, -2])
+def test_sg_copy_finds_every_chunk(C, torch_cuda, lens, n_blocks):
+    """Lists whose items are far from the place that their share of the chunks suggests, one chunk per item, and exactly
+    full chunks; every pair of source and destination alignments occurs."""
+    torch = torch_cuda
+    src = torch.randint(0, 256, (sum(lens) + 64 * len(lens),), dtype=torch.uint8, device="cuda")
+    dst, ref = torch.zeros_like(src), torch.zeros_like(src)
+    items, at = [], 0
+    for k, n in enumerate(lens):
+        s, d = at + k % 16, at + (k // 16 + 3 * k) % 16
+        items.append((src.data_ptr() + s, dst.data_ptr() + d, n))
+        ref[d:d + n] = src[s:s + n]
+        at += (n + 63) // 16 * 16
+    C.sg_copy(items, 0, n_blocks)
+    torch.cuda.synchronize()
+    assert torch.equal(dst, ref)
+
+
 @pytest.mark.parametrize("n_blocks", [-1, -3, -12, 5])
 def test_sg_copy_fat_blocks(C, torch_cuda, n_blocks):
     """Negative block counts run 1024-thread blocks (four chunk groups each); unaligned items take the byte paths."""
