@@ -337,6 +337,8 @@ int gpu_app_init(AppCtx* c) {
   }
   if (s->name == "lstm") {
     if (cudaMalloc(&s->d_scratch, srpc_lstm_scratch_bytes(s->lstm_clusters)) != cudaSuccess) return 0;
+    // no tag left in it by its previous owner may equal one of this app's
+    if (cudaMemsetAsync(s->d_scratch, 0, srpc_lstm_scratch_bytes(s->lstm_clusters), c->work_stream) != cudaSuccess) return 0;
   }
   if (c->launch_type == 3) {
     c->self_push = true;  // the resident kernel stores responses and completes slots itself

@@ -11,6 +11,8 @@
 //                    (32 launches per inference in the original)
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
+
+#include <atomic>
 #include <math.h>
 
 #include "../host/p2p_rpc.h"
@@ -309,118 +311,179 @@ lstm_wavefront_kernel(const g_params* stub, const float* direct_in, float* direc
   }
 }
 
-// ------------------------------------------------------------------ LSTM, whole-GPU wavefront
-// The cluster kernel above gives a layer one SM, whose threads each walk one 1 KB weight row: a wave takes 74 us.  Here
-// every wave is spread over the whole GPU.  A work item is (layer, hidden unit): a warp loads the unit's four gate
-// rows of W and U (8 KB, coalesced 16-byte loads, kept in registers), then for every request of the group forms the
-// four dot products with the layer's input and previous hidden state, reduces them across the warp and lets lane 0
-// update the unit's cell and hidden state.  Up to eight requests share one pass over the weights; larger batches are
-// served group after group.  Waves are separated by a grid-wide barrier (the kernel is launched cooperatively, so all
-// blocks are resident; the wait on the barrier word is bounded).  Layer outputs of a wave live in hbuf[wave parity],
-// which the next wave reads as input (layer below) and as previous state (same layer).
-constexpr int LSTM_GROUP = 8;
-constexpr long long LSTM_BARRIER_CYCLES = 4000000000ll;
+// ------------------------------------------------------------------ LSTM, whole-GPU dataflow
+// The cluster kernel above gives a layer one SM, whose threads each walk one 1 KB weight row: a wave takes 74 us.  Here a
+// layer has LSTM_LAYER_BLOCKS SMs and a warp owns one hidden unit for the whole kernel: its eight gate rows of W and U (8 KB)
+// are loaded once and stay in its registers, so the weights cross the memory system once per launch instead of once per
+// step.  What is left is the chain of 15 exchanges along the anti-diagonals (layer l, step t needs all 256 outputs of
+// (l-1, t) and of (l, t-1)).  Outputs travel as 8-byte {value, tag} words through L2, stored and read whole: a reader that
+// finds the launch's tag has the value with it, so an exchange is one store and one read, with no counter, no fence
+// and no grid-wide barrier, and layers run apart as far as their inputs allow.  The tag is a launch counter in device memory
+// (lstm_bump_kernel adds one before every launch; graph replays count too), so nothing has to be cleared in between.
+// A block stages the vectors of a step in shared memory for its warps; the 4 x NB gate sums of a warp are reduced together
+// (values are halved between lane pairs as they are added).  The kernel is launched cooperatively: all blocks are resident,
+// and every wait is bounded.  Bounded by the exchange latency (about 1.5 us per step with the staging and the arithmetic).
+constexpr int LSTM_GROUP = 8;          // requests per launch
+constexpr int LSTM_LAYER_BLOCKS = 18;  // 8 x 18 = 144 of 148 SMs
+constexpr int LSTM_WARPS = (LH + LSTM_LAYER_BLOCKS - 1) / LSTM_LAYER_BLOCKS;  // hidden units per block
+constexpr int LSTM_THREADS = LSTM_WARPS * 32;
+constexpr long long LSTM_WAIT_CYCLES = 4000000000ll;
 
 struct LstmGridArgs {
   const g_params* stub;
   const float* direct_in;
   float* direct_out;
   const float* weights;
-  float* hbuf;        // [2][LLAYERS][LSTM_GROUP][LH]
-  float* cbuf;        // [LLAYERS][LSTM_GROUP][LH]
-  unsigned* counter;  // zeroed before the launch
-  uint32_t* status;   // may be null
-  int batch;
+  unsigned long long* hbuf;  // [LLAYERS][LSTEPS][LSTM_GROUP][LH] words {value, tag}
+  const unsigned* epoch;     // this launch's tag
+  uint32_t* status;          // may be null
+  int first;                 // request of the window that this launch starts with
+  int batch;                 // requests of this launch, 1 .. NB
   float forget_bias;
 };
 
 __device__ __forceinline__ float dot4(const float4& a, const float4& b) { return a.x * b.x + a.y * b.y + a.z * b.z + a.w * b.w; }
 
-__global__ void __launch_bounds__(256) lstm_grid_kernel(const LstmGridArgs a) {
-  __shared__ unsigned s_ok;
+__device__ __forceinline__ void ld_two_words(const unsigned long long* p, unsigned long long* w0, unsigned long long* w1) {
+  asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(*w0), "=l"(*w1) : "l"(p) : "memory");
+}
+
+__global__ void lstm_bump_kernel(unsigned* epoch) { *epoch += 1; }
+
+template <int NB>
+__global__ void __launch_bounds__(LSTM_THREADS, 1) lstm_grid_kernel(const LstmGridArgs a) {
+  constexpr int NV = 4 * NB;                                     // gate sums per warp
+  constexpr int LOG_NV = NV == 4 ? 2 : (NV == 8 ? 3 : (NV == 16 ? 4 : 5));
+  constexpr int MAXQ = (2 * NB * (LH / 2) + LSTM_THREADS - 1) / LSTM_THREADS;  // word pairs a thread stages per step
+  __shared__ __align__(16) float s_vec[2][2][NB][LH];            // [buffer][input, own layer's previous output][request][unit]
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int gw = blockIdx.x * 8 + warp, nw = gridDim.x * 8;
-  const float* in_base = a.direct_in ? a.direct_in : reinterpret_cast<const float*>(a.stub->req);
-  float* out_base = a.direct_out ? a.direct_out : reinterpret_cast<float*>(a.stub->resp);
-  const size_t per_layer = (size_t)8 * LH * LH + 4 * LH;
-  unsigned target = 0;
-  for (int g0 = 0; g0 < a.batch; g0 += LSTM_GROUP) {
-    const int nb = a.batch - g0 < LSTM_GROUP ? a.batch - g0 : LSTM_GROUP;
-    for (int d = 0; d < LLAYERS + LSTEPS - 1; d++) {
-      const int l_lo = d - (LSTEPS - 1) > 0 ? d - (LSTEPS - 1) : 0, l_hi = d < LLAYERS - 1 ? d : LLAYERS - 1;
-      const int n_items = (l_hi - l_lo + 1) * LH;
-      const float* h_read = a.hbuf + (size_t)((d + 1) & 1) * LLAYERS * LSTM_GROUP * LH;  // what wave d-1 wrote
-      float* h_write = a.hbuf + (size_t)(d & 1) * LLAYERS * LSTM_GROUP * LH;
-      for (int it = gw; it < n_items; it += nw) {
-        const int l = l_lo + it / LH, j = it % LH, t = d - l;
-        const float* W = a.weights + (size_t)l * per_layer;
-        const float* U = W + (size_t)4 * LH * LH;
-        const float* B = U + (size_t)4 * LH * LH;
-        float4 w[4][2], u[4][2];
+  const int l = blockIdx.x / LSTM_LAYER_BLOCKS, part = blockIdx.x - l * LSTM_LAYER_BLOCKS;
+  const int j = part * LSTM_WARPS + warp;                        // this warp's hidden unit
+  const bool unit = j < LH;
+  const unsigned tag = *a.epoch;
+  const float* in_base = (a.direct_in ? a.direct_in : reinterpret_cast<const float*>(a.stub->req)) + (size_t)a.first * LSTEPS * LH;
+  float* out_base = (a.direct_out ? a.direct_out : reinterpret_cast<float*>(a.stub->resp)) + (size_t)a.first * LH;
+  const float* W = a.weights + (size_t)l * ((size_t)8 * LH * LH + 4 * LH);
+  const float* U = W + (size_t)4 * LH * LH;
+  const float* B = U + (size_t)4 * LH * LH;
+  float4 w[4][2], u[4][2];
+  float bias[4];
 #pragma unroll
-        for (int g = 0; g < 4; g++) {
-          const float4* wr = reinterpret_cast<const float4*>(W + ((size_t)g * LH + j) * LH);
-          w[g][0] = __ldg(wr + lane);
-          w[g][1] = __ldg(wr + 32 + lane);
-          if (t > 0) {
-            const float4* ur = reinterpret_cast<const float4*>(U + ((size_t)g * LH + j) * LH);
-            u[g][0] = __ldg(ur + lane);
-            u[g][1] = __ldg(ur + 32 + lane);
-          } else {
-            u[g][0] = u[g][1] = make_float4(0.f, 0.f, 0.f, 0.f);
-          }
-        }
-        const float bi = B[j], bg = B[LH + j], bf = B[2 * LH + j] + a.forget_bias, bo = B[3 * LH + j];
-        for (int b = 0; b < nb; b++) {
-          const float4* xv = l == 0 ? reinterpret_cast<const float4*>(in_base + ((size_t)(g0 + b) * LSTEPS + t) * LH)
-                                    : reinterpret_cast<const float4*>(h_read + ((size_t)(l - 1) * LSTM_GROUP + b) * LH);
-          const float4 x0 = __ldcg(xv + lane), x1 = __ldcg(xv + 32 + lane);
-          float sum[4];
+  for (int g = 0; g < 4; g++) {
+    const float4* wr = reinterpret_cast<const float4*>(W + ((size_t)g * LH + (unit ? j : 0)) * LH);
+    const float4* ur = reinterpret_cast<const float4*>(U + ((size_t)g * LH + (unit ? j : 0)) * LH);
+    w[g][0] = __ldg(wr + lane);
+    w[g][1] = __ldg(wr + 32 + lane);
+    u[g][0] = __ldg(ur + lane);
+    u[g][1] = __ldg(ur + 32 + lane);
+    bias[g] = B[g * LH + (unit ? j : 0)] + (g == 2 ? a.forget_bias : 0.f);
+  }
+  float cell = 0.f;  // of request (lane >> (5 - LOG_NV)) >> 2
+  for (int t = 0; t < LSTEPS; t++) {
+    float(*vec)[NB][LH] = s_vec[t & 1];
+    // ---- stage the step's vectors: pair q = (source, request, two units)
+    const int n_src = t > 0 ? 2 : 1, n_pairs = n_src * NB * (LH / 2);
+    const unsigned long long* src[MAXQ];
+    bool open[MAXQ], any = false;
 #pragma unroll
-          for (int g = 0; g < 4; g++) sum[g] = dot4(w[g][0], x0) + dot4(w[g][1], x1);
-          if (t > 0) {
-            const float4* hv = reinterpret_cast<const float4*>(h_read + ((size_t)l * LSTM_GROUP + b) * LH);
-            const float4 h0 = __ldcg(hv + lane), h1 = __ldcg(hv + 32 + lane);
+    for (int k = 0; k < MAXQ; k++) {
+      const int q = (int)threadIdx.x + k * LSTM_THREADS;
+      const int from = q / (NB * (LH / 2)), b = (q / (LH / 2)) % NB, pr = q % (LH / 2);
+      open[k] = q < n_pairs && b < a.batch;
+      src[k] = nullptr;
+      if (!open[k]) continue;
+      if (from == 0 && l == 0) {
+        const float2 x = *reinterpret_cast<const float2*>(in_base + ((size_t)b * LSTEPS + t) * LH + 2 * pr);
+        *reinterpret_cast<float2*>(&vec[0][b][2 * pr]) = x;
+        open[k] = false;
+      } else {
+        const int ll = from == 0 ? l - 1 : l, tt = from == 0 ? t : t - 1;
+        src[k] = a.hbuf + (((size_t)ll * LSTEPS + tt) * LSTM_GROUP + b) * LH + 2 * pr;
+        any = true;
+      }
+    }
+    bool late = false;
+    const long long t0 = clock64();
+    while (any) {
+      unsigned long long w0[MAXQ], w1[MAXQ];
 #pragma unroll
-            for (int g = 0; g < 4; g++) sum[g] += dot4(u[g][0], h0) + dot4(u[g][1], h1);
-          }
+      for (int k = 0; k < MAXQ; k++)
+        if (open[k]) ld_two_words(src[k], &w0[k], &w1[k]);
+      any = false;
 #pragma unroll
-          for (int o = 16; o; o >>= 1) {
-#pragma unroll
-            for (int g = 0; g < 4; g++) sum[g] += __shfl_xor_sync(0xffffffffu, sum[g], o);
-          }
-          if (lane == 0) {
-            float* cp = a.cbuf + ((size_t)l * LSTM_GROUP + b) * LH + j;
-            const float c_prev = t > 0 ? *cp : 0.f;
-            const float c = sigmoidf_(sum[2] + bf) * c_prev + sigmoidf_(sum[0] + bi) * tanhf(sum[1] + bg);
-            const float h = tanhf(c) * sigmoidf_(sum[3] + bo);
-            *cp = c;
-            h_write[((size_t)l * LSTM_GROUP + b) * LH + j] = h;
-            if (l == LLAYERS - 1 && t == LSTEPS - 1) out_base[(size_t)(g0 + b) * LH + j] = h;
-          }
+      for (int k = 0; k < MAXQ; k++) {
+        if (!open[k]) continue;
+        if ((unsigned)(w0[k] >> 32) == tag && (unsigned)(w1[k] >> 32) == tag) {
+          const int q = (int)threadIdx.x + k * LSTM_THREADS;
+          const int from = q / (NB * (LH / 2)), b = (q / (LH / 2)) % NB, pr = q % (LH / 2);
+          *reinterpret_cast<float2*>(&vec[from][b][2 * pr]) =
+              make_float2(__uint_as_float((unsigned)w0[k]), __uint_as_float((unsigned)w1[k]));
+          open[k] = false;
+        } else {
+          any = true;
         }
       }
-      // grid-wide barrier, bounded
-      __syncthreads();
-      if (threadIdx.x == 0) {
-        target += gridDim.x;
-        __threadfence();
-        atomicAdd(a.counter, 1u);
-        unsigned ok = 1;
-        const long long t0 = clock64();
-        while ((int)(ptx::ld_acquire_gpu(a.counter) - target) < 0) {
-          if (clock64() - t0 > LSTM_BARRIER_CYCLES) {
-            ok = 0;
-            break;
-          }
+      if (any && clock64() - t0 > LSTM_WAIT_CYCLES) {
+        late = true;
+        break;
+      }
+    }
+    if (__syncthreads_or(late ? 1 : 0)) {
+      if (threadIdx.x == 0 && a.status) atomicExch(a.status, 0x4C53u);  // 'LS': a wait of the LSTM ran out
+      return;
+    }
+    // The buffers alternate: a warp overwrites a vector only after the barrier above of the next step, which every warp
+    // reaches when it has read this step's vectors.
+    float v[NV];
+#pragma unroll
+    for (int b = 0; b < NB; b++) {
+      if (b >= a.batch) {
+#pragma unroll
+        for (int g = 0; g < 4; g++) v[b * 4 + g] = 0.f;
+        continue;
+      }
+      const float4* xv = reinterpret_cast<const float4*>(vec[0][b]);
+      const float4 x0 = xv[lane], x1 = xv[32 + lane];
+#pragma unroll
+      for (int g = 0; g < 4; g++) v[b * 4 + g] = dot4(w[g][0], x0) + dot4(w[g][1], x1);
+      if (t > 0) {
+        const float4* hv = reinterpret_cast<const float4*>(vec[1][b]);
+        const float4 h0 = hv[lane], h1 = hv[32 + lane];
+#pragma unroll
+        for (int g = 0; g < 4; g++) v[b * 4 + g] += dot4(u[g][0], h0) + dot4(u[g][1], h1);
+      }
+    }
+    // ---- sums over the warp: while a lane holds several values it keeps one half of them and adds its partner's share of
+    // that half; then lane = value index x 2^(5 - LOG_NV) + replica
+#pragma unroll
+    for (int step = 0; step < 5; step++) {
+      const int off = 16 >> step;
+      if (step < LOG_NV) {
+        const int half = NV >> (step + 1);
+        const bool upper = (lane & off) != 0;
+#pragma unroll
+        for (int k = 0; k < half; k++) {
+          const float mine = upper ? v[k + half] : v[k], give = upper ? v[k] : v[k + half];
+          v[k] = mine + __shfl_xor_sync(0xffffffffu, give, off);
         }
-        s_ok = ok;
+      } else {
+        v[0] += __shfl_xor_sync(0xffffffffu, v[0], off);
       }
-      __syncthreads();
-      if (!s_ok) {
-        if (threadIdx.x == 0 && a.status) atomicExch(a.status, 0x4C53u);  // 'LS': the LSTM's grid barrier ran out
-        return;
-      }
+    }
+    constexpr int REP = 5 - LOG_NV;
+    const int idx = lane >> REP, base = idx & ~3;
+    const float gi = __shfl_sync(0xffffffffu, v[0], (base + 0) << REP) + bias[0];
+    const float gg = __shfl_sync(0xffffffffu, v[0], (base + 1) << REP) + bias[1];
+    const float gf = __shfl_sync(0xffffffffu, v[0], (base + 2) << REP) + bias[2];
+    const float go = __shfl_sync(0xffffffffu, v[0], (base + 3) << REP) + bias[3];
+    cell = sigmoidf_(gf) * cell + sigmoidf_(gi) * tanhf(gg);
+    const float h = tanhf(cell) * sigmoidf_(go);
+    const int b = base >> 2;
+    if (unit && (lane & ((4 << REP) - 1)) == 0 && b < a.batch) {
+      unsigned long long* dst = a.hbuf + (((size_t)l * LSTEPS + t) * LSTM_GROUP + b) * LH + j;
+      const unsigned long long word = ((unsigned long long)tag << 32) | __float_as_uint(h);
+      asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(dst), "l"(word) : "memory");
+      if (l == LLAYERS - 1 && t == LSTEPS - 1) out_base[(size_t)b * LH + j] = h;
     }
   }
 }
@@ -577,53 +640,67 @@ void srpc_parity_preload() {
   (void)cudaFuncGetAttributes(&fa, swap_hdrs_contig_kernel);
   (void)cudaFuncGetAttributes(&fa, lenet_ref_kernel);
   (void)cudaFuncGetAttributes(&fa, lstm_wavefront_kernel);
-  (void)cudaFuncGetAttributes(&fa, lstm_grid_kernel);
+  (void)cudaFuncGetAttributes(&fa, lstm_bump_kernel);
+  (void)cudaFuncGetAttributes(&fa, lstm_grid_kernel<1>);
+  (void)cudaFuncGetAttributes(&fa, lstm_grid_kernel<2>);
+  (void)cudaFuncGetAttributes(&fa, lstm_grid_kernel<4>);
+  (void)cudaFuncGetAttributes(&fa, lstm_grid_kernel<8>);
   (void)cudaGetLastError();
 }
 
-static constexpr size_t kLstmHbufFloats = (size_t)2 * LLAYERS * LSTM_GROUP * LH, kLstmCbufFloats = (size_t)LLAYERS * LSTM_GROUP * LH;
-static size_t lstm_grid_scratch_bytes() { return (kLstmHbufFloats + kLstmCbufFloats) * sizeof(float) + 256; }
+static constexpr size_t kLstmWords = (size_t)LLAYERS * LSTEPS * LSTM_GROUP * LH;
 
 size_t srpc_lstm_scratch_bytes(int max_clusters) {
   const size_t cluster_form = (size_t)max_clusters * LLAYERS * LSTEPS * LH * sizeof(float);
-  return cluster_form > lstm_grid_scratch_bytes() ? cluster_form : lstm_grid_scratch_bytes();
+  const size_t grid_form = kLstmWords * sizeof(unsigned long long) + 256;
+  return cluster_form > grid_form ? cluster_form : grid_form;
 }
 
 cudaError_t srpc_lstm(const void* d_stub, const float* direct_in, float* direct_out, const float* weights, float* scratch,
                       int max_clusters, int batch, float forget_bias, cudaStream_t s) {
   if (batch < 1) return cudaSuccess;
-  // Whole-GPU wavefront (cooperative launch); SPLITRPC_LSTM_CLUSTER=1 or a refused cooperative launch falls back to
-  // the one-cluster-per-request kernel.
+  // Whole-GPU dataflow (cooperative launches, LSTM_GROUP requests each); SPLITRPC_LSTM_CLUSTER=1 or a refused cooperative
+  // launch falls back to the one-cluster-per-request kernel.
   static const int use_cluster = [] { const char* e = getenv("SPLITRPC_LSTM_CLUSTER"); return e ? atoi(e) : 0; }();
-  static int grid_blocks = 0;
+  static std::atomic<int> grid_ok{0};  // 1 all blocks fit the device, -1 they do not
+  int done = 0;
   if (!use_cluster) {
-    if (!grid_blocks) {
+    if (!grid_ok.load(std::memory_order_acquire)) {
       int dev = 0, sms = 0, per_sm = 0, coop = 0;
       cudaGetDevice(&dev);
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
       cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, lstm_grid_kernel, 256, 0);
-      grid_blocks = (coop && sms > 0 && per_sm > 0) ? sms : -1;
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, lstm_grid_kernel<LSTM_GROUP>, LSTM_THREADS, 0);
+      grid_ok.store(coop && sms * per_sm >= LLAYERS * LSTM_LAYER_BLOCKS ? 1 : -1, std::memory_order_release);
     }
-    if (grid_blocks > 0) {
+    if (grid_ok.load(std::memory_order_acquire) > 0) {
       LstmGridArgs a;
       a.stub = (const g_params*)d_stub;
       a.direct_in = direct_in;
       a.direct_out = direct_out;
       a.weights = weights;
-      a.hbuf = scratch;
-      a.cbuf = scratch + kLstmHbufFloats;
-      a.counter = reinterpret_cast<unsigned*>(scratch + kLstmHbufFloats + kLstmCbufFloats);
+      a.hbuf = reinterpret_cast<unsigned long long*>(scratch);
+      unsigned* epoch = reinterpret_cast<unsigned*>(a.hbuf + kLstmWords);
+      a.epoch = epoch;
       a.status = nullptr;
-      a.batch = batch;
       a.forget_bias = forget_bias;
-      cudaError_t e = cudaMemsetAsync(a.counter, 0, sizeof(unsigned), s);
-      if (e != cudaSuccess) return e;
-      void* args[] = {&a};
-      e = cudaLaunchCooperativeKernel((const void*)lstm_grid_kernel, dim3((unsigned)grid_blocks), dim3(256), args, 0, s);
-      if (e == cudaSuccess) return cudaSuccess;
-      (void)cudaGetLastError();
-      grid_blocks = -1;  // not possible on this device or in this context: use the cluster kernel from now on
+      for (; done < batch; done += LSTM_GROUP) {
+        a.first = done;
+        a.batch = batch - done < LSTM_GROUP ? batch - done : LSTM_GROUP;
+        lstm_bump_kernel<<<1, 1, 0, s>>>(epoch);
+        void* args[] = {&a};
+        const void* fn = a.batch == 1   ? (const void*)lstm_grid_kernel<1>
+                         : a.batch == 2 ? (const void*)lstm_grid_kernel<2>
+                         : a.batch <= 4 ? (const void*)lstm_grid_kernel<4>
+                                        : (const void*)lstm_grid_kernel<8>;
+        const cudaError_t e = cudaLaunchCooperativeKernel(fn, dim3(LLAYERS * LSTM_LAYER_BLOCKS), dim3(LSTM_THREADS), args, 0, s);
+        if (e == cudaSuccess) continue;
+        (void)cudaGetLastError();
+        if (done) return e;
+        grid_ok.store(-1, std::memory_order_release);  // not possible in this context: use the cluster kernel from now on
+        break;
+      }
+      if (done) return cudaGetLastError();
     }
   }
   int clusters = batch < max_clusters ? batch : max_clusters;

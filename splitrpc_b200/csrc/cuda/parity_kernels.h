@@ -32,7 +32,8 @@ cudaError_t srpc_lenet_ref(const void* d_stub, const void* direct_in, float* dir
                            const float* fc, const float* fb, int batch, cudaStream_t s);
 
 // 8-layer x 8-step LSTM, hidden 256.  weights: per layer W[4][256][256], U[4][256][256], b[4][256] (gate order
-// input, cell, forget, output).  scratch: srpc_lstm_scratch_bytes(max_clusters) bytes.
+// input, cell, forget, output).  scratch: srpc_lstm_scratch_bytes(max_clusters) bytes, zero
+// before the first call and for the use of one stream.
 size_t srpc_lstm_scratch_bytes(int max_clusters);
 cudaError_t srpc_lstm(const void* d_stub, const float* direct_in, float* direct_out, const float* weights, float* scratch,
                       int max_clusters, int batch, float forget_bias, cudaStream_t s);
