@@ -987,6 +987,11 @@ cudaError_t srpc_conv_bf16_tma(const void* in, const void* weight, const ConvSha
   if (cs.cin % BK || cs.cout % 8) return cudaErrorInvalidValue;
   if (((uintptr_t)in & 15) || ((uintptr_t)weight & 15) || ((uintptr_t)ep.out & 15) || ep.out_fp32) return cudaErrorInvalidValue;
   if (ep.bias && ((uintptr_t)ep.bias & 15)) return cudaErrorInvalidValue;
+  if (srpc_stem_conv_eligible(cs, ep)) {
+    if (cs.in_stub && (cs.in_ring_slots < cs.n || !cs.in_slot_bytes || cs.in_img_stride * 2 != (long)cs.in_slot_bytes))
+      return cudaErrorInvalidValue;
+    return srpc_stem_conv(in, weight, cs, ep, status, stream);
+  }
   TileParams p{};
   p.mode = 1;
   p.oh = cs.oh;

@@ -60,6 +60,12 @@ cudaError_t srpc_gemm_bf16_v2(const void* A, int lda, const void* B, int ldb, in
 cudaError_t srpc_conv_bf16_tma(const void* in, const void* weight, const ConvShape& cs, const GemmEpilogue& ep,
                                uint32_t* status, cudaStream_t stream);
 
+// Convolution over overlapping windows of narrow pixels (stem_conv.cu); srpc_conv_bf16_tma selects it by itself,
+// SPLITRPC_STEM_CONV=0 turns it off.
+bool srpc_stem_conv_eligible(const ConvShape& cs, const GemmEpilogue& ep);
+cudaError_t srpc_stem_conv(const void* in, const void* weight, const ConvShape& cs, const GemmEpilogue& ep, uint32_t* status,
+                           cudaStream_t stream);
+
 // Two-SM variant (CTA pairs, 256 x bn tiles with bn = 128, 192 or 256, tcgen05.mma.cta_group::2) for compute-bound
 // shapes; bf16 output with 16-byte aligned rows only.  srpc_gemm_bf16_v2 selects it by itself; SPLITRPC_GEMM_2SM=0
 // turns it off.
