@@ -2,7 +2,7 @@
 //
 // One CTA serves one (sequence, head) and loops over its 128-query tiles.
 //   scores = Q . K^T      tcgen05.mma, M=128, N=128 per key block, K=64, fp32 in TMEM
-//   P = softmax(scores)   four warps, one query row per thread, read from TMEM,
+//   P = softmax(scores)   eight warps, half a query row per thread, read from TMEM,
 //                         written as bf16 into 128-byte-swizzled shared memory
 //   O = P . V             tcgen05.mma, M=128, N=64, K=SEQ, fp32 in TMEM
 // All operands arrive by TMA (no multicast) from this GPU's memory:
@@ -28,7 +28,8 @@ namespace {
 
 constexpr int HD = 64;          // head dim
 constexpr int QT = 128;         // queries per tile
-constexpr int ATT_THREADS = 160;  // warps 0-3 softmax/epilogue, warp 4 TMA + MMA issue
+constexpr int SOFT_THREADS = 256;            // warps 0-7: softmax and output
+constexpr int ATT_THREADS = SOFT_THREADS + 32;  // warp 8: TMA and MMA issue
 
 template <int SEQ>
 struct AttSmem {
@@ -51,8 +52,21 @@ struct AttSmem {
 // is then [keys, 64] with the head dimension contiguous, i.e. an MN-major B operand of the second product: same
 // 128-byte-swizzled shared-memory tile and descriptor, "B is MN-major" in the instruction descriptor, and a step of 16
 // keys along K is 2048 bytes (two 8-row groups) instead of 32.  No transposed copy of V and no separate V GEMM.
+__device__ __forceinline__ void soft_sync() { asm volatile("bar.sync 1, %0;" ::"n"(SOFT_THREADS) : "memory"); }
+// The same barrier with the AND of the threads' predicates.
+__device__ __forceinline__ bool soft_all(bool pred) {
+  uint32_t out;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 q, %2, 0;\n\t"
+      "barrier.cta.red.and.pred p, 1, %1, q;\n\tselp.u32 %0, 1, 0, p;\n\t}\n"
+      : "=r"(out)
+      : "n"(SOFT_THREADS), "r"((uint32_t)pred)
+      : "memory");
+  return out != 0;
+}
+
 template <int SEQ, bool VMN>
-__global__ void __launch_bounds__(ATT_THREADS)
+__global__ void __launch_bounds__(ATT_THREADS, SEQ == QT ? 3 : 1)
 attention_tc(const __grid_constant__ CUtensorMap tmap_qk, const __grid_constant__ CUtensorMap tmap_vt,
              __nv_bfloat16* out, int ld_out, const float* v_bias, int hidden, float scale_log2e,
              uint32_t* status) {
@@ -66,6 +80,7 @@ attention_tc(const __grid_constant__ CUtensorMap tmap_qk, const __grid_constant_
   __shared__ __align__(8) uint64_t bar_kv, bar_q, bar_s, bar_p, bar_o;
   __shared__ uint32_t tmem_base_smem;
   __shared__ uint32_t s_error;
+  __shared__ float s_max[2][QT], s_sum[2][QT];
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int head = blockIdx.x, seq_idx = blockIdx.y;
@@ -76,14 +91,14 @@ attention_tc(const __grid_constant__ CUtensorMap tmap_qk, const __grid_constant_
     ptx::mbar_init(&bar_kv, 1);
     ptx::mbar_init(&bar_q, 1);
     ptx::mbar_init(&bar_s, 1);
-    ptx::mbar_init(&bar_p, 4);
+    ptx::mbar_init(&bar_p, SOFT_THREADS / 32);
     ptx::mbar_init(&bar_o, 1);
     ptx::fence_mbar_init();
     s_error = 0;
     ptx::prefetch_tmap(&tmap_qk);
     ptx::prefetch_tmap(&tmap_vt);
   }
-  if (warp == 4) {
+  if (warp == SOFT_THREADS / 32) {
     ptx::tmem_alloc(&tmem_base_smem, L::TMEM_COLS);
     ptx::tmem_relinquish();
     ptx::grid_dep_launch();  // after the allocation, see pdl_launch.h
@@ -95,9 +110,11 @@ attention_tc(const __grid_constant__ CUtensorMap tmap_qk, const __grid_constant_
   const uint32_t tmem_s = tmem_base_smem;          // scores: columns [0, SEQ)
   const uint32_t tmem_o = tmem_base_smem + (L::ALIAS ? 0 : SEQ);  // output: columns [SEQ, SEQ+64), or over the scores
 
-  if (warp == 4) {
+  if (warp == SOFT_THREADS / 32) {
     if (ptx::elect_one()) {
-      // K and V^T of this head stay resident for all query tiles.
+      // K and V^T of this head stay resident for all query tiles.  The first Q tile does not wait for them.
+      ptx::mbar_expect_tx(&bar_q, L::Q_BYTES);
+      ptx::tma_load_2d(sQ, &tmap_qk, &bar_q, head * HD, tok0);
       ptx::mbar_expect_tx(&bar_kv, L::K_BYTES + L::VT_BYTES);
       for (int nb = 0; nb < SEQ / 128; nb++)
         ptx::tma_load_2d(sK + nb * 128 * 128, &tmap_qk, &bar_kv, hidden + head * HD, tok0 + nb * 128);
@@ -110,25 +127,31 @@ attention_tc(const __grid_constant__ CUtensorMap tmap_qk, const __grid_constant_
       bool ok = ptx::mbar_wait(&bar_kv, 0);
       const uint32_t idesc_s = ptx::umma_idesc_bf16(QT, 128);
       const uint32_t idesc_o = ptx::umma_idesc_bf16(QT, HD) | (VMN ? (1u << 16) : 0u);  // bit 16: B is MN-major
-      for (int qt = 0; qt < NQT && ok; qt++) {
-        const uint32_t ph = (uint32_t)qt & 1u;
-        // Q tile (the previous tile's score MMAs have completed: bar_s was awaited by the softmax warps and
-        // bar_o, which follows it, by this thread's successors; this thread itself waited bar_p below).
+      const uint32_t q_addr = ptx::smem_u32(sQ), k_addr = ptx::smem_u32(sK), p_addr = ptx::smem_u32(sP), vt_addr = ptx::smem_u32(sVT);
+      auto load_q = [&](int qt) {
         ptx::mbar_expect_tx(&bar_q, L::Q_BYTES);
         ptx::tma_load_2d(sQ, &tmap_qk, &bar_q, head * HD, tok0 + qt * QT);
-        if (!(ok = ptx::mbar_wait(&bar_q, ph))) break;
-        ptx::tc_fence_after();
-        const uint32_t q_addr = ptx::smem_u32(sQ), k_addr = ptx::smem_u32(sK);
+      };
+      auto scores = [&]() {
         for (int nb = 0; nb < SEQ / 128; nb++)
 #pragma unroll
           for (int k = 0; k < HD / 16; k++)
             ptx::umma_bf16(tmem_s + nb * 128, ptx::umma_desc_sw128(q_addr + k * 32),
                            ptx::umma_desc_sw128(k_addr + nb * 128 * 128 + k * 32), idesc_s, k != 0 ? 1u : 0u);
         ptx::umma_commit(&bar_s);
-        // P ready (written by the softmax warps)
+      };
+      ok = ok && ptx::mbar_wait(&bar_q, 0);
+      if (ok) scores();
+      for (int qt = 0; qt < NQT && ok; qt++) {
+        const uint32_t ph = (uint32_t)qt & 1u;
+        // The next Q tile takes this one's place as soon as its scores exist, while the softmax runs.
+        if (qt + 1 < NQT) {
+          if (!(ok = ptx::mbar_wait(&bar_s, ph))) break;
+          load_q(qt + 1);
+        }
+        // P ready (written by the softmax warps, which have read all scores by then)
         if (!(ok = ptx::mbar_wait(&bar_p, ph))) break;
         ptx::tc_fence_after();
-        const uint32_t p_addr = ptx::smem_u32(sP), vt_addr = ptx::smem_u32(sVT);
         for (int kk = 0; kk < SEQ / 16; kk++) {
           const int atom = kk >> 2, sub = kk & 3;
           const uint32_t v_desc_addr = VMN ? vt_addr + kk * 2048 : vt_addr + atom * 64 * 128 + sub * 32;
@@ -136,33 +159,47 @@ attention_tc(const __grid_constant__ CUtensorMap tmap_qk, const __grid_constant_
                          idesc_o, kk != 0 ? 1u : 0u);
         }
         ptx::umma_commit(&bar_o);
+        // The next tile's scores run behind P.V, while the output is written.
+        if (qt + 1 < NQT) {
+          if (!(ok = ptx::mbar_wait(&bar_q, ph ^ 1u))) break;
+          scores();
+        }
       }
       if (!ok) atomicExch(&s_error, 1u);
     }
   } else {
-    const int row = warp * 32 + lane;  // query row inside the tile; warp == TMEM lane quarter
-    const uint32_t lane_base = (uint32_t)(warp * 32) << 16;
+    // Two warps per tensor-memory lane quarter: a thread has one query row and half of its keys; the halves' maxima and
+    // sums meet in shared memory.
+    const int half = warp >> 2, row = (warp & 3) * 32 + lane;
+    constexpr int COLS = SEQ / 2;
+    const int c0 = half * COLS;
+    const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
     for (int qt = 0; qt < NQT; qt++) {
       const uint32_t ph = (uint32_t)qt & 1u;
-      if (*(volatile uint32_t*)&s_error != 0 || !ptx::mbar_wait(&bar_s, ph)) {
-        atomicExch(&s_error, 2u);
+      const bool got = *(volatile uint32_t*)&s_error == 0 && ptx::mbar_wait(&bar_s, ph);
+      if (!soft_all(got)) {
+        if (lane == 0) atomicCAS(&s_error, 0u, 2u);
         break;
       }
       ptx::tc_fence_after();
       // pass 1: row maximum
       float mx = -3.0e38f;
 #pragma unroll 1
-      for (int c = 0; c < SEQ; c += 32) {
-        uint32_t r[32];
-        ptx::tmem_ld_32x32b_x32(tmem_s + lane_base + c, r);
+      for (int c = 0; c < COLS; c += 64) {
+        uint32_t r[64];
+        ptx::tmem_ld_32x32b_x32(tmem_s + lane_base + c0 + c, r);
+        ptx::tmem_ld_32x32b_x32(tmem_s + lane_base + c0 + c + 32, r + 32);
         ptx::tmem_ld_wait();
 #pragma unroll
-        for (int j = 0; j < 32; j++) mx = fmaxf(mx, __uint_as_float(r[j]));
+        for (int j = 0; j < 64; j++) mx = fmaxf(mx, __uint_as_float(r[j]));
       }
+      s_max[half][row] = mx;
+      soft_sync();
+      mx = fmaxf(s_max[0][row], s_max[1][row]);
       // pass 2: exponentials, row sum, P in bf16 to swizzled shared memory
       float sum = 0.f;
 #pragma unroll 1
-      for (int c = 0; c < SEQ; c += 32) {
+      for (int c = c0; c < c0 + COLS; c += 32) {
         uint32_t r[32];
         ptx::tmem_ld_32x32b_x32(tmem_s + lane_base + c, r);
         ptx::tmem_ld_wait();
@@ -184,37 +221,36 @@ attention_tc(const __grid_constant__ CUtensorMap tmap_qk, const __grid_constant_
           *reinterpret_cast<uint4*>(prow + (((chunk0 + j) ^ (row & 7)) << 4)) = q;
         }
       }
+      s_sum[half][row] = sum;
       ptx::tc_fence_before();
       ptx::fence_proxy_async_smem();
       __syncwarp();
       if (lane == 0) ptx::mbar_arrive(&bar_p);
-      // output tile
-      if (!ptx::mbar_wait(&bar_o, ph)) {
-        atomicExch(&s_error, 3u);
+      // output tile: each half writes 32 of the head's 64 columns
+      if (!soft_all(ptx::mbar_wait(&bar_o, ph))) {
+        if (lane == 0) atomicCAS(&s_error, 0u, 3u);
         break;
       }
       ptx::tc_fence_after();
-      const float inv = 1.f / sum;
+      const float inv = 1.f / (s_sum[0][row] + s_sum[1][row]);
       __nv_bfloat16* orow = out + (size_t)(tok0 + qt * QT + row) * ld_out + head * HD;
+      const int c = half * 32;
+      uint32_t r[32];
+      ptx::tmem_ld_32x32b_x32(tmem_o + lane_base + c, r);
+      ptx::tmem_ld_wait();
 #pragma unroll
-      for (int c = 0; c < HD; c += 32) {
-        uint32_t r[32];
-        ptx::tmem_ld_32x32b_x32(tmem_o + lane_base + c, r);
-        ptx::tmem_ld_wait();
+      for (int j = 0; j < 4; j++) {
+        uint4 q;
+        __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&q);
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-          uint4 q;
-          __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&q);
-#pragma unroll
-          for (int t = 0; t < 4; t++) {
-            const int d = c + j * 8 + 2 * t;
-            const float b0 = v_bias ? *(v_bias + head * HD + d) : 0.f;
-            const float b1 = v_bias ? *(v_bias + head * HD + d + 1) : 0.f;
-            h[t] = __floats2bfloat162_rn(__uint_as_float(r[j * 8 + 2 * t]) * inv + b0,
-                                         __uint_as_float(r[j * 8 + 2 * t + 1]) * inv + b1);
-          }
-          *reinterpret_cast<uint4*>(orow + c + j * 8) = q;
+        for (int t = 0; t < 4; t++) {
+          const int d = c + j * 8 + 2 * t;
+          const float b0 = v_bias ? *(v_bias + head * HD + d) : 0.f;
+          const float b1 = v_bias ? *(v_bias + head * HD + d + 1) : 0.f;
+          h[t] = __floats2bfloat162_rn(__uint_as_float(r[j * 8 + 2 * t]) * inv + b0,
+                                       __uint_as_float(r[j * 8 + 2 * t + 1]) * inv + b1);
         }
+        *reinterpret_cast<uint4*>(orow + c + j * 8) = q;
       }
       ptx::tc_fence_before();
     }
@@ -226,7 +262,7 @@ attention_tc(const __grid_constant__ CUtensorMap tmap_qk, const __grid_constant_
     __nanosleep(1000000);
     __syncthreads();
   }
-  if (warp == 4) {
+  if (warp == SOFT_THREADS / 32) {
     ptx::tc_fence_after();
     ptx::tmem_dealloc(tmem_base_smem, L::TMEM_COLS);
   }

@@ -12,13 +12,14 @@
 // is one run of memory; the three positions per row that lie past the output's width are computed and dropped.
 //
 // One persistent CTA per SM.  A work item is a chunk of up to MAX_TILES tiles of one image.
-//   warp 0      weights by TMA once, then one elected lane issues 16 MMAs (128 x 64 x 16) per tile into one of four
+//   warp 0      weights by TMA once, then one elected lane issues 16 MMAs (128 x 64 x 16) per tile into one of eight
 //               accumulators, taps in the order of the generic kernel, so that results are bit-identical to it
 //   warps 1-3   copy the next chunk's pixels with 16-byte cp.async into the other of two buffers
-//   warps 4-11  read accumulators (four warps per tile, alternating tiles), bias, activation, bf16, transpose through a
+//   warps 4-15  read accumulators (four warps per tile, three tiles at a time), bias, activation, bf16, transpose through a
 //               swizzled 4 KB buffer per warp, 512-byte coalesced stores
-// Bound by the tensor pipe's operand reads (48 clocks per MMA at 64 columns: 0.4 us per tile, 18 us for 64 images) and the
-// output (103 MB, 16 us).  Waits are bounded as in gemm_persistent.cu.
+// 64 images: 48 us (71 us in the generic kernel); the output alone takes 16 us of memory time.  What bounds it is shared
+// memory: the operand reads of the MMAs, the pixel copies and the transposing epilogue each take 5 - 10 us off when they are
+// left out, and eight epilogue warps with four accumulators took 53 us.  Waits are bounded as in gemm_persistent.cu.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -41,10 +42,10 @@ constexpr int MAX_PIX = MAX_TILES * BM + (TAPS - 1) * MAX_PITCH + WIN - 1;
 constexpr int PLANE = (MAX_PIX * 16 + 127) / 128 * 128;
 constexpr int BUF_BYTES = 2 * PLANE;
 constexpr int W_BYTES = TAPS * COUT * 128;
-constexpr int LOADERS = 96, EPI_WARPS = 8, THREADS = 32 + LOADERS + EPI_WARPS * 32;
+constexpr int LOADERS = 96, EPI_WARPS = 12, THREADS = 32 + LOADERS + EPI_WARPS * 32;
 constexpr int STAGE_BYTES = 32 * 128;                   // per epilogue warp: 32 pixels x 64 channels
 constexpr int SMEM_BYTES = W_BYTES + 2 * BUF_BYTES + EPI_WARPS * STAGE_BYTES;
-constexpr int ACC = 4;
+constexpr int ACC = 8;
 
 struct StemParams {
   const uint8_t* in;            // image 0 (or the ring's base with in_stub)
@@ -174,7 +175,7 @@ __global__ void __launch_bounds__(THREADS, 1) stem_conv_kernel(const __grid_cons
       ptx::cp_async_wait<0>();
       if (it > 0) hand_over(it - 1);
     } else {
-      // ---------------- epilogue: warps 4-7 take the even tiles, warps 8-11 the odd ones; a warp has 32 positions
+      // ---------------- epilogue: each set of four warps takes every third tile; a warp has 32 positions
       const int ew = warp - 4, set = ew >> 2, quarter = warp & 3;
       uint8_t* stage = s_out + ew * STAGE_BYTES;
       uint32_t tile = 0;
@@ -183,7 +184,7 @@ __global__ void __launch_bounds__(THREADS, 1) stem_conv_kernel(const __grid_cons
         const int img = c / p.chunks_per_img, first = (c - img * p.chunks_per_img) * chunk_pos;
         const int nt = tiles_of(c);
         for (int r = 0; r < nt; r++, tile++) {
-          if ((int)(tile & 1u) != set) continue;
+          if ((int)(tile % 3u) != set) continue;
           const uint32_t acc = tile & (ACC - 1);
           ok = ptx::mbar_wait_warp(&acc_full[acc], (tile / ACC) & 1u);
           if (!ok) break;
