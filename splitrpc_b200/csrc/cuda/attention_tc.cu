@@ -2,7 +2,7 @@
 //
 // One CTA serves one (sequence, head) and loops over its 128-query tiles.
 //   scores = Q . K^T      tcgen05.mma, M=128, N=128 per key block, K=64, fp32 in TMEM
-//   P = softmax(scores)   eight warps, half a query row per thread, read from TMEM,
+//   P = softmax(scores)   8 or 16 warps, 1/2 or 1/4 of a query row per thread, from TMEM,
 //                         written as bf16 into 128-byte-swizzled shared memory
 //   O = P . V             tcgen05.mma, M=128, N=64, K=SEQ, fp32 in TMEM
 // All operands arrive by TMA (no multicast) from this GPU's memory:
@@ -28,8 +28,13 @@ namespace {
 
 constexpr int HD = 64;          // head dim
 constexpr int QT = 128;         // queries per tile
-constexpr int SOFT_THREADS = 256;            // warps 0-7: softmax and output
-constexpr int ATT_THREADS = SOFT_THREADS + 32;  // warp 8: TMA and MMA issue
+// Softmax warps per tensor-memory lane quarter; one more warp issues TMA and MMAs.  Long rows take four: 384 keys need the
+// warps to keep the special-function unit busy (one CTA per SM).  With 128 keys three CTAs share an SM and two are enough.
+template <int SEQ>
+struct AttThreads {
+  static constexpr int SHARES = SEQ == QT ? 2 : 4;  // a thread has one query row and 1/SHARES of its keys
+  static constexpr int SOFT = SHARES * 128, TOTAL = SOFT + 32;
+};
 
 template <int SEQ>
 struct AttSmem {
@@ -52,8 +57,10 @@ struct AttSmem {
 // is then [keys, 64] with the head dimension contiguous, i.e. an MN-major B operand of the second product: same
 // 128-byte-swizzled shared-memory tile and descriptor, "B is MN-major" in the instruction descriptor, and a step of 16
 // keys along K is 2048 bytes (two 8-row groups) instead of 32.  No transposed copy of V and no separate V GEMM.
+template <int SOFT_THREADS>
 __device__ __forceinline__ void soft_sync() { asm volatile("bar.sync 1, %0;" ::"n"(SOFT_THREADS) : "memory"); }
 // The same barrier with the AND of the threads' predicates.
+template <int SOFT_THREADS>
 __device__ __forceinline__ bool soft_all(bool pred) {
   uint32_t out;
   asm volatile(
@@ -66,21 +73,22 @@ __device__ __forceinline__ bool soft_all(bool pred) {
 }
 
 template <int SEQ, bool VMN>
-__global__ void __launch_bounds__(ATT_THREADS, SEQ == QT ? 3 : 1)
+__global__ void __launch_bounds__(AttThreads<SEQ>::TOTAL, SEQ == QT ? 3 : 1)
 attention_tc(const __grid_constant__ CUtensorMap tmap_qk, const __grid_constant__ CUtensorMap tmap_vt,
              __nv_bfloat16* out, int ld_out, const float* v_bias, int hidden, float scale_log2e,
              uint32_t* status) {
   using L = AttSmem<SEQ>;
+  constexpr int SOFT_THREADS = AttThreads<SEQ>::SOFT, SHARES = AttThreads<SEQ>::SHARES;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint8_t* sQ = smem;
   uint8_t* sK = sQ + L::Q_BYTES;
   uint8_t* sVT = sK + L::K_BYTES;
   uint8_t* sP = smem + L::P_OFFSET;
-  __shared__ __align__(8) uint64_t bar_kv, bar_q, bar_s, bar_p, bar_o;
+  __shared__ __align__(8) uint64_t bar_k, bar_v, bar_q, bar_s, bar_p, bar_o;
   __shared__ uint32_t tmem_base_smem;
   __shared__ uint32_t s_error;
-  __shared__ float s_max[2][QT], s_sum[2][QT];
+  __shared__ float s_max[SHARES][QT], s_sum[SHARES][QT];
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int head = blockIdx.x, seq_idx = blockIdx.y;
@@ -88,7 +96,8 @@ attention_tc(const __grid_constant__ CUtensorMap tmap_qk, const __grid_constant_
   constexpr int NQT = SEQ / QT;
 
   if (threadIdx.x == 0) {
-    ptx::mbar_init(&bar_kv, 1);
+    ptx::mbar_init(&bar_k, 1);
+    ptx::mbar_init(&bar_v, 1);
     ptx::mbar_init(&bar_q, 1);
     ptx::mbar_init(&bar_s, 1);
     ptx::mbar_init(&bar_p, SOFT_THREADS / 32);
@@ -111,94 +120,102 @@ attention_tc(const __grid_constant__ CUtensorMap tmap_qk, const __grid_constant_
   const uint32_t tmem_o = tmem_base_smem + (L::ALIAS ? 0 : SEQ);  // output: columns [SEQ, SEQ+64), or over the scores
 
   if (warp == SOFT_THREADS / 32) {
-    if (ptx::elect_one()) {
-      // K and V^T of this head stay resident for all query tiles.  The first Q tile does not wait for them.
+    // The warp walks the tiles together, one elected lane issues: descriptors and addresses stay in uniform registers
+    // (see gemm_persistent.cu).  K and V^T of this head stay resident for all query tiles; the first Q tile does not wait
+    // for V^T.
+    const bool elected = ptx::elect_one();
+    auto load_q = [&](int qt) {
       ptx::mbar_expect_tx(&bar_q, L::Q_BYTES);
-      ptx::tma_load_2d(sQ, &tmap_qk, &bar_q, head * HD, tok0);
-      ptx::mbar_expect_tx(&bar_kv, L::K_BYTES + L::VT_BYTES);
+      ptx::tma_load_2d(sQ, &tmap_qk, &bar_q, head * HD, tok0 + qt * QT);
+    };
+    if (elected) {
+      load_q(0);
+      ptx::mbar_expect_tx(&bar_k, L::K_BYTES);
       for (int nb = 0; nb < SEQ / 128; nb++)
-        ptx::tma_load_2d(sK + nb * 128 * 128, &tmap_qk, &bar_kv, hidden + head * HD, tok0 + nb * 128);
+        ptx::tma_load_2d(sK + nb * 128 * 128, &tmap_qk, &bar_k, hidden + head * HD, tok0 + nb * 128);
+      ptx::mbar_expect_tx(&bar_v, L::VT_BYTES);
       if constexpr (VMN) {
         for (int nb = 0; nb < SEQ / 128; nb++)
-          ptx::tma_load_2d(sVT + nb * 128 * 128, &tmap_qk, &bar_kv, 2 * hidden + head * HD, tok0 + nb * 128);
+          ptx::tma_load_2d(sVT + nb * 128 * 128, &tmap_qk, &bar_v, 2 * hidden + head * HD, tok0 + nb * 128);
       } else {
-        for (int a = 0; a < SEQ / 64; a++) ptx::tma_load_2d(sVT + a * 64 * 128, &tmap_vt, &bar_kv, tok0 + a * 64, head * HD);
+        for (int a = 0; a < SEQ / 64; a++) ptx::tma_load_2d(sVT + a * 64 * 128, &tmap_vt, &bar_v, tok0 + a * 64, head * HD);
       }
-      bool ok = ptx::mbar_wait(&bar_kv, 0);
-      const uint32_t idesc_s = ptx::umma_idesc_bf16(QT, 128);
-      const uint32_t idesc_o = ptx::umma_idesc_bf16(QT, HD) | (VMN ? (1u << 16) : 0u);  // bit 16: B is MN-major
-      const uint32_t q_addr = ptx::smem_u32(sQ), k_addr = ptx::smem_u32(sK), p_addr = ptx::smem_u32(sP), vt_addr = ptx::smem_u32(sVT);
-      auto load_q = [&](int qt) {
-        ptx::mbar_expect_tx(&bar_q, L::Q_BYTES);
-        ptx::tma_load_2d(sQ, &tmap_qk, &bar_q, head * HD, tok0 + qt * QT);
-      };
-      auto scores = [&]() {
-        for (int nb = 0; nb < SEQ / 128; nb++)
+    }
+    const uint32_t idesc_s = ptx::umma_idesc_bf16(QT, 128);
+    const uint32_t idesc_o = ptx::umma_idesc_bf16(QT, HD) | (VMN ? (1u << 16) : 0u);  // bit 16: B is MN-major
+    const uint32_t q_lo = ptx::umma_desc_lo(ptx::smem_u32(sQ)), k_lo = ptx::umma_desc_lo(ptx::smem_u32(sK)),
+                   p_lo = ptx::umma_desc_lo(ptx::smem_u32(sP)), v_lo = ptx::umma_desc_lo(ptx::smem_u32(sVT));
+    auto scores = [&]() {
+      if (!elected) return;
 #pragma unroll
-          for (int k = 0; k < HD / 16; k++)
-            ptx::umma_bf16(tmem_s + nb * 128, ptx::umma_desc_sw128(q_addr + k * 32),
-                           ptx::umma_desc_sw128(k_addr + nb * 128 * 128 + k * 32), idesc_s, k != 0 ? 1u : 0u);
-        ptx::umma_commit(&bar_s);
-      };
-      ok = ok && ptx::mbar_wait(&bar_q, 0);
-      if (ok) scores();
-      for (int qt = 0; qt < NQT && ok; qt++) {
-        const uint32_t ph = (uint32_t)qt & 1u;
-        // The next Q tile takes this one's place as soon as its scores exist, while the softmax runs.
-        if (qt + 1 < NQT) {
-          if (!(ok = ptx::mbar_wait(&bar_s, ph))) break;
-          load_q(qt + 1);
-        }
-        // P ready (written by the softmax warps, which have read all scores by then)
-        if (!(ok = ptx::mbar_wait(&bar_p, ph))) break;
-        ptx::tc_fence_after();
+      for (int nb = 0; nb < SEQ / 128; nb++)
+#pragma unroll
+        for (int k = 0; k < HD / 16; k++)
+          ptx::umma_bf16(tmem_s + nb * 128, ptx::umma_desc_join(q_lo + k * 2), ptx::umma_desc_join(k_lo + nb * (128 * 128 / 16) + k * 2),
+                         idesc_s, k != 0 ? 1u : 0u);
+      ptx::umma_commit(&bar_s);
+    };
+    bool ok = ptx::mbar_wait_warp(&bar_q, 0) && ptx::mbar_wait_warp(&bar_k, 0);
+    if (ok) scores();
+    ok = ok && ptx::mbar_wait_warp(&bar_v, 0);
+    for (int qt = 0; qt < NQT && ok; qt++) {
+      const uint32_t ph = (uint32_t)qt & 1u;
+      // The next Q tile takes this one's place as soon as its scores exist, while the softmax runs.
+      if (qt + 1 < NQT) {
+        if (!(ok = ptx::mbar_wait_warp(&bar_s, ph))) break;
+        if (elected) load_q(qt + 1);
+      }
+      // P ready (written by the softmax warps, which have read all scores by then)
+      if (!(ok = ptx::mbar_wait_warp(&bar_p, ph))) break;
+      ptx::tc_fence_after();
+      if (elected) {
+#pragma unroll
         for (int kk = 0; kk < SEQ / 16; kk++) {
-          const int atom = kk >> 2, sub = kk & 3;
-          const uint32_t v_desc_addr = VMN ? vt_addr + kk * 2048 : vt_addr + atom * 64 * 128 + sub * 32;
-          ptx::umma_bf16(tmem_o, ptx::umma_desc_sw128(p_addr + atom * QT * 128 + sub * 32), ptx::umma_desc_sw128(v_desc_addr),
+          const uint32_t atom = (uint32_t)kk >> 2, sub = (uint32_t)kk & 3u;
+          const uint32_t v_at = VMN ? (uint32_t)kk * (2048 / 16) : atom * (64 * 128 / 16) + sub * 2;
+          ptx::umma_bf16(tmem_o, ptx::umma_desc_join(p_lo + atom * (QT * 128 / 16) + sub * 2), ptx::umma_desc_join(v_lo + v_at),
                          idesc_o, kk != 0 ? 1u : 0u);
         }
         ptx::umma_commit(&bar_o);
-        // The next tile's scores run behind P.V, while the output is written.
-        if (qt + 1 < NQT) {
-          if (!(ok = ptx::mbar_wait(&bar_q, ph ^ 1u))) break;
-          scores();
-        }
       }
-      if (!ok) atomicExch(&s_error, 1u);
+      // The next tile's scores run behind P.V, while the output is written.
+      if (qt + 1 < NQT) {
+        if (!(ok = ptx::mbar_wait_warp(&bar_q, ph ^ 1u))) break;
+        scores();
+      }
     }
+    if (!ok && elected) atomicCAS(&s_error, 0u, 1u);
   } else {
-    // Two warps per tensor-memory lane quarter: a thread has one query row and half of its keys; the halves' maxima and
-    // sums meet in shared memory.
-    const int half = warp >> 2, row = (warp & 3) * 32 + lane;
-    constexpr int COLS = SEQ / 2;
-    const int c0 = half * COLS;
+    // A thread has one query row and a share of its keys; the shares' maxima and sums meet in shared memory.
+    const int share = warp >> 2, row = (warp & 3) * 32 + lane;
+    constexpr int COLS = SEQ / SHARES;
+    const int c0 = share * COLS;
     const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
     for (int qt = 0; qt < NQT; qt++) {
       const uint32_t ph = (uint32_t)qt & 1u;
       const bool got = *(volatile uint32_t*)&s_error == 0 && ptx::mbar_wait(&bar_s, ph);
-      if (!soft_all(got)) {
+      if (!soft_all<SOFT_THREADS>(got)) {
         if (lane == 0) atomicCAS(&s_error, 0u, 2u);
         break;
       }
       ptx::tc_fence_after();
       // pass 1: row maximum
       float mx = -3.0e38f;
-#pragma unroll 1
-      for (int c = 0; c < COLS; c += 64) {
-        uint32_t r[64];
+      for (int c = 0; c < COLS; c += 32) {
+        uint32_t r[32];
         ptx::tmem_ld_32x32b_x32(tmem_s + lane_base + c0 + c, r);
-        ptx::tmem_ld_32x32b_x32(tmem_s + lane_base + c0 + c + 32, r + 32);
         ptx::tmem_ld_wait();
 #pragma unroll
-        for (int j = 0; j < 64; j++) mx = fmaxf(mx, __uint_as_float(r[j]));
+        for (int j = 0; j < 32; j++) mx = fmaxf(mx, __uint_as_float(r[j]));
       }
-      s_max[half][row] = mx;
-      soft_sync();
-      mx = fmaxf(s_max[0][row], s_max[1][row]);
-      // pass 2: exponentials, row sum, P in bf16 to swizzled shared memory
+      s_max[share][row] = mx;
+      soft_sync<SOFT_THREADS>();
+#pragma unroll
+      for (int k = 0; k < SHARES; k++) mx = fmaxf(mx, s_max[k][row]);
+      // pass 2: exponentials, row sum, P in bf16 to swizzled shared memory.  Packed differences and products; the flushed
+      // exponentials (weights below 2^-126 of the row's largest) are lost in the row's sum of at least one anyway.
       float sum = 0.f;
-#pragma unroll 1
+      const float2 neg_mx = make_float2(-mx, -mx), scale2 = make_float2(scale_log2e, scale_log2e);
       for (int c = c0; c < c0 + COLS; c += 32) {
         uint32_t r[32];
         ptx::tmem_ld_32x32b_x32(tmem_s + lane_base + c, r);
@@ -211,8 +228,11 @@ attention_tc(const __grid_constant__ CUtensorMap tmap_qk, const __grid_constant_
           __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&q);
 #pragma unroll
           for (int t = 0; t < 4; t++) {
-            const float e0 = exp2f((__uint_as_float(r[j * 8 + 2 * t]) - mx) * scale_log2e);
-            const float e1 = exp2f((__uint_as_float(r[j * 8 + 2 * t + 1]) - mx) * scale_log2e);
+            const float2 x = make_float2(__uint_as_float(r[j * 8 + 2 * t]), __uint_as_float(r[j * 8 + 2 * t + 1]));
+            const float2 y = __fmul2_rn(__fadd2_rn(x, neg_mx), scale2);
+            float e0, e1;
+            asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e0) : "f"(y.x));
+            asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e1) : "f"(y.y));
             h[t] = __floats2bfloat162_rn(e0, e1);
             // the row sum uses the rounded values that the second product will see
             float2 back = __bfloat1622float2(h[t]);
@@ -221,20 +241,24 @@ attention_tc(const __grid_constant__ CUtensorMap tmap_qk, const __grid_constant_
           *reinterpret_cast<uint4*>(prow + (((chunk0 + j) ^ (row & 7)) << 4)) = q;
         }
       }
-      s_sum[half][row] = sum;
+      s_sum[share][row] = sum;
       ptx::tc_fence_before();
       ptx::fence_proxy_async_smem();
       __syncwarp();
       if (lane == 0) ptx::mbar_arrive(&bar_p);
-      // output tile: each half writes 32 of the head's 64 columns
-      if (!soft_all(ptx::mbar_wait(&bar_o, ph))) {
+      // output tile: the first two shares write 32 of the head's 64 columns each
+      if (!soft_all<SOFT_THREADS>(ptx::mbar_wait(&bar_o, ph))) {
         if (lane == 0) atomicCAS(&s_error, 0u, 3u);
         break;
       }
       ptx::tc_fence_after();
-      const float inv = 1.f / (s_sum[0][row] + s_sum[1][row]);
+      if (share >= 2) continue;
+      float total = s_sum[0][row];
+#pragma unroll
+      for (int k = 1; k < SHARES; k++) total += s_sum[k][row];
+      const float inv = 1.f / total;
       __nv_bfloat16* orow = out + (size_t)(tok0 + qt * QT + row) * ld_out + head * HD;
-      const int c = half * 32;
+      const int c = share * 32;
       uint32_t r[32];
       ptx::tmem_ld_32x32b_x32(tmem_o + lane_base + c, r);
       ptx::tmem_ld_wait();
@@ -294,7 +318,7 @@ cudaError_t launch(const CUtensorMap& tqk, const CUtensorMap& tvt, void* out, in
     attr.set(dev);
   }
   const float scale_log2e = 0.125f * 1.4426950408889634f;
-  return launch_pdl(attention_tc<SEQ, VMN>, dim3(heads, batch), dim3(ATT_THREADS), smem, s, tqk, tvt, (__nv_bfloat16*)out, ld_out, v_bias,
+  return launch_pdl(attention_tc<SEQ, VMN>, dim3(heads, batch), dim3(AttThreads<SEQ>::TOTAL), smem, s, tqk, tvt, (__nv_bfloat16*)out, ld_out, v_bias,
                     hidden, scale_log2e, status);
 }
 
