@@ -115,8 +115,6 @@ struct TileParams {
   int kb_split, stride2;
 };
 
-__device__ __forceinline__ float gelu_f(float x) { return ptx::gelu_erf_fast(x); }
-
 __device__ __forceinline__ void named_bar_sync(int id, int count) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory");
 }
@@ -583,7 +581,11 @@ gemm_conv_persistent(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
           for (int j = 0; j < 32; j++) v[j] = fmaxf(v[j], 0.f);
         } else if (ep.act == GEMM_ACT_GELU) {
 #pragma unroll
-          for (int j = 0; j < 32; j++) v[j] = gelu_f(v[j]);
+          for (int j = 0; j < 32; j += 2) {
+            const float2 g = ptx::gelu_erf_fast2(make_float2(v[j], v[j + 1]));
+            v[j] = g.x;
+            v[j + 1] = g.y;
+          }
         } else if (ep.act == GEMM_ACT_TANH) {
 #pragma unroll
           for (int j = 0; j < 32; j++) v[j] = tanhf(v[j]);
@@ -699,6 +701,7 @@ struct MapKey {
   uint32_t box[5];
   uint32_t es[5];
   int rank;
+  uint32_t swizzle;
   bool operator==(const MapKey& o) const { return std::memcmp(this, &o, sizeof(MapKey)) == 0; }
 };
 struct MapKeyHash {
@@ -713,13 +716,14 @@ struct MapKeyHash {
 // Tensor maps are cached: encoding costs microseconds and the same layers run
 // for every batch.
 cudaError_t get_map(CUtensorMap* out, const void* ptr, int rank, const uint64_t* dims, const uint64_t* strides_bytes,
-                    const uint32_t* box, const uint32_t* estr) {
+                    const uint32_t* box, const uint32_t* estr, CUtensorMapSwizzle swizzle = CU_TENSOR_MAP_SWIZZLE_128B) {
   static std::mutex mu;
   static std::unordered_map<MapKey, CUtensorMap, MapKeyHash> cache;
   MapKey k;
   std::memset(&k, 0, sizeof(k));
   k.ptr = ptr;
   k.rank = rank;
+  k.swizzle = (uint32_t)swizzle;
   for (int i = 0; i < rank; i++) {
     k.d[i] = dims[i];
     k.box[i] = box[i];
@@ -743,7 +747,7 @@ cudaError_t get_map(CUtensorMap* out, const void* ptr, int rank, const uint64_t*
     if (i + 1 < rank) gs[i] = strides_bytes[i];
   }
   CUresult r = d->TensorMapEncodeTiled(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, (cuuint32_t)rank, const_cast<void*>(ptr), gd, gs,
-                                       bx, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                                       bx, es, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
                                        CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return cudaErrorInvalidValue;
   if (cache.size() > 4096) cache.clear();
@@ -751,11 +755,12 @@ cudaError_t get_map(CUtensorMap* out, const void* ptr, int rank, const uint64_t*
   return cudaSuccess;
 }
 
+// Rows of the box are 128 bytes of shared memory under the 128-byte swizzle and 64 bytes under the 64-byte one.
 cudaError_t map_2d(CUtensorMap* m, const void* ptr, uint64_t inner, uint64_t outer, uint64_t row_stride_bytes,
                    uint32_t box_inner, uint32_t box_outer) {
   uint64_t dims[2] = {inner, outer}, st[1] = {row_stride_bytes};
   uint32_t box[2] = {box_inner, box_outer}, es[2] = {1, 1};
-  return get_map(m, ptr, 2, dims, st, box, es);
+  return get_map(m, ptr, 2, dims, st, box, es, box_inner == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B);
 }
 
 // SMs that the persistent kernels size their grids for.  A persistent kernel has one block per SM and a fixed tile

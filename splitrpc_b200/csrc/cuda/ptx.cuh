@@ -133,6 +133,24 @@ __device__ __forceinline__ float gelu_erf_fast(float x) {
   return x * (x < 0.f ? h : 1.0f - h);
 }
 
+// The same for two values with packed arithmetic: every operation and rounding of gelu_erf_fast, half the instructions.
+__device__ __forceinline__ float2 gelu_erf_fast2(float2 x) {
+  const float2 ax = __fmul2_rn(make_float2(fabsf(x.x), fabsf(x.y)), make_float2(0.70710678118654752f, 0.70710678118654752f));
+  const float2 d = __ffma2_rn(make_float2(0.3275911f, 0.3275911f), ax, make_float2(1.0f, 1.0f));
+  float2 t, e;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(t.x) : "f"(d.x));
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(t.y) : "f"(d.y));
+  float2 p = __ffma2_rn(t, make_float2(1.061405429f, 1.061405429f), make_float2(-1.453152027f, -1.453152027f));
+  p = __ffma2_rn(p, t, make_float2(1.421413741f, 1.421413741f));
+  p = __ffma2_rn(p, t, make_float2(-0.284496736f, -0.284496736f));
+  p = __ffma2_rn(p, t, make_float2(0.254829592f, 0.254829592f));
+  const float2 g = __fmul2_rn(__fmul2_rn(make_float2(-1.4426950408889634f, -1.4426950408889634f), ax), ax);
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e.x) : "f"(g.x));
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e.y) : "f"(g.y));
+  const float2 h = __fmul2_rn(__fmul2_rn(__fmul2_rn(make_float2(0.5f, 0.5f), p), t), e);  // 0.5 * erfc(|x| / sqrt 2)
+  return __fmul2_rn(x, make_float2(x.x < 0.f ? h.x : 1.0f - h.x, x.y < 0.f ? h.y : 1.0f - h.y));
+}
+
 // ---------------------------------------------------------------- proxies / fences
 __device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void fence_proxy_async_all() { asm volatile("fence.proxy.async;" ::: "memory"); }
