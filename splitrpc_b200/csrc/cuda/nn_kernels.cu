@@ -200,18 +200,33 @@ __global__ void __launch_bounds__(256) global_avgpool(const __nv_bfloat16* in, _
 
 // Skinny fully connected layer: out[m, n] = sum_k a[m, k] * w[n, k] + bias[n] for a handful of rows, fp32 output.  A
 // tensor-core tile would be 128 rows x 64 columns: with 64 rows that leaves 16 CTAs each walking all of K.  Here a
-// block owns FC_NB output columns and FC_ROWS rows: the weight rows are staged in shared memory as fp32 once (two
+// block owns FC_NB output columns and 16 * RPT rows: the weight rows are staged in shared memory as fp32 once (two
 // planes of float4 per column, so that the sixteen k-slices a warp reads together are contiguous), thread
-// (row pair, kq) walks every sixteenth 8-element slice of its two rows of `a` with the next slice's loads in flight, and
-// the sixteen partial sums of a row meet through shuffles.
-constexpr int FC_NB = 8, FC_ROWS = 32;
-__global__ void __launch_bounds__(256, 2) fc_skinny(const __nv_bfloat16* a, int lda, const __nv_bfloat16* w,
+// (row group, kq) walks every sixteenth 8-element slice of its RPT rows of `a` with the next slice's loads in flight, and
+// the sixteen partial sums of a row meet through shuffles.  A slice's weights are read from shared memory once for the
+// RPT rows: with two rows those reads were the limit (64 x 1000 x 2048: 15.6 us), with four it takes 12 us, of which the FMAs
+// are 4.  Two rows stay for up to 32 rows, where twice the blocks share the work.  The order of every sum is the same.
+constexpr int FC_NB = 8;
+template <int RPT>
+__global__ void __launch_bounds__(256, RPT == 2 ? 2 : 1) fc_skinny(const __nv_bfloat16* a, int lda, const __nv_bfloat16* w,
                                                  int ldw, const float* bias, float* out, int ldo, int M,
                                                  int N, int K) {
   ptx::grid_dep_launch();
   ptx::grid_dep_wait();
   extern __shared__ __align__(16) float4 s_w[];  // [FC_NB][2][K/8]
   const int n0 = blockIdx.x * FC_NB, kvn = K / 8;
+  const int kq = threadIdx.x & 15;
+  const int row0 = blockIdx.y * (16 * RPT) + (threadIdx.x >> 4) * RPT;
+  // rows past M read row M-1 again (their results are not stored): no branch inside the loop
+  const __nv_bfloat16* ar[RPT];
+#pragma unroll
+  for (int r = 0; r < RPT; r++) ar[r] = a + (size_t)min(row0 + r, M - 1) * lda;
+  auto load = [&](const __nv_bfloat16* r, int kv) {
+    return kv < kvn ? *(reinterpret_cast<const uint4*>(r + kv * 8)) : make_uint4(0, 0, 0, 0);
+  };
+  uint4 qa[RPT];  // the first slice of the rows travels beside the weights
+#pragma unroll
+  for (int r = 0; r < RPT; r++) qa[r] = load(ar[r], kq);
   for (int base = 0; base < FC_NB * kvn; base += 256 * 8) {
     uint4 q[8];  // eight loads in flight per thread: the weights usually come from DRAM
 #pragma unroll
@@ -233,71 +248,46 @@ __global__ void __launch_bounds__(256, 2) fc_skinny(const __nv_bfloat16* a, int 
     }
   }
   __syncthreads();
-  const int kq = threadIdx.x & 15;
-  const int row0 = blockIdx.y * FC_ROWS + (threadIdx.x >> 4) * 2;
-  // rows past M read row M-1 again (their results are not stored): no branch inside the loop
-  const __nv_bfloat16* ar0 = a + (size_t)min(row0, M - 1) * lda;
-  const __nv_bfloat16* ar1 = a + (size_t)min(row0 + 1, M - 1) * lda;
   // packed fp32 FMAs (two per instruction): lane x of an accumulator sums the even k, lane y the odd k
-  float2 acc0[FC_NB], acc1[FC_NB];
+  float2 acc[RPT][FC_NB];
 #pragma unroll
-  for (int j = 0; j < FC_NB; j++) acc0[j] = acc1[j] = make_float2(0.f, 0.f);
-  auto step = [&](const uint4& c0, const uint4& c1, int kv) {
-    float2 x0[4], x1[4];
-    const __nv_bfloat162* h0 = reinterpret_cast<const __nv_bfloat162*>(&c0);
-    const __nv_bfloat162* h1 = reinterpret_cast<const __nv_bfloat162*>(&c1);
+  for (int r = 0; r < RPT; r++)
 #pragma unroll
-    for (int t = 0; t < 4; t++) {
-      x0[t] = __bfloat1622float2(h0[t]);
-      x1[t] = __bfloat1622float2(h1[t]);
+    for (int j = 0; j < FC_NB; j++) acc[r][j] = make_float2(0.f, 0.f);
+  for (int kv = kq; kv < kvn; kv += 16) {
+    float2 x[RPT][4];
+#pragma unroll
+    for (int r = 0; r < RPT; r++) {
+      const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&qa[r]);
+#pragma unroll
+      for (int t = 0; t < 4; t++) x[r][t] = __bfloat1622float2(h[t]);
     }
+#pragma unroll
+    for (int r = 0; r < RPT; r++) qa[r] = load(ar[r], kv + 16);  // in flight during this slice's arithmetic
 #pragma unroll
     for (int j = 0; j < FC_NB; j++) {
       const float4 w0 = s_w[(j * 2) * kvn + kv], w1 = s_w[(j * 2 + 1) * kvn + kv];
-      const float2 wa = make_float2(w0.x, w0.y), wb = make_float2(w0.z, w0.w), wc = make_float2(w1.x, w1.y),
-                   wd = make_float2(w1.z, w1.w);
-      acc0[j] = __ffma2_rn(x0[0], wa, acc0[j]);
-      acc1[j] = __ffma2_rn(x1[0], wa, acc1[j]);
-      acc0[j] = __ffma2_rn(x0[1], wb, acc0[j]);
-      acc1[j] = __ffma2_rn(x1[1], wb, acc1[j]);
-      acc0[j] = __ffma2_rn(x0[2], wc, acc0[j]);
-      acc1[j] = __ffma2_rn(x1[2], wc, acc1[j]);
-      acc0[j] = __ffma2_rn(x0[3], wd, acc0[j]);
-      acc1[j] = __ffma2_rn(x1[3], wd, acc1[j]);
-    }
-  };
-  auto load = [&](const __nv_bfloat16* r, int kv) {
-    return kv < kvn ? *(reinterpret_cast<const uint4*>(r + kv * 8)) : make_uint4(0, 0, 0, 0);
-  };
-  // two slices per trip, the next trip's four loads issued before this trip's arithmetic
-  uint4 qa0 = load(ar0, kq), qa1 = load(ar1, kq), qb0 = load(ar0, kq + 16), qb1 = load(ar1, kq + 16);
-  for (int kv = kq; kv < kvn; kv += 32) {
-    const uint4 ca0 = qa0, ca1 = qa1, cb0 = qb0, cb1 = qb1;
-    qa0 = load(ar0, kv + 32);
-    qa1 = load(ar1, kv + 32);
-    qb0 = load(ar0, kv + 48);
-    qb1 = load(ar1, kv + 48);
-    step(ca0, ca1, kv);
-    if (kv + 16 < kvn) step(cb0, cb1, kv + 16);
-  }
-  float s0[FC_NB], s1[FC_NB];
+      const float2 wq[4] = {make_float2(w0.x, w0.y), make_float2(w0.z, w0.w), make_float2(w1.x, w1.y), make_float2(w1.z, w1.w)};
 #pragma unroll
-  for (int j = 0; j < FC_NB; j++) {
-    s0[j] = acc0[j].x + acc0[j].y;
-    s1[j] = acc1[j].x + acc1[j].y;
+      for (int t = 0; t < 4; t++)
 #pragma unroll
-    for (int d = 1; d < 16; d <<= 1) {
-      s0[j] += __shfl_xor_sync(0xffffffffu, s0[j], d);
-      s1[j] += __shfl_xor_sync(0xffffffffu, s1[j], d);
+        for (int r = 0; r < RPT; r++) acc[r][j] = __ffma2_rn(x[r][t], wq[t], acc[r][j]);
     }
   }
-  // lane kq stores column kq & 7 of row kq >> 3
 #pragma unroll
-  for (int j = 0; j < FC_NB; j++) {
-    if ((kq & 7) == j && n0 + j < N) {
-      const int row = row0 + (kq >> 3);
-      if (row < M) out[(size_t)row * ldo + n0 + j] = ((kq >> 3) ? s1[j] : s0[j]) + (bias ? bias[n0 + j] : 0.f);
+  for (int r = 0; r < RPT; r++) {
+    float s[FC_NB];
+#pragma unroll
+    for (int j = 0; j < FC_NB; j++) {
+      s[j] = acc[r][j].x + acc[r][j].y;
+#pragma unroll
+      for (int d = 1; d < 16; d <<= 1) s[j] += __shfl_xor_sync(0xffffffffu, s[j], d);
     }
+    // lane kq stores column kq & 7 of the rows r with r mod 2 = kq >> 3
+#pragma unroll
+    for (int j = 0; j < FC_NB; j++)
+      if ((kq & 7) == j && (kq >> 3) == (r & 1) && n0 + j < N && row0 + r < M)
+        out[(size_t)(row0 + r) * ldo + n0 + j] = s[j] + (bias ? bias[n0 + j] : 0.f);
   }
 }
 
@@ -625,12 +615,18 @@ cudaError_t nn_fc_skinny(const void* a, int lda, const void* w, int ldw, const f
   static PerDeviceFlag attr_set;
   const int dev = PerDeviceFlag::current();
   if (attr_set.needed(dev)) {
-    cudaError_t e = cudaFuncSetAttribute(fc_skinny, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    cudaError_t e = cudaFuncSetAttribute(fc_skinny<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(fc_skinny<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     if (e != cudaSuccess) return e;
     attr_set.set(dev);
   }
-  return launch_pdl(fc_skinny, dim3((N + FC_NB - 1) / FC_NB, (M + FC_ROWS - 1) / FC_ROWS), dim3(256), smem, s, (const
-                    __nv_bfloat16*)a, lda, (const __nv_bfloat16*)w, ldw, bias, out, ldo, M, N, K);
+  const dim3 block(256);
+  const unsigned cols = (unsigned)((N + FC_NB - 1) / FC_NB);
+  if (M <= 32)
+    return launch_pdl(fc_skinny<2>, dim3(cols, (M + 31) / 32), block, smem, s, (const __nv_bfloat16*)a, lda, (const __nv_bfloat16*)w,
+                      ldw, bias, out, ldo, M, N, K);
+  return launch_pdl(fc_skinny<4>, dim3(cols, (M + 63) / 64), block, smem, s, (const __nv_bfloat16*)a, lda, (const __nv_bfloat16*)w, ldw,
+                    bias, out, ldo, M, N, K);
 }
 cudaError_t nn_softmax_response(const float* logits, int rows, int n, int ld, const void* d_stub, void* direct_out,
                                 size_t resp_stride, int write_argmax, uint32_t* counter, uint32_t* flag, uint32_t flag_value,
