@@ -277,8 +277,9 @@ gemm_conv_persistent(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
   // The state lives across two calls: the first fills one (initially free) stage each right after the barriers exist,
   // before the block-wide set-up barrier, so that the first operands are already in flight while tensor memory is being
   // allocated; the second runs the rest of the schedule.
-  constexpr int PRODUCERS = 2;
-  const int producer = warp == 0 ? 0 : (warp == Threads<BN>::TOTAL / 32 - 1 ? 1 : -1);
+  // (A ring of one stage, which the widest load groups of a short filter leave, has one producer.)
+  const int producers = nst >= 2 ? 2 : 1;
+  const int producer = warp == 0 ? 0 : (warp == Threads<BN>::TOTAL / 32 - 1 && producers == 2 ? 1 : -1);
   int pr_s = producer, pr_kb = producer, pr_j = 0;
   uint32_t pr_ph = 0;
   int img_off = 0;
@@ -326,8 +327,8 @@ gemm_conv_persistent(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
     }
     if (!p.b_stationary && !p.reuse) ptx::tma_load_2d(sa + A_BYTES, &tmap_b, &full_bar[pr_s], pr_kb * BK, pr_tc.n_idx * BN);
     if (pr_j == 0 && pr_kb == 0) GEMM_TRACE(2);
-    pr_kb += PRODUCERS;
-    pr_s += PRODUCERS;
+    pr_kb += producers;
+    pr_s += producers;
     if (pr_s >= nst) {
       pr_s -= nst;
       pr_ph ^= 1u;

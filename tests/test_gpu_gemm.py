@@ -95,6 +95,18 @@ def test_two_input_pointwise_conv(env, n, oh, c1, h2, c2, cout, stride2):
     assert _rel_err(torch, out, torch.relu(ref)) < 1e-2
 
 
+@pytest.mark.parametrize("n,h,w,cout,r,s", [(1, 20, 16, 128, 4, 1), (1, 11, 14, 72, 4, 1), (1, 20, 16, 128, 2, 1), (1, 20, 16, 200, 3, 1), (2, 20, 16, 64, 4, 1)])
+def test_conv_with_few_wide_load_groups(env, n, h, w, cout, r, s):
+    """Short filters on small images: all row taps of a column travel in one load group, and the ring holds one to three."""
+    torch, ops = env
+    x = torch.randn(n, h, w, 64, device="cuda").bfloat16()
+    f = (torch.randn(cout, r, s, 64, device="cuda") / (64 * r * s) ** 0.5).bfloat16()
+    out = ops.conv2d_nhwc(x, f)
+    ops.check_status()
+    ref = torch.nn.functional.conv2d(x.double().permute(0, 3, 1, 2), f.double().permute(0, 3, 1, 2)).permute(0, 2, 3, 1)
+    assert out.shape == ref.shape and ((out.double() - ref).norm() / ref.norm()).item() < 2.0 ** -8  # one rounding to bf16
+
+
 @pytest.mark.parametrize("n,h,cin,cout,r,stride,pad", [(2, 56, 64, 64, 3, 1, 1), (4, 28, 128, 128, 3, 1, 1),
                                                        (2, 56, 256, 128, 1, 2, 0), (3, 14, 256, 256, 3, 1, 1),
                                                        (2, 7, 512, 512, 3, 1, 1), (2, 56, 64, 256, 1, 1, 0),
