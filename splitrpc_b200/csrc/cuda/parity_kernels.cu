@@ -322,9 +322,12 @@ lstm_wavefront_kernel(const g_params* stub, const float* direct_in, float* direc
 // (lstm_bump_kernel adds one before every launch; graph replays count too), so nothing has to be cleared in between.
 // A block stages the vectors of a step in shared memory for its warps; the 4 x NB gate sums of a warp are reduced together
 // (values are halved between lane pairs as they are added).  The kernel is launched cooperatively: all blocks are resident,
-// and every wait is bounded.  Bounded by the exchange latency (about 1.5 us per step with the staging and the arithmetic).
+// and every wait is bounded.  30.6 / 39.4 / 50.6 / 74.8 us for 1 / 2 / 4 / 8 requests back to back (61.8 / 84.0 / 128.9 / 216.7 us with a
+// grid barrier per wave); what is left is the exchange latency, 2 us per step for one request, and 0.4 us per further request.
 constexpr int LSTM_GROUP = 8;          // requests per launch
-constexpr int LSTM_LAYER_BLOCKS = 18;  // 8 x 18 = 144 of 148 SMs
+// 8 x 16 = 128 of 148 SMs.  A cooperative launch waits until all its blocks fit, and a block takes all registers of its SM; the
+// resident copy engine (16 blocks that do not leave between requests) and the other resident kernels need the rest.
+constexpr int LSTM_LAYER_BLOCKS = 16;
 constexpr int LSTM_WARPS = (LH + LSTM_LAYER_BLOCKS - 1) / LSTM_LAYER_BLOCKS;  // hidden units per block
 constexpr int LSTM_THREADS = LSTM_WARPS * 32;
 constexpr long long LSTM_WAIT_CYCLES = 4000000000ll;

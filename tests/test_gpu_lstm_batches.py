@@ -46,3 +46,28 @@ def test_batches_and_repeated_runs(C, launch_type):
         want = _exact(w, x)
         # 64 cells of 512-term fp32 sums in a row; measured 2e-7 of the result's norm
         assert np.linalg.norm(got.cpu().numpy() - want) < 2e-6 * np.linalg.norm(want), n
+
+
+def test_beside_the_resident_copy_engine(C):
+    """The cooperative launch needs 128 SMs to itself while the resident copy engine (copy type 1) holds blocks on 16 of them."""
+    import torch
+
+    torch.cuda.set_device(0)
+    rng = np.random.default_rng(8)
+    w = [(rng.standard_normal(s) * 0.08).astype(np.float32) for _ in range(L) for s in ((4, H, H), (4, H, H), (4, H))]
+    C.set_rpc_mtu(8192)
+    sp, cp = C.make_loopback_pair(8192, 512, "pinned")
+    app = C.make_app("lstm", 0, T * H * 4, H * 4, w, 64, 1, 8, copy_type=1)
+    srv = C.Server(sp, req_size=T * H * 4, resp_size=H * 4, server_mode=2, max_batch=8)
+    srv.add_replica(app)
+    srv.start()
+    cli = C.Client(cp, req_size=T * H * 4, resp_size=H * 4, total=64, warmup=0, payload="uniform", verify=True, n_payloads=4)
+    try:
+        assert cli.run_closed_loop(8) and cli.received == 64
+        assert srv.worker_stats(0)["wait_timeouts"] == 0
+    finally:
+        srv.stop()
+    for k in range(4):
+        x = np.frombuffer(cli.payload(k), dtype=np.float32).reshape(1, T, H)
+        got = np.frombuffer(cli.response(k), dtype=np.float32)
+        np.testing.assert_allclose(got, _exact(w, x)[0], rtol=1e-4, atol=1e-6)
