@@ -204,8 +204,9 @@ __global__ void __launch_bounds__(256) global_avgpool(const __nv_bfloat16* in, _
 // planes of float4 per column, so that the sixteen k-slices a warp reads together are contiguous), thread
 // (row group, kq) walks every sixteenth 8-element slice of its RPT rows of `a` with the next slice's loads in flight, and
 // the sixteen partial sums of a row meet through shuffles.  A slice's weights are read from shared memory once for the
-// RPT rows: with two rows those reads were the limit (64 x 1000 x 2048: 15.6 us), with four it takes 12 us, of which the FMAs
-// are 4.  Two rows stay for up to 32 rows, where twice the blocks share the work.  The order of every sum is the same.
+// RPT rows: with two rows those reads bound 64 x 1000 x 2048 (15.2 us), with four it takes 13.3 us, of which the FMAs are 4.  Two
+// rows stay for up to 32 rows (about 10 us), where there are enough of them for one block per column group anyway.  The order of
+// every sum is the same.
 constexpr int FC_NB = 8;
 template <int RPT>
 __global__ void __launch_bounds__(256, RPT == 2 ? 2 : 1) fc_skinny(const __nv_bfloat16* a, int lda, const __nv_bfloat16* w,
@@ -224,9 +225,13 @@ __global__ void __launch_bounds__(256, RPT == 2 ? 2 : 1) fc_skinny(const __nv_bf
   auto load = [&](const __nv_bfloat16* r, int kv) {
     return kv < kvn ? *(reinterpret_cast<const uint4*>(r + kv * 8)) : make_uint4(0, 0, 0, 0);
   };
-  uint4 qa[RPT];  // the first slice of the rows travels beside the weights
+  // AHEAD slices of every row are in flight, the first ones beside the weights (four rows: more than one slice measured slower).
+  constexpr int AHEAD = RPT == 2 ? 2 : 1;
+  uint4 qa[AHEAD][RPT];
 #pragma unroll
-  for (int r = 0; r < RPT; r++) qa[r] = load(ar[r], kq);
+  for (int d = 0; d < AHEAD; d++)
+#pragma unroll
+    for (int r = 0; r < RPT; r++) qa[d][r] = load(ar[r], kq + 16 * d);
   for (int base = 0; base < FC_NB * kvn; base += 256 * 8) {
     uint4 q[8];  // eight loads in flight per thread: the weights usually come from DRAM
 #pragma unroll
@@ -254,24 +259,29 @@ __global__ void __launch_bounds__(256, RPT == 2 ? 2 : 1) fc_skinny(const __nv_bf
   for (int r = 0; r < RPT; r++)
 #pragma unroll
     for (int j = 0; j < FC_NB; j++) acc[r][j] = make_float2(0.f, 0.f);
-  for (int kv = kq; kv < kvn; kv += 16) {
-    float2 x[RPT][4];
+  for (int kv0 = kq; kv0 < kvn; kv0 += 16 * AHEAD) {
 #pragma unroll
-    for (int r = 0; r < RPT; r++) {
-      const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&qa[r]);
+    for (int d = 0; d < AHEAD; d++) {
+      const int kv = kv0 + 16 * d;
+      if (kv >= kvn) break;
+      float2 x[RPT][4];
 #pragma unroll
-      for (int t = 0; t < 4; t++) x[r][t] = __bfloat1622float2(h[t]);
-    }
+      for (int r = 0; r < RPT; r++) {
+        const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&qa[d][r]);
 #pragma unroll
-    for (int r = 0; r < RPT; r++) qa[r] = load(ar[r], kv + 16);  // in flight during this slice's arithmetic
+        for (int t = 0; t < 4; t++) x[r][t] = __bfloat1622float2(h[t]);
+      }
 #pragma unroll
-    for (int j = 0; j < FC_NB; j++) {
-      const float4 w0 = s_w[(j * 2) * kvn + kv], w1 = s_w[(j * 2 + 1) * kvn + kv];
-      const float2 wq[4] = {make_float2(w0.x, w0.y), make_float2(w0.z, w0.w), make_float2(w1.x, w1.y), make_float2(w1.z, w1.w)};
+      for (int r = 0; r < RPT; r++) qa[d][r] = load(ar[r], kv + 16 * AHEAD);  // in flight during the arithmetic
 #pragma unroll
-      for (int t = 0; t < 4; t++)
+      for (int j = 0; j < FC_NB; j++) {
+        const float4 w0 = s_w[(j * 2) * kvn + kv], w1 = s_w[(j * 2 + 1) * kvn + kv];
+        const float2 wq[4] = {make_float2(w0.x, w0.y), make_float2(w0.z, w0.w), make_float2(w1.x, w1.y), make_float2(w1.z, w1.w)};
 #pragma unroll
-        for (int r = 0; r < RPT; r++) acc[r][j] = __ffma2_rn(x[r][t], wq[t], acc[r][j]);
+        for (int t = 0; t < 4; t++)
+#pragma unroll
+          for (int r = 0; r < RPT; r++) acc[r][j] = __ffma2_rn(x[r][t], wq[t], acc[r][j]);
+      }
     }
   }
 #pragma unroll
@@ -442,7 +452,7 @@ __global__ void __launch_bounds__(256) layernorm_rows_warp(const __nv_bfloat16* 
     }
   }
   // The parameters are fetched while the row's sums travel through the warp: read where they are used, after the
-  // reductions, they cost every row a second round trip (4096 x 768: 5.0 -> 4.2 us beside the neighbouring kernels).
+  // reductions, they cost every row a second round trip (4096 x 768 back to back 4.4 -> 4.1 us).
   float4 g4[2 * VPL], b4[2 * VPL];
 #pragma unroll
   for (int i = 0; i < VPL; i++) {
@@ -620,11 +630,14 @@ cudaError_t nn_fc_skinny(const void* a, int lda, const void* w, int ldw, const f
     if (e != cudaSuccess) return e;
     attr_set.set(dev);
   }
+  // One block per SM where that is enough for all of them (more than half of an SM's shared memory): blocks that start while
+  // the kernel before still runs would otherwise be stacked two to an SM beside empty ones (32 rows: 13.6 us then, about 10 us now).
+  const size_t spread = 116 * 1024;
   const dim3 block(256);
   const unsigned cols = (unsigned)((N + FC_NB - 1) / FC_NB);
   if (M <= 32)
-    return launch_pdl(fc_skinny<2>, dim3(cols, (M + 31) / 32), block, smem, s, (const __nv_bfloat16*)a, lda, (const __nv_bfloat16*)w,
-                      ldw, bias, out, ldo, M, N, K);
+    return launch_pdl(fc_skinny<2>, dim3(cols), block, cols <= 148 && smem < spread ? spread : smem, s, (const __nv_bfloat16*)a,
+                      lda, (const __nv_bfloat16*)w, ldw, bias, out, ldo, M, N, K);
   return launch_pdl(fc_skinny<4>, dim3(cols, (M + 63) / 64), block, smem, s, (const __nv_bfloat16*)a, lda, (const __nv_bfloat16*)w, ldw,
                     bias, out, ldo, M, N, K);
 }
