@@ -205,11 +205,11 @@ __global__ void __launch_bounds__(256) global_avgpool(const __nv_bfloat16* in, _
 // (row group, kq) walks every sixteenth 8-element slice of its RPT rows of `a` with the next slice's loads in flight, and
 // the sixteen partial sums of a row meet through shuffles.  A slice's weights are read from shared memory once for the
 // RPT rows: with two rows those reads bound 64 x 1000 x 2048 (15.2 us), with four it takes 13.3 us, of which the FMAs are 4.  Two
-// rows stay for up to 32 rows (about 10 us), where there are enough of them for one block per column group anyway.  The order of
+// rows stay for up to 32 rows (9.1 us), where there are enough of them for one block per column group anyway.  The order of
 // every sum is the same.
 constexpr int FC_NB = 8;
 template <int RPT>
-__global__ void __launch_bounds__(256, RPT == 2 ? 2 : 1) fc_skinny(const __nv_bfloat16* a, int lda, const __nv_bfloat16* w,
+__global__ void __launch_bounds__(256, 1) fc_skinny(const __nv_bfloat16* a, int lda, const __nv_bfloat16* w,
                                                  int ldw, const float* bias, float* out, int ldo, int M,
                                                  int N, int K) {
   ptx::grid_dep_launch();
@@ -631,7 +631,7 @@ cudaError_t nn_fc_skinny(const void* a, int lda, const void* w, int ldw, const f
     attr_set.set(dev);
   }
   // One block per SM where that is enough for all of them (more than half of an SM's shared memory): blocks that start while
-  // the kernel before still runs would otherwise be stacked two to an SM beside empty ones (32 rows: 13.6 us then, about 10 us now).
+  // the kernel before still runs would otherwise be stacked two to an SM beside empty ones (32 rows: 13.6 us then, 9.1 us now).
   const size_t spread = 116 * 1024;
   const dim3 block(256);
   const unsigned cols = (unsigned)((N + FC_NB - 1) / FC_NB);
