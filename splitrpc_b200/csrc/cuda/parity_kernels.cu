@@ -322,14 +322,19 @@ lstm_wavefront_kernel(const g_params* stub, const float* direct_in, float* direc
 // (lstm_bump_kernel adds one before every launch; graph replays count too), so nothing has to be cleared in between.
 // A block stages the vectors of a step in shared memory for its warps; the 4 x NB gate sums of a warp are reduced together
 // (values are halved between lane pairs as they are added).  The kernel is launched cooperatively: all blocks are resident,
-// and every wait is bounded.  30.6 / 39.4 / 50.6 / 74.8 us for 1 / 2 / 4 / 8 requests back to back (61.8 / 84.0 / 128.9 / 216.7 us with a
+// and every wait is bounded.  32.0 / 39.0 / 50.3 / 79.4 us for 1 / 2 / 4 / 8 requests back to back (61.8 / 84.0 / 128.9 / 216.7 us with a
 // grid barrier per wave); what is left is the exchange latency, 2 us per step for one request, and 0.4 us per further request.
 constexpr int LSTM_GROUP = 8;          // requests per launch
-// 8 x 16 = 128 of 148 SMs.  A cooperative launch waits until all its blocks fit, and a block takes all registers of its SM; the
-// resident copy engine (16 blocks that do not leave between requests) and the other resident kernels need the rest.
-constexpr int LSTM_LAYER_BLOCKS = 16;
+constexpr int LSTM_LAYER_BLOCKS = 16;  // 8 x 16 = 128 of 148 SMs
 constexpr int LSTM_WARPS = (LH + LSTM_LAYER_BLOCKS - 1) / LSTM_LAYER_BLOCKS;  // hidden units per block
 constexpr int LSTM_THREADS = LSTM_WARPS * 32;
+// A cooperative launch waits until all its blocks fit, and the blocks of resident copy engines (16 each) do not leave between
+// requests: with 128 registers a block of this kernel took all of its SM, and two engines left it 116 SMs.  512 threads x 104
+// registers leave room for one engine block on every SM (256 threads, held to 48 registers by its launch bounds, sg_kernels.cu);
+// the 20 SMs that no block needs may hold any number.  Two requests' sums at a time keep the warp within 104 registers
+// (all at once with 128: 31.0 / 40.0 / 51.7 / 72.0 us; 96 registers spill: 37.2 / 39.3 / 55.4 / 93.5 us).
+constexpr int LSTM_REGS = 104;
+static_assert(LSTM_THREADS * LSTM_REGS + 256 * 48 <= 65536, "a block and a resident copy block share an SM's registers");
 constexpr long long LSTM_WAIT_CYCLES = 4000000000ll;
 
 struct LstmGridArgs {
@@ -354,10 +359,12 @@ __device__ __forceinline__ void ld_two_words(const unsigned long long* p, unsign
 __global__ void lstm_bump_kernel(unsigned* epoch) { *epoch += 1; }
 
 template <int NB>
-__global__ void __launch_bounds__(LSTM_THREADS, 1) lstm_grid_kernel(const LstmGridArgs a) {
-  constexpr int NV = 4 * NB;                                     // gate sums per warp
-  constexpr int LOG_NV = NV == 4 ? 2 : (NV == 8 ? 3 : (NV == 16 ? 4 : 5));
-  constexpr int MAXQ = (2 * NB * (LH / 2) + LSTM_THREADS - 1) / LSTM_THREADS;  // word pairs a thread stages per step
+__global__ void __maxnreg__(LSTM_REGS) lstm_grid_kernel(const LstmGridArgs a) {
+  constexpr int P = NB == 1 ? 1 : 2, PASSES = NB / P;            // requests whose sums a warp forms together
+  constexpr int PV = 4 * P, REP = 32 / PV;                       // their gate sums, lanes per sum after the reduction
+  constexpr int ROWS = LSTM_THREADS / (LH / 2);                  // vectors that the block stages at once
+  constexpr int MAXQ = (2 * NB + ROWS - 1) / ROWS;               // word pairs a thread stages per step
+  static_assert(LSTM_THREADS % (LH / 2) == 0 && (NB % ROWS == 0 || MAXQ == 1), "constant distance between a thread's vectors");
   __shared__ __align__(16) float s_vec[2][2][NB][LH];            // [buffer][input, own layer's previous output][request][unit]
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int l = blockIdx.x / LSTM_LAYER_BLOCKS, part = blockIdx.x - l * LSTM_LAYER_BLOCKS;
@@ -370,7 +377,6 @@ __global__ void __launch_bounds__(LSTM_THREADS, 1) lstm_grid_kernel(const LstmGr
   const float* U = W + (size_t)4 * LH * LH;
   const float* B = U + (size_t)4 * LH * LH;
   float4 w[4][2], u[4][2];
-  float bias[4];
 #pragma unroll
   for (int g = 0; g < 4; g++) {
     const float4* wr = reinterpret_cast<const float4*>(W + ((size_t)g * LH + (unit ? j : 0)) * LH);
@@ -379,47 +385,46 @@ __global__ void __launch_bounds__(LSTM_THREADS, 1) lstm_grid_kernel(const LstmGr
     w[g][1] = __ldg(wr + 32 + lane);
     u[g][0] = __ldg(ur + lane);
     u[g][1] = __ldg(ur + 32 + lane);
-    bias[g] = B[g * LH + (unit ? j : 0)] + (g == 2 ? a.forget_bias : 0.f);
   }
-  float cell = 0.f;  // of request (lane >> (5 - LOG_NV)) >> 2
+  // After the reductions a lane has gate `gate` of request `req`; with the other gates it computes that request's cell.
+  const int gate = (lane / REP) & 3, req = (lane & (PASSES - 1)) * P + lane / (4 * REP), src_lane = lane - gate * REP;
+  const bool stores = unit && gate == 0 && (lane & (REP - 1)) < PASSES && req < a.batch;
+  const float bias = B[gate * LH + (unit ? j : 0)] + (gate == 2 ? a.forget_bias : 0.f);
+  // Staging: a thread takes two units of every ROWS-th of the step's 2 x NB vectors.  Both sources lie on one line through
+  // hbuf, so each further vector of a thread is the first one's address plus a constant.
+  const int row0 = (int)threadIdx.x / (LH / 2), pr2 = 2 * ((int)threadIdx.x % (LH / 2));
+  const int from0 = row0 / NB, b0 = row0 % NB;
+  const int words0 = (((l - 1 + from0) * LSTEPS - from0) * LSTM_GROUP + b0) * LH + pr2;  // at step 0; + LSTM_GROUP * LH per step
+  float cell = 0.f;
   for (int t = 0; t < LSTEPS; t++) {
     float(*vec)[NB][LH] = s_vec[t & 1];
-    // ---- stage the step's vectors: pair q = (source, request, two units)
-    const int n_src = t > 0 ? 2 : 1, n_pairs = n_src * NB * (LH / 2);
-    const unsigned long long* src[MAXQ];
+    // ---- stage the step's vectors (source 0: the layer below or the request, 1: this layer's previous output)
     bool open[MAXQ], any = false;
 #pragma unroll
     for (int k = 0; k < MAXQ; k++) {
-      const int q = (int)threadIdx.x + k * LSTM_THREADS;
-      const int from = q / (NB * (LH / 2)), b = (q / (LH / 2)) % NB, pr = q % (LH / 2);
-      open[k] = q < n_pairs && b < a.batch;
-      src[k] = nullptr;
-      if (!open[k]) continue;
-      if (from == 0 && l == 0) {
-        const float2 x = *reinterpret_cast<const float2*>(in_base + ((size_t)b * LSTEPS + t) * LH + 2 * pr);
-        *reinterpret_cast<float2*>(&vec[0][b][2 * pr]) = x;
+      const int from = from0 + k * ROWS / NB, b = b0 + k * ROWS % NB;
+      open[k] = from <= (t > 0 ? 1 : 0) && b < a.batch;
+      if (open[k] && from == 0 && l == 0) {
+        *reinterpret_cast<float2*>(&vec[0][b][pr2]) = *reinterpret_cast<const float2*>(in_base + ((size_t)b * LSTEPS + t) * LH + pr2);
         open[k] = false;
-      } else {
-        const int ll = from == 0 ? l - 1 : l, tt = from == 0 ? t : t - 1;
-        src[k] = a.hbuf + (((size_t)ll * LSTEPS + tt) * LSTM_GROUP + b) * LH + 2 * pr;
-        any = true;
       }
+      any |= open[k];
     }
+    const unsigned long long* words = a.hbuf + (words0 + t * LSTM_GROUP * LH);
     bool late = false;
     const long long t0 = clock64();
     while (any) {
       unsigned long long w0[MAXQ], w1[MAXQ];
 #pragma unroll
       for (int k = 0; k < MAXQ; k++)
-        if (open[k]) ld_two_words(src[k], &w0[k], &w1[k]);
+        if (open[k])
+          ld_two_words(words + (k * ROWS / NB) * ((LSTEPS - 1) * LSTM_GROUP * LH) + (k * ROWS % NB) * LH, &w0[k], &w1[k]);
       any = false;
 #pragma unroll
       for (int k = 0; k < MAXQ; k++) {
         if (!open[k]) continue;
         if ((unsigned)(w0[k] >> 32) == tag && (unsigned)(w1[k] >> 32) == tag) {
-          const int q = (int)threadIdx.x + k * LSTM_THREADS;
-          const int from = q / (NB * (LH / 2)), b = (q / (LH / 2)) % NB, pr = q % (LH / 2);
-          *reinterpret_cast<float2*>(&vec[from][b][2 * pr]) =
+          *reinterpret_cast<float2*>(&vec[from0 + k * ROWS / NB][b0 + k * ROWS % NB][pr2]) =
               make_float2(__uint_as_float((unsigned)w0[k]), __uint_as_float((unsigned)w1[k]));
           open[k] = false;
         } else {
@@ -437,56 +442,55 @@ __global__ void __launch_bounds__(LSTM_THREADS, 1) lstm_grid_kernel(const LstmGr
     }
     // The buffers alternate: a warp overwrites a vector only after the barrier above of the next step, which every warp
     // reaches when it has read this step's vectors.
-    float v[NV];
+    // Sums over the warp, P requests at a time: while a lane holds several values it keeps one half of them and adds its
+    // partner's share of that half; then lane = value index x REP + replica, and of a value's replicas one keeps each pass.
+    float sum = 0.f;
 #pragma unroll
-    for (int b = 0; b < NB; b++) {
-      if (b >= a.batch) {
+    for (int p = 0; p < PASSES; p++) {
+      if (p * P >= a.batch) break;
+      float v[PV];
 #pragma unroll
-        for (int g = 0; g < 4; g++) v[b * 4 + g] = 0.f;
-        continue;
-      }
-      const float4* xv = reinterpret_cast<const float4*>(vec[0][b]);
-      const float4 x0 = xv[lane], x1 = xv[32 + lane];
+      for (int b = 0; b < P; b++) {
+        const float4* xv = reinterpret_cast<const float4*>(vec[0][p * P + b]);
+        const float4 x0 = xv[lane], x1 = xv[32 + lane];
 #pragma unroll
-      for (int g = 0; g < 4; g++) v[b * 4 + g] = dot4(w[g][0], x0) + dot4(w[g][1], x1);
-      if (t > 0) {
-        const float4* hv = reinterpret_cast<const float4*>(vec[1][b]);
-        const float4 h0 = hv[lane], h1 = hv[32 + lane];
+        for (int g = 0; g < 4; g++) v[b * 4 + g] = dot4(w[g][0], x0) + dot4(w[g][1], x1);
+        if (t > 0) {
+          const float4* hv = reinterpret_cast<const float4*>(vec[1][p * P + b]);
+          const float4 h0 = hv[lane], h1 = hv[32 + lane];
 #pragma unroll
-        for (int g = 0; g < 4; g++) v[b * 4 + g] += dot4(u[g][0], h0) + dot4(u[g][1], h1);
-      }
-    }
-    // ---- sums over the warp: while a lane holds several values it keeps one half of them and adds its partner's share of
-    // that half; then lane = value index x 2^(5 - LOG_NV) + replica
-#pragma unroll
-    for (int step = 0; step < 5; step++) {
-      const int off = 16 >> step;
-      if (step < LOG_NV) {
-        const int half = NV >> (step + 1);
-        const bool upper = (lane & off) != 0;
-#pragma unroll
-        for (int k = 0; k < half; k++) {
-          const float mine = upper ? v[k + half] : v[k], give = upper ? v[k] : v[k + half];
-          v[k] = mine + __shfl_xor_sync(0xffffffffu, give, off);
+          for (int g = 0; g < 4; g++) v[b * 4 + g] += dot4(u[g][0], h0) + dot4(u[g][1], h1);
         }
-      } else {
-        v[0] += __shfl_xor_sync(0xffffffffu, v[0], off);
       }
+#pragma unroll
+      for (int step = 0; step < 5; step++) {
+        const int off = 16 >> step;
+        const int half = PV >> (step + 1);
+        if (half > 0) {
+          const bool upper = (lane & off) != 0;
+#pragma unroll
+          for (int k = 0; k < half; k++) {
+            const float mine = upper ? v[k + half] : v[k], give = upper ? v[k] : v[k + half];
+            v[k] = mine + __shfl_xor_sync(0xffffffffu, give, off);
+          }
+        } else {
+          v[0] += __shfl_xor_sync(0xffffffffu, v[0], off);
+        }
+      }
+      if (PASSES == 1 || (lane & (PASSES - 1)) == p) sum = v[0];
     }
-    constexpr int REP = 5 - LOG_NV;
-    const int idx = lane >> REP, base = idx & ~3;
-    const float gi = __shfl_sync(0xffffffffu, v[0], (base + 0) << REP) + bias[0];
-    const float gg = __shfl_sync(0xffffffffu, v[0], (base + 1) << REP) + bias[1];
-    const float gf = __shfl_sync(0xffffffffu, v[0], (base + 2) << REP) + bias[2];
-    const float go = __shfl_sync(0xffffffffu, v[0], (base + 3) << REP) + bias[3];
+    sum += bias;
+    const float gi = __shfl_sync(0xffffffffu, sum, src_lane);
+    const float gg = __shfl_sync(0xffffffffu, sum, src_lane + REP);
+    const float gf = __shfl_sync(0xffffffffu, sum, src_lane + 2 * REP);
+    const float go = __shfl_sync(0xffffffffu, sum, src_lane + 3 * REP);
     cell = sigmoidf_(gf) * cell + sigmoidf_(gi) * tanhf(gg);
     const float h = tanhf(cell) * sigmoidf_(go);
-    const int b = base >> 2;
-    if (unit && (lane & ((4 << REP) - 1)) == 0 && b < a.batch) {
-      unsigned long long* dst = a.hbuf + (((size_t)l * LSTEPS + t) * LSTM_GROUP + b) * LH + j;
+    if (stores) {
+      unsigned long long* dst = a.hbuf + (((size_t)l * LSTEPS + t) * LSTM_GROUP + req) * LH + j;
       const unsigned long long word = ((unsigned long long)tag << 32) | __float_as_uint(h);
       asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(dst), "l"(word) : "memory");
-      if (l == LLAYERS - 1 && t == LSTEPS - 1) out_base[(size_t)b * LH + j] = h;
+      if (l == LLAYERS - 1 && t == LSTEPS - 1) out_base[(size_t)req * LH + j] = h;
     }
   }
 }

@@ -425,7 +425,8 @@ __global__ void __launch_bounds__(1024) sg_stem_s2d(const SgItem* __restrict__ i
 // valid.  The exit flag and the idle limit are looked at on every poll, before the doorbell, so a block always leaves
 // within one poll of being asked to, whatever the doorbell says.  Blocks never wait for one another: each finishes its
 // share, and the block that brings the arrival counter to gridDim.x publishes `done`.
-__global__ void __launch_bounds__(256) sg_persistent(SgCtrl* ctrl, uint32_t* counter) {
+// (At most 48 registers: the LSTM's blocks, which must all be resident at once, count on room beside one block of this kernel.)
+__global__ void __launch_bounds__(256, 5) sg_persistent(SgCtrl* ctrl, uint32_t* counter) {
   __shared__ uint32_t s_cmd, s_seq;
   __shared__ SgItem s_items[SG_PERSISTENT_ITEMS];
   uint32_t seen = ctrl->done;  // submissions up to `done` were served by an earlier launch

@@ -48,8 +48,10 @@ def test_batches_and_repeated_runs(C, launch_type):
         assert np.linalg.norm(got.cpu().numpy() - want) < 2e-6 * np.linalg.norm(want), n
 
 
-def test_beside_the_resident_copy_engine(C):
-    """The cooperative launch needs 128 SMs to itself while the resident copy engine (copy type 1) holds blocks on 16 of them."""
+@pytest.mark.parametrize("n_engines", [1, 2])
+def test_beside_resident_copy_engines(C, n_engines):
+    """The cooperative launch needs 128 SMs while every resident copy engine (copy type 1) holds blocks on 16 of them.  A launch
+    that did not fit would wait until an engine leaves at its idle limit of 200 ms."""
     import torch
 
     torch.cuda.set_device(0)
@@ -57,14 +59,17 @@ def test_beside_the_resident_copy_engine(C):
     w = [(rng.standard_normal(s) * 0.08).astype(np.float32) for _ in range(L) for s in ((4, H, H), (4, H, H), (4, H))]
     C.set_rpc_mtu(8192)
     sp, cp = C.make_loopback_pair(8192, 512, "pinned")
-    app = C.make_app("lstm", 0, T * H * 4, H * 4, w, 64, 1, 8, copy_type=1)
+    apps = [C.make_app("lstm", 0, T * H * 4, H * 4, w, 64, 1, 8, copy_type=1) for _ in range(n_engines)]
     srv = C.Server(sp, req_size=T * H * 4, resp_size=H * 4, server_mode=2, max_batch=8)
-    srv.add_replica(app)
+    for app in apps:
+        srv.add_replica(app)
     srv.start()
-    cli = C.Client(cp, req_size=T * H * 4, resp_size=H * 4, total=64, warmup=0, payload="uniform", verify=True, n_payloads=4)
+    cli = C.Client(cp, req_size=T * H * 4, resp_size=H * 4, total=192, warmup=32, payload="uniform", verify=True, n_payloads=4)
     try:
-        assert cli.run_closed_loop(8) and cli.received == 64
-        assert srv.worker_stats(0)["wait_timeouts"] == 0
+        assert cli.run_closed_loop(8) and cli.received == 192
+        stats = [srv.worker_stats(k) for k in range(n_engines)]
+        assert all(s["wait_timeouts"] == 0 and s["num_batches"] > 0 for s in stats)
+        assert cli.post_process()["p99_sojournTime_us"] < 50e3
     finally:
         srv.stop()
     for k in range(4):
