@@ -39,6 +39,9 @@ struct GpuAppState {
   uint32_t* h_pt_status = nullptr;
   uint64_t idle_ns = 200000000ull;
   float* d_scratch = nullptr;           // lstm: inter-layer hand-off buffer
+  uint32_t* h_status = nullptr;         // lstm: mapped word, non-zero after a wait between blocks has run out
+  uint32_t* d_status = nullptr;
+  uint64_t wait_ms = 2000;              // lstm: limit of such a wait
   int lstm_clusters = 16;
 };
 
@@ -314,7 +317,7 @@ void launch_kernels(AppCtx* c, int batch) {
     const float* b = s->d_weights;
     srpc_lenet_ref(c->d_stub, nullptr, nullptr, b + s->w_off[0], b + s->w_off[1], b + s->w_off[2], b + s->w_off[3], batch, q);
   } else if (s->name == "lstm") {
-    srpc_lstm(c->d_stub, nullptr, nullptr, s->d_weights, s->d_scratch, s->lstm_clusters, batch, 0.0f, q);
+    srpc_lstm(c->d_stub, nullptr, nullptr, s->d_weights, s->d_scratch, s->lstm_clusters, batch, 0.0f, s->d_status, s->wait_ms, q);
   }
 }
 
@@ -337,6 +340,9 @@ int gpu_app_init(AppCtx* c) {
   }
   if (s->name == "lstm") {
     if (cudaMalloc(&s->d_scratch, srpc_lstm_scratch_bytes(s->lstm_clusters)) != cudaSuccess) return 0;
+    if (cudaHostAlloc(&s->h_status, 4, cudaHostAllocMapped) != cudaSuccess) return 0;
+    if (cudaHostGetDevicePointer((void**)&s->d_status, s->h_status, 0) != cudaSuccess) return 0;
+    *s->h_status = 0;
     // no tag left in it by its previous owner may equal one of this app's
     if (cudaMemsetAsync(s->d_scratch, 0, srpc_lstm_scratch_bytes(s->lstm_clusters), c->work_stream) != cudaSuccess) return 0;
   }
@@ -396,6 +402,12 @@ int gpu_app_run(AppCtx* c) {
 
 int gpu_app_complete(AppCtx* c) {
   if (c->launch_type == 3) c->ResetAppRunStatus();
+  GpuAppState* s = st(c);
+  if (s->h_status && *(volatile uint32_t*)s->h_status) {
+    *(volatile uint32_t*)s->h_status = 0;
+    c->last_status = -1;
+    srpc_log(SRPC_LOG_ERROR, "app '%s': a wait between blocks ran out, the batch has no result", s->name.c_str());
+  }
   return 1;
 }
 
@@ -410,6 +422,7 @@ int gpu_app_cleanup(AppCtx* c) {
   for (auto& kv : s->graphs) cudaGraphExecDestroy(kv.second);
   if (s->d_weights) cudaFree(s->d_weights);
   if (s->d_scratch) cudaFree(s->d_scratch);
+  if (s->h_status) cudaFreeHost(s->h_status);
   delete s;
   c->app_ctx_internal = nullptr;
   return 1;
@@ -442,6 +455,7 @@ GpuAppHandle srpc_make_gpu_app(const char* name, int device_id, size_t req_size,
   s->name = nm;
   s->req_size = req_size;
   s->resp_size = resp_size;
+  s->wait_ms = readEnvInfo<uint64_t>("P2P_RPC_APP_WAIT_MS", 2000);
   s->idle_ns = (uint64_t)readEnvInfo<uint64_t>("P2P_RPC_APP_IDLE_MS", 200) * 1000000ull;
   const size_t want = nm == "lenet5" ? 10 : (nm == "lenet_ref" ? 4 : (nm == "lstm" ? 24 : 0));
   if (want) {

@@ -335,7 +335,6 @@ constexpr int LSTM_THREADS = LSTM_WARPS * 32;
 // (all at once with 128: 31.0 / 40.0 / 51.7 / 72.0 us; 96 registers spill: 37.2 / 39.3 / 55.4 / 93.5 us).
 constexpr int LSTM_REGS = 104;
 static_assert(LSTM_THREADS * LSTM_REGS + 256 * 48 <= 65536, "a block and a resident copy block share an SM's registers");
-constexpr long long LSTM_WAIT_CYCLES = 4000000000ll;
 
 struct LstmGridArgs {
   const g_params* stub;
@@ -344,7 +343,8 @@ struct LstmGridArgs {
   const float* weights;
   unsigned long long* hbuf;  // [LLAYERS][LSTEPS][LSTM_GROUP][LH] words {value, tag}
   const unsigned* epoch;     // this launch's tag
-  uint32_t* status;          // may be null
+  volatile uint32_t* status; // may be null
+  long long wait_cycles;     // limit of one wait
   int first;                 // request of the window that this launch starts with
   int batch;                 // requests of this launch, 1 .. NB
   float forget_bias;
@@ -431,13 +431,18 @@ __global__ void __maxnreg__(LSTM_REGS) lstm_grid_kernel(const LstmGridArgs a) {
           any = true;
         }
       }
-      if (any && clock64() - t0 > LSTM_WAIT_CYCLES) {
+      if (any && clock64() - t0 > a.wait_cycles) {
         late = true;
         break;
       }
     }
     if (__syncthreads_or(late ? 1 : 0)) {
-      if (threadIdx.x == 0 && a.status) atomicExch(a.status, 0x4C53u);  // 'LS': a wait of the LSTM ran out
+      // Every block that waits for this one's words gives up in turn; the last layer's blocks leave no number of an earlier
+      // batch behind in the rows that they do not compute.
+      if (l == LLAYERS - 1)
+        for (int i = (int)threadIdx.x; i < a.batch * LSTM_WARPS; i += LSTM_THREADS)
+          out_base[(size_t)(i / LSTM_WARPS) * LH + part * LSTM_WARPS + i % LSTM_WARPS] = __int_as_float(0x7fffffff);
+      if (threadIdx.x == 0 && a.status) *a.status = 0x4C53u;  // 'LS': a wait of the LSTM ran out
       return;
     }
     // The buffers alternate: a warp overwrites a vector only after the barrier above of the next step, which every warp
@@ -664,7 +669,7 @@ size_t srpc_lstm_scratch_bytes(int max_clusters) {
 }
 
 cudaError_t srpc_lstm(const void* d_stub, const float* direct_in, float* direct_out, const float* weights, float* scratch,
-                      int max_clusters, int batch, float forget_bias, cudaStream_t s) {
+                      int max_clusters, int batch, float forget_bias, uint32_t* status, uint64_t wait_ms, cudaStream_t s) {
   if (batch < 1) return cudaSuccess;
   // Whole-GPU dataflow (cooperative launches, LSTM_GROUP requests each); SPLITRPC_LSTM_CLUSTER=1 or a refused cooperative
   // launch falls back to the one-cluster-per-request kernel.
@@ -689,12 +694,14 @@ cudaError_t srpc_lstm(const void* d_stub, const float* direct_in, float* direct_
       a.hbuf = reinterpret_cast<unsigned long long*>(scratch);
       unsigned* epoch = reinterpret_cast<unsigned*>(a.hbuf + kLstmWords);
       a.epoch = epoch;
-      a.status = nullptr;
+      a.status = status;
+      a.wait_cycles = (long long)(wait_ms < 1000000 ? wait_ms : 1000000) * 2000000;  // at 2 GHz
       a.forget_bias = forget_bias;
       for (; done < batch; done += LSTM_GROUP) {
         a.first = done;
         a.batch = batch - done < LSTM_GROUP ? batch - done : LSTM_GROUP;
         lstm_bump_kernel<<<1, 1, 0, s>>>(epoch);
+        if (const cudaError_t e = cudaGetLastError(); e != cudaSuccess) return e;  // the words of the launch before would pass for this one's
         void* args[] = {&a};
         const void* fn = a.batch == 1   ? (const void*)lstm_grid_kernel<1>
                          : a.batch == 2 ? (const void*)lstm_grid_kernel<2>
@@ -707,7 +714,7 @@ cudaError_t srpc_lstm(const void* d_stub, const float* direct_in, float* direct_
         grid_ok.store(-1, std::memory_order_release);  // not possible in this context: use the cluster kernel from now on
         break;
       }
-      if (done) return cudaGetLastError();
+      if (done) return cudaSuccess;
     }
   }
   int clusters = batch < max_clusters ? batch : max_clusters;

@@ -33,10 +33,11 @@ cudaError_t srpc_lenet_ref(const void* d_stub, const void* direct_in, float* dir
 
 // 8-layer x 8-step LSTM, hidden 256.  weights: per layer W[4][256][256], U[4][256][256], b[4][256] (gate order
 // input, cell, forget, output).  scratch: srpc_lstm_scratch_bytes(max_clusters) bytes, zero
-// before the first call and for the use of one stream.
+// before the first call and for the use of one stream.  When a wait between blocks runs out (limit wait_ms), the rows that were
+// not computed are NaN and *status (mapped host memory or null) is non-zero.
 size_t srpc_lstm_scratch_bytes(int max_clusters);
 cudaError_t srpc_lstm(const void* d_stub, const float* direct_in, float* direct_out, const float* weights, float* scratch,
-                      int max_clusters, int batch, float forget_bias, cudaStream_t s);
+                      int max_clusters, int batch, float forget_bias, uint32_t* status, uint64_t wait_ms, cudaStream_t s);
 
 // Loads this file's kernels on the current device, so that none of them is loaded lazily at a first launch that
 // happens while a stream is parked on a doorbell.

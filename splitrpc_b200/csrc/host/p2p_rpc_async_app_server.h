@@ -290,8 +290,9 @@ class P2pRpcAsyncAppServer {
   bool do_sync(int appIdx) {
     P2pRpcAppInfo* a = all_apps[appIdx];
     bool ok = a->app_ctx->WaitForAppRunComplete();
+    a->app_ctx->last_status = 0;
     if (a->app_complete) a->app_complete(a->app_ctx);
-    return ok;
+    return ok && a->app_ctx->last_status == 0;  // the app may report a device-side wait that ran out
   }
   // Runs slot rr_idx (and the curr_batch_size-1 slots after it) to completion
   // without checking that the slots are ready.
@@ -445,7 +446,12 @@ class P2pRpcAsyncAppServer {
       a->consumer_seq += (uint64_t)bs;
       update_batch_size(appIdx);
       c->ResetAppRunStatus();
+      c->last_status = 0;
       if (a->app_complete) a->app_complete(c);
+      if (c->last_status != 0) {
+        std::lock_guard<std::mutex> g(stats_mu_);
+        stats_[appIdx].wait_timeouts++;
+      }
       armed = false;
     }
     if (armed && c->device_id >= 0) {

@@ -333,8 +333,9 @@ class P2pRpcAppServer {
   bool sync(int instance = 0) {
     P2pRpcAppInfo* a = apps_[instance].get();
     bool ok = a->app_ctx->WaitForAppRunComplete();
+    a->app_ctx->last_status = 0;
     if (a->app_complete) a->app_complete(a->app_ctx);
-    return ok;
+    return ok && a->app_ctx->last_status == 0;
   }
   bool do_work_sync(p2p_rpc_rr* rr, int instance = 0) {
     do_work(rr, instance);

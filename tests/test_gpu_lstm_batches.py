@@ -48,6 +48,66 @@ def test_batches_and_repeated_runs(C, launch_type):
         assert np.linalg.norm(got.cpu().numpy() - want) < 2e-6 * np.linalg.norm(want), n
 
 
+@pytest.mark.parametrize("launch_type", [1, 4])
+def test_a_wait_that_runs_out_is_reported(C, monkeypatch, launch_type):
+    """With a limit of zero the blocks of the upper layers give up at their first look: the run fails, its rows are NaN, and the
+    device serves the next app as before."""
+    import torch
+
+    torch.cuda.set_device(0)
+    rng = np.random.default_rng(9)
+    w = [(rng.standard_normal(s) * 0.08).astype(np.float32) for _ in range(L) for s in ((4, H, H), (4, H, H), (4, H))]
+    C.set_rpc_mtu(8192)
+    x = rng.standard_normal((3, T, H)).astype(np.float32)
+    d = torch.from_numpy(x).cuda()
+
+    def run(app):
+        C.memcpy_async(app.req_ring[0], d.data_ptr(), x.nbytes, 0)
+        torch.cuda.synchronize()
+        _, resp = C.local_bench(app, 1, 3)
+        got = torch.zeros(3, H, device="cuda")
+        C.memcpy_async(got.data_ptr(), resp[0], 3 * H * 4, 0)
+        torch.cuda.synchronize()
+        return got.cpu().numpy()
+
+    good = C.make_app("lstm", 0, T * H * 4, H * 4, w, 64, launch_type, 8)
+    want = run(good)
+    np.testing.assert_allclose(want, _exact(w, x), rtol=1e-4, atol=1e-6)
+    monkeypatch.setenv("P2P_RPC_APP_WAIT_MS", "0")
+    bad = C.make_app("lstm", 0, T * H * 4, H * 4, w, 64, launch_type, 8)
+    monkeypatch.delenv("P2P_RPC_APP_WAIT_MS")
+    for _ in range(2):
+        with pytest.raises(RuntimeError):
+            run(bad)
+    got = torch.zeros(3, H, device="cuda")
+    C.memcpy_async(got.data_ptr(), bad.resp_ring[0], 3 * H * 4, 0)
+    torch.cuda.synchronize()
+    assert bool(got.isnan().all())
+    np.testing.assert_array_equal(run(good), want)
+
+
+@pytest.mark.parametrize("server_mode", [1, 2])
+def test_a_wait_that_runs_out_counts_as_the_workers(C, monkeypatch, server_mode):
+    import torch
+
+    torch.cuda.set_device(0)
+    rng = np.random.default_rng(10)
+    w = [(rng.standard_normal(s) * 0.08).astype(np.float32) for _ in range(L) for s in ((4, H, H), (4, H, H), (4, H))]
+    C.set_rpc_mtu(8192)
+    sp, cp = C.make_loopback_pair(8192, 512, "pinned")
+    monkeypatch.setenv("P2P_RPC_APP_WAIT_MS", "0")
+    app = C.make_app("lstm", 0, T * H * 4, H * 4, w, 64, 1, 1)
+    srv = C.Server(sp, req_size=T * H * 4, resp_size=H * 4, server_mode=server_mode, max_batch=1)
+    srv.add_replica(app)
+    srv.start()
+    cli = C.Client(cp, req_size=T * H * 4, resp_size=H * 4, total=8, warmup=0, payload="uniform", n_payloads=1)
+    try:
+        assert cli.run_closed_loop(1) and cli.received == 8
+        assert srv.worker_stats(0)["wait_timeouts"] >= 8
+    finally:
+        srv.stop()
+
+
 @pytest.mark.parametrize("n_engines", [1, 2])
 def test_beside_resident_copy_engines(C, n_engines):
     """The cooperative launch needs 128 SMs while every resident copy engine (copy type 1) holds blocks on 16 of them.  A launch
