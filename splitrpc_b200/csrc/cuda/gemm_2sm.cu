@@ -108,6 +108,7 @@ struct TileOrder {
   int tiles_m2, tiles_n;
   int group_m;   // 256-row blocks per group
   int m_rot2;    // rotation of the 256-row blocks (tensor-parallel: which rank's rows come first)
+  int late_trigger;  // the next kernel starts behind this CTA's last load only (pdl_launch.h)
 };
 
 // j-th tile of this cluster, grouped so that tiles in flight share A and B blocks in L2.
@@ -179,7 +180,7 @@ gemm_2sm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
   if (warp == 1) {
     ptx::tmem_alloc_2sm(&tmem_base_smem, TMEM_COLS);
     ptx::tmem_relinquish_2sm();
-    ptx::grid_dep_launch();  // after the allocation, see pdl_launch.h
+    if (!order.late_trigger) ptx::grid_dep_launch();  // after the allocation, see pdl_launch.h
   }
   ptx::tc_fence_before();
   __syncthreads();
@@ -232,6 +233,10 @@ gemm_2sm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
           ph ^= 1u;
         }
       }
+    }
+    if (order.late_trigger && warp == 0) {
+      __syncwarp();
+      ptx::grid_dep_launch();
     }
   } else if (warp == 1) {
     // ---------------- MMA issue (leader only): the warp walks the schedule together, one elected lane issues, so that
@@ -515,6 +520,7 @@ cudaError_t launch_2sm(const void* A, int lda, const void* B, int ldb, int M, in
   o.clusters = std::min(o.tiles_m2 * o.tiles_n, std::min(max_clusters, srpc_gemm_grid_sms() / 2));
   o.group_m = 4;
   o.m_rot2 = 0;
+  o.late_trigger = srpc_gemm_reserved_sms() > 0;
   return launch_pdl(gemm_2sm_kernel<BN, false>, dim3(2 * o.clusters), dim3(C::THREADS), C::SMEM_BYTES, stream, ta, tb, to, M, N, K,
                     o, ep, status, TpParams{});
 }
@@ -543,6 +549,7 @@ cudaError_t launch_2sm_tp(const void* A, int lda, const void* B, int ldb, int M,
     to = ta;  // never used: the epilogue stores to the owners' slots
   }
   TileOrder o;
+  o.late_trigger = 0;
   o.tiles_m2 = M / (2 * BM);
   o.tiles_n = (N + BN - 1) / BN;
   o.clusters = std::min(o.tiles_m2 * o.tiles_n, max_clusters - copy_clusters);

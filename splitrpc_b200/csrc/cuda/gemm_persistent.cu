@@ -111,6 +111,7 @@ struct TileParams {
   const void* in_stub;
   unsigned long long in_ring_base;
   unsigned int in_slot_bytes;
+  int late_trigger;  // the next kernel starts behind this CTA's last load only (pdl_launch.h); filled in by launch()
   // two-input 1x1 convolution: k-blocks from kb_split on come from the second input (pixel stride2, no padding)
   int kb_split, stride2;
 };
@@ -351,7 +352,7 @@ gemm_conv_persistent(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
   if (warp == 1) {
     ptx::tmem_alloc(&tmem_base_smem, ACC * ACC_STRIDE);
     ptx::tmem_relinquish();
-    ptx::grid_dep_launch();  // after the allocation, see pdl_launch.h
+    if (!p.late_trigger) ptx::grid_dep_launch();  // after the allocation, see pdl_launch.h
   }
   ptx::tc_fence_before();
   __syncthreads();
@@ -373,6 +374,10 @@ gemm_conv_persistent(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
         while (pr_more && pr_j == j && pr_kb < p.num_kb) produce_one();
         if (!pr_more) break;
       }
+    if (producer == 0 && p.late_trigger) {
+      __syncwarp();
+      ptx::grid_dep_launch();
+    }
   } else if (warp == 1) {
     // The whole warp walks the schedule and waits together; one elected lane issues.  Every value that a tcgen05
     // instruction takes lives in uniform registers then; with the loop inside the elected lane's branch each of them was
@@ -807,6 +812,7 @@ cudaError_t launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorM
   p.fd_tiles_h = make_fastdiv((uint32_t)(p.tiles_h > 0 ? p.tiles_h : 1));
   p.fd_cblocks = make_fastdiv((uint32_t)(p.cblocks > 0 ? p.cblocks : 1));
   p.fd_s = make_fastdiv((uint32_t)(p.s > 0 ? p.s : 1));
+  p.late_trigger = srpc_gemm_reserved_sms() > 0;
   static const int allow_bs = [] { const char* e = getenv("SPLITRPC_GEMM_BSTAT"); return e ? atoi(e) : 1; }();
   // The panel may take the ring's memory as long as three A stages remain (a 3x3 convolution over 64 channels keeps its
   // nine 8 KB filter taps resident: otherwise every CTA re-reads the same few L2 lines for every tile).

@@ -56,6 +56,7 @@ struct StemParams {
   int tiles;                    // tiles of the largest chunk
   int chunks_per_img;
   int relu;
+  int late_trigger;             // the next kernel starts behind this CTA's last load only (pdl_launch.h)
   const float* bias;
   __nv_bfloat16* out;
 };
@@ -88,7 +89,7 @@ __global__ void __launch_bounds__(THREADS, 1) stem_conv_kernel(const __grid_cons
     __syncwarp();
     ptx::tmem_alloc(&tmem_base_smem, ACC * COUT);
     ptx::tmem_relinquish();
-    ptx::grid_dep_launch();  // after the allocation, see pdl_launch.h
+    if (!p.late_trigger) ptx::grid_dep_launch();  // after the allocation, see pdl_launch.h
   }
   ptx::tc_fence_before();
   __syncthreads();
@@ -174,6 +175,10 @@ __global__ void __launch_bounds__(THREADS, 1) stem_conv_kernel(const __grid_cons
       }
       ptx::cp_async_wait<0>();
       if (it > 0) hand_over(it - 1);
+      if (p.late_trigger && warp == 1) {
+        __syncwarp();
+        ptx::grid_dep_launch();
+      }
     } else {
       // ---------------- epilogue: each set of four warps takes every third tile; a warp has 32 positions
       const int ew = warp - 4, set = ew >> 2, quarter = warp & 3;
@@ -280,6 +285,7 @@ cudaError_t srpc_stem_conv(const void* in, const void* weight, const ConvShape& 
   p.oh = cs.oh;
   p.n = cs.n;
   p.relu = ep.act == GEMM_ACT_RELU;
+  p.late_trigger = srpc_gemm_reserved_sms() > 0;
   p.bias = ep.bias;
   p.out = (__nv_bfloat16*)ep.out;
   // Tiles per chunk: few for small batches, so that every SM has a chunk; a chunk costs the rows shared with its neighbour

@@ -3,6 +3,126 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 
+_LAUNCHES = ("gemm", "fc_skinny", "conv2d_nhwc", "conv1x1_dual", "stem_s2d", "stem_conv", "maxpool3x3s2", "global_avgpool",
+             "softmax_response", "layernorm", "bert_embed_ln", "attention_tc_qkv")
+
+
+def _model(name):
+    """A model, its input and a function that runs it into ``out``."""
+    import torch
+    from splitrpc_b200.models.bert import BertClassifier, BertConfig
+    from splitrpc_b200.models.resnet import ResNet50
+
+    g = torch.Generator(device="cuda").manual_seed(3)
+    if name == "resnet":
+        m, x = ResNet50(device=0, max_batch=5), torch.randn(5, 3, 224, 224, device="cuda", generator=g)
+        return m, torch.empty(5, 1000, device="cuda"), lambda out: m.forward(5, x=x, out=out)
+    seq = int(name[4:])
+    m = BertClassifier(BertConfig(layers=2, hidden=768, heads=12, ffn=3072, vocab=500), seq=seq, device=0, max_batch=9)
+    ids = torch.randint(0, 500, (9, seq), device="cuda", generator=g, dtype=torch.int32)
+    return m, torch.empty(9, 2, device="cuda"), lambda out: m.forward(9, ids=ids, out=out)
+
+
+def _want(name, run, out, monkeypatch):
+    """The result with every launch waited for."""
+    import torch
+    from splitrpc_b200 import ops
+
+    with monkeypatch.context() as mp:
+        for f in _LAUNCHES:
+            def waited(*a, _f=getattr(ops, f), **k):
+                r = _f(*a, **k)
+                torch.cuda.synchronize()
+                return r
+            mp.setattr(ops, f, waited)
+        run(out)
+    return out.clone()
+
+
+@pytest.mark.parametrize("reserve", [0, 12])
+@pytest.mark.parametrize("name", ["resnet", "bert128", "bert384"])
+def test_model_keeps_its_order(C, monkeypatch, name, reserve):
+    """Every kernel of the models in a chain, two chains beside each other on two streams, and a copy kernel beside both."""
+    import torch
+    from splitrpc_b200 import ops
+
+    torch.cuda.set_device(0)
+    C.gemm_reserve_sms(reserve)
+    try:
+        chains = []
+        for _ in range(2):
+            m, out, run = _model(name)
+            want = _want(name, run, out, monkeypatch)
+            s, g = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+            with torch.cuda.graph(g, stream=s):
+                run(out)
+            chains.append((s, g, out, want, run, m))
+        src = torch.randint(0, 256, (64 << 20,), dtype=torch.uint8).pin_memory()
+        dst = torch.empty(64 << 20, dtype=torch.uint8, device="cuda")
+        copies = torch.cuda.Stream()
+        h = C.sg_list_create([(src.data_ptr() + o, dst.data_ptr() + o, 8192) for o in range(0, 64 << 20, 8192)])
+        for eager in (False, True):
+            for s, g, out, want, run, m in chains:
+                out.zero_()
+            dst.zero_()
+            torch.cuda.synchronize()
+            C.sg_list_launch(h, 0, -12, copies.cuda_stream)
+            for _ in range(3):
+                for s, g, out, want, run, m in chains:
+                    with torch.cuda.stream(s):
+                        run(out) if eager else g.replay()
+            torch.cuda.synchronize()
+            ops.check_status()
+            for s, g, out, want, run, m in chains:
+                assert torch.equal(out, want)
+            assert torch.equal(dst.cpu(), src)
+        C.sg_list_destroy(h)
+    finally:
+        C.gemm_reserve_sms(0)
+
+
+@pytest.mark.parametrize("mnk", [(16384, 8192, 8192), (32768, 1000, 8192)])
+def test_reserved_sms_stay_free(C, mnk):
+    """Beside a chain of long persistent kernels that leave twelve SMs out, a copy kernel of twelve blocks starts at once; it
+    must not wait for the end of a kernel because blocks of the next one sit on those SMs."""
+    import time
+    import torch
+    from splitrpc_b200 import ops
+
+    torch.cuda.set_device(0)
+    M, N, K = mnk
+    a, b = torch.randn(M, K, device="cuda").bfloat16(), torch.randn(N, K, device="cuda").bfloat16()
+    out = torch.empty(M, N, device="cuda").bfloat16()
+    src, dst = torch.ones(12 * 16384, dtype=torch.uint8, device="cuda"), torch.zeros(12 * 16384, dtype=torch.uint8, device="cuda")
+    h = C.sg_list_create([(src.data_ptr(), dst.data_ptr(), src.numel())])
+    long, short = torch.cuda.Stream(), torch.cuda.Stream()
+    ev = lambda: torch.cuda.Event(enable_timing=True)
+    C.gemm_reserve_sms(12)
+    try:
+        with torch.cuda.stream(long):
+            ops.gemm(a, b, out=out)  # first launches load the kernels
+        C.sg_list_launch(h, 0, -12, short.cuda_stream)
+        torch.cuda.synchronize()
+        t = []
+        for i in range(15):
+            begin, end, first, last = ev(), ev(), ev(), ev()
+            with torch.cuda.stream(long):
+                first.record()
+                for _ in range(3):
+                    ops.gemm(a, b, out=out)
+                last.record()
+            time.sleep(1e-4 * (1 + i % 5))
+            begin.record(short)
+            C.sg_list_launch(h, 0, -12, short.cuda_stream)
+            end.record(short)
+            torch.cuda.synchronize()
+            t.append(begin.elapsed_time(end) / (first.elapsed_time(last) / 3))
+        # as a share of one long kernel's time: a few per cent, half a kernel and more when it waits for a boundary
+        assert sorted(t)[len(t) // 2] < 0.2, t
+    finally:
+        C.gemm_reserve_sms(0)
+        C.sg_list_destroy(h)
+
 
 @pytest.mark.parametrize("rows", [1, 128, 1000, 4096])
 @pytest.mark.parametrize("graph", [False, True])
