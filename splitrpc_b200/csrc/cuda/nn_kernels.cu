@@ -10,6 +10,7 @@
 #include <stdint.h>
 
 #include "../host/p2p_rpc_app.h"
+#include "gemm_tcgen05.h"
 #include "nn_kernels.h"
 #include "pdl_launch.h"
 #include "per_device.h"
@@ -204,12 +205,12 @@ __global__ void __launch_bounds__(256) global_avgpool(const __nv_bfloat16* in, _
 // planes of float4 per column, so that the sixteen k-slices a warp reads together are contiguous), thread
 // (row group, kq) walks every sixteenth 8-element slice of its RPT rows of `a` with the next slice's loads in flight, and
 // the sixteen partial sums of a row meet through shuffles.  A slice's weights are read from shared memory once for the
-// RPT rows: with two rows those reads bound 64 x 1000 x 2048 (15.2 us), with four it takes 13.3 us, of which the FMAs are 4.  Two
-// rows stay for up to 32 rows (9.1 us), where there are enough of them for one block per column group anyway.  The order of
-// every sum is the same.
+// RPT rows: with two rows those reads bound 64 x 1000 x 2048 (15.2 us), with four it takes 12.9 us, of which the FMAs are 4.  Two
+// rows stay for up to 32 rows (8.9 us), where there are enough of them for one block per column group anyway.  PER_SM: blocks
+// that the registers leave room for on an SM, see nn_fc_skinny.  The order of every sum is the same in all forms.
 constexpr int FC_NB = 8;
-template <int RPT>
-__global__ void __launch_bounds__(256, 1) fc_skinny(const __nv_bfloat16* a, int lda, const __nv_bfloat16* w,
+template <int RPT, int PER_SM>
+__global__ void __launch_bounds__(256, PER_SM) fc_skinny(const __nv_bfloat16* a, int lda, const __nv_bfloat16* w,
                                                  int ldw, const float* bias, float* out, int ldo, int M,
                                                  int N, int K) {
   ptx::grid_dep_launch();
@@ -625,21 +626,27 @@ cudaError_t nn_fc_skinny(const void* a, int lda, const void* w, int ldw, const f
   static PerDeviceFlag attr_set;
   const int dev = PerDeviceFlag::current();
   if (attr_set.needed(dev)) {
-    cudaError_t e = cudaFuncSetAttribute(fc_skinny<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(fc_skinny<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    cudaError_t e = cudaFuncSetAttribute(fc_skinny<2, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(fc_skinny<4, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(fc_skinny<2, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(fc_skinny<4, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     if (e != cudaSuccess) return e;
     attr_set.set(dev);
   }
-  // One block per SM where that is enough for all of them (more than half of an SM's shared memory): blocks that start while
-  // the kernel before still runs would otherwise be stacked two to an SM beside empty ones (32 rows: 13.6 us then, 9.1 us now).
+  // While the blocks fit the SMs one each, a block takes the registers it likes, and up to 32 rows also more than half of an
+  // SM's shared memory: blocks that start while the kernel before still runs would otherwise be stacked two to an SM
+  // beside empty ones (32 x 1000 x 2048: 13.6 us then, 8.9 us now).  With more blocks than SMs two share an SM, at 128
+  // registers, where two blocks' weights fit its shared memory (K up to 3616).  One per SM against two, us:
+  // 32 x 1192 x 512 8.2 / 6.4, 32 x 4096 x 2048 32.9 / 28.4, 64 x 1192 x 512 12.6 / 10.0, 128 x 1000 x 512 12.9 / 10.2, 64 x 8192 x 768 50.4 / 38.3.
   const size_t spread = 116 * 1024;
-  const dim3 block(256);
-  const unsigned cols = (unsigned)((N + FC_NB - 1) / FC_NB);
-  if (M <= 32)
-    return launch_pdl(fc_skinny<2>, dim3(cols), block, cols <= 148 && smem < spread ? spread : smem, s, (const __nv_bfloat16*)a,
-                      lda, (const __nv_bfloat16*)w, ldw, bias, out, ldo, M, N, K);
-  return launch_pdl(fc_skinny<4>, dim3(cols, (M + 63) / 64), block, smem, s, (const __nv_bfloat16*)a, lda, (const __nv_bfloat16*)w, ldw,
-                    bias, out, ldo, M, N, K);
+  const int sms = srpc_gemm_grid_sms(), rpt = M <= 32 ? 2 : 4;
+  const dim3 grid((unsigned)((N + FC_NB - 1) / FC_NB), (unsigned)((M + 16 * rpt - 1) / (16 * rpt)));
+  const bool one_each = (uint64_t)grid.x * grid.y <= (uint64_t)sms, two_fit = smem <= 113 * 1024;
+  auto go = [&](auto* kernel, size_t shared) {
+    return launch_pdl(kernel, grid, dim3(256), shared, s, (const __nv_bfloat16*)a, lda, (const __nv_bfloat16*)w, ldw, bias, out, ldo, M, N, K);
+  };
+  if (rpt == 2) return one_each ? go(fc_skinny<2, 1>, smem < spread ? spread : smem) : (two_fit ? go(fc_skinny<2, 2>, smem) : go(fc_skinny<2, 1>, smem));
+  return one_each || !two_fit ? go(fc_skinny<4, 1>, smem) : go(fc_skinny<4, 2>, smem);
 }
 cudaError_t nn_softmax_response(const float* logits, int rows, int n, int ld, const void* d_stub, void* direct_out,
                                 size_t resp_stride, int write_argmax, uint32_t* counter, uint32_t* flag, uint32_t flag_value,

@@ -56,6 +56,27 @@ def test_nn_layers_match_pytorch(torch_cuda):
     assert got[..., 7].abs().max() == 0 and col[:, 168:].abs().max() == 0
 
 
+@pytest.mark.parametrize("m_rows", [1, 16, 32, 33, 64, 65, 130])
+@pytest.mark.parametrize("n_cols,k", [(8, 8), (1000, 24), (1184, 520), (1192, 512), (4100, 2048), (1200, 3616), (1200, 3624), (77, 6400)])
+def test_fc_skinny_forms(torch_cuda, m_rows, n_cols, k):
+    """Two and four rows per thread, one and two blocks per SM: around 32 and 64 rows, around one block per SM (148 x 8 columns),
+    around the K whose weights fit an SM twice (3616), and K that leave some of a row's sixteen threads without a slice."""
+    torch = torch_cuda
+    from splitrpc_b200 import ops
+
+    g = torch.Generator(device="cuda").manual_seed(m_rows * n_cols + k)
+    a = torch.randn(m_rows, k + 8, device="cuda", generator=g).bfloat16()[:, :k]
+    w = torch.randn(n_cols, k + 16, device="cuda", generator=g).bfloat16()[:, :k]
+    bias = torch.randn(n_cols, device="cuda", generator=g)
+    out = torch.full((m_rows + 1, n_cols + 3), 7.0, device="cuda")
+    ops.fc_skinny(a, w, bias=bias, out=out[:m_rows, :n_cols])
+    want = a.double() @ w.double().t() + bias.double()
+    # k products and a bias in fp32, whatever the order: fewer than k + 8 roundings of partial sums
+    bound = (a.double().abs() @ w.double().abs().t() + bias.double().abs()) * ((k + 8) * 2.0 ** -24)
+    assert bool(((out[:m_rows, :n_cols].double() - want).abs() <= bound).all())
+    assert bool((out[m_rows] == 7).all()) and bool((out[:, n_cols:] == 7).all())
+
+
 def test_space_to_depth_stem_matches_conv2d(torch_cuda):
     """stem_s2d + stem_conv (4x1 taps over overlapping 64-channel windows) against an fp32 7x7/2 convolution."""
     torch = torch_cuda
