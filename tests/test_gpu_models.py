@@ -77,6 +77,35 @@ def test_fc_skinny_forms(torch_cuda, m_rows, n_cols, k):
     assert bool((out[m_rows] == 7).all()) and bool((out[:, n_cols:] == 7).all())
 
 
+@pytest.mark.parametrize("seq", [128, 384])
+@pytest.mark.parametrize("exponent", [-120, -126.3, -128, -131])
+def test_attention_keeps_subnormal_weights(torch_cuda, seq, exponent):
+    """One key far above the others in every row and values that make the others' weights count: weights just above and below
+    2^-126 of the row's largest."""
+    torch = torch_cuda
+    from splitrpc_b200 import ops
+
+    heads, B = 2, 3
+    H = heads * 64
+    qkv = torch.zeros(B * seq, 3, heads, 64, device="cuda")
+    qkv[:, 0, :, 0] = 16
+    lead = -exponent * 0.6931471805599453 * 8 / 16  # score / 8 in nats
+    best = torch.arange(B, device="cuda") * seq + torch.tensor([0, 40, seq - 1], device="cuda")
+    qkv[best, 1, :, 0] = lead
+    qkv[:, 2] = torch.rand(B * seq, heads, 64, device="cuda") + 0.5
+    qkv[:, 2] *= 2.0 ** 100
+    qkv[best, 2] = 0
+    qkv = qkv.bfloat16()
+    out = ops.attention_tc_qkv(qkv.view(B * seq, 3 * H), B, seq, heads)
+    ops.check_status()
+    q, k, v = (qkv[:, i].double().view(B, seq, heads, 64).transpose(1, 2) for i in range(3))
+    want = (torch.softmax(q @ k.transpose(-1, -2) / 8, -1) @ v).transpose(1, 2).reshape(B * seq, H)
+    # a bf16 weight w has a spacing of 2^-133 below 2^-126; the exponent itself is rounded to fp32 (2^-18 near 128)
+    w = torch.exp(-torch.tensor(16 * qkv[best[0], 1, 0, 0].item() / 8, dtype=torch.float64)).item()
+    rel = max(2.0 ** -8, 2.0 ** -134 / w) + 2.0 ** -8 + 2.0 ** -17
+    assert ((out.double() - want).abs() <= rel * want.abs()).all()
+
+
 def test_space_to_depth_stem_matches_conv2d(torch_cuda):
     """stem_s2d + stem_conv (4x1 taps over overlapping 64-channel windows) against an fp32 7x7/2 convolution."""
     torch = torch_cuda
