@@ -322,7 +322,7 @@ lstm_wavefront_kernel(const g_params* stub, const float* direct_in, float* direc
 // (lstm_bump_kernel adds one before every launch; graph replays count too), so nothing has to be cleared in between.
 // A block stages the vectors of a step in shared memory for its warps; the 4 x NB gate sums of a warp are reduced together
 // (values are halved between lane pairs as they are added).  The kernel is launched cooperatively: all blocks are resident,
-// and every wait is bounded.  32.0 / 39.0 / 50.3 / 79.4 us for 1 / 2 / 4 / 8 requests back to back (61.8 / 84.0 / 128.9 / 216.7 us with a
+// and every wait is bounded.  29.4 / 36.2 / 51.4 / 77.8 us for 1 / 2 / 4 / 8 requests back to back (61.8 / 84.0 / 128.9 / 216.7 us with a
 // grid barrier per wave); what is left is the exchange latency, 2 us per step for one request, and 0.4 us per further request.
 constexpr int LSTM_GROUP = 8;          // requests per launch
 constexpr int LSTM_LAYER_BLOCKS = 16;  // 8 x 16 = 128 of 148 SMs
@@ -332,7 +332,7 @@ constexpr int LSTM_THREADS = LSTM_WARPS * 32;
 // requests: with 128 registers a block of this kernel took all of its SM, and two engines left it 116 SMs.  512 threads x 104
 // registers leave room for one engine block on every SM (256 threads, held to 48 registers by its launch bounds, sg_kernels.cu);
 // the 20 SMs that no block needs may hold any number.  Two requests' sums at a time keep the warp within 104 registers
-// (all at once with 128: 31.0 / 40.0 / 51.7 / 72.0 us; 96 registers spill: 37.2 / 39.3 / 55.4 / 93.5 us).
+// (all at once with 128: 30.4 / 38.9 / 49.1 / 69.5 us; four at a time with 104: 29.4 / 36.2 / 52.4 / 80.5 us; 96 registers spill more).
 constexpr int LSTM_REGS = 104;
 static_assert(LSTM_THREADS * LSTM_REGS + 256 * 48 <= 65536, "a block and a resident copy block share an SM's registers");
 
@@ -354,6 +354,20 @@ __device__ __forceinline__ float dot4(const float4& a, const float4& b) { return
 
 __device__ __forceinline__ void ld_two_words(const unsigned long long* p, unsigned long long* w0, unsigned long long* w1) {
   asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(*w0), "=l"(*w1) : "l"(p) : "memory");
+}
+
+// One step of a sum over the warp: of 2 x half values a lane keeps half, those of its side of `off`, and adds its partner's
+// share of them; with one value left both add the whole.
+template <int N>
+__device__ __forceinline__ void keep_half(float (&v)[N], int half, int off) {
+  const bool upper = (threadIdx.x & off) != 0;
+  if (half == 0) v[0] += __shfl_xor_sync(0xffffffffu, v[0], off);
+#pragma unroll
+  for (int k = 0; k < N / 2; k++) {
+    if (k >= half) break;
+    const float mine = upper ? v[k + half] : v[k], give = upper ? v[k] : v[k + half];
+    v[k] = mine + __shfl_xor_sync(0xffffffffu, give, off);
+  }
 }
 
 __global__ void lstm_bump_kernel(unsigned* epoch) { *epoch += 1; }
@@ -387,14 +401,17 @@ __global__ void __maxnreg__(LSTM_REGS) lstm_grid_kernel(const LstmGridArgs a) {
     u[g][1] = __ldg(ur + 32 + lane);
   }
   // After the reductions a lane has gate `gate` of request `req`; with the other gates it computes that request's cell.
-  const int gate = (lane / REP) & 3, req = (lane & (PASSES - 1)) * P + lane / (4 * REP), src_lane = lane - gate * REP;
-  const bool stores = unit && gate == 0 && (lane & (REP - 1)) < PASSES && req < a.batch;
+  const int lane_of_sum = lane & (REP - 1), gate = (lane / REP) & 3, src_lane = lane - gate * REP;
+  const int req = lane_of_sum / (REP / PASSES) * P + lane / (4 * REP);
+  const bool stores = unit && gate == 0 && lane_of_sum % (REP / PASSES) == 0 && req < a.batch;
   const float bias = B[gate * LH + (unit ? j : 0)] + (gate == 2 ? a.forget_bias : 0.f);
   // Staging: a thread takes two units of every ROWS-th of the step's 2 x NB vectors.  Both sources lie on one line through
   // hbuf, so each further vector of a thread is the first one's address plus a constant.
   const int row0 = (int)threadIdx.x / (LH / 2), pr2 = 2 * ((int)threadIdx.x % (LH / 2));
   const int from0 = row0 / NB, b0 = row0 % NB;
   const int words0 = (((l - 1 + from0) * LSTEPS - from0) * LSTM_GROUP + b0) * LH + pr2;  // at step 0; + LSTM_GROUP * LH per step
+  for (int i = (int)threadIdx.x; i < 4 * NB * LH; i += LSTM_THREADS)  // vectors of absent requests are multiplied all the same
+    if (i / LH % NB >= a.batch) (&s_vec[0][0][0][0])[i] = 0.f;
   float cell = 0.f;
   for (int t = 0; t < LSTEPS; t++) {
     float(*vec)[NB][LH] = s_vec[t & 1];
@@ -447,12 +464,11 @@ __global__ void __maxnreg__(LSTM_REGS) lstm_grid_kernel(const LstmGridArgs a) {
     }
     // The buffers alternate: a warp overwrites a vector only after the barrier above of the next step, which every warp
     // reaches when it has read this step's vectors.
-    // Sums over the warp, P requests at a time: while a lane holds several values it keeps one half of them and adds its
-    // partner's share of that half; then lane = value index x REP + replica, and of a value's replicas one keeps each pass.
-    float sum = 0.f;
+    // Sums over the warp: while a lane holds several values it keeps one half of them and adds its partner's share of that
+    // half, first among the PV sums of P requests, then among the passes; what is left of the 32 lanes are replicas.
+    float sum[PASSES];
 #pragma unroll
     for (int p = 0; p < PASSES; p++) {
-      if (p * P >= a.batch) break;
       float v[PV];
 #pragma unroll
       for (int b = 0; b < P; b++) {
@@ -468,27 +484,16 @@ __global__ void __maxnreg__(LSTM_REGS) lstm_grid_kernel(const LstmGridArgs a) {
         }
       }
 #pragma unroll
-      for (int step = 0; step < 5; step++) {
-        const int off = 16 >> step;
-        const int half = PV >> (step + 1);
-        if (half > 0) {
-          const bool upper = (lane & off) != 0;
-#pragma unroll
-          for (int k = 0; k < half; k++) {
-            const float mine = upper ? v[k + half] : v[k], give = upper ? v[k] : v[k + half];
-            v[k] = mine + __shfl_xor_sync(0xffffffffu, give, off);
-          }
-        } else {
-          v[0] += __shfl_xor_sync(0xffffffffu, v[0], off);
-        }
-      }
-      if (PASSES == 1 || (lane & (PASSES - 1)) == p) sum = v[0];
+      for (int half = PV / 2, off = 16; half > 0; half /= 2, off /= 2) keep_half(v, half, off);
+      sum[p] = v[0];
     }
-    sum += bias;
-    const float gi = __shfl_sync(0xffffffffu, sum, src_lane);
-    const float gg = __shfl_sync(0xffffffffu, sum, src_lane + REP);
-    const float gf = __shfl_sync(0xffffffffu, sum, src_lane + 2 * REP);
-    const float go = __shfl_sync(0xffffffffu, sum, src_lane + 3 * REP);
+#pragma unroll
+    for (int half = PASSES / 2, off = REP / 2; off > 0; half /= 2, off /= 2) keep_half(sum, half, off);
+    sum[0] += bias;
+    const float gi = __shfl_sync(0xffffffffu, sum[0], src_lane);
+    const float gg = __shfl_sync(0xffffffffu, sum[0], src_lane + REP);
+    const float gf = __shfl_sync(0xffffffffu, sum[0], src_lane + 2 * REP);
+    const float go = __shfl_sync(0xffffffffu, sum[0], src_lane + 3 * REP);
     cell = sigmoidf_(gf) * cell + sigmoidf_(gi) * tanhf(gg);
     const float h = tanhf(cell) * sigmoidf_(go);
     if (stores) {
