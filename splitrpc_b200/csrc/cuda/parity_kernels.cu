@@ -18,6 +18,7 @@
 #include "../host/p2p_rpc.h"
 #include "../host/p2p_rpc_app.h"
 #include "parity_kernels.h"
+#include "per_device.h"
 #include "ptx.cuh"
 
 namespace cg = cooperative_groups;
@@ -679,7 +680,8 @@ cudaError_t srpc_lstm(const void* d_stub, const float* direct_in, float* direct_
   // Whole-GPU dataflow (cooperative launches, LSTM_GROUP requests each); SPLITRPC_LSTM_CLUSTER=1 or a refused cooperative
   // launch falls back to the one-cluster-per-request kernel.
   static const int use_cluster = [] { const char* e = getenv("SPLITRPC_LSTM_CLUSTER"); return e ? atoi(e) : 0; }();
-  static std::atomic<int> grid_ok{0};  // 1 all blocks fit the device, -1 they do not
+  static std::atomic<signed char> grid_forms[64];  // per device: 1 all blocks fit it, -1 they do not, 0 not known yet
+  std::atomic<signed char>& grid_ok = grid_forms[PerDeviceFlag::current()];
   int done = 0;
   if (!use_cluster) {
     if (!grid_ok.load(std::memory_order_acquire)) {
@@ -716,7 +718,7 @@ cudaError_t srpc_lstm(const void* d_stub, const float* direct_in, float* direct_
         if (e == cudaSuccess) continue;
         (void)cudaGetLastError();
         if (done) return e;
-        grid_ok.store(-1, std::memory_order_release);  // not possible in this context: use the cluster kernel from now on
+        grid_ok.store(-1, std::memory_order_release);  // not possible on this device: use the cluster kernel from now on
         break;
       }
       if (done) return cudaSuccess;
