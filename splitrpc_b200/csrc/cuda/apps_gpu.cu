@@ -39,7 +39,7 @@ struct GpuAppState {
   uint32_t* h_pt_status = nullptr;
   uint64_t idle_ns = 200000000ull;
   float* d_scratch = nullptr;           // lstm: inter-layer hand-off buffer
-  uint32_t* h_status = nullptr;         // lstm: mapped word, non-zero after a wait between blocks has run out
+  uint32_t* h_status = nullptr;         // lstm: mapped word, non-zero after a wait between blocks has run out or a launch has failed
   uint32_t* d_status = nullptr;
   uint64_t wait_ms = 2000;              // lstm: limit of such a wait
   int lstm_clusters = 16;
@@ -317,7 +317,9 @@ void launch_kernels(AppCtx* c, int batch) {
     const float* b = s->d_weights;
     srpc_lenet_ref(c->d_stub, nullptr, nullptr, b + s->w_off[0], b + s->w_off[1], b + s->w_off[2], b + s->w_off[3], batch, q);
   } else if (s->name == "lstm") {
-    srpc_lstm(c->d_stub, nullptr, nullptr, s->d_weights, s->d_scratch, s->lstm_clusters, batch, 0.0f, s->d_status, s->wait_ms, q);
+    // a group of a larger batch that was not launched has no other way to be noticed
+    if (srpc_lstm(c->d_stub, nullptr, nullptr, s->d_weights, s->d_scratch, s->lstm_clusters, batch, 0.0f, s->d_status, s->wait_ms, q) != cudaSuccess)
+      *(volatile uint32_t*)s->h_status = 0x4C45u;
   }
 }
 
@@ -406,7 +408,7 @@ int gpu_app_complete(AppCtx* c) {
   if (s->h_status && *(volatile uint32_t*)s->h_status) {
     *(volatile uint32_t*)s->h_status = 0;
     c->last_status = -1;
-    srpc_log(SRPC_LOG_ERROR, "app '%s': a wait between blocks ran out, the batch has no result", s->name.c_str());
+    srpc_log(SRPC_LOG_ERROR, "app '%s': a wait between blocks ran out or a launch failed, the batch has no result", s->name.c_str());
   }
   return 1;
 }
