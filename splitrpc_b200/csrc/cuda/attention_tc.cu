@@ -44,8 +44,8 @@ struct AttSmem {
   static constexpr int P_BYTES = (SEQ / 64) * QT * 128;   // SEQ/64 atoms of 128 rows x 64 keys
   // With a single query tile (SEQ == 128) Q and K are dead once the scores exist, and the scores are dead once P is
   // written: P takes the place of Q|K in shared memory and the output accumulator the place of the scores in tensor
-  // memory.  48 KB and 128 columns per CTA let four CTAs share an SM, so every (sequence, head) of a 32 x 12 batch is
-  // resident at once and the SM interleaves their load -> MMA -> softmax -> MMA chains.
+  // memory.  48 KB, 128 columns and the launch bounds let three CTAs share an SM, so every (sequence, head) of a 32 x 12
+  // batch is resident at once (384 of 444) and the SM interleaves their load -> MMA -> softmax -> MMA chains.
   static constexpr bool ALIAS = SEQ == QT;
   static constexpr int P_OFFSET = ALIAS ? 0 : Q_BYTES + K_BYTES + VT_BYTES;
   static constexpr int TOTAL = ALIAS ? Q_BYTES + K_BYTES + VT_BYTES : Q_BYTES + K_BYTES + VT_BYTES + P_BYTES;

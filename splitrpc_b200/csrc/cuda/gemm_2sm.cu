@@ -55,13 +55,12 @@ template <int BN>
 struct Cfg {
   static constexpr int B_BYTES = (BN / 2) * BK * 2;  // this CTA's half of the B rows
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-  // (Measured: 4096 x 3072 x 768 with GELU 26.5 -> 24.2 us, 4096 x 768 x 3072 with residual 20.3 -> 18.8 us, 6144 x 4096 x 1024 with
-  // GELU 48.1 -> 44.8 us; before, all warps met at barriers twice per pass and one thread issued every store.)
   // Output staging.  Every epilogue warp has a block of its own, one or two chunks of 32 rows x 32 columns (2 KB), so that
   // no warp waits for another one between reading its part of the accumulator and handing it to its TMA store.  The
   // 256-wide tile has one chunk per warp: the memory goes to a sixth operand stage, and the k loop runs at (round-trip
-  // latency) / (stages); five stages cost 6144 x 3072 x 1024 6 %.  (Peer stores use the same memory as one block of
-  // PASS_COLS columns per pass.)
+  // latency) / (stages); five stages cost 6144 x 3072 x 1024 6 %.  Against barriers of all warps twice per pass and one thread
+  // that issues every store: 4096 x 3072 x 768 with GELU 26.5 -> 23.9 us, 4096 x 768 x 3072 with residual 20.3 -> 18.5 us, 6144 x 4096 x
+  // 1024 with GELU 48.1 -> 44.3 us.  (Peer stores use the same memory as one block of PASS_COLS columns per pass.)
   static constexpr int PASSES = BN == 256 ? 2 : 1;
   static constexpr int PASS_COLS = BN / PASSES;
   static constexpr int STAGES = BN == 256 ? 6 : (BN == 192 ? 6 : 7);

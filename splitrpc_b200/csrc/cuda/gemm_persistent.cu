@@ -7,15 +7,16 @@
 //   warp 0 and the last warp   one thread each issues the TMA loads of every second
 //            k-block of this CTA's tiles, running ahead through a STAGES-deep
 //            shared-memory ring that is not drained at tile boundaries;
-//   warp 1   one elected thread issues tcgen05.mma into one of two TMEM
-//            accumulators (2 x BN columns), so tile i+1 accumulates while tile i
-//            is being written out;
-//   warps 2-9 read the accumulator with tcgen05.ld (two warps per TMEM lane
-//            quarter, half of the columns each), release it at once, apply bias /
-//            residual (prefetched before the accumulator is ready) / activation,
-//            stage the bf16 tile in one of two 128-byte-swizzled shared-memory
-//            buffers and hand it to a TMA store (full-line coalesced writes,
-//            bounds clipped by the tensor map).
+//   warp 1   walks the schedule as one and waits; one elected lane issues
+//            tcgen05.mma into one of ACC TMEM accumulators (BN columns each), so
+//            tile i+1 accumulates while tile i is being written out;
+//   warps from 2 on (8, 12 or 16 of them, two to four per TMEM lane quarter, see
+//            Threads) read the accumulator with tcgen05.ld, release it at once,
+//            apply bias / residual (prefetched before the accumulator is ready) /
+//            activation and stage the bf16 tile in one of OB 128-byte-swizzled
+//            shared-memory buffers;
+//   the warp after them hands finished tiles to TMA stores (full-line coalesced
+//            writes, bounds clipped by the tensor map) and prefetches residual tiles.
 // In convolution mode the A operand needs no im2col and no gather: a tile is a
 // PW x PH x PN patch of output pixels, and the rows for filter tap (fr, fs) are
 // one 4-D TMA box over the NHWC input shifted by the tap offset, with element
@@ -53,7 +54,7 @@ constexpr int OUT_BUFS = 3;
 constexpr int MAX_OUT_BUFS = 4;
 // How many tiles ahead the residual tile is loaded (see TileParams::res_tma).
 constexpr int RES_DIST = 2;
-// warp 0 TMA, warp 1 MMA, then two epilogue warps per TMEM lane quarter (each takes half of the tile's columns)
+// warp 0 TMA, warp 1 MMA, then two to four epilogue warps per TMEM lane quarter (they share the tile's columns)
 template <int BN>
 struct Threads {
   // BN = 256 / 192: four / three warps per quarter, 64 columns each
@@ -115,10 +116,6 @@ struct TileParams {
   // two-input 1x1 convolution: k-blocks from kb_split on come from the second input (pixel stride2, no padding)
   int kb_split, stride2;
 };
-
-__device__ __forceinline__ void named_bar_sync(int id, int count) {
-  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory");
-}
 
 // Barrier over `count` threads that also returns the AND of their predicates.
 __device__ __forceinline__ bool named_bar_all(int id, int count, bool pred) {
@@ -335,7 +332,6 @@ gemm_conv_persistent(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
       pr_ph ^= 1u;
     }
   };
-  if (warp == 0) __syncwarp();
   const bool produces = producer >= 0 && layout_ok && lane == 0;
   if (producer == 0 && lane == 0) {
     ptx::grid_dep_wait();  // set-up above overlaps the kernel before; its results are read below
@@ -442,7 +438,7 @@ gemm_conv_persistent(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
     }
     if (!ok && elected) atomicCAS(&s_error, 0u, (uint32_t)GEMM_ERR_MMA_WAIT);
   } else if (warp < 2 + Threads<BN>::EPI / 32) {
-    // ---------------- epilogue warps (8): warp pair (w, w+4) shares a TMEM lane quarter and splits the columns
+    // ---------------- epilogue warps: those of one TMEM lane quarter (w, w+4, ...) split the columns
     constexpr int CPW = BN / (Threads<BN>::EPI / 128);  // columns per warp
     constexpr bool LEAN = BN >= 192 || Threads<BN>::EPI > 256;     // 14-18 warps per CTA: keep the accumulator in registers one chunk at a time
     constexpr int NCH = CPW / 32;        // 32-column chunks per warp
@@ -878,8 +874,8 @@ int srpc_gemm_trace_read(unsigned long long* out, int n) {
 // operand delivery (32 - 48 KB per k-block and SM), the two-SM tiles (256 rows per SM pair, gemm_2sm.cu) take a third less
 // of it.  With these figures 6144 x 1024 x 4096 takes pairs of 256 x 192 tiles (50.3 -> 42.6 us), 6144 x 1024 x 1024 too
 // (22.3 -> 17.9 us), 1024 x 768 x 3072 takes 64 columns (16.4 -> 15.1 us).  Below eight k-blocks memory and the epilogue
-// decide; the older figures pick the right shapes there.  Returns the width; *two_sm says which kernel, *cost_us the estimate.
-static int pick_tile(int M, int N, int num_kb, bool bf16_out, bool allow_two_sm, bool* two_sm, double* cost_us = nullptr) {
+// decide; the older figures pick the right shapes there (pairs are no candidates).  Returns the width; *two_sm says which kernel.
+static int pick_tile(int M, int N, int num_kb, bool bf16_out, bool allow_two_sm, bool* two_sm) {
   static const int allow256 = [] { const char* e = getenv("SPLITRPC_GEMM_BN256"); return e ? atoi(e) : 1; }();
   static const int allow192 = [] { const char* e = getenv("SPLITRPC_GEMM_BN192"); return e ? atoi(e) : 1; }();
   *two_sm = false;
@@ -889,7 +885,7 @@ static int pick_tile(int M, int N, int num_kb, bool bf16_out, bool allow_two_sm,
     bool pair;
   };
   const int sms = num_sms();
-  const Cand cands[7] = {{256, 256, sms / 2, 0.35, 0.40, true},  {192, 256, sms / 2, 0.29, 0.40, true}, {128, 256, sms / 2, 0.23, 0.40, true},
+  const Cand cands[7] = {{256, 256, sms / 2, 0.35, 0.35, true},  {192, 256, sms / 2, 0.29, 0.29, true}, {128, 256, sms / 2, 0.23, 0.23, true},
                          {256, 128, sms, 0.43, 0.49, false},     {192, 128, sms, 0.335, 0.37, false},   {128, 128, sms, 0.25, 0.27, false},
                          {64, 128, sms, 0.21, 0.27, false}};
   int best = N <= 64 ? 64 : 128;
@@ -911,7 +907,6 @@ static int pick_tile(int M, int N, int num_kb, bool bf16_out, bool allow_two_sm,
       *two_sm = c.pair;
     }
   }
-  if (cost_us) *cost_us = best_cost;
   return best;
 }
 

@@ -357,7 +357,7 @@ __global__ void __launch_bounds__(256) sg_cast_bf16(const SgItem* __restrict__ i
 
 // Gather fused with the deserialisation of a ResNet request: the fragments of an fp32 3 x 224 x 224 image are read
 // where the NIC put them and written, normalised and cast to bf16, in the space-to-depth layout that the stem
-// convolution reads through TMA (see stem_s2d in nn_kernels.cu for the layout).  The copy list is the ordinary one:
+// convolution reads (see stem_s2d in nn_kernels.cu for the layout).  The copy list is the ordinary one:
 // an item's destination address says which ring slot and which byte offset of the request the bytes belong to, so
 // fragments may arrive split and in any order.  The slot then holds the [115][115][16] bf16 tensor (423,200 bytes,
 // less than the 602,112-byte request it replaces); border pixels and padding channels are never written and keep
