@@ -323,19 +323,20 @@ lstm_wavefront_kernel(const g_params* stub, const float* direct_in, float* direc
 // (lstm_bump_kernel adds one before every launch; graph replays count too), so nothing has to be cleared in between.
 // A block stages the vectors of a step in shared memory for its warps; the 4 x NB gate sums of a warp are reduced together
 // (values are halved between lane pairs as they are added).  The kernel is launched cooperatively: all blocks are resident,
-// and every wait is bounded.  29.4 / 36.2 / 51.4 / 77.8 us for 1 / 2 / 4 / 8 requests back to back (61.8 / 84.0 / 128.9 / 216.7 us with a
+// and every wait is bounded.  30.3 / 35.6 / 47.4 / 79.4 us for 1 / 2 / 4 / 8 requests back to back (61.8 / 84.0 / 128.9 / 216.7 us with a
 // grid barrier per wave); what is left is the exchange latency, 2 us per step for one request, and 0.4 us per further request.
 constexpr int LSTM_GROUP = 8;          // requests per launch
 constexpr int LSTM_LAYER_BLOCKS = 16;  // 8 x 16 = 128 of 148 SMs
 constexpr int LSTM_WARPS = (LH + LSTM_LAYER_BLOCKS - 1) / LSTM_LAYER_BLOCKS;  // hidden units per block
 constexpr int LSTM_THREADS = LSTM_WARPS * 32;
 // A cooperative launch waits until all its blocks fit, and the blocks of resident copy engines (16 each) do not leave between
-// requests: with 128 registers a block of this kernel took all of its SM, and two engines left it 116 SMs.  512 threads x 104
-// registers leave room for one engine block on every SM (256 threads, held to 48 registers by its launch bounds, sg_kernels.cu);
-// the 20 SMs that no block needs may hold any number.  Two requests' sums at a time keep the warp within 104 registers
-// (all at once with 128: 30.4 / 38.9 / 49.1 / 69.5 us; four at a time with 104: 29.4 / 36.2 / 52.4 / 80.5 us; 96 registers spill more).
-constexpr int LSTM_REGS = 104;
-static_assert(LSTM_THREADS * LSTM_REGS + 256 * 48 <= 65536, "a block and a resident copy block share an SM's registers");
+// requests: with 128 registers a block of this kernel took all of its SM, and two engines left it 116 SMs.  512 threads x 112
+// registers leave room for one engine block on every SM (256 threads, held to 32 registers by its launch bounds, sg_kernels.cu);
+// the 20 SMs that no block needs may hold any number.  Two requests' sums at a time keep the warp within 112 registers.
+// 1 / 2 / 4 / 5 / 8 requests: 30.3 / 35.6 / 47.4 / 58.0 / 79.4 us; all sums at once with 128 registers 30.5 / 39.3 / 49.9 / 57.1 / 74.7 us; with 104
+// registers 30.5 / 41.3 / 55.1 / 65.5 / 82.8 us, with 96 it spills more.
+constexpr int LSTM_REGS = 112;
+static_assert(LSTM_THREADS * LSTM_REGS + 256 * 32 <= 65536, "a block and a resident copy block share an SM's registers");
 
 struct LstmGridArgs {
   const g_params* stub;
@@ -411,8 +412,6 @@ __global__ void __maxnreg__(LSTM_REGS) lstm_grid_kernel(const LstmGridArgs a) {
   const int row0 = (int)threadIdx.x / (LH / 2), pr2 = 2 * ((int)threadIdx.x % (LH / 2));
   const int from0 = row0 / NB, b0 = row0 % NB;
   const int words0 = (((l - 1 + from0) * LSTEPS - from0) * LSTM_GROUP + b0) * LH + pr2;  // at step 0; + LSTM_GROUP * LH per step
-  for (int i = (int)threadIdx.x; i < 4 * NB * LH; i += LSTM_THREADS)  // vectors of absent requests are multiplied all the same
-    if (i / LH % NB >= a.batch) (&s_vec[0][0][0][0])[i] = 0.f;
   float cell = 0.f;
   for (int t = 0; t < LSTEPS; t++) {
     float(*vec)[NB][LH] = s_vec[t & 1];
@@ -473,6 +472,11 @@ __global__ void __maxnreg__(LSTM_REGS) lstm_grid_kernel(const LstmGridArgs a) {
       float v[PV];
 #pragma unroll
       for (int b = 0; b < P; b++) {
+        if (p * P + b > NB / 2 && p * P + b >= a.batch) {  // (a launch has more than NB / 2 requests)
+#pragma unroll
+          for (int g = 0; g < 4; g++) v[b * 4 + g] = 0.f;
+          continue;
+        }
         const float4* xv = reinterpret_cast<const float4*>(vec[0][p * P + b]);
         const float4 x0 = xv[lane], x1 = xv[32 + lane];
 #pragma unroll

@@ -26,8 +26,8 @@ class P2pRpcSgGpuEngine : public P2pRpcSgEngine {
   // Blocks per copy kernel.  A list whose sources sit in host memory is bound by the PCIe link and needs only enough
   // loads in flight to cover its latency.  When the model's persistent kernels leave r SMs out of their grids
   // (srpc_gemm_reserve_sms), the copy runs as r blocks of 1024 threads (written -r): twelve reach the link rate, and
-  // the model beside it runs as fast as alone (measured: ResNet-50 graph 1.68 ms with the copy, 1.63 ms alone, against
-  // 1.98 ms when the copy's 48 blocks of 256 threads each hold an SM that a persistent kernel counts on).  Lists
+  // the model beside it runs as fast as alone (measured: ResNet-50 graph 1.16 ms with the copy, 1.13 ms alone, against
+  // 1.57 ms when the copy's 48 blocks of 256 threads each hold an SM that a persistent kernel counts on).  Lists
   // that read device memory get four blocks of 256 threads per SM.  P2P_RPC_SG_BLOCKS overrides both
   // (negative = 1024-thread blocks).
   int n_blocks_ = readEnvInfo<int>("P2P_RPC_SG_BLOCKS", 0);

@@ -425,15 +425,23 @@ __global__ void __launch_bounds__(1024) sg_stem_s2d(const SgItem* __restrict__ i
 // valid.  The exit flag and the idle limit are looked at on every poll, before the doorbell, so a block always leaves
 // within one poll of being asked to, whatever the doorbell says.  Blocks never wait for one another: each finishes its
 // share, and the block that brings the arrival counter to gridDim.x publishes `done`.
-// (At most 48 registers: the LSTM's blocks, which must all be resident at once, count on room beside one block of this kernel.)
-__global__ void __launch_bounds__(256, 5) sg_persistent(SgCtrl* ctrl, uint32_t* counter) {
-  __shared__ uint32_t s_cmd, s_seq;
+// At most 32 registers: the LSTM's blocks, which must all be resident at once, count on room beside one block of this kernel.
+// What only the polling thread looks at therefore lives in shared memory.
+constexpr uint32_t PERSISTENT_THREADS = 256;
+__global__ void __launch_bounds__(PERSISTENT_THREADS, 8) sg_persistent(SgCtrl* ctrl, uint32_t* counter) {
+  __shared__ uint32_t s_cmd;
+  __shared__ volatile uint32_t s_seen;              // the newest submission that this block has taken on
+  __shared__ volatile uint64_t s_last, s_idle_limit;
   __shared__ SgItem s_items[SG_PERSISTENT_ITEMS];
-  uint32_t seen = ctrl->done;  // submissions up to `done` were served by an earlier launch
-  uint64_t last = ptx::globaltimer_ns();
-  const uint64_t idle_limit = ctrl->idle_limit_ns;
+  if (threadIdx.x == 0) {
+    s_seen = ctrl->done;  // submissions up to `done` were served by an earlier launch
+    s_last = ptx::globaltimer_ns();
+    s_idle_limit = ctrl->idle_limit_ns;
+  }
   for (;;) {
     if (threadIdx.x == 0) {
+      const uint64_t last = s_last, idle_limit = s_idle_limit;
+      const uint32_t seen = s_seen;
       uint32_t cmd = 0;  // 0 keep polling, 1 work, 2 leave
       for (int spin = 0; spin < 4096; spin++) {
         if (ptx::ld_relaxed_sys(&ctrl->exit_flag) || ptx::globaltimer_ns() - last > idle_limit) {
@@ -442,7 +450,7 @@ __global__ void __launch_bounds__(256, 5) sg_persistent(SgCtrl* ctrl, uint32_t* 
         }
         const uint32_t db = ptx::ld_acquire_sys(&ctrl->doorbell);
         if ((int32_t)(db - seen) > 0) {
-          s_seq = db;
+          s_seen = db;
           cmd = 1;
           break;
         }
@@ -451,11 +459,10 @@ __global__ void __launch_bounds__(256, 5) sg_persistent(SgCtrl* ctrl, uint32_t* 
       s_cmd = cmd;
     }
     __syncthreads();
-    const uint32_t cmd = s_cmd, seq = s_seq;
+    const uint32_t cmd = s_cmd;
     __syncthreads();
     if (cmd == 2) break;
     if (cmd == 0) continue;
-    seen = seq;
     uint32_t n_items = ctrl->n_items, n_chunks = ctrl->n_chunks;
     if (n_items > SG_PERSISTENT_ITEMS) n_items = SG_PERSISTENT_ITEMS;
     // One pass over PCIe brings the list into shared memory; lookups stay on chip.
@@ -467,7 +474,7 @@ __global__ void __launch_bounds__(256, 5) sg_persistent(SgCtrl* ctrl, uint32_t* 
     __syncthreads();
     for (uint32_t c = blockIdx.x; c < n_chunks; c += gridDim.x) {
       ChunkRef r = chunk_ref(s_items, n_items, c, n_chunks);
-      copy_chunk_simt(r.src, r.dst, r.len, threadIdx.x, blockDim.x);
+      copy_chunk_simt(r.src, r.dst, r.len, threadIdx.x, PERSISTENT_THREADS);
     }
     __threadfence_system();
     __syncthreads();
@@ -476,9 +483,9 @@ __global__ void __launch_bounds__(256, 5) sg_persistent(SgCtrl* ctrl, uint32_t* 
       if (prev + 1 == gridDim.x) {
         atomicExch(counter, 0u);
         __threadfence_system();
-        ptx::st_release_sys(&ctrl->done, seen);
+        ptx::st_release_sys(&ctrl->done, s_seen);
       }
-      last = ptx::globaltimer_ns();
+      s_last = ptx::globaltimer_ns();
     }
   }
   if (threadIdx.x == 0) atomicAdd_system(const_cast<uint32_t*>(&ctrl->exited), 1u);
@@ -605,6 +612,6 @@ cudaError_t sg_launch_stem_s2d(const SgItem* d_items, uint32_t n_items, uint32_t
 
 cudaError_t sg_launch_persistent(SgCtrl* d_ctrl, uint32_t* d_counter, int n_blocks, cudaStream_t stream) {
   sg_kernel_setup();
-  sg_persistent<<<n_blocks, 256, 0, stream>>>(d_ctrl, d_counter);
+  sg_persistent<<<n_blocks, PERSISTENT_THREADS, 0, stream>>>(d_ctrl, d_counter);
   return cudaGetLastError();
 }
