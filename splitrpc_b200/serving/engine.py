@@ -93,7 +93,7 @@ class ModelServer(_GraphModelApp):
         """``reserve_sms``: SMs that the model's persistent kernels leave out of their grids, for the scatter-gather
         kernel that pulls the next batch out of host memory while the current one is computed.  A persistent kernel
         counts on one block per SM: with a foreign block on only a few SMs it takes twice as long (ResNet-50 graph
-        1.98 ms instead of 1.63 ms), with twelve SMs set aside it runs at 1.68 ms beside the copy.
+        1.57 ms instead of 1.13 ms), with twelve SMs set aside it runs at 1.16 ms beside the copy.
 
         ``n_replicas``: how many replicas this ingress will feed in total (sizes the arenas and the request pool)."""
         super().__init__(model, device, max_batch, copy_type, pool_size, batch_sizes, reserve_sms, fused_ingress)

@@ -33,7 +33,7 @@ def test_batches_and_repeated_runs(C, launch_type):
     C.set_rpc_mtu(8192)
     app = C.make_app("lstm", 0, T * H * 4, H * 4, w, 64, launch_type, 17)
     base = app.req_ring[0]
-    for n in (1, 2, 3, 4, 5, 8, 9, 17, 2, 1):  # short batches after long ones must not see their words
+    for n in (1, 2, 3, 4, 5, 6, 7, 8, 9, 17, 2, 1):  # short batches after long ones must not see their words
         x = rng.standard_normal((n, T, H)).astype(np.float32)
         d = torch.from_numpy(x).cuda()
         C.memcpy_async(base, d.data_ptr(), x.nbytes, 0)
