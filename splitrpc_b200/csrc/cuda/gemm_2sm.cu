@@ -1,17 +1,16 @@
 // Two-SM persistent GEMM:  D[M,N] = act(A[M,K] . B[N,K]^T + bias + residual), bf16 in and out, fp32 accumulation.
 //
-// The compute-bound shapes of the one-SM kernel (gemm_persistent.cu) stall on operand delivery: a 128 x 256 tile
-// pulls 48 KB through the L2 -> SM path per 64-deep k-block, and at full tensor rate that is more than the path
-// carries, so the tensor pipe idles a third of the time.  Here two CTAs of a cluster (an SM pair) compute one
-// 256 x 256 tile with tcgen05.mma.cta_group::2: each CTA loads its own 128 rows of A and only HALF of the B rows
-// (32 KB per k-block), the leader CTA's single MMA thread issues one instruction that reads both CTAs' shared memory
-// and writes 128 accumulator rows into each CTA's tensor memory.
+// The compute-bound shapes of the one-SM kernel (gemm_persistent.cu) stall on shared memory: for a 128 x 256 tile and a
+// 64-deep k-block the loads write 48 KB and the MMAs read 48 KB, 768 cycles at 128 bytes per clock where the tensor pipe takes
+// 512.  Here two CTAs of a cluster (an SM pair) compute one 256 x 256 tile with tcgen05.mma.cta_group::2: each CTA loads its own
+// 128 rows of A and only HALF of the B rows (32 KB per k-block), one instruction of the leader CTA reads both CTAs' shared
+// memory and writes 128 accumulator rows into each CTA's tensor memory.
 //
 // Protocol (both CTAs run the same code; rank 0 of the pair is the leader):
-//   producer   two threads of each CTA, in turn, load its A rows and its half of B for every k-block into a stage ring.  The
+//   producer   two warps of each CTA, in turn, load its A rows and its half of B for every k-block into a stage ring.  The
 //              "full" barrier of a stage is the LEADER's: the leader's producer posts the expected byte count of both
 //              CTAs, and both CTAs' TMA loads (cp.async.bulk.tensor ... cta_group::2, no multicast) count on it.
-//   MMA        one thread of the leader waits for a full stage, issues four 256 x 256 x 16 MMAs and commits them to
+//   MMA        one warp of the leader waits for a full stage, issues four 256 x 256 x 16 MMAs and commits them to
 //              the stage's "empty" barrier in BOTH CTAs (tcgen05.commit with a two-CTA mask), then, per tile, to both
 //              CTAs' "accumulator full" barriers.  Two accumulators (2 x 256 columns) alternate between tiles.
 //   epilogue   16 warps per CTA read their CTA's 128 accumulator rows (tcgen05.ld), 32 rows x 64 columns each, add bias
@@ -51,23 +50,34 @@ constexpr int OUT_HALF_BYTES = BM * 128;    // 128 rows x 64 bf16 columns
 constexpr int OUT_CHUNK_BYTES = 32 * 64;    // 32 rows x 32 bf16 columns
 
 // Tile widths 128 / 192 / 256: one epilogue warp per 64 columns and TMEM lane quarter, as many stages as fit.
-template <int BN>
+//
+// What bounds the k loop: shared memory.  Loads write (128 + BN / 2) x 128 bytes per k-block and SM, MMAs read (128 + BN) x
+// 128, and both together move 128 bytes per clock: 640 cycles for BN = 256 against 512 of the tensor pipe.
+//
+// What a launch costs beside it, and what was done about it (4096 x 2304 x 768, two tiles of 3.5 us each per pair): a
+// cluster barrier with release / acquire takes 0.85 us, twice per launch, and so does every release to the peer, 0.6 us per
+// tile: none of the three orders memory here (relaxed forms, see ptx.cuh).  The epilogue reads the accumulator as 8 x 8
+// fragments: bias and residual are then packed pairs of columns, where a thread with a whole row needs every bias value of
+// the tile broadcast to it through the pipe that the MMAs' operands take; with stmatrix behind it the last
+// tile's epilogue takes 2.4 us instead of 3.9.  Together (us before -> now): 4096 x 2304 x 768 14.9 -> 12.4, 4096 x 3072 x 768
+// with GELU 24.0 -> 20.0, 4096 x 768 x 3072 with residual 18.9 -> 15.8, 6144 x 1024 x 1024 16.2 -> 12.9, 12544 x 256 x 1024 12.0 -> 10.3.
+// Not better: stores of 32 bytes per lane instead of TMA stores (17.5 us for the first), 64 columns per store (one operand
+// stage less, 13.2 us).
+//
+// Output staging: every epilogue warp has a block of its own, one or two chunks of 32 rows x 32 columns (2 KB), so that no warp
+// waits for another one between reading its part of the accumulator and handing it to its TMA store.  The 256-wide tile has
+// one chunk per warp: the memory goes to a sixth operand stage.  (Peer stores use the same memory as one block of PASS_COLS
+// columns per pass.)
+template <int BN, bool TP>
 struct Cfg {
-  static constexpr int B_BYTES = (BN / 2) * BK * 2;  // this CTA's half of the B rows
-  static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-  // Output staging.  Every epilogue warp has a block of its own, one or two chunks of 32 rows x 32 columns (2 KB), so that
-  // no warp waits for another one between reading its part of the accumulator and handing it to its TMA store.  The
-  // 256-wide tile has one chunk per warp: the memory goes to a sixth operand stage, and the k loop runs at (round-trip
-  // latency) / (stages); five stages cost 6144 x 3072 x 1024 6 %.  Against barriers of all warps twice per pass and one thread
-  // that issues every store: 4096 x 3072 x 768 with GELU 26.5 -> 23.9 us, 4096 x 768 x 3072 with residual 20.3 -> 18.5 us, 6144 x 4096 x
-  // 1024 with GELU 48.1 -> 44.3 us.  (Peer stores use the same memory as one block of PASS_COLS columns per pass.)
+  static constexpr int STAGE_BYTES = A_BYTES + (BN / 2) * BK * 2;  // A rows and this CTA's half of the B rows
   static constexpr int PASSES = BN == 256 ? 2 : 1;
   static constexpr int PASS_COLS = BN / PASSES;
-  static constexpr int STAGES = BN == 256 ? 6 : (BN == 192 ? 6 : 7);
   static constexpr int OUT_BYTES = (PASS_COLS / 64) * OUT_HALF_BYTES;
+  static constexpr int CHUNK_BUFS = OUT_BYTES / ((2 * BN) / 32) / OUT_CHUNK_BYTES;
+  static constexpr int STAGES = (224 * 1024 - OUT_BYTES) / STAGE_BYTES;
   static constexpr int EPI_THREADS = 2 * BN;
   static constexpr int THREADS = 64 + EPI_THREADS + 32;  // TMA, MMA, epilogue, second TMA warp
-  static constexpr int CHUNK_BUFS = OUT_BYTES / (EPI_THREADS / 32) / OUT_CHUNK_BYTES;
   static constexpr int ACC_STRIDE = BN == 192 ? 256 : BN;  // TMEM columns between the two accumulators
   static constexpr int TMEM_COLS = 2 * ACC_STRIDE;
   static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + OUT_BYTES;
@@ -126,14 +136,13 @@ __device__ __forceinline__ bool pair_tile(int j, const TileOrder& o, PairTile* o
 }
 
 template <int BN, bool TP>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Cfg<BN>::THREADS, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Cfg<BN, TP>::THREADS, 1)
 gemm_2sm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                 const __grid_constant__ CUtensorMap tmap_out, int M, int N, int K, const TileOrder order, GemmEpilogue ep,
                 uint32_t* status, const TpParams tp_in) {
-  constexpr int B_BYTES = Cfg<BN>::B_BYTES, STAGE_BYTES = Cfg<BN>::STAGE_BYTES, STAGES = Cfg<BN>::STAGES;
-  constexpr int EPI_THREADS = Cfg<BN>::EPI_THREADS, ACC_STRIDE = Cfg<BN>::ACC_STRIDE, TMEM_COLS = Cfg<BN>::TMEM_COLS;
-  constexpr int PASSES = Cfg<BN>::PASSES, PASS_COLS = Cfg<BN>::PASS_COLS, CHUNK_BUFS = Cfg<BN>::CHUNK_BUFS;
-  (void)B_BYTES;
+  using C = Cfg<BN, TP>;
+  constexpr int STAGE_BYTES = C::STAGE_BYTES, STAGES = C::STAGES, EPI_THREADS = C::EPI_THREADS, ACC_STRIDE = C::ACC_STRIDE;
+  constexpr int PASSES = C::PASSES, PASS_COLS = C::PASS_COLS;
   extern __shared__ __align__(1024) uint8_t smem[];
   TpParams tp = tp_in;
   if constexpr (TP) {
@@ -177,28 +186,31 @@ gemm_2sm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
     ptx::prefetch_tmap(&tmap_out);
   }
   if (warp == 1) {
-    ptx::tmem_alloc_2sm(&tmem_base_smem, TMEM_COLS);
+    ptx::tmem_alloc_2sm(&tmem_base_smem, C::TMEM_COLS);
     ptx::tmem_relinquish_2sm();
     if (!order.late_trigger) ptx::grid_dep_launch();  // after the allocation, see pdl_launch.h
   }
   ptx::tc_fence_before();
   __syncthreads();
-  ptx::cluster_sync_all();  // the peer's barriers exist before anything signals them
-  ptx::grid_dep_wait();     // set-up above overlaps the kernel before; its results are read below
+  // The peer's barriers must exist before anything signals them; every role waits for that where it first matters.
+  ptx::cluster_arrive_relaxed();
   ptx::tc_fence_after();
   const uint32_t tmem_base = tmem_base_smem;
-  if (threadIdx.x == 0) GEMM2_TRACE(1);
 
-  if (warp == 0 || warp == Cfg<BN>::THREADS / 32 - 1) {
-    // ---------------- producers: one lane each of two warps per CTA take the k-blocks in turn (see gemm_persistent.cu)
+  if (warp == 0 || warp == C::THREADS / 32 - 1) {
+    // ---------------- producers: two warps per CTA take the k-blocks in turn (see gemm_persistent.cu).  Each walks the schedule
+    // as one and an elected lane issues, so that the operands of the loads stay in uniform registers (an iteration of
+    // the loads alone: 240 ns in one lane's branch, 200 ns this way).
     constexpr int PRODUCERS = 2;
-    int kb = warp == 0 ? 0 : 1, s = kb, j = 0;
+    const bool elected = ptx::elect_one();
+    int kb = warp == 0 ? 0 : 1, s = kb, j = 0, seq = kb;  // seq: position in this cluster's sequence of k-blocks
     uint32_t ph = 0;
     PairTile t;
-    bool ok = layout_ok && lane == 0;
+    bool ok = layout_ok, first = true;
     while (ok) {
       for (; kb >= num_kb; kb -= num_kb) j++;
-      if (!pair_tile(j, order, &t) || *(volatile uint32_t*)&s_error != 0) break;
+      ok = __all_sync(0xffffffffu, *(volatile uint32_t*)&s_error == 0);
+      if (!ok || !pair_tile(j, order, &t)) break;
       const int row0 = (t.m2 * 2 + (int)rank) * BM;
       const int brow0 = t.n * BN + (int)rank * (BN / 2);
       if constexpr (TP) {
@@ -206,26 +218,40 @@ gemm_2sm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
           // Rows of a peer arrive through the copier clusters of this launch, one 128-row block at a time.
           const int m_idx = t.m2 * 2 + (int)rank;
           if (m_idx / tp.mblocks_per_rank != tp.rank) {
-            if (!tpdev::wait_flag_gpu(tp.mblock_ready + m_idx, tp.epoch)) {
-              atomicExch(&s_error, GEMM_ERR_TP_BLOCK_WAIT);
+            if (elected) {
+              ok = tpdev::wait_flag_gpu(tp.mblock_ready + m_idx, tp.epoch);
+              ptx::fence_proxy_async_all();  // the copier's writes -> this thread's TMA reads
+            }
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok) {
+              if (elected) atomicExch(&s_error, GEMM_ERR_TP_BLOCK_WAIT);
               break;
             }
-            ptx::fence_proxy_async_all();  // the copier's writes -> this thread's TMA reads
           }
         }
       }
       for (; kb < num_kb; kb += PRODUCERS) {
-        if (!ptx::mbar_wait(&empty_bar[s], ph ^ 1u)) {
-          atomicExch(&s_error, GEMM_ERR_PRODUCER_WAIT);
-          ok = false;
+        ok = ptx::mbar_wait_warp(&empty_bar[s], ph ^ 1u);
+        if (!ok) {
+          if (elected) atomicExch(&s_error, GEMM_ERR_PRODUCER_WAIT);
           break;
         }
         const uint32_t full_leader = ptx::mapa_shared(ptx::smem_u32(&full_bar[s]), 0);
-        if (leader) ptx::mbar_expect_tx(&full_bar[s], 2u * STAGE_BYTES);
         uint8_t* sa = smem + (size_t)s * STAGE_BYTES;
-        ptx::tma_load_2d_2sm(sa, &tmap_a, full_leader, kb * BK, row0);
-        ptx::tma_load_2d_2sm(sa + A_BYTES, &tmap_b, full_leader, kb * BK, brow0);
-        if (j == 0 && kb == 0) GEMM2_TRACE(2);
+        if (first) {
+          // everything above overlaps the kernel before; its results are read below
+          ptx::cluster_wait();
+          if (lane == 0 && warp == 0) GEMM2_TRACE(1);
+          ptx::grid_dep_wait();
+          first = false;
+        }
+        if (elected) {
+          if (leader) ptx::mbar_expect_tx(&full_bar[s], 2u * STAGE_BYTES);
+          ptx::tma_load_2d_2sm(sa, &tmap_a, full_leader, kb * BK, row0);
+          ptx::tma_load_2d_2sm(sa + A_BYTES, &tmap_b, full_leader, kb * BK, brow0);
+        }
+        if (j == 0 && kb == 0 && lane == 0) GEMM2_TRACE(2);
+        seq += PRODUCERS;
         s += PRODUCERS;
         if (s >= STAGES) {
           s -= STAGES;
@@ -237,9 +263,26 @@ gemm_2sm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
       __syncwarp();
       ptx::grid_dep_launch();
     }
+    if (first) ptx::cluster_wait();  // this warp had no k-block
+    // The leader's MMAs signal the stages of both CTAs, and none of those signals may still be on its way when this CTA leaves:
+    // wait as for the STAGES k-blocks behind the last one (this warp's share of them).
+    if (ok) {
+      const int tiles = order.tiles_m2 * order.tiles_n, first_tile = (int)(blockIdx.x >> 1);
+      const int total = first_tile < tiles ? ((tiles - first_tile + order.clusters - 1) / order.clusters) * num_kb : 0;
+      for (int i = seq - total; ok && i < STAGES; i += PRODUCERS) {
+        ok = ptx::mbar_wait_warp(&empty_bar[s], ph ^ 1u);
+        s += PRODUCERS;
+        if (s >= STAGES) {
+          s -= STAGES;
+          ph ^= 1u;
+        }
+      }
+      if (!ok && elected) atomicCAS(&s_error, 0u, (uint32_t)GEMM_ERR_PRODUCER_WAIT);
+    }
   } else if (warp == 1) {
     // ---------------- MMA issue (leader only): the warp walks the schedule together, one elected lane issues, so that
     // descriptors and addresses stay in uniform registers (see gemm_persistent.cu)
+    ptx::cluster_wait();
     if (leader) {
       const bool elected = ptx::elect_one();
       const uint32_t idesc = ptx::umma_idesc_bf16(2 * BM, BN);
@@ -280,19 +323,26 @@ gemm_2sm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
         ok = *(volatile uint32_t*)&s_error == 0;
         ok = __all_sync(0xffffffffu, ok);
       }
+      // the peer's last hand-backs have arrived before this CTA leaves
+      for (int i = 0; ok && i < 2; i++, local++) ok = ptx::mbar_wait_warp(&tmem_empty_bar[local & 1u], ((local >> 1) & 1u) ^ 1u);
       if (!ok && elected) atomicCAS(&s_error, 0u, (uint32_t)GEMM_ERR_MMA_WAIT);
     }
   } else {
     // ---------------- epilogue: a warp has 32 rows (its TMEM lane quarter) x two chunks of 32 columns of the tile and goes through
     // them on its own: residual and bias on their way before the accumulator is ready, its own TMA stores.
+    ptx::grid_dep_wait();
+    ptx::cluster_wait();
     const int warp_q = warp & 3;
     const int cgroup = (warp - 2) >> 2;      // 0 .. EPI_THREADS/128 - 1
-    const int row = warp_q * 32 + lane;      // row of this CTA's half tile
     const int et = threadIdx.x - 64;
-    const bool vec_res = ep.residual && ((ep.ldr & 7) == 0) && (((uintptr_t)ep.residual & 15) == 0);
-    uint8_t* stage = stage_out + (size_t)(warp - 2) * CHUNK_BUFS * OUT_CHUNK_BYTES;
+    // This thread's accumulator elements: columns 8 g + fc, + 1 (g = 0 .. 3) of rows fr + 8 i (i = 0 .. 3) of the warp's 32 rows.
+    const int fr = lane >> 2, fc = (lane & 3) * 2;
+    const bool vec_res = ep.residual && ((ep.ldr & 1) == 0) && (((uintptr_t)ep.residual & 3) == 0);
     // column of chunk ch inside the tile
-    auto chunk_col = [&](int ch) { return PASSES == 2 ? ch * PASS_COLS + cgroup * 32 : (cgroup * 2 + ch) * 32; };
+    auto chunk_col = [&](int ch) { return PASSES == 2 && TP ? ch * PASS_COLS + cgroup * 32 : (cgroup * 2 + ch) * 32; };
+    uint8_t* stage = stage_out + (size_t)(warp - 2) * C::CHUNK_BUFS * OUT_CHUNK_BYTES;
+    // what this lane names in stmatrix: matrices 0, 1 = rows 0 .. 7, 8 .. 15 of one column group, 2, 3 = of the next one
+    const int st_row = (lane & 7) + (lane & 8), st_cg = lane >> 4;
     uint32_t local = 0;
     PairTile t;
     bool peer_store = false;
@@ -301,23 +351,30 @@ gemm_2sm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
     for (int j = 0; ok && pair_tile(j, order, &t); j++, local++) {
       const uint32_t acc = local & 1u;
       const int row0 = (t.m2 * 2 + (int)rank) * BM;
-      const int m = row0 + row;
-      const bool row_ok = m < M;
+      const int m0 = row0 + warp_q * 32;  // first row of this warp
       const int n0 = t.n * BN;
-      const __nv_bfloat16* rp = ep.residual ? ep.residual + (size_t)(row_ok ? m : 0) * ep.ldr + n0 : nullptr;
-      uint4 rq[4];
-      auto load_residual = [&](int ch) {
-        if (vec_res && row_ok && n0 + chunk_col(ch) + 32 <= N) {
+      // Residual and bias are on their way before the accumulator is ready.
+      uint32_t rq[2][16];
+      if (vec_res) {
 #pragma unroll
-          for (int q = 0; q < 4; q++) rq[q] = *(reinterpret_cast<const uint4*>(rp + chunk_col(ch)) + q);
+        for (int ch = 0; ch < 2; ch++) {
+          const int col0 = n0 + chunk_col(ch);
+          if (col0 + 32 <= N) {
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+              const int m = m0 + fr + 8 * i;
+              if (m < M) {
+                const __nv_bfloat16* rp = ep.residual + (size_t)m * ep.ldr + col0 + fc;
+#pragma unroll
+                for (int g = 0; g < 4; g++) rq[ch][i * 4 + g] = *reinterpret_cast<const uint32_t*>(rp + g * 8);
+              }
+            }
+          }
         }
-      };
-      if (ep.residual) load_residual(0);
-      float bias_l[2] = {0.f, 0.f};  // lane = column of the chunk; handed round by shuffles when it is added
+      }
       if (ep.bias) {
-#pragma unroll
-        for (int ch = 0; ch < 2; ch++)
-          if (n0 + chunk_col(ch) + lane < N) bias_l[ch] = ep.bias[n0 + chunk_col(ch) + lane];
+        const int cb = n0 + chunk_col(lane >> 4) + (lane & 15) * 2;
+        if (cb < N) asm volatile("prefetch.global.L1 [%0];" ::"l"(ep.bias + cb));
       }
       ok = *(volatile uint32_t*)&s_error == 0 && ptx::mbar_wait(&tmem_full_bar[acc], (local >> 1) & 1u);
       ok = __all_sync(0xffffffffu, ok);
@@ -332,71 +389,83 @@ gemm_2sm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
       for (int ch = 0; ch < 2; ch++) {
         const int c = chunk_col(ch);  // column inside the tile
         const int col0 = n0 + c;
+        const uint32_t t_addr = tmem_base + acc * ACC_STRIDE + ((uint32_t)(warp_q * 32) << 16) + (uint32_t)c;
         uint32_t r[32];
-        ptx::tmem_ld_32x32b_x32(tmem_base + acc * ACC_STRIDE + ((uint32_t)(warp_q * 32) << 16) + (uint32_t)c, r);
+        ptx::tmem_ld_16x256b_x4(t_addr, r);
+        ptx::tmem_ld_16x256b_x4(t_addr + (16u << 16), r + 16);
+        float2 b2[4];
+        if (ep.bias) {
+#pragma unroll
+          for (int g = 0; g < 4; g++) {
+            const int col = col0 + g * 8 + fc;
+            if (col + 1 < N) b2[g] = *reinterpret_cast<const float2*>(ep.bias + col);
+            else b2[g] = make_float2(col < N ? ep.bias[col] : 0.f, 0.f);
+          }
+        }
         ptx::tmem_ld_wait();
-        if (ch == 1) {  // last read: hand the accumulator back to the leader's MMA thread
+        if (ch == 1) {  // last read: hand the accumulator back to the leader's MMA warp
           ptx::tc_fence_before();
           __syncwarp();
           if (lane == 0) ptx::mbar_arrive_cluster(ptx::mapa_shared(ptx::smem_u32(&tmem_empty_bar[acc]), 0));
         }
-        float v[32];
+        float2 v[16];  // [row group i][column group g]
 #pragma unroll
-        for (int q = 0; q < 32; q++) v[q] = __uint_as_float(r[q]);
+        for (int i = 0; i < 4; i++)
+#pragma unroll
+          for (int g = 0; g < 4; g++) {
+            const int at = (i >> 1) * 16 + g * 4 + (i & 1) * 2;
+            v[i * 4 + g] = make_float2(__uint_as_float(r[at]), __uint_as_float(r[at + 1]));
+          }
         if (ep.bias) {
 #pragma unroll
-          for (int q = 0; q < 32; q++) v[q] += __shfl_sync(0xffffffffu, bias_l[ch], q);
+          for (int q = 0; q < 16; q++) v[q] = __fadd2_rn(v[q], b2[q & 3]);
         }
-        if (ep.residual && row_ok && col0 < N) {
-          if (vec_res && col0 + 32 <= N) {
+        if (vec_res && col0 + 32 <= N) {
 #pragma unroll
-            for (int q = 0; q < 4; q++) {
-              const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&rq[q]);
+          for (int q = 0; q < 16; q++) v[q] = __fadd2_rn(v[q], __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&rq[ch][q])));
+        } else if (ep.residual) {
 #pragma unroll
-              for (int u = 0; u < 4; u++) {
-                const float2 f = __bfloat1622float2(h[u]);
-                v[q * 8 + 2 * u] += f.x;
-                v[q * 8 + 2 * u + 1] += f.y;
-              }
-            }
-          } else {
-#pragma unroll
-            for (int q = 0; q < 32; q++)
-              if (col0 + q < N) v[q] += __bfloat162float(rp[c + q]);
+          for (int q = 0; q < 16; q++) {
+            const int m = m0 + fr + 8 * (q >> 2), col = col0 + (q & 3) * 8 + fc;
+            const __nv_bfloat16* rp = ep.residual + (size_t)m * ep.ldr + col;
+            if (m < M && col < N) v[q].x += __bfloat162float(rp[0]);
+            if (m < M && col + 1 < N) v[q].y += __bfloat162float(rp[1]);
           }
         }
-        if (ep.residual && ch == 0) load_residual(1);
         if (ep.act == GEMM_ACT_RELU) {
 #pragma unroll
-          for (int q = 0; q < 32; q++) v[q] = fmaxf(v[q], 0.f);
+          for (int q = 0; q < 16; q++) v[q] = make_float2(fmaxf(v[q].x, 0.f), fmaxf(v[q].y, 0.f));
         } else if (ep.act == GEMM_ACT_GELU) {
 #pragma unroll
-          for (int q = 0; q < 32; q += 2) {
-            const float2 g = ptx::gelu_erf_fast2(make_float2(v[q], v[q + 1]));
-            v[q] = g.x;
-            v[q + 1] = g.y;
-          }
+          for (int q = 0; q < 16; q++) v[q] = ptx::gelu_erf_fast2(v[q]);
         } else if (ep.act == GEMM_ACT_TANH) {
 #pragma unroll
-          for (int q = 0; q < 32; q++) v[q] = tanhf(v[q]);
+          for (int q = 0; q < 16; q++) v[q] = make_float2(tanhf(v[q].x), tanhf(v[q].y));
         }
-        uint4 o[4];
+        uint32_t o[16];
 #pragma unroll
-        for (int q = 0; q < 4; q++) {
-          __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&o[q]);
-#pragma unroll
-          for (int u = 0; u < 4; u++) h[u] = __floats2bfloat162_rn(v[q * 8 + 2 * u], v[q * 8 + 2 * u + 1]);
+        for (int q = 0; q < 16; q++) {
+          const __nv_bfloat162 h = __floats2bfloat162_rn(v[q].x, v[q].y);
+          o[q] = *reinterpret_cast<const uint32_t*>(&h);
         }
+        // Rows of `row_bytes`, 16-byte pieces exchanged within a row by piece XOR swz(row): piece `first` + column group.
+        auto put = [&](uint8_t* base, int row_bytes, int first, auto swz) {
+#pragma unroll
+          for (int h = 0; h < 2; h++)
+#pragma unroll
+            for (int g = 0; g < 4; g += 2) {
+              const int rr = h * 16 + st_row;
+              const uint32_t addr = ptx::smem_u32(base) + (uint32_t)(rr * row_bytes + (((first + g + st_cg) ^ swz(rr)) << 4));
+              ptx::stmatrix_x4(addr, o[(2 * h) * 4 + g], o[(2 * h + 1) * 4 + g], o[(2 * h) * 4 + g + 1], o[(2 * h + 1) * 4 + g + 1]);
+            }
+        };
         if constexpr (TP) {
           if (peer_store) {
             // The tile goes to the slot this rank owns on the rank that owns these rows (rows per rank are a multiple
             // of 128, so a CTA's half tile has one owner), PASS_COLS columns at a time.
             const int pass = PASSES == 2 ? ch : 0, cp = c - pass * PASS_COLS;  // column inside the pass
             if (PASSES == 2 || ch == 0) named_bar_sync(1, EPI_THREADS);        // the previous pass has been read
-            uint8_t* half = stage_out + (size_t)(cp >> 6) * OUT_HALF_BYTES + (size_t)row * 128;
-            const int chunk0 = (cp & 63) >> 3;
-#pragma unroll
-            for (int q = 0; q < 4; q++) *reinterpret_cast<uint4*>(half + (((chunk0 + q) ^ (row & 7)) << 4)) = o[q];
+            put(stage_out + (size_t)(cp >> 6) * OUT_HALF_BYTES + (size_t)(warp_q * 32) * 128, 128, (cp & 63) >> 3, [](int rr) { return rr & 7; });
             if (PASSES == 1 && ch == 0) continue;
             named_bar_sync(1, EPI_THREADS);
             const int m_idx = t.m2 * 2 + (int)rank;
@@ -431,22 +500,18 @@ gemm_2sm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
             continue;
           }
         }
-        // This chunk's block of the staging memory: its last store must have finished reading it.
-        uint8_t* block = stage + (CHUNK_BUFS == 2 ? ch * OUT_CHUNK_BYTES : 0);
-        if (lane == 0) ptx::bulk_wait_read<CHUNK_BUFS - 1>();
+        // A chunk is a block of 32 rows of 64 bytes under the 64-byte swizzle; its last store must have been read.
+        uint8_t* block = stage + (C::CHUNK_BUFS == 2 ? ch * OUT_CHUNK_BYTES : 0);
+        if (lane == 0) ptx::bulk_wait_read<C::CHUNK_BUFS - 1>();
         __syncwarp();
-#pragma unroll
-        for (int q = 0; q < 4; q++) {  // rows of 64 bytes, 64-byte swizzle: 16-byte piece XOR (128-byte line number mod 4)
-          const uint32_t at = (uint32_t)(lane * 64 + q * 16);
-          *reinterpret_cast<uint4*>(block + (at ^ (((at >> 7) & 3u) << 4))) = o[q];
-        }
+        put(block, 64, 0, [](int rr) { return (rr >> 1) & 3; });
         ptx::fence_proxy_async_smem();
         __syncwarp();
         if (lane == 0) {
-          if (col0 < N && row0 + warp_q * 32 < M) ptx::tma_store_2d(&tmap_out, block, col0, row0 + warp_q * 32);
+          if (col0 < N && m0 < M) ptx::tma_store_2d(&tmap_out, block, col0, m0);
           ptx::bulk_commit();
-          if (j == 0 && et == 0 && ch == 1) GEMM2_TRACE(6);
         }
+        if (j == 0 && et == 0 && ch == 1) GEMM2_TRACE(6);
       }
     }
     if (et == 0) GEMM2_TRACE(7);
@@ -459,10 +524,13 @@ gemm_2sm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
     if (threadIdx.x == 0 && status) atomicExch(status, s_error);
     __nanosleep(1000000);  // let loads that are still in flight land before the block leaves
   }
-  ptx::cluster_sync_all();  // the peer no longer reads this CTA's shared memory nor signals its barriers
+  // Every signal to this CTA has arrived (above) and the peer's MMAs no longer read its shared memory (its last accumulator was
+  // complete); tensor memory is given back by both CTAs together.
+  ptx::cluster_arrive_relaxed();
+  ptx::cluster_wait();
   if (warp == 1) {
     ptx::tc_fence_after();
-    ptx::tmem_dealloc_2sm(tmem_base, TMEM_COLS);
+    ptx::tmem_dealloc_2sm(tmem_base, C::TMEM_COLS);
   }
 }
 
@@ -470,7 +538,7 @@ gemm_2sm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
 // Clusters of two CTAs that can be resident at once (queried once per instantiation and device).
 template <int BN, bool TP>
 cudaError_t max_clusters_2sm(int* out) {
-  using C = Cfg<BN>;
+  using C = Cfg<BN, TP>;
   static std::atomic<int> per_device[64];
   const int dev = PerDeviceFlag::current();
   int max_clusters = per_device[dev].load(std::memory_order_acquire);
@@ -502,7 +570,7 @@ cudaError_t max_clusters_2sm(int* out) {
 template <int BN>
 cudaError_t launch_2sm(const void* A, int lda, const void* B, int ldb, int M, int N, int K, const GemmEpilogue& ep,
                        uint32_t* status, cudaStream_t stream) {
-  using C = Cfg<BN>;
+  using C = Cfg<BN, false>;
   int max_clusters = 0;
   cudaError_t e = max_clusters_2sm<BN, false>(&max_clusters);
   if (e != cudaSuccess) return e;
@@ -528,7 +596,7 @@ cudaError_t launch_2sm(const void* A, int lda, const void* B, int ldb, int M, in
 template <int BN>
 cudaError_t launch_2sm_tp(const void* A, int lda, const void* B, int ldb, int M, int N, int K, const GemmEpilogue& ep,
                           TpParams tp, uint32_t* status, cudaStream_t stream) {
-  using C = Cfg<BN>;
+  using C = Cfg<BN, true>;
   static_assert(C::SMEM_BYTES >= tpdev::COPY_SLOTS * tpdev::COPY_CHUNK, "the copier's ring lives in the operand stages");
   int max_clusters = 0;
   cudaError_t e = max_clusters_2sm<BN, true>(&max_clusters);

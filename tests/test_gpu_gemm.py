@@ -67,6 +67,27 @@ def test_gemm_wide_tiles_with_epilogue(env, M, N, K):
     assert _rel_err(torch, out, ref) < 1e-2
 
 
+@pytest.mark.parametrize("M,N,K", [(4352, 1536, 512), (4097, 1032, 768), (3000, 1000, 832), (2600, 768, 1096), (2049, 128, 2048)])
+@pytest.mark.parametrize("ldr_extra", [0, 1, 6])
+def test_gemm_pair_tiles_ragged(env, M, N, K, ldr_extra):
+    """Edges of the CTA-pair tiles: last rows and columns, K remainders, one to three tiles per pair, residual rows of any stride."""
+    torch, ops = env
+    a = (torch.randn(M, K, device="cuda") * 0.3).bfloat16()
+    b = (torch.randn(N, K, device="cuda") * 0.3).bfloat16()
+    bias = torch.randn(N, device="cuda")
+    res = torch.randn(M, N + ldr_extra, device="cuda").bfloat16()[:, :N]
+    buf = torch.full((M + 1, N + 8), 7.0, device="cuda", dtype=torch.bfloat16)
+    for act in (None, "relu", "gelu"):
+        out = ops.gemm(a, b, bias=bias, residual=res, act=act, out=buf[:M, :N])
+        ops.check_status()
+        ref = a.double() @ b.double().t() + bias.double() + res.double()
+        ref = torch.relu(ref) if act == "relu" else (torch.nn.functional.gelu(ref) if act == "gelu" else ref)
+        # half a unit of bf16 (2^-9 of the value) twice, and the fp32 sums: K 2^-24 times the sum of |products| (about 0.09 K)
+        assert ((out.double() - ref).abs() <= ref.abs() * 2.0 ** -8 + K * K * 0.09 * 2.0 ** -24 + 1e-6).all()
+        assert (buf[M] == 7.0).all() and (buf[:, N:] == 7.0).all()
+
+
+
 def test_gelu_epilogue_matches_erf_definition(env):
     """The epilogue's rational erfc approximation against torch's exact GELU over a wide range of inputs."""
     torch, ops = env
