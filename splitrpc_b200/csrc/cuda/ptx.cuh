@@ -133,22 +133,27 @@ __device__ __forceinline__ float gelu_erf_fast(float x) {
   return x * (x < 0.f ? h : 1.0f - h);
 }
 
-// The same for two values with packed arithmetic: every operation and rounding of gelu_erf_fast, half the instructions.
+// The same approximation for two values, in the form x Phi(x) = max(x, 0) - |x| erfc(|x| / sqrt 2) / 2: no selection by the sign,
+// constants folded (2 MIN, 2 MAX, 11 packed operations, 4 MUFU for two values; the GELU epilogue of a 128 x 256 half tile
+// is bound by them).  |x| is capped where the second term has long been zero, so that infinities give infinity and 0; NaN stays.
 __device__ __forceinline__ float2 gelu_erf_fast2(float2 x) {
-  const float2 ax = __fmul2_rn(make_float2(fabsf(x.x), fabsf(x.y)), make_float2(0.70710678118654752f, 0.70710678118654752f));
-  const float2 d = __ffma2_rn(make_float2(0.3275911f, 0.3275911f), ax, make_float2(1.0f, 1.0f));
-  float2 t, e;
+  float2 t, e, relu;
+  const float2 a = make_float2(fminf(fabsf(x.x), 64.f), fminf(fabsf(x.y), 64.f));
+  const float2 d = __ffma2_rn(make_float2(0.23164190f, 0.23164190f), a, make_float2(1.0f, 1.0f));  // 0.3275911 / sqrt 2
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(t.x) : "f"(d.x));
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(t.y) : "f"(d.y));
-  float2 p = __ffma2_rn(t, make_float2(1.061405429f, 1.061405429f), make_float2(-1.453152027f, -1.453152027f));
-  p = __ffma2_rn(p, t, make_float2(1.421413741f, 1.421413741f));
-  p = __ffma2_rn(p, t, make_float2(-0.284496736f, -0.284496736f));
-  p = __ffma2_rn(p, t, make_float2(0.254829592f, 0.254829592f));
-  const float2 g = __fmul2_rn(__fmul2_rn(make_float2(-1.4426950408889634f, -1.4426950408889634f), ax), ax);
+  // the polynomial times -1/2
+  float2 p = __ffma2_rn(t, make_float2(-0.5307027145f, -0.5307027145f), make_float2(0.7265760135f, 0.7265760135f));
+  p = __ffma2_rn(p, t, make_float2(-0.7107068705f, -0.7107068705f));
+  p = __ffma2_rn(p, t, make_float2(0.142248368f, 0.142248368f));
+  p = __ffma2_rn(p, t, make_float2(-0.127414796f, -0.127414796f));
+  p = __fmul2_rn(p, t);
+  const float2 g = __fmul2_rn(__fmul2_rn(a, make_float2(-0.72134752044f, -0.72134752044f)), a);  // -x^2 / 2 in powers of two
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e.x) : "f"(g.x));
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e.y) : "f"(g.y));
-  const float2 h = __fmul2_rn(__fmul2_rn(__fmul2_rn(make_float2(0.5f, 0.5f), p), t), e);  // 0.5 * erfc(|x| / sqrt 2)
-  return __fmul2_rn(x, make_float2(x.x < 0.f ? h.x : 1.0f - h.x, x.y < 0.f ? h.y : 1.0f - h.y));
+  asm("max.NaN.f32 %0, %1, 0f00000000;" : "=f"(relu.x) : "f"(x.x));
+  asm("max.NaN.f32 %0, %1, 0f00000000;" : "=f"(relu.y) : "f"(x.y));
+  return __ffma2_rn(__fmul2_rn(p, e), a, relu);
 }
 
 // ---------------------------------------------------------------- 8 x 8 matrices of 16-bit values to shared memory
