@@ -86,17 +86,6 @@ struct Cfg {
 __device__ __forceinline__ void named_bar_sync(int id, int count) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory");
 }
-__device__ __forceinline__ bool named_bar_all(int id, int count, bool pred) {
-  uint32_t out;
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 q, %3, 0;\n\t"
-      "barrier.cta.red.and.pred p, %1, %2, q;\n\tselp.u32 %0, 1, 0, p;\n\t}\n"
-      : "=r"(out)
-      : "r"(id), "r"(count), "r"((uint32_t)pred)
-      : "memory");
-  return out != 0;
-}
-
 // Optional phase time stamps of block 0 (build with -DSRPC_GEMM_TRACE), read back through srpc_gemm_trace_read.
 #ifdef SRPC_GEMM_TRACE
 __device__ unsigned long long g_gemm2_trace[16];
@@ -353,7 +342,7 @@ gemm_2sm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
       const int row0 = (t.m2 * 2 + (int)rank) * BM;
       const int m0 = row0 + warp_q * 32;  // first row of this warp
       const int n0 = t.n * BN;
-      // Residual and bias are on their way before the accumulator is ready.
+      // Residual and bias arrive before the accumulator is ready.
       uint32_t rq[2][16];
       if (vec_res) {
 #pragma unroll
@@ -372,13 +361,20 @@ gemm_2sm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
           }
         }
       }
+      float2 b2[2][4];
       if (ep.bias) {
-        const int cb = n0 + chunk_col(lane >> 4) + (lane & 15) * 2;
-        if (cb < N) asm volatile("prefetch.global.L1 [%0];" ::"l"(ep.bias + cb));
+#pragma unroll
+        for (int ch = 0; ch < 2; ch++)
+#pragma unroll
+          for (int g = 0; g < 4; g++) {
+            const int col = n0 + chunk_col(ch) + g * 8 + fc;
+            if (col + 1 < N) b2[ch][g] = *reinterpret_cast<const float2*>(ep.bias + col);
+            else b2[ch][g] = make_float2(col < N ? ep.bias[col] : 0.f, 0.f);
+          }
       }
       ok = *(volatile uint32_t*)&s_error == 0 && ptx::mbar_wait(&tmem_full_bar[acc], (local >> 1) & 1u);
       ok = __all_sync(0xffffffffu, ok);
-      if (TP && peer_store) ok = named_bar_all(2, EPI_THREADS, ok);
+      if (TP && peer_store) ok = ptx::named_bar_all(2, EPI_THREADS, ok);
       if (!ok) {
         if (lane == 0) atomicCAS(&s_error, 0u, (uint32_t)GEMM_ERR_EPILOGUE_WAIT);
         break;
@@ -393,15 +389,6 @@ gemm_2sm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
         uint32_t r[32];
         ptx::tmem_ld_16x256b_x4(t_addr, r);
         ptx::tmem_ld_16x256b_x4(t_addr + (16u << 16), r + 16);
-        float2 b2[4];
-        if (ep.bias) {
-#pragma unroll
-          for (int g = 0; g < 4; g++) {
-            const int col = col0 + g * 8 + fc;
-            if (col + 1 < N) b2[g] = *reinterpret_cast<const float2*>(ep.bias + col);
-            else b2[g] = make_float2(col < N ? ep.bias[col] : 0.f, 0.f);
-          }
-        }
         ptx::tmem_ld_wait();
         if (ch == 1) {  // last read: hand the accumulator back to the leader's MMA warp
           ptx::tc_fence_before();
@@ -418,7 +405,7 @@ gemm_2sm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
           }
         if (ep.bias) {
 #pragma unroll
-          for (int q = 0; q < 16; q++) v[q] = __fadd2_rn(v[q], b2[q & 3]);
+          for (int q = 0; q < 16; q++) v[q] = __fadd2_rn(v[q], b2[ch][q & 3]);
         }
         if (vec_res && col0 + 32 <= N) {
 #pragma unroll

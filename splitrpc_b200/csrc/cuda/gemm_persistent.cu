@@ -52,6 +52,8 @@ constexpr int UMMA_K = 16;
 // the pace of memory-bound shapes.
 constexpr int OUT_BUFS = 3;
 constexpr int MAX_OUT_BUFS = 4;
+// Width of the output patch of convolutions with row-tap reuse: an image row inside the box is one swizzle atom.
+constexpr int REUSE_PW = 8;
 // How many tiles ahead the residual tile is loaded (see TileParams::res_tma).
 constexpr int RES_DIST = 2;
 // warp 0 TMA, warp 1 MMA, then two to four epilogue warps per TMEM lane quarter (they share the tile's columns)
@@ -117,22 +119,6 @@ struct TileParams {
   int kb_split, stride2;
 };
 
-// Barrier over `count` threads that also returns the AND of their predicates.
-__device__ __forceinline__ bool named_bar_all(int id, int count, bool pred) {
-  uint32_t out;
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 q, %3, 0;\n\t"
-      "barrier.cta.red.and.pred p, %1, %2, q;\n\tselp.u32 %0, 1, 0, p;\n\t}\n"
-      : "=r"(out)
-      : "r"(id), "r"(count), "r"((uint32_t)pred)
-      : "memory");
-  return out != 0;
-}
-
-__device__ __forceinline__ void tma_load_4d_box(void* smem_dst, const CUtensorMap* m, uint64_t* bar, int c0, int c1, int c2,
-                                                int c3) {
-  ptx::tma_load_4d(smem_dst, m, bar, c0, c1, c2, c3);
-}
 __device__ __forceinline__ void tma_store_4d(const CUtensorMap* m, const void* smem_src, int c0, int c1, int c2, int c3) {
   asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.tile.bulk_group [%0, {%2, %3, %4, %5}], [%1];" ::"l"(m),
                "r"(ptx::smem_u32(smem_src)), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
@@ -267,12 +253,11 @@ gemm_conv_persistent(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
     if (use_tma_store) ptx::prefetch_tmap(&tmap_out);
     if (p.res_tma) ptx::prefetch_tmap(&tmap_res);
   }
-  // TMA producers: the elected lanes of warp 0 and of the last warp take the k-blocks of this CTA's schedule in turn (even
-  // ones, odd ones).  One of them needs about 250 ns per k-block (wait for the stage, post the byte count, issue two
-  // loads), as long as the tensor pipe takes for the widest tile and twice as long as for a 128-wide one.  Measured with
-  // two producers and the uniform MMA loop below: 258 -> 211 ns per k-block of a single 128 x 128 tile; 3x3 convolutions of
-  // 64 images: 56x56x64 44.0 -> 30.3 us, 14x14x256 25.7 -> 22.3 us, 7x7x512 39.9 -> 22.9 us.
-  // The state lives across two calls: the first fills one (initially free) stage each right after the barriers exist,
+  // TMA producers: warp 0 and the last warp take the k-blocks of this CTA's schedule in turn (even ones, odd ones).  Each walks
+  // the schedule as one and an elected lane issues, so that the operands of the loads stay in uniform registers: an iteration
+  // (wait for the stage, post the byte count, two loads) takes 200 ns this way and 240 ns in one lane's branch, and a k-block of
+  // the narrow tiles is consumed in 150 - 250 ns.  One producer instead of two: 258 ns per k-block of a lone 128 x 128 tile.
+  // The state lives across two calls: the first fills one (initially free) stage right after the barriers exist,
   // before the block-wide set-up barrier, so that the first operands are already in flight while tensor memory is being
   // allocated; the second runs the rest of the schedule.
   // (A ring of one stage, which the widest load groups of a short filter leave, has one producer.)
@@ -283,48 +268,56 @@ gemm_conv_persistent(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
   int img_off = 0;
   TileCoord pr_tc;
   bool pr_more = false;
+  const bool pr_elected = producer >= 0 && ptx::elect_one();
   // Moves to the tile that holds k-block pr_kb; false when the schedule is through.
   auto producer_tile = [&]() {
     while (pr_kb >= p.num_kb) {
       pr_kb -= p.num_kb;
       pr_j++;
     }
-    return get_tile(p, pr_j, &pr_tc) && *(volatile uint32_t*)&s_error == 0;
+    return get_tile(p, pr_j, &pr_tc) && __all_sync(0xffffffffu, *(volatile uint32_t*)&s_error == 0);
   };
   const uint32_t b_tx = (uint32_t)(b_per_stage * B_BYTES);
   auto produce_one = [&]() {
-    if (!ptx::mbar_wait(&empty_bar[pr_s], pr_ph ^ 1u)) {
-      atomicExch(&s_error, GEMM_ERR_PRODUCER_WAIT);
+    if (!ptx::mbar_wait_warp(&empty_bar[pr_s], pr_ph ^ 1u)) {
+      if (pr_elected) atomicExch(&s_error, GEMM_ERR_PRODUCER_WAIT);
       pr_more = false;
       return;
     }
     uint8_t* sa = a_ring + (size_t)pr_s * a_stride;
+    uint64_t* full = &full_bar[pr_s];
     if (p.mode == 0) {
-      ptx::mbar_expect_tx(&full_bar[pr_s], (uint32_t)A_BYTES + b_tx);
-      ptx::tma_load_2d(sa, &tmap_a, &full_bar[pr_s], pr_kb * BK, pr_tc.m_idx * BM);
+      if (pr_elected) {
+        ptx::mbar_expect_tx(full, (uint32_t)A_BYTES + b_tx);
+        ptx::tma_load_2d(sa, &tmap_a, full, pr_kb * BK, pr_tc.m_idx * BM);
+        if (!p.b_stationary) ptx::tma_load_2d(sa + A_BYTES, &tmap_b, full, pr_kb * BK, pr_tc.n_idx * BN);
+      }
     } else {
-      ptx::mbar_expect_tx(&full_bar[pr_s], p.a_box_bytes + b_tx);
       const int tap = (int)fdiv(p.fd_cblocks, (uint32_t)pr_kb), cb = pr_kb - tap * p.cblocks;
       if (p.reuse) {
         // load group (fs, cb): the box covers filter rows 0 .. r-1 at once
         const int fs = tap;
-        tma_load_4d_box(sa, &tmap_a, &full_bar[pr_s], cb * BK, pr_tc.w0 + fs - p.pad, pr_tc.h0 - p.pad, pr_tc.img0 + img_off);
-        if (!p.b_stationary)
-          for (int fr = 0; fr < p.r; fr++)
-            ptx::tma_load_2d(sa + A_BYTES + fr * B_BYTES, &tmap_b, &full_bar[pr_s], ((fr * p.s + fs) * p.cblocks + cb) * BK,
-                             pr_tc.n_idx * BN);
-      } else if (pr_kb >= p.kb_split) {
-        // second input of a two-input 1x1 convolution (its map travels in the residual map's place)
-        tma_load_4d_box(sa, &tmap_res, &full_bar[pr_s], (pr_kb - p.kb_split) * BK, pr_tc.w0 * p.stride2, pr_tc.h0 * p.stride2,
-                        pr_tc.img0);
-      } else {
-        const int fr = (int)fdiv(p.fd_s, (uint32_t)tap), fs = tap - fr * p.s;
-        tma_load_4d_box(sa, &tmap_a, &full_bar[pr_s], cb * BK, pr_tc.w0 * p.stride + fs - p.pad, pr_tc.h0 * p.stride + fr - p.pad,
-                        pr_tc.img0 + img_off);
+        if (pr_elected) {
+          ptx::mbar_expect_tx(full, p.a_box_bytes + b_tx);
+          ptx::tma_load_4d(sa, &tmap_a, full, cb * BK, pr_tc.w0 + fs - p.pad, pr_tc.h0 - p.pad, pr_tc.img0 + img_off);
+          if (!p.b_stationary)
+            for (int fr = 0; fr < p.r; fr++)
+              ptx::tma_load_2d(sa + A_BYTES + fr * B_BYTES, &tmap_b, full, ((fr * p.s + fs) * p.cblocks + cb) * BK, pr_tc.n_idx * BN);
+        }
+      } else if (pr_elected) {
+        ptx::mbar_expect_tx(full, p.a_box_bytes + b_tx);
+        if (pr_kb >= p.kb_split) {
+          // second input of a two-input 1x1 convolution (its map travels in the residual map's place)
+          ptx::tma_load_4d(sa, &tmap_res, full, (pr_kb - p.kb_split) * BK, pr_tc.w0 * p.stride2, pr_tc.h0 * p.stride2, pr_tc.img0);
+        } else {
+          const int fr = (int)fdiv(p.fd_s, (uint32_t)tap), fs = tap - fr * p.s;
+          ptx::tma_load_4d(sa, &tmap_a, full, cb * BK, pr_tc.w0 * p.stride + fs - p.pad, pr_tc.h0 * p.stride + fr - p.pad,
+                           pr_tc.img0 + img_off);
+        }
+        if (!p.b_stationary) ptx::tma_load_2d(sa + A_BYTES, &tmap_b, full, pr_kb * BK, pr_tc.n_idx * BN);
       }
     }
-    if (!p.b_stationary && !p.reuse) ptx::tma_load_2d(sa + A_BYTES, &tmap_b, &full_bar[pr_s], pr_kb * BK, pr_tc.n_idx * BN);
-    if (pr_j == 0 && pr_kb == 0) GEMM_TRACE(2);
+    if (pr_j == 0 && pr_kb == 0 && lane == 0) GEMM_TRACE(2);
     pr_kb += producers;
     pr_s += producers;
     if (pr_s >= nst) {
@@ -332,18 +325,17 @@ gemm_conv_persistent(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
       pr_ph ^= 1u;
     }
   };
-  const bool produces = producer >= 0 && layout_ok && lane == 0;
-  if (producer == 0 && lane == 0) {
+  if (producer == 0) {
+    pr_more = layout_ok && producer_tile();
     ptx::grid_dep_wait();  // set-up above overlaps the kernel before; its results are read below
     if (p.in_stub)
       img_off = (int)((*reinterpret_cast<const unsigned long long*>(p.in_stub) - p.in_ring_base) / p.in_slot_bytes);
-    TileCoord tc;
-    if (layout_ok && p.b_stationary && get_tile(p, 0, &tc)) {
+    if (pr_more && p.b_stationary && pr_elected) {
       ptx::mbar_expect_tx(&bpanel_bar, (uint32_t)panel_bytes);
       for (int kb = 0; kb < p.panel_kb; kb++)
-        ptx::tma_load_2d(smem + (size_t)kb * B_BYTES, &tmap_b, &bpanel_bar, kb * BK, tc.n_idx * BN);
+        ptx::tma_load_2d(smem + (size_t)kb * B_BYTES, &tmap_b, &bpanel_bar, kb * BK, pr_tc.n_idx * BN);
     }
-    if (layout_ok && (pr_more = producer_tile())) produce_one();
+    if (pr_more) produce_one();
   }
   if (warp == 1) {
     ptx::tmem_alloc(&tmem_base_smem, ACC * ACC_STRIDE);
@@ -364,7 +356,7 @@ gemm_conv_persistent(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
       pr_more = true;
     }
     // the rest of this producer's k-blocks, paced by the MMA warp through the empty barriers
-    if (produces && pr_more)
+    if (layout_ok && pr_more)
       while (producer_tile()) {
         const int j = pr_j;
         while (pr_more && pr_j == j && pr_kb < p.num_kb) produce_one();
@@ -385,6 +377,8 @@ gemm_conv_persistent(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
     const uint32_t ring_lo = ptx::umma_desc_lo(ptx::smem_u32(a_ring)), stride_lo = (uint32_t)a_stride >> 4;
     const uint32_t panel_lo = ptx::umma_desc_lo(ptx::smem_u32(smem));
     constexpr uint32_t K_LO = UMMA_K * 2 / 16;  // descriptor step from one 16-deep slice to the next
+    constexpr uint32_t REUSE_ROW_LO = REUSE_PW * 128 / 16;  // to the next image row inside a reused box
+    const uint32_t b_row_lo = (uint32_t)(p.b_stationary ? p.num_kb * B_BYTES : B_BYTES) / 16;  // to the next filter row
     uint32_t local = 0;
     int s = 0;
     uint32_t ph = 0;
@@ -403,16 +397,24 @@ gemm_conv_persistent(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
         if (j == 0 && kb == 0 && lane == 0) GEMM_TRACE(3);
         const uint32_t sa = ring_lo + (uint32_t)s * stride_lo;
         if (p.reuse) {
-          const int fs = kb / p.cblocks, cb = kb - fs * p.cblocks;
-          for (int fr = 0; fr < p.r; fr++) {
-            const uint32_t sa_fr = sa + (uint32_t)(fr * p.pw * 128 / 16);  // fr image rows further into the box
-            const uint32_t sb = p.b_stationary ? panel_lo + (uint32_t)((fr * p.s + fs) * p.cblocks + cb) * (B_BYTES / 16)
-                                               : sa + (uint32_t)(A_BYTES + fr * B_BYTES) / 16;
-            if (elected) {
+          // r filter rows: A a patch row further into the box, B the next filter row of this (filter column, channel block).
+          // One unrolled run of MMAs per load group: issuing them was what a 64-wide tile took its time for (56 ns per MMA, 27 now;
+          // 64 images of 56 x 56 x 64 29.5 -> 23.9 us, 28 x 28 x 128 22.2 -> 20.3, 14 x 14 x 256 21.6 -> 18.7).
+          const uint32_t sb = p.b_stationary ? panel_lo + (uint32_t)kb * (B_BYTES / 16) : sa + A_BYTES / 16;
+          if (elected) {
+            if (p.r == 3) {
 #pragma unroll
-              for (int k = 0; k < BK / UMMA_K; k++)
-                ptx::umma_bf16(d_tmem, ptx::umma_desc_join(sa_fr + k * K_LO), ptx::umma_desc_join(sb + k * K_LO), idesc,
-                               (kb | fr | k) != 0 ? 1u : 0u);
+              for (int fr = 0; fr < 3; fr++)
+#pragma unroll
+                for (int k = 0; k < BK / UMMA_K; k++)
+                  ptx::umma_bf16(d_tmem, ptx::umma_desc_join(sa + fr * REUSE_ROW_LO + k * K_LO),
+                                 ptx::umma_desc_join(sb + fr * b_row_lo + k * K_LO), idesc, (kb | fr | k) != 0 ? 1u : 0u);
+            } else {
+              for (int fr = 0; fr < p.r; fr++)
+#pragma unroll
+                for (int k = 0; k < BK / UMMA_K; k++)
+                  ptx::umma_bf16(d_tmem, ptx::umma_desc_join(sa + fr * REUSE_ROW_LO + k * K_LO),
+                                 ptx::umma_desc_join(sb + fr * b_row_lo + k * K_LO), idesc, (kb | fr | k) != 0 ? 1u : 0u);
             }
           }
         } else {
@@ -498,7 +500,7 @@ gemm_conv_persistent(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
         if (res_tma && mine) mine = ptx::mbar_wait(&res_full_bar[local % OB], (local / OB) & 1u);
         else if (use_tma_store && mine) mine = ptx::mbar_wait(&out_empty_bar[local % OB], ((local / OB) & 1u) ^ 1u);
       }
-      if (!named_bar_all(2, EPI_THREADS, mine)) {
+      if (!ptx::named_bar_all(2, EPI_THREADS, mine)) {
         if (lane == 0) atomicExch(&s_error, GEMM_ERR_EPILOGUE_WAIT);
         break;
       }
@@ -1032,7 +1034,7 @@ cudaError_t srpc_conv_bf16_tma(const void* in, const void* weight, const ConvSha
   int bn;
   if (reuse) {
     p.reuse = 1;
-    p.pw = 8;
+    p.pw = REUSE_PW;
     p.ph = std::min(cs.oh, 16 - (cs.r - 1));
     p.pn = 1;
     p.num_kb = cs.s * p.cblocks;  // load groups
