@@ -63,6 +63,7 @@ const SrpcDriverApi* srpc_driver_api() {
     get("cuStreamWriteValue32", (void**)&api.StreamWriteValue32);
     get("cuStreamWriteValue64", (void**)&api.StreamWriteValue64);
     get("cuTensorMapEncodeTiled", (void**)&api.TensorMapEncodeTiled);
+    get("cuTensorMapEncodeIm2col", (void**)&api.TensorMapEncodeIm2col);
     get("cuDeviceGetAttribute", (void**)&api.DeviceGetAttribute);
     get("cuMemExportToShareableHandle", (void**)&api.MemExportToShareableHandle);
     get("cuMemImportFromShareableHandle", (void**)&api.MemImportFromShareableHandle);

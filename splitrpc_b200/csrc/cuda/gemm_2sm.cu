@@ -31,6 +31,7 @@
 #include <algorithm>
 #include <cstdlib>
 
+#include "fast_div.h"
 #include "gemm_tcgen05.h"
 #include "pdl_launch.h"
 #include "per_device.h"
@@ -39,13 +40,14 @@
 
 cudaError_t srpc_tensor_map_2d(CUtensorMap* m, const void* ptr, uint64_t inner, uint64_t outer, uint64_t row_stride_bytes,
                                uint32_t box_inner, uint32_t box_outer);
+cudaError_t srpc_tensor_map_im2col(CUtensorMap* m, const void* ptr, int n, int h, int w, int c, int r, int s, int stride, int pad,
+                                   int pixels);
 
 namespace {
 
 constexpr int BM = 128;   // rows per CTA; a pair computes 256
 constexpr int BK = 64;
 constexpr int UMMA_K = 16;
-constexpr int A_BYTES = BM * BK * 2;
 constexpr int OUT_HALF_BYTES = BM * 128;    // 128 rows x 64 bf16 columns
 constexpr int OUT_CHUNK_BYTES = 32 * 64;    // 32 rows x 32 bf16 columns
 
@@ -68,19 +70,29 @@ constexpr int OUT_CHUNK_BYTES = 32 * 64;    // 32 rows x 32 bf16 columns
 // waits for another one between reading its part of the accumulator and handing it to its TMA store.  The 256-wide tile has
 // one chunk per warp: the memory goes to a sixth operand stage.  (Peer stores use the same memory as one block of PASS_COLS
 // columns per pass.)
-template <int BN, bool TP>
+// Rows per CTA: 128, or 64 for products with few tiles (RPC).  With 64 rows the accumulator's columns lie in two halves one
+// below the other in tensor memory (lanes 0 - 63: columns 0 .. BN / 2 - 1, lanes 64 - 127: the others), a k-block takes 55 - 76 ns of
+// the tensor pipe instead of 150, and two of them share a stage, since a turn of the MMA loop takes 134 ns whatever it issues.
+template <int BN, int RPC, bool TP>
 struct Cfg {
-  static constexpr int STAGE_BYTES = A_BYTES + (BN / 2) * BK * 2;  // A rows and this CTA's half of the B rows
+  static constexpr int KPS = RPC == 64 || BN == 64 ? 2 : 1;         // k-blocks per stage
+  static constexpr int A_BYTES = RPC * BK * 2;
+  static constexpr int KB_BYTES = A_BYTES + (BN / 2) * BK * 2;      // A rows and this CTA's half of the B rows
+  static constexpr int STAGE_BYTES = KPS * KB_BYTES;
   static constexpr int PASSES = BN == 256 ? 2 : 1;
   static constexpr int PASS_COLS = BN / PASSES;
-  static constexpr int OUT_BYTES = (PASS_COLS / 64) * OUT_HALF_BYTES;
-  static constexpr int CHUNK_BUFS = OUT_BYTES / ((2 * BN) / 32) / OUT_CHUNK_BYTES;
+  static constexpr int QC = RPC == 128 ? BN : BN / 2;               // columns of a TMEM lane quarter
+  static constexpr int NCH = RPC == 128 && BN >= 128 ? 2 : 1;       // 32-column chunks per epilogue warp
+  static constexpr int EPI_WARPS = 4 * QC / (32 * NCH);
+  static constexpr int CHUNK_BUFS = BN == 256 ? 1 : 2;
+  static constexpr int OUT_BYTES = EPI_WARPS * CHUNK_BUFS * OUT_CHUNK_BYTES;
   static constexpr int STAGES = (224 * 1024 - OUT_BYTES) / STAGE_BYTES;
-  static constexpr int EPI_THREADS = 2 * BN;
+  static constexpr int EPI_THREADS = 32 * EPI_WARPS;
   static constexpr int THREADS = 64 + EPI_THREADS + 32;  // TMA, MMA, epilogue, second TMA warp
-  static constexpr int ACC_STRIDE = BN == 192 ? 256 : BN;  // TMEM columns between the two accumulators
+  static constexpr int ACC_STRIDE = QC == 192 ? 256 : QC;  // TMEM columns between the two accumulators
   static constexpr int TMEM_COLS = 2 * ACC_STRIDE;
   static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + OUT_BYTES;
+  static_assert(!TP || (RPC == 128 && OUT_BYTES == (PASS_COLS / 64) * OUT_HALF_BYTES), "peer stores stage whole passes");
 };
 
 __device__ __forceinline__ void named_bar_sync(int id, int count) {
@@ -104,33 +116,51 @@ struct PairTile {
 struct TileOrder {
   int clusters;  // clusters that compute tiles (the grid may hold copier clusters after them)
   int tiles_m2, tiles_n;
-  int group_m;   // 256-row blocks per group
-  int m_rot2;    // rotation of the 256-row blocks (tensor-parallel: which rank's rows come first)
+  int group_m;   // pair row blocks per group
+  int m_rot2;    // rotation of the pair row blocks (tensor-parallel: which rank's rows come first)
   int late_trigger;  // the next kernel starts behind this CTA's last load only (pdl_launch.h)
+  FastDiv fd_group, fd_gm;  // by group_m * tiles_n and group_m
 };
 
 // j-th tile of this cluster, grouped so that tiles in flight share A and B blocks in L2.
 __device__ __forceinline__ bool pair_tile(int j, const TileOrder& o, PairTile* out) {
   const int tile = (int)(blockIdx.x >> 1) + j * o.clusters;
   if (tile >= o.tiles_m2 * o.tiles_n) return false;
-  const int per_group = o.group_m * o.tiles_n;
-  const int g = tile / per_group, in_g = tile - g * per_group;
+  const int g = (int)fdiv(o.fd_group, (uint32_t)tile), in_g = tile - g * o.group_m * o.tiles_n;
   const int m_first = g * o.group_m;
-  const int gm = (o.tiles_m2 - m_first) < o.group_m ? (o.tiles_m2 - m_first) : o.group_m;
-  int m2 = m_first + in_g % gm + o.m_rot2;
-  if (m2 >= o.tiles_m2) m2 -= o.tiles_m2;
-  out->m2 = m2;
-  out->n = in_g / gm;
+  int m2;
+  if (o.tiles_m2 - m_first >= o.group_m) {
+    out->n = (int)fdiv(o.fd_gm, (uint32_t)in_g);
+    m2 = m_first + in_g - out->n * o.group_m;
+  } else {  // last, shorter group
+    const int gm = o.tiles_m2 - m_first;
+    out->n = in_g / gm;
+    m2 = m_first + in_g - out->n * gm;
+  }
+  m2 += o.m_rot2;
+  out->m2 = m2 >= o.tiles_m2 ? m2 - o.tiles_m2 : m2;
   return true;
 }
 
-template <int BN, bool TP>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Cfg<BN, TP>::THREADS, 1)
+// Where the rows of A come from.  GEMM: a matrix.  Convolution: row i of the product is output pixel i (rows and images in
+// sequence), its A row for filter tap (fr, fs) the pixel that the tap meets, read through an im2col tensor map; k-blocks from
+// kb_split on come from a second input (two-input 1x1 convolution) by tmap_a2.
+struct ASource {
+  int im2col, im2col2;  // of the first / second input
+  int kb_split;
+  int stride, pad, stride2;
+  FastDiv fd_img, fd_ow;      // by output pixels per image and per row
+  FastDiv fd_cblocks, fd_s;   // by channel blocks and filter columns
+};
+
+template <int BN, int RPC, bool TP>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Cfg<BN, RPC, TP>::THREADS, 1)
 gemm_2sm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
-                const __grid_constant__ CUtensorMap tmap_out, int M, int N, int K, const TileOrder order, GemmEpilogue ep,
-                uint32_t* status, const TpParams tp_in) {
-  using C = Cfg<BN, TP>;
-  constexpr int STAGE_BYTES = C::STAGE_BYTES, STAGES = C::STAGES, EPI_THREADS = C::EPI_THREADS, ACC_STRIDE = C::ACC_STRIDE;
+                const __grid_constant__ CUtensorMap tmap_out, const __grid_constant__ CUtensorMap tmap_a2, int M, int N, int K,
+                const TileOrder order, const ASource src, GemmEpilogue ep, uint32_t* status, const TpParams tp_in) {
+  using C = Cfg<BN, RPC, TP>;
+  constexpr int A_BYTES = C::A_BYTES, KB_BYTES = C::KB_BYTES, KPS = C::KPS, STAGE_BYTES = C::STAGE_BYTES, STAGES = C::STAGES;
+  constexpr int EPI_THREADS = C::EPI_THREADS, ACC_STRIDE = C::ACC_STRIDE, NCH = C::NCH;
   constexpr int PASSES = C::PASSES, PASS_COLS = C::PASS_COLS;
   extern __shared__ __align__(1024) uint8_t smem[];
   TpParams tp = tp_in;
@@ -153,7 +183,7 @@ gemm_2sm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = ptx::cluster_ctarank();
   const bool leader = rank == 0;
-  const int num_kb = (K + BK - 1) / BK;
+  const int num_kb = (K + BK - 1) / BK, num_st = (num_kb + KPS - 1) / KPS;  // k-blocks, stages of them
   // The swizzled tiles and their descriptors need a 1024-byte aligned base; the layout is the same in both CTAs, so
   // both take the same decision.
   const bool layout_ok = (ptx::smem_u32(smem) & 1023u) == 0;
@@ -173,6 +203,7 @@ gemm_2sm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
     ptx::prefetch_tmap(&tmap_a);
     ptx::prefetch_tmap(&tmap_b);
     ptx::prefetch_tmap(&tmap_out);
+    if (src.kb_split < num_kb) ptx::prefetch_tmap(&tmap_a2);
   }
   if (warp == 1) {
     ptx::tmem_alloc_2sm(&tmem_base_smem, C::TMEM_COLS);
@@ -192,16 +223,23 @@ gemm_2sm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
     // the loads alone: 240 ns in one lane's branch, 200 ns this way).
     constexpr int PRODUCERS = 2;
     const bool elected = ptx::elect_one();
-    int kb = warp == 0 ? 0 : 1, s = kb, j = 0, seq = kb;  // seq: position in this cluster's sequence of k-blocks
+    int st = warp == 0 ? 0 : 1, s = st, j = 0, seq = st;  // stage of the tile; seq: position in this cluster's sequence of stages
     uint32_t ph = 0;
     PairTile t;
     bool ok = layout_ok, first = true;
     while (ok) {
-      for (; kb >= num_kb; kb -= num_kb) j++;
+      for (; st >= num_st; st -= num_st) j++;
       ok = __all_sync(0xffffffffu, *(volatile uint32_t*)&s_error == 0);
       if (!ok || !pair_tile(j, order, &t)) break;
-      const int row0 = (t.m2 * 2 + (int)rank) * BM;
+      const int row0 = (t.m2 * 2 + (int)rank) * RPC;
       const int brow0 = t.n * BN + (int)rank * (BN / 2);
+      int img = 0, y = 0, x = 0;  // output pixel of the first row
+      if ((src.im2col | src.im2col2) && row0 < M) {  // (rows behind the last pixel: any pixels, the results are not stored)
+        img = (int)fdiv(src.fd_img, (uint32_t)row0);
+        const int in_img = row0 - img * (int)src.fd_img.d;
+        y = (int)fdiv(src.fd_ow, (uint32_t)in_img);
+        x = in_img - y * (int)src.fd_ow.d;
+      }
       if constexpr (TP) {
         if (tp.mblock_ready) {
           // Rows of a peer arrive through the copier clusters of this launch, one 128-row block at a time.
@@ -219,7 +257,7 @@ gemm_2sm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
           }
         }
       }
-      for (; kb < num_kb; kb += PRODUCERS) {
+      for (; st < num_st; st += PRODUCERS) {
         ok = ptx::mbar_wait_warp(&empty_bar[s], ph ^ 1u);
         if (!ok) {
           if (elected) atomicExch(&s_error, GEMM_ERR_PRODUCER_WAIT);
@@ -234,12 +272,30 @@ gemm_2sm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
           ptx::grid_dep_wait();
           first = false;
         }
-        if (elected) {
-          if (leader) ptx::mbar_expect_tx(&full_bar[s], 2u * STAGE_BYTES);
-          ptx::tma_load_2d_2sm(sa, &tmap_a, full_leader, kb * BK, row0);
-          ptx::tma_load_2d_2sm(sa + A_BYTES, &tmap_b, full_leader, kb * BK, brow0);
+        const int blocks = KPS == 1 || st * KPS + 1 < num_kb ? KPS : 1;
+        if (elected && leader) ptx::mbar_expect_tx(&full_bar[s], 2u * KB_BYTES * blocks);
+#pragma unroll
+        for (int b = 0; b < KPS; b++) {
+          if (b >= blocks) break;
+          const int kb = st * KPS + b;
+          if (!src.im2col && kb < src.kb_split) {
+            if (elected) ptx::tma_load_2d_2sm(sa + b * KB_BYTES, &tmap_a, full_leader, kb * BK, row0);
+          } else if (kb < src.kb_split) {
+            const int tap = (int)fdiv(src.fd_cblocks, (uint32_t)kb), cb = kb - tap * (int)src.fd_cblocks.d;
+            const int fr = (int)fdiv(src.fd_s, (uint32_t)tap), fs = tap - fr * (int)src.fd_s.d;
+            if (elected)
+              ptx::tma_load_im2col_2sm(sa + b * KB_BYTES, &tmap_a, full_leader, cb * BK, x * src.stride - src.pad, y * src.stride - src.pad,
+                                       img, (uint16_t)fs, (uint16_t)fr);
+          } else if (src.im2col2) {
+            if (elected)
+              ptx::tma_load_im2col_2sm(sa + b * KB_BYTES, &tmap_a2, full_leader, (kb - src.kb_split) * BK, x * src.stride2, y * src.stride2, img,
+                                       0, 0);
+          } else if (elected) {
+            ptx::tma_load_2d_2sm(sa + b * KB_BYTES, &tmap_a2, full_leader, (kb - src.kb_split) * BK, row0);
+          }
+          if (elected) ptx::tma_load_2d_2sm(sa + b * KB_BYTES + A_BYTES, &tmap_b, full_leader, kb * BK, brow0);
         }
-        if (j == 0 && kb == 0 && lane == 0) GEMM2_TRACE(2);
+        if (j == 0 && st == 0 && lane == 0) GEMM2_TRACE(2);
         seq += PRODUCERS;
         s += PRODUCERS;
         if (s >= STAGES) {
@@ -254,10 +310,10 @@ gemm_2sm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
     }
     if (first) ptx::cluster_wait();  // this warp had no k-block
     // The leader's MMAs signal the stages of both CTAs, and none of those signals may still be on its way when this CTA leaves:
-    // wait as for the STAGES k-blocks behind the last one (this warp's share of them).
+    // wait as for the STAGES stages behind the last one (this warp's share of them).
     if (ok) {
       const int tiles = order.tiles_m2 * order.tiles_n, first_tile = (int)(blockIdx.x >> 1);
-      const int total = first_tile < tiles ? ((tiles - first_tile + order.clusters - 1) / order.clusters) * num_kb : 0;
+      const int total = first_tile < tiles ? ((tiles - first_tile + order.clusters - 1) / order.clusters) * num_st : 0;
       for (int i = seq - total; ok && i < STAGES; i += PRODUCERS) {
         ok = ptx::mbar_wait_warp(&empty_bar[s], ph ^ 1u);
         s += PRODUCERS;
@@ -274,7 +330,7 @@ gemm_2sm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
     ptx::cluster_wait();
     if (leader) {
       const bool elected = ptx::elect_one();
-      const uint32_t idesc = ptx::umma_idesc_bf16(2 * BM, BN);
+      const uint32_t idesc = ptx::umma_idesc_bf16(2 * RPC, BN);
       const uint32_t ring_lo = ptx::umma_desc_lo(ptx::smem_u32(smem));
       constexpr uint32_t K_LO = UMMA_K * 2 / 16;
       int s = 0;
@@ -287,18 +343,22 @@ gemm_2sm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
         if (!ok) break;
         ptx::tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * ACC_STRIDE;
-        for (int kb = 0; kb < num_kb; kb++) {
+        for (int st = 0; st < num_st; st++) {
           ok = ptx::mbar_wait_warp(&full_bar[s], ph);
           if (!ok) break;
-          if (j == 0 && kb == 0 && lane == 0) GEMM2_TRACE(3);
-          if (j == 0 && kb == 8 && lane == 0) GEMM2_TRACE(10);
-          if (j == 0 && kb == 24 && lane == 0) GEMM2_TRACE(11);
+          if (j == 0 && st == 0 && lane == 0) GEMM2_TRACE(3);
+          if (j == 0 && st == 8 && lane == 0) GEMM2_TRACE(10);
+          if (j == 0 && st == 24 && lane == 0) GEMM2_TRACE(11);
           const uint32_t sa = ring_lo + (uint32_t)s * (STAGE_BYTES / 16), sb = sa + A_BYTES / 16;
           if (elected) {
 #pragma unroll
-            for (int k = 0; k < BK / UMMA_K; k++)
-              ptx::umma_bf16_2sm(d_tmem, ptx::umma_desc_join(sa + k * K_LO), ptx::umma_desc_join(sb + k * K_LO), idesc,
-                                 (kb | k) != 0 ? 1u : 0u);
+            for (int b = 0; b < KPS; b++) {
+              if (KPS > 1 && b > 0 && st * KPS + b >= num_kb) break;
+#pragma unroll
+              for (int k = 0; k < BK / UMMA_K; k++)
+                ptx::umma_bf16_2sm(d_tmem, ptx::umma_desc_join(sa + b * (KB_BYTES / 16) + k * K_LO),
+                                   ptx::umma_desc_join(sb + b * (KB_BYTES / 16) + k * K_LO), idesc, (st | b | k) != 0 ? 1u : 0u);
+            }
             ptx::umma_commit_2sm(&empty_bar[s], 3);  // frees the stage in both CTAs
           }
           if (++s == STAGES) {
@@ -323,12 +383,15 @@ gemm_2sm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
     ptx::cluster_wait();
     const int warp_q = warp & 3;
     const int cgroup = (warp - 2) >> 2;      // 0 .. EPI_THREADS/128 - 1
+    // first row and column of this warp's lane quarter in the CTA's part of the tile
+    const int q_row = RPC == 128 ? warp_q * 32 : (warp_q & 1) * 32, q_col = RPC == 128 ? 0 : (warp_q >> 1) * (BN / 2);
     const int et = threadIdx.x - 64;
     // This thread's accumulator elements: columns 8 g + fc, + 1 (g = 0 .. 3) of rows fr + 8 i (i = 0 .. 3) of the warp's 32 rows.
     const int fr = lane >> 2, fc = (lane & 3) * 2;
-    const bool vec_res = ep.residual && ((ep.ldr & 1) == 0) && (((uintptr_t)ep.residual & 3) == 0);
-    // column of chunk ch inside the tile
-    auto chunk_col = [&](int ch) { return PASSES == 2 && TP ? ch * PASS_COLS + cgroup * 32 : (cgroup * 2 + ch) * 32; };
+    // pairs of residual columns (a pair is inside the matrix or outside)
+    const bool vec_res = ep.residual && (((ep.ldr | N) & 1) == 0) && (((uintptr_t)ep.residual & 3) == 0);
+    // column of chunk ch inside the lane quarter
+    auto chunk_col = [&](int ch) { return PASSES == 2 && TP ? ch * PASS_COLS + cgroup * 32 : (cgroup * NCH + ch) * 32; };
     uint8_t* stage = stage_out + (size_t)(warp - 2) * C::CHUNK_BUFS * OUT_CHUNK_BYTES;
     // what this lane names in stmatrix: matrices 0, 1 = rows 0 .. 7, 8 .. 15 of one column group, 2, 3 = of the next one
     const int st_row = (lane & 7) + (lane & 8), st_cg = lane >> 4;
@@ -339,32 +402,36 @@ gemm_2sm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
     bool ok = layout_ok;
     for (int j = 0; ok && pair_tile(j, order, &t); j++, local++) {
       const uint32_t acc = local & 1u;
-      const int row0 = (t.m2 * 2 + (int)rank) * BM;
-      const int m0 = row0 + warp_q * 32;  // first row of this warp
-      const int n0 = t.n * BN;
+      const int m0 = (t.m2 * 2 + (int)rank) * RPC + q_row;  // first row of this warp
+      const int n0 = t.n * BN + q_col;
       // Residual and bias arrive before the accumulator is ready.
-      uint32_t rq[2][16];
+      uint32_t rq[NCH][16];
       if (vec_res) {
 #pragma unroll
-        for (int ch = 0; ch < 2; ch++) {
-          const int col0 = n0 + chunk_col(ch);
-          if (col0 + 32 <= N) {
+        for (int ch = 0; ch < NCH; ch++) {
+          const int col = n0 + chunk_col(ch) + fc;
+          const bool whole = n0 + chunk_col(ch) + 32 <= N;
 #pragma unroll
-            for (int i = 0; i < 4; i++) {
-              const int m = m0 + fr + 8 * i;
-              if (m < M) {
-                const __nv_bfloat16* rp = ep.residual + (size_t)m * ep.ldr + col0 + fc;
+          for (int i = 0; i < 4; i++) {
+            const int m = m0 + fr + 8 * i;
+            if (m < M) {
+              const __nv_bfloat16* rp = ep.residual + (size_t)m * ep.ldr + col;
+              if (whole) {
 #pragma unroll
                 for (int g = 0; g < 4; g++) rq[ch][i * 4 + g] = *reinterpret_cast<const uint32_t*>(rp + g * 8);
+              } else {
+#pragma unroll
+                for (int g = 0; g < 4; g++)
+                  if (col + g * 8 < N) rq[ch][i * 4 + g] = *reinterpret_cast<const uint32_t*>(rp + g * 8);
               }
             }
           }
         }
       }
-      float2 b2[2][4];
+      float2 b2[NCH][4];
       if (ep.bias) {
 #pragma unroll
-        for (int ch = 0; ch < 2; ch++)
+        for (int ch = 0; ch < NCH; ch++)
 #pragma unroll
           for (int g = 0; g < 4; g++) {
             const int col = n0 + chunk_col(ch) + g * 8 + fc;
@@ -382,15 +449,15 @@ gemm_2sm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
       ptx::tc_fence_after();
       if (j == 0 && et == 0) GEMM2_TRACE(5);
 #pragma unroll
-      for (int ch = 0; ch < 2; ch++) {
-        const int c = chunk_col(ch);  // column inside the tile
+      for (int ch = 0; ch < NCH; ch++) {
+        const int c = chunk_col(ch);  // column inside the lane quarter
         const int col0 = n0 + c;
         const uint32_t t_addr = tmem_base + acc * ACC_STRIDE + ((uint32_t)(warp_q * 32) << 16) + (uint32_t)c;
         uint32_t r[32];
         ptx::tmem_ld_16x256b_x4(t_addr, r);
         ptx::tmem_ld_16x256b_x4(t_addr + (16u << 16), r + 16);
         ptx::tmem_ld_wait();
-        if (ch == 1) {  // last read: hand the accumulator back to the leader's MMA warp
+        if (ch == NCH - 1) {  // last read: hand the accumulator back to the leader's MMA warp
           ptx::tc_fence_before();
           __syncwarp();
           if (lane == 0) ptx::mbar_arrive_cluster(ptx::mapa_shared(ptx::smem_u32(&tmem_empty_bar[acc]), 0));
@@ -407,7 +474,7 @@ gemm_2sm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
 #pragma unroll
           for (int q = 0; q < 16; q++) v[q] = __fadd2_rn(v[q], b2[ch][q & 3]);
         }
-        if (vec_res && col0 + 32 <= N) {
+        if (vec_res) {
 #pragma unroll
           for (int q = 0; q < 16; q++) v[q] = __fadd2_rn(v[q], __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&rq[ch][q])));
         } else if (ep.residual) {
@@ -488,7 +555,7 @@ gemm_2sm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
           }
         }
         // A chunk is a block of 32 rows of 64 bytes under the 64-byte swizzle; its last store must have been read.
-        uint8_t* block = stage + (C::CHUNK_BUFS == 2 ? ch * OUT_CHUNK_BYTES : 0);
+        uint8_t* block = stage + (C::CHUNK_BUFS == 2 ? (NCH == 2 ? ch : (int)(local & 1u)) * OUT_CHUNK_BYTES : 0);
         if (lane == 0) ptx::bulk_wait_read<C::CHUNK_BUFS - 1>();
         __syncwarp();
         put(block, 64, 0, [](int rr) { return (rr >> 1) & 3; });
@@ -498,7 +565,7 @@ gemm_2sm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
           if (col0 < N && m0 < M) ptx::tma_store_2d(&tmap_out, block, col0, m0);
           ptx::bulk_commit();
         }
-        if (j == 0 && et == 0 && ch == 1) GEMM2_TRACE(6);
+        if (j == 0 && et == 0 && ch == NCH - 1) GEMM2_TRACE(6);
       }
     }
     if (et == 0) GEMM2_TRACE(7);
@@ -523,14 +590,14 @@ gemm_2sm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
 
 
 // Clusters of two CTAs that can be resident at once (queried once per instantiation and device).
-template <int BN, bool TP>
+template <int BN, int RPC, bool TP>
 cudaError_t max_clusters_2sm(int* out) {
-  using C = Cfg<BN, TP>;
+  using C = Cfg<BN, RPC, TP>;
   static std::atomic<int> per_device[64];
   const int dev = PerDeviceFlag::current();
   int max_clusters = per_device[dev].load(std::memory_order_acquire);
   if (!max_clusters) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_2sm_kernel<BN, TP>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES);
+    cudaError_t e = cudaFuncSetAttribute(gemm_2sm_kernel<BN, RPC, TP>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2 * 74);
@@ -544,7 +611,7 @@ cudaError_t max_clusters_2sm(int* out) {
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
     int n = 0;
-    e = cudaOccupancyMaxActiveClusters(&n, gemm_2sm_kernel<BN, TP>, &cfg);
+    e = cudaOccupancyMaxActiveClusters(&n, gemm_2sm_kernel<BN, RPC, TP>, &cfg);
     if (e != cudaSuccess) return e;
     if (n < 1) return cudaErrorInvalidConfiguration;
     max_clusters = n;
@@ -554,39 +621,101 @@ cudaError_t max_clusters_2sm(int* out) {
   return cudaSuccess;
 }
 
-template <int BN>
-cudaError_t launch_2sm(const void* A, int lda, const void* B, int ldb, int M, int N, int K, const GemmEpilogue& ep,
-                       uint32_t* status, cudaStream_t stream) {
-  using C = Cfg<BN, false>;
+// A matrix of rows as the only source.
+ASource matrix_source(int num_kb) {
+  ASource src = {};
+  src.kb_split = num_kb;
+  src.stride = src.stride2 = 1;
+  src.fd_img = src.fd_ow = src.fd_cblocks = src.fd_s = make_fastdiv(1);
+  return src;
+}
+
+void order_tiles(TileOrder* o, int M, int N, int rows, int bn, int max_clusters, int group_m) {
+  o->tiles_m2 = (M + rows - 1) / rows;
+  o->tiles_n = (N + bn - 1) / bn;
+  o->clusters = std::min(o->tiles_m2 * o->tiles_n, max_clusters);
+  o->group_m = group_m;
+  o->fd_group = make_fastdiv((uint32_t)(group_m * o->tiles_n));
+  o->fd_gm = make_fastdiv((uint32_t)group_m);
+}
+
+// What a launch reads its A rows from: makes the tensor maps for tiles of `rows_per_cta` rows per CTA.
+struct AInput {
+  const void* a = nullptr;
+  int lda = 0;
+  const ConvShape* cs = nullptr;
+};
+cudaError_t a_maps(const AInput& in, int M, int K, int rows_per_cta, ASource* src, CUtensorMap* ta, CUtensorMap* ta2) {
+  *src = matrix_source((K + BK - 1) / BK);
+  if (!in.cs) {
+    cudaError_t e = srpc_tensor_map_2d(ta, in.a, (uint64_t)K, (uint64_t)M, (uint64_t)in.lda * 2, BK, (uint32_t)rows_per_cta);
+    *ta2 = *ta;
+    return e;
+  }
+  const ConvShape& cs = *in.cs;
+  src->kb_split = cs.r * cs.s * cs.cin / BK;
+  src->im2col = cs.r != 1 || cs.s != 1 || cs.stride != 1 || cs.pad != 0;
+  src->stride = cs.stride;
+  src->pad = cs.pad;
+  src->fd_img = make_fastdiv((uint32_t)(cs.oh * cs.ow));
+  src->fd_ow = make_fastdiv((uint32_t)cs.ow);
+  src->fd_cblocks = make_fastdiv((uint32_t)(cs.cin / BK));
+  src->fd_s = make_fastdiv((uint32_t)cs.s);
+  cudaError_t e = src->im2col ? srpc_tensor_map_im2col(ta, in.a, cs.n, cs.h, cs.w, cs.cin, cs.r, cs.s, cs.stride, cs.pad, rows_per_cta)
+                              : srpc_tensor_map_2d(ta, in.a, (uint64_t)cs.cin, (uint64_t)M, (uint64_t)cs.cin * 2, BK, (uint32_t)rows_per_cta);
+  *ta2 = *ta;
+  if (e != cudaSuccess || !cs.in2) return e;
+  src->im2col2 = cs.stride2 != 1;
+  src->stride2 = cs.stride2;
+  return src->im2col2 ? srpc_tensor_map_im2col(ta2, cs.in2, cs.n, cs.h2, cs.w2, cs.cin2, 1, 1, cs.stride2, 0, rows_per_cta)
+                      : srpc_tensor_map_2d(ta2, cs.in2, (uint64_t)cs.cin2, (uint64_t)M, (uint64_t)cs.cin2 * 2, BK, (uint32_t)rows_per_cta);
+}
+
+template <int BN, int RPC>
+cudaError_t launch_2sm(const AInput& in, const void* B, int ldb, int M, int N, int K, const GemmEpilogue& ep, uint32_t* status,
+                       cudaStream_t stream) {
+  using C = Cfg<BN, RPC, false>;
   int max_clusters = 0;
-  cudaError_t e = max_clusters_2sm<BN, false>(&max_clusters);
+  cudaError_t e = max_clusters_2sm<BN, RPC, false>(&max_clusters);
   if (e != cudaSuccess) return e;
-  CUtensorMap ta, tb, to;
-  e = srpc_tensor_map_2d(&ta, A, (uint64_t)K, (uint64_t)M, (uint64_t)lda * 2, BK, BM);
+  CUtensorMap ta, tb, to, ta2;
+  ASource src;
+  e = a_maps(in, M, K, RPC, &src, &ta, &ta2);
   if (e != cudaSuccess) return e;
   e = srpc_tensor_map_2d(&tb, B, (uint64_t)K, (uint64_t)N, (uint64_t)ldb * 2, BK, BN / 2);
   if (e != cudaSuccess) return e;
   e = srpc_tensor_map_2d(&to, ep.out, (uint64_t)N, (uint64_t)M, (uint64_t)ep.ldo * 2, 32, 32);
   if (e != cudaSuccess) return e;
   TileOrder o;
-  o.tiles_m2 = (M + 2 * BM - 1) / (2 * BM);
-  o.tiles_n = (N + BN - 1) / BN;
-  o.clusters = std::min(o.tiles_m2 * o.tiles_n, std::min(max_clusters, srpc_gemm_grid_sms() / 2));
-  o.group_m = 4;
+  order_tiles(&o, M, N, 2 * RPC, BN, std::min(max_clusters, srpc_gemm_grid_sms() / 2), 4);
   o.m_rot2 = 0;
   o.late_trigger = srpc_gemm_reserved_sms() > 0;
-  return launch_pdl(gemm_2sm_kernel<BN, false>, dim3(2 * o.clusters), dim3(C::THREADS), C::SMEM_BYTES, stream, ta, tb, to, M, N, K,
-                    o, ep, status, TpParams{});
+  return launch_pdl(gemm_2sm_kernel<BN, RPC, false>, dim3(2 * o.clusters), dim3(C::THREADS), C::SMEM_BYTES, stream, ta, tb, to, ta2, M,
+                    N, K, o, src, ep, status, TpParams{});
+}
+
+cudaError_t launch_shape(int bn, int rows, const AInput& in, const void* B, int ldb, int M, int N, int K, const GemmEpilogue& ep,
+                         uint32_t* status, cudaStream_t stream) {
+  if (rows == 256) {
+    if (bn == 256) return launch_2sm<256, 128>(in, B, ldb, M, N, K, ep, status, stream);
+    if (bn == 192) return launch_2sm<192, 128>(in, B, ldb, M, N, K, ep, status, stream);
+    if (bn == 128) return launch_2sm<128, 128>(in, B, ldb, M, N, K, ep, status, stream);
+    if (bn == 64) return launch_2sm<64, 128>(in, B, ldb, M, N, K, ep, status, stream);
+  } else if (rows == 128) {
+    if (bn == 128) return launch_2sm<128, 64>(in, B, ldb, M, N, K, ep, status, stream);
+    if (bn == 64) return launch_2sm<64, 64>(in, B, ldb, M, N, K, ep, status, stream);
+  }
+  return cudaErrorInvalidValue;
 }
 
 // Tensor-parallel launch: `tp` arrives with mblocks_per_rank / mblock_bytes filled in and an even n_copy.
 template <int BN>
 cudaError_t launch_2sm_tp(const void* A, int lda, const void* B, int ldb, int M, int N, int K, const GemmEpilogue& ep,
                           TpParams tp, uint32_t* status, cudaStream_t stream) {
-  using C = Cfg<BN, true>;
+  using C = Cfg<BN, BM, true>;
   static_assert(C::SMEM_BYTES >= tpdev::COPY_SLOTS * tpdev::COPY_CHUNK, "the copier's ring lives in the operand stages");
   int max_clusters = 0;
-  cudaError_t e = max_clusters_2sm<BN, true>(&max_clusters);
+  cudaError_t e = max_clusters_2sm<BN, BM, true>(&max_clusters);
   if (e != cudaSuccess) return e;
   max_clusters = std::min(max_clusters, srpc_gemm_grid_sms() / 2);
   const int copy_clusters = tp.n_copy / 2;
@@ -602,19 +731,18 @@ cudaError_t launch_2sm_tp(const void* A, int lda, const void* B, int ldb, int M,
   } else {
     to = ta;  // never used: the epilogue stores to the owners' slots
   }
-  TileOrder o;
-  o.late_trigger = 0;
-  o.tiles_m2 = M / (2 * BM);
-  o.tiles_n = (N + BN - 1) / BN;
-  o.clusters = std::min(o.tiles_m2 * o.tiles_n, max_clusters - copy_clusters);
   const int m2_per_rank = tp.mblocks_per_rank / 2;
-  o.group_m = 1;
+  int group_m = 1;
   for (int g = 2; g <= 4; g++)
-    if (m2_per_rank % g == 0) o.group_m = g;  // groups never straddle two ranks' rows
+    if (m2_per_rank % g == 0) group_m = g;  // groups never straddle two ranks' rows
+  TileOrder o;
+  order_tiles(&o, M, N, 2 * BM, BN, max_clusters - copy_clusters, group_m);
+  o.late_trigger = 0;
   // all-gather: own rows first (they are here already); reduce-scatter: own rows last (the peers' cross NVLink)
   o.m_rot2 = (tp.rs ? (tp.rank + 1) % tp.tp : tp.rank) * m2_per_rank;
   tp.tiles_per_owner = tp.mblocks_per_rank * o.tiles_n;
-  gemm_2sm_kernel<BN, true><<<2 * (o.clusters + copy_clusters), C::THREADS, C::SMEM_BYTES, stream>>>(ta, tb, to, M, N, K, o, ep, status, tp);
+  gemm_2sm_kernel<BN, BM, true><<<2 * (o.clusters + copy_clusters), C::THREADS, C::SMEM_BYTES, stream>>>(
+      ta, tb, to, ta, M, N, K, o, matrix_source((K + BK - 1) / BK), ep, status, tp);
   return cudaGetLastError();
 }
 
@@ -632,22 +760,41 @@ int srpc_gemm2_trace_read(unsigned long long* out, int n) {
 #endif
 }
 
-bool srpc_gemm_2sm_eligible(int M, int N, int K, const GemmEpilogue& ep) {
+bool srpc_gemm_2sm_eligible(int K, const GemmEpilogue& ep) {
   static const int allow = [] { const char* e = getenv("SPLITRPC_GEMM_2SM"); return e ? atoi(e) : 1; }();
   if (!allow || ep.out_fp32 || (ep.ldo % 8) || ((uintptr_t)ep.out & 15)) return false;
   if (ep.bias && ((uintptr_t)ep.bias & 15)) return false;
-  return M >= 256 && N >= 128 && K >= 64;
+  return K >= 64;
 }
 
-cudaError_t srpc_gemm_bf16_2sm(const void* A, int lda, const void* B, int ldb, int M, int N, int K, int bn, const GemmEpilogue& ep,
-                               uint32_t* status, cudaStream_t stream) {
+cudaError_t srpc_gemm_bf16_2sm(const void* A, int lda, const void* B, int ldb, int M, int N, int K, int bn, int rows,
+                               const GemmEpilogue& ep, uint32_t* status, cudaStream_t stream) {
   if (M <= 0 || N <= 0 || K <= 0) return cudaErrorInvalidValue;
   if ((lda % 8) || (ldb % 8) || (K % 8) || ((uintptr_t)A & 15) || ((uintptr_t)B & 15)) return cudaErrorInvalidValue;
-  if (!srpc_gemm_2sm_eligible(M, N, K, ep)) return cudaErrorInvalidValue;
-  if (bn == 256) return launch_2sm<256>(A, lda, B, ldb, M, N, K, ep, status, stream);
-  if (bn == 192) return launch_2sm<192>(A, lda, B, ldb, M, N, K, ep, status, stream);
-  if (bn == 128) return launch_2sm<128>(A, lda, B, ldb, M, N, K, ep, status, stream);
-  return cudaErrorInvalidValue;
+  if (!srpc_gemm_2sm_eligible(K, ep)) return cudaErrorInvalidValue;
+  AInput in;
+  in.a = A;
+  in.lda = lda;
+  return launch_shape(bn, rows, in, B, ldb, M, N, K, ep, status, stream);
+}
+
+// Dense inputs only: no window that overlaps its neighbours, no request ring; corners and steps within what an im2col tensor map holds.
+bool srpc_conv_2sm_eligible(const ConvShape& cs, const GemmEpilogue& ep) {
+  if (cs.in_stub || cs.in_pix_stride || cs.in_row_stride || cs.in_img_stride || (cs.cin % BK) || (cs.in2 && (cs.cin2 % BK))) return false;
+  if (cs.stride < 1 || cs.stride > 8 || cs.pad < 0 || cs.pad > 127 || cs.r < 1 || cs.s < 1 || cs.r > 128 || cs.s > 128) return false;
+  if (cs.in2 && (cs.stride2 < 1 || cs.stride2 > 8)) return false;
+  if (cs.oh != (cs.h + 2 * cs.pad - cs.r) / cs.stride + 1 || cs.ow != (cs.w + 2 * cs.pad - cs.s) / cs.stride + 1) return false;
+  return srpc_gemm_2sm_eligible(cs.r * cs.s * cs.cin, ep);
+}
+
+cudaError_t srpc_conv_bf16_2sm(const void* input, const void* weight, const ConvShape& cs, int bn, int rows, const GemmEpilogue& ep,
+                               uint32_t* status, cudaStream_t stream) {
+  if (!srpc_conv_2sm_eligible(cs, ep) || cs.n <= 0 || cs.cout <= 0) return cudaErrorInvalidValue;
+  AInput in;
+  in.a = input;
+  in.cs = &cs;
+  const int K = cs.r * cs.s * cs.cin + (cs.in2 ? cs.cin2 : 0);
+  return launch_shape(bn, rows, in, weight, K, cs.n * cs.oh * cs.ow, cs.cout, K, ep, status, stream);
 }
 
 // Tensor-parallel entry point (see gemm_tp.h).  Takes the shapes where a rank's rows are whole 256-row pair tiles.

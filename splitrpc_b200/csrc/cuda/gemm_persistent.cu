@@ -32,6 +32,7 @@
 #include <mutex>
 #include <unordered_map>
 
+#include "fast_div.h"
 #include "gemm_tcgen05.h"
 #include "pdl_launch.h"
 #include "ptx.cuh"
@@ -63,22 +64,6 @@ struct Threads {
   static constexpr int EPI = BN == 256 ? 512 : (BN == 192 ? 384 : (BN == 128 ? SRPC_EPI128 : 256));
   static constexpr int TOTAL = 64 + EPI + 64;  // + the store warp, the second producer warp
 };
-
-// Division by a launch-time constant as multiply-high + shift (dividends below 2^24): every thread of every role
-// decodes a tile index per tile, and with small tiles the hardware divisions were a quarter of a microsecond per tile.
-struct FastDiv {
-  uint32_t mul, shr, d;
-};
-static inline FastDiv make_fastdiv(uint32_t d) {
-  FastDiv f;
-  f.d = d ? d : 1;
-  uint32_t l = 0;
-  while ((1u << l) < f.d) l++;
-  f.shr = l;
-  f.mul = (uint32_t)((((uint64_t)1 << 32) * (((uint64_t)1 << l) - f.d)) / f.d + 1);
-  return f;
-}
-__device__ __forceinline__ uint32_t fdiv(const FastDiv& f, uint32_t n) { return (__umulhi(f.mul, n) + n) >> f.shr; }
 
 struct TileParams {
   int mode;          // 0 GEMM, 1 convolution
@@ -719,10 +704,25 @@ struct MapKeyHash {
 
 // Tensor maps are cached: encoding costs microseconds and the same layers run
 // for every batch.
-cudaError_t get_map(CUtensorMap* out, const void* ptr, int rank, const uint64_t* dims, const uint64_t* strides_bytes,
-                    const uint32_t* box, const uint32_t* estr, CUtensorMapSwizzle swizzle = CU_TENSOR_MAP_SWIZZLE_128B) {
+template <typename Encode>
+cudaError_t cached_map(CUtensorMap* out, const MapKey& k, Encode encode) {
   static std::mutex mu;
   static std::unordered_map<MapKey, CUtensorMap, MapKeyHash> cache;
+  std::lock_guard<std::mutex> g(mu);
+  auto it = cache.find(k);
+  if (it != cache.end()) {
+    *out = it->second;
+    return cudaSuccess;
+  }
+  const cudaError_t e = encode(out);
+  if (e != cudaSuccess) return e;
+  if (cache.size() > 4096) cache.clear();
+  cache.emplace(k, *out);
+  return cudaSuccess;
+}
+
+cudaError_t get_map(CUtensorMap* out, const void* ptr, int rank, const uint64_t* dims, const uint64_t* strides_bytes,
+                    const uint32_t* box, const uint32_t* estr, CUtensorMapSwizzle swizzle = CU_TENSOR_MAP_SWIZZLE_128B) {
   MapKey k;
   std::memset(&k, 0, sizeof(k));
   k.ptr = ptr;
@@ -734,29 +734,22 @@ cudaError_t get_map(CUtensorMap* out, const void* ptr, int rank, const uint64_t*
     k.es[i] = estr[i];
     if (i + 1 < rank) k.st[i] = strides_bytes[i];
   }
-  std::lock_guard<std::mutex> g(mu);
-  auto it = cache.find(k);
-  if (it != cache.end()) {
-    *out = it->second;
-    return cudaSuccess;
-  }
-  const SrpcDriverApi* d = srpc_driver_api();
-  if (!d->TensorMapEncodeTiled) return cudaErrorNotSupported;
-  cuuint64_t gd[5], gs[4];
-  cuuint32_t bx[5], es[5];
-  for (int i = 0; i < rank; i++) {
-    gd[i] = dims[i];
-    bx[i] = box[i];
-    es[i] = estr[i];
-    if (i + 1 < rank) gs[i] = strides_bytes[i];
-  }
-  CUresult r = d->TensorMapEncodeTiled(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, (cuuint32_t)rank, const_cast<void*>(ptr), gd, gs,
-                                       bx, es, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
-                                       CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) return cudaErrorInvalidValue;
-  if (cache.size() > 4096) cache.clear();
-  cache.emplace(k, *out);
-  return cudaSuccess;
+  return cached_map(out, k, [&](CUtensorMap* m) {
+    const SrpcDriverApi* d = srpc_driver_api();
+    if (!d->TensorMapEncodeTiled) return cudaErrorNotSupported;
+    cuuint64_t gd[5], gs[4];
+    cuuint32_t bx[5], es[5];
+    for (int i = 0; i < rank; i++) {
+      gd[i] = dims[i];
+      bx[i] = box[i];
+      es[i] = estr[i];
+      if (i + 1 < rank) gs[i] = strides_bytes[i];
+    }
+    const CUresult r = d->TensorMapEncodeTiled(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, (cuuint32_t)rank, const_cast<void*>(ptr), gd, gs,
+                                               bx, es, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                                               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
+  });
 }
 
 // Rows of the box are 128 bytes of shared memory under the 128-byte swizzle and 64 bytes under the 64-byte one.
@@ -858,6 +851,32 @@ cudaError_t srpc_tensor_map_2d(CUtensorMap* m, const void* ptr, uint64_t inner, 
   return map_2d(m, ptr, inner, outer, row_stride_bytes, box_inner, box_outer);
 }
 
+// Dense NHWC tensor read by an r x s filter: `pixels` output pixels x 64 channels per load, zero outside the image.
+cudaError_t srpc_tensor_map_im2col(CUtensorMap* m, const void* ptr, int n, int h, int w, int c, int r, int s, int stride, int pad,
+                                   int pixels) {
+  MapKey k;
+  std::memset(&k, 0, sizeof(k));
+  k.ptr = ptr;
+  k.rank = 4 | 0x100;  // no tiled map has this rank
+  const uint64_t dims[4] = {(uint64_t)c, (uint64_t)w, (uint64_t)h, (uint64_t)n};
+  for (int i = 0; i < 4; i++) k.d[i] = dims[i];
+  const uint32_t shape[5] = {(uint32_t)r, (uint32_t)s, (uint32_t)stride, (uint32_t)pad, (uint32_t)pixels};
+  for (int i = 0; i < 5; i++) k.box[i] = shape[i];
+  return cached_map(m, k, [&](CUtensorMap* out) {
+    const SrpcDriverApi* d = srpc_driver_api();
+    if (!d->TensorMapEncodeIm2col) return cudaErrorNotSupported;
+    const cuuint64_t gd[4] = {dims[0], dims[1], dims[2], dims[3]};
+    const cuuint64_t gs[3] = {(cuuint64_t)c * 2, (cuuint64_t)w * c * 2, (cuuint64_t)h * w * c * 2};
+    // first and last filter position over the image, as offsets from its corners (w, then h)
+    const int lower[2] = {-pad, -pad}, upper[2] = {pad - (s - 1), pad - (r - 1)};
+    const cuuint32_t es[4] = {1, (cuuint32_t)stride, (cuuint32_t)stride, 1};
+    const CUresult e = d->TensorMapEncodeIm2col(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(ptr), gd, gs, lower, upper, BK,
+                                                (cuuint32_t)pixels, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                                                CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return e == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
+  });
+}
+
 int srpc_gemm_trace_read(unsigned long long* out, int n) {
 #ifdef SRPC_GEMM_TRACE
   if (n > 16) n = 16;
@@ -870,51 +889,47 @@ int srpc_gemm_trace_read(unsigned long long* out, int n) {
 #endif
 }
 
-// Tile shape.  Narrow outputs take 64 columns.  Otherwise the shape with the lowest estimated time wins: rounds of
-// tiles over the SMs (or SM pairs) x (k-blocks x time per k-block + hand-over).  The per-k-block times are measured with
-// every SM busy (rounds x k-blocks of 4096 .. 6144 x 768 .. 4096 products with K = 768 .. 4096): the one-SM tiles are bound by
-// operand delivery (32 - 48 KB per k-block and SM), the two-SM tiles (256 rows per SM pair, gemm_2sm.cu) take a third less
-// of it.  With these figures 6144 x 1024 x 4096 takes pairs of 256 x 192 tiles (50.3 -> 42.6 us), 6144 x 1024 x 1024 too
-// (22.3 -> 17.9 us), 1024 x 768 x 3072 takes 64 columns (16.4 -> 15.1 us).  Below eight k-blocks memory and the epilogue
-// decide; the older figures pick the right shapes there (pairs are no candidates).  Returns the width; *two_sm says which kernel.
-static int pick_tile(int M, int N, int num_kb, bool bf16_out, bool allow_two_sm, bool* two_sm) {
+// Tile shape: the one with the lowest estimated time, a launch plus rounds of tiles over the SMs (or SM pairs) x (k-blocks x time
+// per k-block + hand-over, more with a residual or GELU).  The figures are a fit to 200 products and convolutions of 49 .. 200704 rows,
+// 8 .. 8192 columns and K 64 .. 8192, each measured with every shape; the choice is within 0.5 % of the best one on average, 9 % at
+// worst.  Pairs win nearly everywhere (us, one-SM against pairs): 128 x 768 x 3072 14.2 against 8.1, 512 x 768 x 768 6.8 and 4.4,
+// 4096 x 768 x 768 10.8 and 7.6; the one-SM kernel is left with fp32 and unaligned outputs and with the shapes that stream a
+// residual (srpc_gemm_bf16_v2).  Every shape sums a result's products in the same order, so that a row does not depend on the
+// batch that it is computed in.
+struct TileShape {
+  int bn, rows;  // columns; rows of a CTA pair, 0: the one-SM kernel (128 rows)
+};
+static TileShape pick_tile(int M, int N, int num_kb, const GemmEpilogue& ep, bool one_sm, bool pairs) {
   static const int allow256 = [] { const char* e = getenv("SPLITRPC_GEMM_BN256"); return e ? atoi(e) : 1; }();
   static const int allow192 = [] { const char* e = getenv("SPLITRPC_GEMM_BN192"); return e ? atoi(e) : 1; }();
-  *two_sm = false;
   struct Cand {
-    int bn, rows, units;
-    double t_kb, t_short;  // microseconds per 64-deep k-block; the same for the choice among short k loops
-    bool pair;
+    int bn, rows;
+    double fixed, kb, round, res, gelu;  // microseconds per launch, k-block, tile; more per tile with a residual, with GELU
   };
+  static const Cand cands[10] = {
+      {256, 256, 3.26, 0.269, 1.34, 2.23, 1.53}, {192, 256, 2.97, 0.208, 1.14, 0.86, 0.95}, {128, 256, 2.62, 0.160, 1.07, 0.67, 0.60},
+      {64, 256, 2.69, 0.132, 0.67, 0.40, 0.40},  {128, 128, 2.52, 0.123, 0.64, 0.33, 0.29}, {64, 128, 2.43, 0.116, 0.52, 0.17, 0.10},
+      {256, 0, 4.30, 0.309, 1.69, 2.89, 1.38},   {192, 0, 4.13, 0.231, 1.30, 2.19, 1.01},   {128, 0, 3.82, 0.213, 0.88, 1.39, 0.61},
+      {64, 0, 3.49, 0.192, 0.72, 0.61, 0.36}};
   const int sms = num_sms();
-  const Cand cands[7] = {{256, 256, sms / 2, 0.35, 0.35, true},  {192, 256, sms / 2, 0.29, 0.29, true}, {128, 256, sms / 2, 0.23, 0.23, true},
-                         {256, 128, sms, 0.43, 0.49, false},     {192, 128, sms, 0.335, 0.37, false},   {128, 128, sms, 0.25, 0.27, false},
-                         {64, 128, sms, 0.21, 0.27, false}};
-  int best = N <= 64 ? 64 : 128;
+  const bool bf16_out = ep.out_fp32 == 0;
+  TileShape best = {N <= 64 ? 64 : 128, 0};
   double best_cost = 1e30;
   for (const Cand& c : cands) {
-    if (N <= 64 && c.bn != 64) continue;
-    if (N > 64 && c.bn == 64 && num_kb < 8) continue;
-    // pairs only where the k loop dominates: short-K shapes are bound by memory and keep the B-stationary schedule
-    if (c.pair && !(allow_two_sm && M >= 256 && num_kb >= 8)) continue;
-    if (c.bn == 256 && !(allow256 && bf16_out && N >= 256 && ((N % 256) == 0 || N >= 1024))) continue;
-    if (c.bn == 192 && !(allow192 && bf16_out && N >= 192 && ((N % 192) == 0 || N >= 1024))) continue;
-    if (c.pair && c.bn == 128 && (N % 128) != 0 && N < 1024) continue;
-    const long tiles = (long)((M + c.rows - 1) / c.rows) * ((N + c.bn - 1) / c.bn);
-    const long rounds = (tiles + c.units - 1) / c.units;
-    const double cost = (double)rounds * (num_kb * (num_kb >= 8 ? c.t_kb : c.t_short) + 0.25) + (c.pair ? 0.8 : 0.0);  // pairs: cluster set-up
-    if (cost < best_cost * 0.98) {  // near-ties go to the candidate listed first
+    if (c.rows ? !pairs : !one_sm) continue;
+    if (c.bn > 64 && N <= c.bn - 64) continue;  // more than a third of the tile would be empty
+    if (c.bn == 256 && !(allow256 && bf16_out)) continue;
+    if (c.bn == 192 && !(allow192 && bf16_out)) continue;
+    const int rows = c.rows ? c.rows : BM, units = c.rows ? sms / 2 : sms;
+    const long tiles = (long)((M + rows - 1) / rows) * ((N + c.bn - 1) / c.bn);
+    const long rounds = (tiles + units - 1) / units;
+    const double cost = c.fixed + (double)rounds * (num_kb * c.kb + c.round + (ep.residual ? c.res : 0) + (ep.act == GEMM_ACT_GELU ? c.gelu : 0));
+    if (cost < best_cost) {
       best_cost = cost;
-      best = c.bn;
-      *two_sm = c.pair;
+      best = {c.bn, c.rows};
     }
   }
   return best;
-}
-
-static int pick_bn(int N, int tiles_m, int num_kb, bool bf16_out) {
-  bool two_sm;
-  return pick_tile(tiles_m * BM, N, num_kb, bf16_out, false, &two_sm);
 }
 
 cudaError_t srpc_gemm_bf16_v2(const void* A, int lda, const void* B, int ldb, int M, int N, int K, const GemmEpilogue& ep,
@@ -925,15 +940,19 @@ cudaError_t srpc_gemm_bf16_v2(const void* A, int lda, const void* B, int ldb, in
   int use_tma_store = (!ep.out_fp32 && (ep.ldo % 8) == 0 && ((uintptr_t)ep.out & 15) == 0) ? 1 : 0;
   static const int allow_res_tma = [] { const char* e = getenv("SPLITRPC_GEMM_RES_TMA"); return e ? atoi(e) : 1; }();
   static const int res_tma_max_k = [] { const char* e = getenv("SPLITRPC_GEMM_RES_TMA_MAXK"); return e ? atoi(e) : 512; }();
-  // Short-K shapes are bound by memory and gain from the prefetched residual; with a long K the plain residual loads of
-  // the epilogue hide behind the next tile's MMAs and the tile width matters more.
+  // Short-K shapes of many tiles are bound by memory and gain from the residual that TMA prefetches tiles ahead (us, against the
+  // best pair tiles: 200704 x 256 x 64 42 and 63, 12544 x 1024 x 256 14.2 and 15.4; 62720 x 256 x 64 13.7 and 20).  Fewer than four
+  // rounds are bound by the launch and the first and last tile (3136 x 2048 x 512 12.7 and 10.4, 980 x 1024 x 256 5.8 and 4.2), and
+  // with a long K the plain residual loads of the epilogue hide behind the next tile's MMAs.
+  const int rt_bn = N <= 64 ? 64 : 128;
+  const bool many_tiles = (long)((M + BM - 1) / BM) * ((N + rt_bn - 1) / rt_bn) > 3l * num_sms();
+  const bool pairs = srpc_gemm_2sm_eligible(K, ep);
   const bool res_tma = allow_res_tma && use_tma_store == 1 && ep.residual && (ep.ldr % 8) == 0 &&
-                       ((uintptr_t)ep.residual & 15) == 0 && K <= res_tma_max_k;
+                       ((uintptr_t)ep.residual & 15) == 0 && K <= res_tma_max_k && (many_tiles || !pairs);
   // The residual ring lives in the output staging buffers, which the wide tiles have only one of.
-  bool two_sm = false;
-  const int bn = res_tma ? (N <= 64 ? 64 : 128)
-                         : pick_tile(M, N, (K + BK - 1) / BK, ep.out_fp32 == 0, srpc_gemm_2sm_eligible(M, N, K, ep), &two_sm);
-  if (two_sm) return srpc_gemm_bf16_2sm(A, lda, B, ldb, M, N, K, bn, ep, status, stream);
+  const TileShape ts = res_tma ? TileShape{rt_bn, 0} : pick_tile(M, N, (K + BK - 1) / BK, ep, true, pairs);
+  const int bn = ts.bn;
+  if (ts.rows) return srpc_gemm_bf16_2sm(A, lda, B, ldb, M, N, K, bn, ts.rows, ep, status, stream);
   TileParams p{};
   p.mode = 0;
   p.res_tma = res_tma ? 1 : 0;
@@ -1001,6 +1020,19 @@ cudaError_t srpc_conv_bf16_tma(const void* in, const void* weight, const ConvSha
       return cudaErrorInvalidValue;
     return srpc_stem_conv(in, weight, cs, ep, status, stream);
   }
+  GemmEpilogue ep2 = ep;
+  ep2.ldo = cs.cout;
+  if (ep2.residual) ep2.ldr = cs.cout;
+  if (cs.in2) {
+    // out = act(W1 . in + W2 . in2(strided) + bias): the weight rows hold [W1 | W2]
+    if (cs.r != 1 || cs.s != 1 || cs.pad != 0 || cs.in_stub || cs.cin2 % BK || cs.stride2 < 1 || ((uintptr_t)cs.in2 & 15))
+      return cudaErrorInvalidValue;
+    if ((cs.h2 - 1) / cs.stride2 + 1 != cs.oh || (cs.w2 - 1) / cs.stride2 + 1 != cs.ow) return cudaErrorInvalidValue;
+  }
+  if (srpc_conv_2sm_eligible(cs, ep2)) {
+    const TileShape ts = pick_tile(cs.n * cs.oh * cs.ow, cs.cout, (cs.r * cs.s * cs.cin + (cs.in2 ? cs.cin2 : 0)) / BK, ep2, false, true);
+    return srpc_conv_bf16_2sm(in, weight, cs, ts.bn, ts.rows, ep2, status, stream);
+  }
   TileParams p{};
   p.mode = 1;
   p.oh = cs.oh;
@@ -1016,10 +1048,6 @@ cudaError_t srpc_conv_bf16_tma(const void* in, const void* weight, const ConvSha
   p.kb_split = p.num_kb;
   p.stride2 = 1;
   if (cs.in2) {
-    // out = act(W1 . in + W2 . in2(strided) + bias): the weight rows hold [W1 | W2]
-    if (cs.r != 1 || cs.s != 1 || cs.pad != 0 || cs.in_stub || cs.cin2 % BK || cs.stride2 < 1 || ((uintptr_t)cs.in2 & 15))
-      return cudaErrorInvalidValue;
-    if ((cs.h2 - 1) / cs.stride2 + 1 != cs.oh || (cs.w2 - 1) / cs.stride2 + 1 != cs.ow) return cudaErrorInvalidValue;
     p.K += cs.cin2;
     p.num_kb += cs.cin2 / BK;
     p.stride2 = cs.stride2;
@@ -1046,7 +1074,7 @@ cudaError_t srpc_conv_bf16_tma(const void* in, const void* weight, const ConvSha
   p.tiles_h = (cs.oh + p.ph - 1) / p.ph;
   p.tiles_m = p.tiles_w * p.tiles_h * ((cs.n + p.pn - 1) / p.pn);
   if (reuse) bn = cs.cout <= 64 ? 64 : 128;  // r B tiles travel with every A box: wider tiles leave too few stages
-  else bn = pick_bn(cs.cout, p.tiles_m, p.num_kb, true);
+  else bn = pick_tile(p.tiles_m * BM, cs.cout, p.num_kb, ep2, true, false).bn;
   p.tiles_n = (cs.cout + bn - 1) / bn;
   const int box_rows = reuse ? p.ph + cs.r - 1 : p.ph * cs.stride;
   p.a_box_bytes = reuse ? (uint32_t)(box_rows * p.pw) * 128u : (uint32_t)p.rows_used * 128u;
@@ -1088,8 +1116,5 @@ cudaError_t srpc_conv_bf16_tma(const void* in, const void* weight, const ConvSha
     e = get_map(&to, ep.out, 4, dims, st, box, es);
     if (e != cudaSuccess) return e;
   }
-  GemmEpilogue ep2 = ep;
-  ep2.ldo = cs.cout;
-  if (ep2.residual) ep2.ldr = cs.cout;
   return dispatch(bn, ta, tb, to, ta2, p, ep2, 1, status, stream);
 }

@@ -66,12 +66,15 @@ bool srpc_stem_conv_eligible(const ConvShape& cs, const GemmEpilogue& ep);
 cudaError_t srpc_stem_conv(const void* in, const void* weight, const ConvShape& cs, const GemmEpilogue& ep, uint32_t* status,
                            cudaStream_t stream);
 
-// Two-SM variant (CTA pairs, 256 x bn tiles with bn = 128, 192 or 256, tcgen05.mma.cta_group::2) for compute-bound
-// shapes; bf16 output with 16-byte aligned rows only.  srpc_gemm_bf16_v2 selects it by itself; SPLITRPC_GEMM_2SM=0
-// turns it off.
-bool srpc_gemm_2sm_eligible(int M, int N, int K, const GemmEpilogue& ep);
-cudaError_t srpc_gemm_bf16_2sm(const void* A, int lda, const void* B, int ldb, int M, int N, int K, int bn,
+// Two-SM variant (CTA pairs, tcgen05.mma.cta_group::2): tiles of `rows` = 256 rows by bn = 64, 128, 192 or 256 columns, or of 128
+// rows by 64 or 128; bf16 output with 16-byte aligned rows only.  The convolution form reads dense NHWC inputs through im2col
+// tensor maps.  srpc_gemm_bf16_v2 and srpc_conv_bf16_tma select them by themselves; SPLITRPC_GEMM_2SM=0 turns them off.
+bool srpc_gemm_2sm_eligible(int K, const GemmEpilogue& ep);
+cudaError_t srpc_gemm_bf16_2sm(const void* A, int lda, const void* B, int ldb, int M, int N, int K, int bn, int rows,
                                const GemmEpilogue& ep, uint32_t* status, cudaStream_t stream);
+bool srpc_conv_2sm_eligible(const ConvShape& cs, const GemmEpilogue& ep);
+cudaError_t srpc_conv_bf16_2sm(const void* input, const void* weight, const ConvShape& cs, int bn, int rows, const GemmEpilogue& ep,
+                               uint32_t* status, cudaStream_t stream);
 
 // Leaves `n` SMs out of the grids of the persistent kernels (see num_sms in gemm_persistent.cu); takes effect for
 // launches (and graph captures) made afterwards.  srpc_gemm_grid_sms returns the SM count the grids are sized for.

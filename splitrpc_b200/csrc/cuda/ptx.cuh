@@ -366,6 +366,17 @@ __device__ __forceinline__ void tma_load_2d_2sm(void* smem_dst, const CUtensorMa
       : "memory");
 }
 
+// The same through an im2col tensor map over an NHWC tensor: the pixels that filter tap (off_h, off_w) meets for consecutive output
+// pixels (across rows and images), the first of which starts at (w, h, n); zero outside the image and behind the last one.
+__device__ __forceinline__ void tma_load_im2col_2sm(void* smem_dst, const CUtensorMap* m, uint32_t bar_cluster_addr, int c, int w,
+                                                    int h, int n, uint16_t off_w, uint16_t off_h) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.cta_group::2.shared::cluster.global.im2col.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, "
+      "%6}], [%2], {%7, %8};" ::"r"(smem_u32(smem_dst)),
+      "l"(m), "r"(bar_cluster_addr), "r"(c), "r"(w), "r"(h), "r"(n), "h"(off_w), "h"(off_h)
+      : "memory");
+}
+
 // Reads 32 consecutive fp32 columns of this warp's 32 TMEM lanes: thread t gets
 // lane (warp%4)*32 + t, columns [col, col+32).
 __device__ __forceinline__ void tmem_ld_32x32b_x32(uint32_t taddr, uint32_t* r) {

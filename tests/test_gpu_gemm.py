@@ -148,3 +148,47 @@ def test_conv_implicit_gemm(env, n, h, cin, cout, r, stride, pad):
     ref2 = torch.relu(torch.nn.functional.conv2d(x.float().permute(0, 3, 1, 2), w.float().permute(0, 3, 1, 2), bias, stride,
                                                  pad).permute(0, 2, 3, 1) + res.float())
     assert _rel_err(torch, out2, ref2) < 1e-2
+
+
+@pytest.mark.parametrize("M", [1, 64, 65, 128, 129, 200, 300])
+@pytest.mark.parametrize("N,K", [(8, 64), (72, 200), (64, 1096), (136, 72), (1000, 512)])
+def test_gemm_few_rows(env, M, N, K):
+    """Pair tiles of 64 rows per CTA: rows of one CTA only, column halves, odd numbers of k-blocks, a K remainder."""
+    torch, ops = env
+    a = (torch.randn(M, K, device="cuda") * 0.3).bfloat16()
+    b = (torch.randn(N, K, device="cuda") * 0.3).bfloat16()
+    bias = torch.randn(N, device="cuda")
+    res = torch.randn(M, N, device="cuda").bfloat16()
+    buf = torch.full((M + 1, N + 8), 7.0, device="cuda", dtype=torch.bfloat16)
+    for r in (None, res):
+        out = ops.gemm(a, b, bias=bias, residual=r, act="gelu", out=buf[:M, :N])
+        ops.check_status()
+        ref = a.double() @ b.double().t() + bias.double()
+        ref = torch.nn.functional.gelu(ref if r is None else ref + r.double())
+        # bounds as in test_gemm_pair_tiles_ragged
+        assert ((out.double() - ref).abs() <= ref.abs() * 2.0 ** -8 + K * K * 0.09 * 2.0 ** -24 + 1e-6).all()
+        assert (buf[M] == 7.0).all() and (buf[:, N:] == 7.0).all()
+
+
+@pytest.mark.parametrize("h,w,cin,cout,r,s,stride,pad", [(14, 14, 64, 128, 3, 3, 1, 1), (19, 23, 64, 136, 2, 5, 1, 2), (19, 23, 128, 72, 5, 2, 2, 3),
+                                                         (15, 15, 64, 64, 3, 1, 1, 0), (30, 30, 64, 64, 7, 7, 4, 3), (9, 9, 128, 64, 1, 1, 3, 0),
+                                                         (7, 7, 512, 512, 3, 3, 1, 1), (5, 5, 64, 8, 3, 3, 2, 1)])
+def test_conv_linear_pixels(env, h, w, cin, cout, r, s, stride, pad):
+    """Tiles of consecutive output pixels across rows and images: filters of any form, partial last tiles; an image gives the same
+    bits in every batch."""
+    torch, ops = env
+    x = torch.randn(11, h, w, cin, device="cuda").bfloat16()
+    wt = (torch.randn(cout, r, s, cin, device="cuda") * 0.05).bfloat16()
+    bias = torch.randn(cout, device="cuda")
+    ref = torch.nn.functional.conv2d(x.permute(0, 3, 1, 2).double(), wt.permute(0, 3, 1, 2).double(), bias.double(), stride, pad).permute(0, 2, 3, 1)
+    res = torch.randn(ref.shape, device="cuda").bfloat16()
+    K = r * s * cin
+    whole = ops.conv2d_nhwc(x, wt, bias=bias, residual=res, stride=stride, pad=pad, act="relu")
+    ops.check_status()
+    want = torch.relu(ref + res.double())
+    # as above, with products of about 0.04 on average
+    assert ((whole.double() - want).abs() <= want.abs() * 2.0 ** -8 + K * K * 0.04 * 2.0 ** -24 + 1e-6).all()
+    for n in (1, 2, 5):
+        part = ops.conv2d_nhwc(x[:n].contiguous(), wt, bias=bias, residual=res[:n].contiguous(), stride=stride, pad=pad, act="relu")
+        assert torch.equal(part, whole[:n])
+    ops.check_status()
