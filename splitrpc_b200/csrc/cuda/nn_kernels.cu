@@ -199,26 +199,40 @@ __global__ void __launch_bounds__(256) global_avgpool(const __nv_bfloat16* in, _
   *reinterpret_cast<__nv_bfloat162*>(out + (size_t)b * c + ch) = __floats2bfloat162_rn(s0 / hw, s1 / hw);
 }
 
-// Skinny fully connected layer: out[m, n] = sum_k a[m, k] * w[n, k] + bias[n] for a handful of rows, fp32 output.  A
-// tensor-core tile would be 128 rows x 64 columns: with 64 rows that leaves 16 CTAs each walking all of K.  Here a
-// block owns FC_NB output columns and 16 * RPT rows: the weight rows are staged in shared memory as fp32 once (two
-// planes of float4 per column, so that the sixteen k-slices a warp reads together are contiguous), thread
-// (row group, kq) walks every sixteenth 8-element slice of its RPT rows of `a` with the next slice's loads in flight, and
-// the sixteen partial sums of a row meet through shuffles.  A slice's weights are read from shared memory once for the
-// RPT rows: with two rows those reads bound 64 x 1000 x 2048 (15.2 us), with four it takes 12.9 us, of which the FMAs are 4.  Two
-// rows stay for up to 32 rows (8.9 us), where there are enough of them for one block per column group anyway.  PER_SM: blocks
-// that the registers leave room for on an SM, see nn_fc_skinny.  The order of every sum is the same in all forms.
-constexpr int FC_NB = 8;
+// Skinny fully connected layer: out[m, n] = sum_k a[m, k] * w[n, k] + bias[n] for a handful of rows, fp32 output and fp32 sums
+// (the tensor cores' accumulator rounds more).  A block owns FC_NB output columns and 16 * RPT rows: a warp copies the weights of
+// one column into shared memory, in four parts of K that arrive behind one another, so that the arithmetic starts with the first;
+// thread (row group, kq) walks every sixteenth 8-element slice of its RPT rows of `a` with the next slice's loads in flight, and
+// the sixteen partial sums of a row meet through shuffles that halve the list of values at every step.  A slice's weights are
+// read from shared memory and converted once for the RPT rows.  Two rows stay for up to 32 rows, where there are enough of them
+// for one block per column group anyway.  PER_SM: blocks that the registers leave room for on an SM, see nn_fc_skinny.
+// Us, before (weights staged whole, as fp32, before any arithmetic; 128 shuffles per thread) and now: 64 x 1000 x 2048 12.85 and
+// 11.75, 64 x 1192 x 512 9.9 and 7.4, 128 x 1000 x 512 10.1 and 7.6, 64 x 8192 x 768 38 and 31, 32 x 1192 x 512 6.4 and 5.2.  The loop
+// is bound by what it reads through the L1 / shared-memory path (9.5 of the first, the FMAs are 4.2): deeper prefetch, twice the
+// warps or scalar FMAs change nothing.  The order of every sum is the same in all forms.
+constexpr int FC_NB = 8, FC_PARTS = 4;
 template <int RPT, int PER_SM>
 __global__ void __launch_bounds__(256, PER_SM) fc_skinny(const __nv_bfloat16* a, int lda, const __nv_bfloat16* w,
                                                  int ldw, const float* bias, float* out, int ldo, int M,
                                                  int N, int K) {
+  static_assert(FC_NB == 8 && FC_PARTS == 4, "one warp per column, three steps over the columns; four waits below");
   ptx::grid_dep_launch();
   ptx::grid_dep_wait();
-  extern __shared__ __align__(16) float4 s_w[];  // [FC_NB][2][K/8]
-  const int n0 = blockIdx.x * FC_NB, kvn = K / 8;
+  extern __shared__ __align__(16) uint4 s_w[];  // [FC_NB][K/8]
+  const int n0 = blockIdx.x * FC_NB, kvn = K / 8, turns = (kvn + 15) / 16;
   const int kq = threadIdx.x & 15;
   const int row0 = blockIdx.y * (16 * RPT) + (threadIdx.x >> 4) * RPT;
+  {
+    const int col = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const bool in = n0 + col < N;
+    const __nv_bfloat16* wr = w + (size_t)(in ? n0 + col : 0) * ldw;
+#pragma unroll
+    for (int part = 0; part < FC_PARTS; part++) {
+      const int end = min(kvn, turns * (part + 1) / FC_PARTS * 16);
+      for (int kv = turns * part / FC_PARTS * 16 + lane; kv < end; kv += 32) ptx::cp_async_16(s_w + col * kvn + kv, wr + kv * 8, in);
+      ptx::cp_async_commit();
+    }
+  }
   // rows past M read row M-1 again (their results are not stored): no branch inside the loop
   const __nv_bfloat16* ar[RPT];
 #pragma unroll
@@ -226,79 +240,80 @@ __global__ void __launch_bounds__(256, PER_SM) fc_skinny(const __nv_bfloat16* a,
   auto load = [&](const __nv_bfloat16* r, int kv) {
     return kv < kvn ? *(reinterpret_cast<const uint4*>(r + kv * 8)) : make_uint4(0, 0, 0, 0);
   };
-  // AHEAD slices of every row are in flight, the first ones beside the weights (four rows: more than one slice measured slower).
+  // AHEAD slices of every row are in flight, the first ones beside the weights.
   constexpr int AHEAD = RPT == 2 ? 2 : 1;
   uint4 qa[AHEAD][RPT];
 #pragma unroll
   for (int d = 0; d < AHEAD; d++)
 #pragma unroll
     for (int r = 0; r < RPT; r++) qa[d][r] = load(ar[r], kq + 16 * d);
-  for (int base = 0; base < FC_NB * kvn; base += 256 * 8) {
-    uint4 q[8];  // eight loads in flight per thread: the weights usually come from DRAM
-#pragma unroll
-    for (int u = 0; u < 8; u++) {
-      const int i = base + u * 256 + threadIdx.x, col = i / kvn, kv = i - col * kvn;
-      q[u] = make_uint4(0, 0, 0, 0);
-      if (i < FC_NB * kvn && n0 + col < N) q[u] = *(reinterpret_cast<const uint4*>(w + (size_t)(n0 + col) * ldw + kv * 8));
-    }
-#pragma unroll
-    for (int u = 0; u < 8; u++) {
-      const int i = base + u * 256 + threadIdx.x, col = i / kvn, kv = i - col * kvn;
-      const __nv_bfloat162* hq = reinterpret_cast<const __nv_bfloat162*>(&q[u]);
-      const float2 f0 = __bfloat1622float2(hq[0]), f1 = __bfloat1622float2(hq[1]), f2 = __bfloat1622float2(hq[2]),
-                   f3 = __bfloat1622float2(hq[3]);
-      if (i < FC_NB * kvn) {
-        s_w[(col * 2) * kvn + kv] = make_float4(f0.x, f0.y, f1.x, f1.y);
-        s_w[(col * 2 + 1) * kvn + kv] = make_float4(f2.x, f2.y, f3.x, f3.y);
-      }
-    }
-  }
-  __syncthreads();
-  // packed fp32 FMAs (two per instruction): lane x of an accumulator sums the even k, lane y the odd k
+  // packed fp32 FMAs (two per instruction): element x of an accumulator sums the even k, element y the odd k
   float2 acc[RPT][FC_NB];
 #pragma unroll
   for (int r = 0; r < RPT; r++)
 #pragma unroll
     for (int j = 0; j < FC_NB; j++) acc[r][j] = make_float2(0.f, 0.f);
-  for (int kv0 = kq; kv0 < kvn; kv0 += 16 * AHEAD) {
+  auto slice = [&](int kv, uint4 (&q)[RPT]) {
+    float2 x[RPT][4];
 #pragma unroll
-    for (int d = 0; d < AHEAD; d++) {
-      const int kv = kv0 + 16 * d;
-      if (kv >= kvn) break;
-      float2 x[RPT][4];
+    for (int r = 0; r < RPT; r++) {
+      const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&q[r]);
 #pragma unroll
-      for (int r = 0; r < RPT; r++) {
-        const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&qa[d][r]);
-#pragma unroll
-        for (int t = 0; t < 4; t++) x[r][t] = __bfloat1622float2(h[t]);
-      }
-#pragma unroll
-      for (int r = 0; r < RPT; r++) qa[d][r] = load(ar[r], kv + 16 * AHEAD);  // in flight during the arithmetic
-#pragma unroll
-      for (int j = 0; j < FC_NB; j++) {
-        const float4 w0 = s_w[(j * 2) * kvn + kv], w1 = s_w[(j * 2 + 1) * kvn + kv];
-        const float2 wq[4] = {make_float2(w0.x, w0.y), make_float2(w0.z, w0.w), make_float2(w1.x, w1.y), make_float2(w1.z, w1.w)};
-#pragma unroll
-        for (int t = 0; t < 4; t++)
-#pragma unroll
-          for (int r = 0; r < RPT; r++) acc[r][j] = __ffma2_rn(x[r][t], wq[t], acc[r][j]);
-      }
+      for (int t = 0; t < 4; t++) x[r][t] = __bfloat1622float2(h[t]);
     }
-  }
 #pragma unroll
-  for (int r = 0; r < RPT; r++) {
-    float s[FC_NB];
+    for (int r = 0; r < RPT; r++) q[r] = load(ar[r], kv + 16 * AHEAD);  // in flight during the arithmetic
 #pragma unroll
     for (int j = 0; j < FC_NB; j++) {
-      s[j] = acc[r][j].x + acc[r][j].y;
+      const uint4 wv = s_w[j * kvn + kv];
+      const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&wv);
 #pragma unroll
-      for (int d = 1; d < 16; d <<= 1) s[j] += __shfl_xor_sync(0xffffffffu, s[j], d);
+      for (int t = 0; t < 4; t++) {
+        const float2 wq = __bfloat1622float2(h[t]);
+#pragma unroll
+        for (int r = 0; r < RPT; r++) acc[r][j] = __ffma2_rn(x[r][t], wq, acc[r][j]);
+      }
     }
-    // lane kq stores column kq & 7 of the rows r with r mod 2 = kq >> 3
+  };
+  int turn = 0;
 #pragma unroll
-    for (int j = 0; j < FC_NB; j++)
-      if ((kq & 7) == j && (kq >> 3) == (r & 1) && n0 + j < N && row0 + r < M)
-        out[(size_t)(row0 + r) * ldo + n0 + j] = s[j] + (bias ? bias[n0 + j] : 0.f);
+  for (int part = 0; part < FC_PARTS; part++) {
+    if (part == 0) ptx::cp_async_wait<3>();
+    else if (part == 1) ptx::cp_async_wait<2>();
+    else if (part == 2) ptx::cp_async_wait<1>();
+    else ptx::cp_async_wait<0>();
+    __syncthreads();
+    const int end = turns * (part + 1) / FC_PARTS;
+#pragma unroll 1
+    for (; turn < end; turn++) {
+      if (turn * 16 + kq >= kvn) continue;
+      if (AHEAD > 1 && (turn & 1)) slice(turn * 16 + kq, qa[AHEAD - 1]);  // slice `turn` is in qa[turn mod AHEAD]
+      else slice(turn * 16 + kq, qa[0]);
+    }
+  }
+  // The sums over the sixteen lanes of a row group: at every step a lane keeps the half of its values that its lane number names
+  // and gets the partner's share of them.  Lane kq ends with column kq & 7 of the rows r with r mod 2 = kq >> 3.
+  float s[RPT][FC_NB];
+#pragma unroll
+  for (int r = 0; r < RPT; r++)
+#pragma unroll
+    for (int j = 0; j < FC_NB; j++) s[r][j] = acc[r][j].x + acc[r][j].y;
+#pragma unroll
+  for (int d = 1, n = FC_NB / 2; d < 8; d <<= 1, n >>= 1)
+#pragma unroll
+    for (int r = 0; r < RPT; r++)
+#pragma unroll
+      for (int j = 0; j < FC_NB / 2; j++)
+        if (j < n) {
+          const float even = s[r][2 * j], odd = s[r][2 * j + 1];
+          s[r][j] = ((kq & d) ? odd : even) + __shfl_xor_sync(0xffffffffu, (kq & d) ? even : odd, d);
+        }
+  const int col = n0 + (kq & 7);
+#pragma unroll
+  for (int r = 0; r < RPT; r += 2) {
+    const float v = ((kq & 8) ? s[r + 1][0] : s[r][0]) + __shfl_xor_sync(0xffffffffu, (kq & 8) ? s[r][0] : s[r + 1][0], 8);
+    const int row = row0 + r + (kq >> 3);
+    if (col < N && row < M) out[(size_t)row * ldo + col] = v + (bias ? bias[col] : 0.f);
   }
 }
 
@@ -621,32 +636,32 @@ cudaError_t nn_global_avgpool(const void* in, void* out, int n, int hw, int c, c
 }
 cudaError_t nn_fc_skinny(const void* a, int lda, const void* w, int ldw, const float* bias, float* out, int ldo, int M, int N, int K,
                          cudaStream_t s) {
-  const size_t smem = (size_t)FC_NB * K * sizeof(float);
-  if (K % 8 || lda % 8 || ldw % 8 || (((uintptr_t)a | (uintptr_t)w) & 15) || smem > 200 * 1024 || M <= 0) return cudaErrorInvalidValue;
+  const size_t smem = (size_t)FC_NB * K * sizeof(__nv_bfloat16);
+  if (K % 8 || lda % 8 || ldw % 8 || (((uintptr_t)a | (uintptr_t)w) & 15) || smem > 100 * 1024 || M <= 0) return cudaErrorInvalidValue;
   static PerDeviceFlag attr_set;
   const int dev = PerDeviceFlag::current();
   if (attr_set.needed(dev)) {
-    cudaError_t e = cudaFuncSetAttribute(fc_skinny<2, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(fc_skinny<4, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(fc_skinny<2, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(fc_skinny<4, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    cudaError_t e = cudaFuncSetAttribute(fc_skinny<2, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 116 * 1024);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(fc_skinny<4, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 116 * 1024);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(fc_skinny<2, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 116 * 1024);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(fc_skinny<4, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 116 * 1024);
     if (e != cudaSuccess) return e;
     attr_set.set(dev);
   }
   // While the blocks fit the SMs one each, a block takes the registers it likes, and up to 32 rows also more than half of an
   // SM's shared memory: blocks that start while the kernel before still runs would otherwise be stacked two to an SM
   // beside empty ones (32 x 1000 x 2048: 13.6 us then, 8.9 us now).  With more blocks than SMs two share an SM, at 128
-  // registers, where two blocks' weights fit its shared memory (K up to 3616).  One per SM against two, us:
-  // 32 x 1192 x 512 8.2 / 6.4, 32 x 4096 x 2048 32.9 / 28.4, 64 x 1192 x 512 12.6 / 10.0, 128 x 1000 x 512 12.9 / 10.2, 64 x 8192 x 768 50.4 / 38.3.
+  // registers.  One per SM against two, us (weights staged whole): 32 x 1192 x 512 8.2 / 6.4, 32 x 4096 x 2048 32.9 / 28.4,
+  // 64 x 1192 x 512 12.6 / 10.0, 128 x 1000 x 512 12.9 / 10.2, 64 x 8192 x 768 50.4 / 38.3.
   const size_t spread = 116 * 1024;
   const int sms = srpc_gemm_grid_sms(), rpt = M <= 32 ? 2 : 4;
   const dim3 grid((unsigned)((N + FC_NB - 1) / FC_NB), (unsigned)((M + 16 * rpt - 1) / (16 * rpt)));
-  const bool one_each = (uint64_t)grid.x * grid.y <= (uint64_t)sms, two_fit = smem <= 113 * 1024;
+  const bool one_each = (uint64_t)grid.x * grid.y <= (uint64_t)sms;
   auto go = [&](auto* kernel, size_t shared) {
     return launch_pdl(kernel, grid, dim3(256), shared, s, (const __nv_bfloat16*)a, lda, (const __nv_bfloat16*)w, ldw, bias, out, ldo, M, N, K);
   };
-  if (rpt == 2) return one_each ? go(fc_skinny<2, 1>, smem < spread ? spread : smem) : (two_fit ? go(fc_skinny<2, 2>, smem) : go(fc_skinny<2, 1>, smem));
-  return one_each || !two_fit ? go(fc_skinny<4, 1>, smem) : go(fc_skinny<4, 2>, smem);
+  if (rpt == 2) return one_each ? go(fc_skinny<2, 1>, spread) : go(fc_skinny<2, 2>, smem);
+  return one_each ? go(fc_skinny<4, 1>, smem) : go(fc_skinny<4, 2>, smem);
 }
 cudaError_t nn_softmax_response(const float* logits, int rows, int n, int ld, const void* d_stub, void* direct_out,
                                 size_t resp_stride, int write_argmax, uint32_t* counter, uint32_t* flag, uint32_t flag_value,
