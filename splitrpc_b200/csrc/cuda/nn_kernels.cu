@@ -436,66 +436,96 @@ __global__ void __launch_bounds__(256) layernorm_rows(const __nv_bfloat16* x,
     y[row * hidden + i] = __float2bfloat16((v[cnt] - mean) * rstd * gamma[i] + beta[i]);
 }
 
-// Warp-per-row LayerNorm for hidden sizes that are multiples of 256 (up to 2048): each lane owns hidden/32 values as
-// 16-byte vectors, the row never leaves registers, and both reductions are warp shuffles.
-template <int VPL>  // uint4 vectors per lane: hidden = VPL * 256
-__global__ void __launch_bounds__(256) layernorm_rows_warp(const __nv_bfloat16* x,
-                                                           const __nv_bfloat16* residual,
-                                                           const float* gamma, const float* beta,
-                                                           __nv_bfloat16* y, int rows, float eps) {
+// LayerNorm for hidden sizes of 256, 512, 768 and 1024: a thread has eight columns of R rows, so that a row's 8 bytes of
+// parameters per column are read once for R rows (a warp with a row of its own read twice as many bytes of parameters as of the
+// row); rows never leave registers, both reductions halve their list of rows at every step through the warp and meet in
+// shared memory.  Us, a warp per row against this: 6144 x 1024 6.6 and 5.35, 4096 x 768 3.95 and 3.55, 2048 x 1024 4.6 and 2.8,
+// 1024 x 768 2.9 and 2.2, 128 x 768 2.05 and 1.5 (1184 x 768, eight rows for every SM, 2.1 and 2.3).
+template <int VPL, int R>  // hidden = VPL * 256, one warp per 256 columns
+__global__ void __launch_bounds__(32 * VPL) layernorm_rows_vec(const __nv_bfloat16* x, const __nv_bfloat16* residual, const float* gamma,
+                                                               const float* beta, __nv_bfloat16* y, int rows, float eps) {
+  static_assert(R == 2 || R == 4, "a power of two; the steps of the reduction below");
   ptx::grid_dep_launch();
   ptx::grid_dep_wait();
   constexpr int HIDDEN = VPL * 256;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int row = blockIdx.x * 8 + warp;
-  if (row >= rows) return;
-  const uint4* xr = reinterpret_cast<const uint4*>(x + (size_t)row * HIDDEN);
-  const uint4* rr = residual ? reinterpret_cast<const uint4*>(residual + (size_t)row * HIDDEN) : nullptr;
-  float v[VPL * 8];
-  float s = 0.f;
+  __shared__ __align__(16) float sh[2][VPL][R];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, c0 = threadIdx.x * 8;
+  const int row0 = blockIdx.x * R;
+  uint4 q[R], q2[R];
 #pragma unroll
-  for (int i = 0; i < VPL; i++) {
-    uint4 q = xr[i * 32 + lane];
-    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&q);
-    uint4 q2 = rr ? rr[i * 32 + lane] : make_uint4(0u, 0u, 0u, 0u);
-    const __nv_bfloat162* h2 = reinterpret_cast<const __nv_bfloat162*>(&q2);
+  for (int r = 0; r < R; r++) {
+    const size_t at = (size_t)min(row0 + r, rows - 1) * HIDDEN + c0;
+    q[r] = *reinterpret_cast<const uint4*>(x + at);
+    q2[r] = residual ? *reinterpret_cast<const uint4*>(residual + at) : make_uint4(0u, 0u, 0u, 0u);
+  }
+  float4 g4[2], b4[2];
+#pragma unroll
+  for (int i = 0; i < 2; i++) {
+    g4[i] = *reinterpret_cast<const float4*>(gamma + c0 + 4 * i);
+    b4[i] = *reinterpret_cast<const float4*>(beta + c0 + 4 * i);
+  }
+  // Sums of s[r] over the block: lane l of a warp ends with row l mod R, the warps' shares meet in shared memory.
+  auto block_sums = [&](float (&s)[R], int buf) {
+#pragma unroll
+    for (int d = 1, n = R / 2; d < 32; d <<= 1, n >>= 1) {
+      if (n >= 1) {
+#pragma unroll
+        for (int r = 0; r < R / 2; r++)
+          if (r < n) {
+            const float even = s[2 * r], odd = s[2 * r + 1];
+            s[r] = ((lane & d) ? odd : even) + __shfl_xor_sync(0xffffffffu, (lane & d) ? even : odd, d);
+          }
+      } else {
+        s[0] += __shfl_xor_sync(0xffffffffu, s[0], d);
+      }
+    }
+    if (lane < R) sh[buf][warp][lane] = s[0];
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+      s[r] = sh[buf][0][r];
+#pragma unroll
+      for (int w = 1; w < VPL; w++) s[r] += sh[buf][w][r];
+    }
+  };
+  float v[R][8], s[R];
+#pragma unroll
+  for (int r = 0; r < R; r++) {
+    const __nv_bfloat162 *h = reinterpret_cast<const __nv_bfloat162*>(&q[r]), *h2 = reinterpret_cast<const __nv_bfloat162*>(&q2[r]);
+    s[r] = 0.f;
 #pragma unroll
     for (int t = 0; t < 4; t++) {
-      float2 f = __bfloat1622float2(h[t]), g = __bfloat1622float2(h2[t]);
-      v[i * 8 + 2 * t] = f.x + g.x;
-      v[i * 8 + 2 * t + 1] = f.y + g.y;
-      s += v[i * 8 + 2 * t] + v[i * 8 + 2 * t + 1];
+      const float2 f = __bfloat1622float2(h[t]), g = __bfloat1622float2(h2[t]);
+      v[r][2 * t] = f.x + g.x;
+      v[r][2 * t + 1] = f.y + g.y;
+      s[r] += v[r][2 * t] + v[r][2 * t + 1];
     }
   }
-  // The parameters are fetched while the row's sums travel through the warp: read where they are used, after the
-  // reductions, they cost every row a second round trip (4096 x 768 back to back 4.4 -> 4.1 us).
-  float4 g4[2 * VPL], b4[2 * VPL];
+  block_sums(s, 0);
+  float u[R];
 #pragma unroll
-  for (int i = 0; i < VPL; i++) {
-    const int c0 = (i * 32 + lane) * 8;
-    g4[2 * i] = *reinterpret_cast<const float4*>(gamma + c0);
-    g4[2 * i + 1] = *reinterpret_cast<const float4*>(gamma + c0 + 4);
-    b4[2 * i] = *reinterpret_cast<const float4*>(beta + c0);
-    b4[2 * i + 1] = *reinterpret_cast<const float4*>(beta + c0 + 4);
+  for (int r = 0; r < R; r++) {
+    const float mean = s[r] * (1.f / HIDDEN);
+    u[r] = 0.f;
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+      v[r][k] -= mean;
+      u[r] += v[r][k] * v[r][k];
+    }
   }
-  const float mean = warp_sum(s) * (1.f / HIDDEN);
-  float q = 0.f;
+  block_sums(u, 1);
+  const float gg[8] = {g4[0].x, g4[0].y, g4[0].z, g4[0].w, g4[1].x, g4[1].y, g4[1].z, g4[1].w};
+  const float bb[8] = {b4[0].x, b4[0].y, b4[0].z, b4[0].w, b4[1].x, b4[1].y, b4[1].z, b4[1].w};
 #pragma unroll
-  for (int k = 0; k < VPL * 8; k++) q += (v[k] - mean) * (v[k] - mean);
-  const float rstd = rsqrtf(warp_sum(q) * (1.f / HIDDEN) + eps);
-  uint4* yr = reinterpret_cast<uint4*>(y + (size_t)row * HIDDEN);
-#pragma unroll
-  for (int i = 0; i < VPL; i++) {
-    const float4 g0 = g4[2 * i], g1 = g4[2 * i + 1], b0 = b4[2 * i], b1 = b4[2 * i + 1];
-    const float gg[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
-    const float bb[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+  for (int r = 0; r < R; r++) {
+    if (row0 + r >= rows) break;
+    const float rstd = rsqrtf(u[r] * (1.f / HIDDEN) + eps);
     uint4 o;
     __nv_bfloat162* ho = reinterpret_cast<__nv_bfloat162*>(&o);
 #pragma unroll
     for (int t = 0; t < 4; t++)
-      ho[t] = __floats2bfloat162_rn((v[i * 8 + 2 * t] - mean) * rstd * gg[2 * t] + bb[2 * t],
-                                    (v[i * 8 + 2 * t + 1] - mean) * rstd * gg[2 * t + 1] + bb[2 * t + 1]);
-    yr[i * 32 + lane] = o;
+      ho[t] = __floats2bfloat162_rn(v[r][2 * t] * rstd * gg[2 * t] + bb[2 * t], v[r][2 * t + 1] * rstd * gg[2 * t + 1] + bb[2 * t + 1]);
+    *reinterpret_cast<uint4*>(y + (size_t)(row0 + r) * HIDDEN + c0) = o;
   }
 }
 
@@ -674,17 +704,20 @@ cudaError_t nn_layernorm(const void* x, const void* residual, const float* gamma
                          int hidden, float eps, cudaStream_t s) {
   if (hidden > 2048) return cudaErrorInvalidValue;
   const bool aligned = (((uintptr_t)x | (uintptr_t)y | (uintptr_t)residual | (uintptr_t)gamma | (uintptr_t)beta) & 15) == 0;
-  const int grid = (rows + 7) / 8;
   const __nv_bfloat16 *xp = (const __nv_bfloat16*)x, *rp = (const __nv_bfloat16*)residual;
   __nv_bfloat16* yp = (__nv_bfloat16*)y;
-  if (aligned && hidden == 768) return launch_pdl(layernorm_rows_warp<3>, dim3(grid), dim3(256), 0, s, xp, rp, gamma, beta, yp,
-                                                  rows, eps);
-  if (aligned && hidden == 1024) return launch_pdl(layernorm_rows_warp<4>, dim3(grid), dim3(256), 0, s, xp, rp, gamma, beta, yp,
-                                                   rows, eps);
-  if (aligned && hidden == 512) return launch_pdl(layernorm_rows_warp<2>, dim3(grid), dim3(256), 0, s, xp, rp, gamma, beta, yp,
-                                                  rows, eps);
-  if (aligned && hidden == 256) return launch_pdl(layernorm_rows_warp<1>, dim3(grid), dim3(256), 0, s, xp, rp, gamma, beta, yp,
-                                                  rows, eps);
+  if (aligned && rows > 0 && hidden % 256 == 0 && hidden <= 1024) {
+    // Four rows per block once that gives every SM three of them, two for fewer rows (us, two against four: 6144 x 1024 5.8 / 5.35,
+    // 2048 x 1024 3.1 / 2.8, 1184 x 768 2.3 / 2.5); eight: 5.8 for the first, 121 registers.
+    const bool many = rows >= 12 * srpc_gemm_grid_sms();
+    auto go = [&](auto* kernel, int r) {
+      return launch_pdl(kernel, dim3((rows + r - 1) / r), dim3(hidden / 8), 0, s, xp, rp, gamma, beta, yp, rows, eps);
+    };
+    if (hidden == 256) return many ? go(layernorm_rows_vec<1, 4>, 4) : go(layernorm_rows_vec<1, 2>, 2);
+    if (hidden == 512) return many ? go(layernorm_rows_vec<2, 4>, 4) : go(layernorm_rows_vec<2, 2>, 2);
+    if (hidden == 768) return many ? go(layernorm_rows_vec<3, 4>, 4) : go(layernorm_rows_vec<3, 2>, 2);
+    return many ? go(layernorm_rows_vec<4, 4>, 4) : go(layernorm_rows_vec<4, 2>, 2);
+  }
   return launch_pdl(layernorm_rows, dim3(rows), dim3(256), 0, s, xp, rp, gamma, beta, yp, hidden, eps);
 }
 cudaError_t nn_bert_embed_ln(const void* d_stub, const int* direct_ids, size_t req_stride, int batch, int seq, const void* word,

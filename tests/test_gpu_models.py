@@ -282,3 +282,23 @@ def test_model_server_end_to_end_resnet(torch_cuda, fused_ingress):
     torch.cuda.synchronize()
     got = torch.from_numpy(np.frombuffer(cli.response(5), dtype=np.float32).copy())  # request 5 used payload 5 % 4 == 1
     torch.testing.assert_close(got, direct[0].cpu(), rtol=1e-3, atol=1e-5)
+
+
+@pytest.mark.parametrize("hidden", [256, 512, 768, 1024])
+@pytest.mark.parametrize("rows", [1, 2, 3, 127, 1775, 1777, 2051])
+def test_layernorm_rows_per_block(torch_cuda, rows, hidden):
+    """Two and four rows per block, last blocks with rows missing, residual added or not, rows with a large offset."""
+    torch = torch_cuda
+    from splitrpc_b200 import ops
+
+    x = (torch.randn(rows, hidden, device="cuda") + 20.0).bfloat16()
+    res = torch.randn(rows, hidden, device="cuda").bfloat16()
+    g, b = torch.randn(hidden, device="cuda"), torch.randn(hidden, device="cuda")
+    buf = torch.full((rows + 1, hidden), 7.0, device="cuda", dtype=torch.bfloat16)
+    for r in (None, res):
+        ops.layernorm(x, g, b, residual=r, out=buf[:rows])
+        xd = x.double() if r is None else x.double() + r.double()
+        ref = torch.nn.functional.layer_norm(xd, (hidden,), g.double(), b.double(), 1e-12)
+        # bf16 rounding of the result (2^-9 of it), and the fp32 mean and deviations of values about 20 times their spread
+        assert ((buf[:rows].double() - ref).abs() <= ref.abs() * 2.0 ** -8 + g.abs().double() * 2e-5 + 1e-6).all()
+        assert (buf[rows] == 7.0).all()
