@@ -332,61 +332,76 @@ __global__ void __launch_bounds__(256) softmax_response(const float* logits, int
                                                         const RespPushCtx* push) {
   ptx::grid_dep_launch();
   ptx::grid_dep_wait();
-  __shared__ float sh[32];
-  __shared__ float s_max, s_sum;
-  __shared__ int s_arg;
-  const int row = blockIdx.x;
+  __shared__ float sh_max[8], sh_sum[8];
+  __shared__ int sh_arg[8];
+  const int row = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const float* x = logits + (size_t)row * ld;
-  // One thread reads the stub and the push block (mapped host memory: every read is a PCIe round trip) for the block.
+  // One thread reads the stub and the push block (mapped host memory: every read is a PCIe round trip) for the block; the target is
+  // needed behind the last barrier.  The logits stay in registers (a row of up to 2048), and every thread puts the warps'
+  // shares together by itself: two barriers instead of eight and one read of the row instead of three (64 x 1000: 3.2 -> 1.85 us).
   __shared__ RespPushTarget s_target;
   if (threadIdx.x == 0) {
     uint8_t* b = (direct_out ? direct_out : stub->resp) + (size_t)row * resp_stride;
     s_target = (!direct_out && push) ? resp_push_target(push, (uint32_t)row, b) : RespPushTarget{b, nullptr, nullptr};
   }
-  __syncthreads();
-  const RespPushTarget target = s_target;
-  uint8_t* base = target.dst;
+  constexpr int REGS = 8;
+  float v[REGS];
   float m = -FLT_MAX;
   int am = 0;
-  for (int i = threadIdx.x; i < n; i += blockDim.x)
+#pragma unroll
+  for (int k = 0; k < REGS; k++) {
+    const int i = threadIdx.x + k * 256;
+    v[k] = i < n ? x[i] : -INFINITY;
+  }
+#pragma unroll
+  for (int k = 0; k < REGS; k++)
+    if (v[k] > m) {
+      m = v[k];
+      am = threadIdx.x + k * 256;
+    }
+  for (int i = threadIdx.x + REGS * 256; i < n; i += 256)
     if (x[i] > m) {
       m = x[i];
       am = i;
     }
-  // block arg-max
-  float wm = warp_max(m);
-  unsigned ball = __ballot_sync(0xffffffffu, m == wm);
-  int src = __ffs(ball) - 1;
-  int wam = __shfl_sync(0xffffffffu, am, src);
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31, nw = blockDim.x >> 5;
-  __shared__ int sh_i[32];
-  if (l == 0) {
-    sh[w] = wm;
-    sh_i[w] = wam;
+  const float wm = warp_max(m);
+  const int src = __ffs(__ballot_sync(0xffffffffu, m == wm)) - 1;
+  const int wam = __shfl_sync(0xffffffffu, am, src);
+  if (lane == 0) {
+    sh_max[warp] = wm;
+    sh_arg[warp] = wam;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    float bm = sh[0];
-    int bi = sh_i[0];
-    for (int k = 1; k < nw; k++)
-      if (sh[k] > bm) {
-        bm = sh[k];
-        bi = sh_i[k];
-      }
-    s_max = bm;
-    s_arg = bi;
+  float mx = sh_max[0];
+  int arg = sh_arg[0];
+#pragma unroll
+  for (int k = 1; k < 8; k++)
+    if (sh_max[k] > mx) {
+      mx = sh_max[k];
+      arg = sh_arg[k];
+    }
+  float sum = 0.f;
+#pragma unroll
+  for (int k = 0; k < REGS; k++) {
+    v[k] = __expf(v[k] - mx);
+    if (threadIdx.x + k * 256 < n) sum += v[k];
   }
+  for (int i = threadIdx.x + REGS * 256; i < n; i += 256) sum += __expf(x[i] - mx);
+  sum = warp_sum(sum);
+  if (lane == 0) sh_sum[warp] = sum;
   __syncthreads();
-  const float mx = s_max;
-  float s = 0.f;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) s += __expf(x[i] - mx);
-  s = block_sum(s, sh);
-  if (threadIdx.x == 0) s_sum = s;
-  __syncthreads();
-  const float inv = 1.f / s_sum;
+  sum = sh_sum[0];
+#pragma unroll
+  for (int k = 1; k < 8; k++) sum += sh_sum[k];
+  const float inv = 1.f / sum;
+  const RespPushTarget target = s_target;
+  uint8_t* base = target.dst;
   float* o = reinterpret_cast<float*>(base);
-  for (int i = threadIdx.x; i < n; i += blockDim.x) o[i] = __expf(x[i] - mx) * inv;
-  if (write_argmax && threadIdx.x == 0) reinterpret_cast<int*>(base)[n] = s_arg;
+#pragma unroll
+  for (int k = 0; k < REGS; k++)
+    if (threadIdx.x + k * 256 < n) o[threadIdx.x + k * 256] = v[k] * inv;
+  for (int i = threadIdx.x + REGS * 256; i < n; i += 256) o[i] = __expf(x[i] - mx) * inv;
+  if (write_argmax && threadIdx.x == 0) reinterpret_cast<int*>(base)[n] = arg;
   if (target.state) {
     __syncthreads();
     if (threadIdx.x == 0) resp_push_complete(target);
