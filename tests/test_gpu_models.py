@@ -302,3 +302,22 @@ def test_layernorm_rows_per_block(torch_cuda, rows, hidden):
         # bf16 rounding of the result (2^-9 of it), and the fp32 mean and deviations of values about 20 times their spread
         assert ((buf[:rows].double() - ref).abs() <= ref.abs() * 2.0 ** -8 + g.abs().double() * 2e-5 + 1e-6).all()
         assert (buf[rows] == 7.0).all()
+
+
+@pytest.mark.parametrize("batch,seq,hidden", [(1, 1, 768), (1, 3, 1024), (5, 7, 768), (14, 127, 768), (14, 127, 1024)])
+def test_embedding_layernorm_tokens_per_block(torch_cuda, batch, seq, hidden):
+    """Two and four tokens per block, last blocks with tokens missing, blocks across sequences, ids outside the vocabulary."""
+    torch = torch_cuda
+    from splitrpc_b200 import ops
+
+    vocab = 50
+    word, pos, typ = (torch.randn(n, hidden, device="cuda").bfloat16() for n in (vocab, seq, 2))
+    g, b = torch.randn(hidden, device="cuda"), torch.randn(hidden, device="cuda")
+    ids = torch.randint(-5, vocab + 5, (batch, seq), device="cuda", dtype=torch.int32)
+    buf = torch.full((batch * seq + 1, hidden), 7.0, device="cuda", dtype=torch.bfloat16)
+    ops.bert_embed_ln(buf[: batch * seq], batch, seq, word, pos, typ, g, b, ids=ids)
+    x = word.double()[ids.long().clamp(0, vocab - 1)] + pos.double() + typ.double()[0]
+    ref = torch.nn.functional.layer_norm(x, (hidden,), g.double(), b.double(), 1e-12).view(batch * seq, hidden)
+    # bf16 rounding of the result, and the fp32 sums of a row
+    assert ((buf[: batch * seq].double() - ref).abs() <= ref.abs() * 2.0 ** -8 + 1e-5).all()
+    assert (buf[batch * seq] == 7.0).all()
