@@ -14,12 +14,13 @@
 // One persistent CTA per SM.  A work item is a chunk of up to MAX_TILES tiles of one image.
 //   warp 0      weights by TMA once, then one elected lane issues 16 MMAs (128 x 64 x 16) per tile into one of eight
 //               accumulators, taps in the order of the generic kernel, so that results are bit-identical to it
-//   warps 1-3   copy the next chunk's pixels with 16-byte cp.async into the other of two buffers
-//   warps 4-15  read accumulators (four warps per tile, three tiles at a time), bias, activation, bf16, transpose through a
-//               swizzled 4 KB buffer per warp, 512-byte coalesced stores
-// 64 images: 48 us (71 us in the generic kernel); the output alone takes 16 us of memory time.  What bounds it is shared
-// memory: the operand reads of the MMAs, the pixel copies and the transposing epilogue each take 5 - 10 us off when they are
-// left out, and eight epilogue warps with four accumulators took 53 us.  Waits are bounded as in gemm_persistent.cu.
+//   warps 1-3   move the next chunk's pixels through registers into the other of two buffers
+//   warps 4-15  read accumulators as 8 x 8 fragments (four warps per tile, three tiles at a time), bias from registers,
+//               activation, bf16, transpose through a swizzled 4 KB buffer per warp (stmatrix), 512-byte coalesced stores
+// 64 images: 37.8 us, 32 images 19.7 (71 us for 64 in the generic kernel; the output alone takes 16 us of memory time).  What
+// bounds it is shared memory: 48.2 us with a bias read from shared memory per value and pixels copied by cp.async, 41.8 with
+// the fragment epilogue alone; without the pixel copies it would be 31.5, with a quarter of the MMAs 33, without stores 39.
+// Waits are bounded as in gemm_persistent.cu.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -117,7 +118,8 @@ __global__ void __launch_bounds__(THREADS, 1) stem_conv_kernel(const __grid_cons
       const uint32_t idesc = ptx::umma_idesc_bf16(BM, COUT);
       const uint32_t w_lo = ptx::umma_desc_lo(ptx::smem_u32(s_w));
       // unswizzled K-major operand: core matrices along K are a plane apart, 8-pixel groups 128 bytes
-      const uint64_t a_hi = (uint64_t)((128u >> 4) | (1u << 14)) << 32;
+      constexpr uint32_t a_hi = (128u >> 4) | (1u << 14);
+      const uint32_t pitch = (uint32_t)p.pitch;
       uint32_t tile = 0;
       int it = 0;
       for (int c = blockIdx.x; ok && c < n_chunks; c += gridDim.x, it++) {
@@ -131,11 +133,13 @@ __global__ void __launch_bounds__(THREADS, 1) stem_conv_kernel(const __grid_cons
           ok = ptx::mbar_wait_warp(&acc_empty[acc], ((tile / ACC) & 1u) ^ 1u);
           if (!ok) break;
           ptx::tc_fence_after();
+          const uint32_t a0 = a_lo + (uint32_t)(r * BM);
           if (elected) {
+#pragma unroll
             for (int fr = 0; fr < TAPS; fr++)
 #pragma unroll
               for (int j = 0; j < WIN; j++)
-                ptx::umma_bf16(tmem + acc * COUT, a_hi | (a_lo + (uint32_t)(r * BM + fr * p.pitch + j)),
+                ptx::umma_bf16(tmem + acc * COUT, ((uint64_t)a_hi << 32) | (a0 + fr * pitch + j),
                                ptx::umma_desc_join(w_lo + (uint32_t)(fr * COUT * 128 / 16 + j * 2)), idesc, (fr | j) != 0 ? 1u : 0u);
             ptx::umma_commit(&acc_full[acc]);
           }
@@ -144,37 +148,40 @@ __global__ void __launch_bounds__(THREADS, 1) stem_conv_kernel(const __grid_cons
       }
       if (!ok && elected) atomicCAS(&s_error, 0u, (uint32_t)GEMM_ERR_MMA_WAIT);
     } else if (warp < 1 + LOADERS / 32) {
-      // ---------------- pixels of chunk c into buffer it & 1; the copies of one chunk are in flight while the previous one
-      // is handed over
-      const int lt = threadIdx.x - 32;
+      // ---------------- pixels of chunk c into buffer it & 1.  A warp moves 16 pixels at a time through registers: its eight-lane
+      // groups store 128 bytes of one plane each.  (cp.async writes a pixel's two halves, which lie in different planes, 16 bytes
+      // at a time: 10 us of 64 images' 42 were that.)
+      const int lw = warp - 1, plane = (lane >> 3) & 1, px_in_unit = (lane & 7) + ((lane >> 4) << 3);
       const uint8_t* img0 = p.in_stub ? *reinterpret_cast<uint8_t* const*>(p.in_stub) : p.in;
       const int img_pix = p.pitch * p.in_rows;
-      auto hand_over = [&](int it) {
-        ptx::fence_proxy_async_smem();
-        ptx::mbar_arrive(&full_bar[it & 1]);
-      };
       int it = 0;
       for (int c = blockIdx.x; c < n_chunks; c += gridDim.x, it++) {
-        if (!ptx::mbar_wait(&empty_bar[it & 1], ((it >> 1) & 1) ^ 1u)) {
-          atomicCAS(&s_error, 0u, (uint32_t)GEMM_ERR_PRODUCER_WAIT);
+        if (!ptx::mbar_wait_warp(&empty_bar[it & 1], ((it >> 1) & 1) ^ 1u)) {
+          if (lane == 0) atomicCAS(&s_error, 0u, (uint32_t)GEMM_ERR_PRODUCER_WAIT);
           break;
         }
         const int img = c / p.chunks_per_img, first = (c - img * p.chunks_per_img) * chunk_pos;
         const int n_pix = tiles_of(c) * BM + (TAPS - 1) * p.pitch + WIN - 1;
-        const uint8_t* src = img0 + (size_t)img * p.img_bytes + (size_t)first * 32;
-        uint8_t* dst = s_in + (it & 1) * BUF_BYTES;
-        for (int q = lt; q < 2 * n_pix; q += LOADERS) {
-          const bool inside = first + (q >> 1) < img_pix;  // past the image: zeros
-          ptx::cp_async_16(dst + (q & 1) * PLANE + (q >> 1) * 16, inside ? src + (size_t)q * 16 : img0, inside);
+        const int inside = min(n_pix, img_pix - first);  // past the image: zeros
+        const uint8_t* src = img0 + (size_t)img * p.img_bytes + (size_t)first * 32 + plane * 16;
+        uint8_t* dst = s_in + (it & 1) * BUF_BYTES + plane * PLANE;
+        constexpr int AHEAD = 8;  // loads in flight per thread
+        for (int base = lw * 16 + px_in_unit; base < n_pix; base += AHEAD * LOADERS / 2) {
+          uint4 q[AHEAD];
+#pragma unroll
+          for (int k = 0; k < AHEAD; k++) {
+            const int px = base + k * (LOADERS / 2);
+            q[k] = px < inside ? *reinterpret_cast<const uint4*>(src + (size_t)px * 32) : make_uint4(0u, 0u, 0u, 0u);
+          }
+#pragma unroll
+          for (int k = 0; k < AHEAD; k++) {
+            const int px = base + k * (LOADERS / 2);
+            if (px < n_pix) *reinterpret_cast<uint4*>(dst + px * 16) = q[k];
+          }
         }
-        ptx::cp_async_commit();
-        if (it > 0) {
-          ptx::cp_async_wait<1>();
-          hand_over(it - 1);
-        }
+        ptx::fence_proxy_async_smem();
+        ptx::mbar_arrive(&full_bar[it & 1]);
       }
-      ptx::cp_async_wait<0>();
-      if (it > 0) hand_over(it - 1);
       if (p.late_trigger && warp == 1) {
         __syncwarp();
         ptx::grid_dep_launch();
@@ -183,6 +190,9 @@ __global__ void __launch_bounds__(THREADS, 1) stem_conv_kernel(const __grid_cons
       // ---------------- epilogue: each set of four warps takes every third tile; a warp has 32 positions
       const int ew = warp - 4, set = ew >> 2, quarter = warp & 3;
       uint8_t* stage = s_out + ew * STAGE_BYTES;
+      float2 bias[8];
+#pragma unroll
+      for (int g = 0; g < 8; g++) bias[g] = make_float2(s_bias[g * 8 + (lane & 3) * 2], s_bias[g * 8 + (lane & 3) * 2 + 1]);
       uint32_t tile = 0;
       bool ok = true;
       for (int c = blockIdx.x; ok && c < n_chunks; c += gridDim.x) {
@@ -194,30 +204,30 @@ __global__ void __launch_bounds__(THREADS, 1) stem_conv_kernel(const __grid_cons
           ok = ptx::mbar_wait_warp(&acc_full[acc], (tile / ACC) & 1u);
           if (!ok) break;
           ptx::tc_fence_after();
-          uint32_t v[2][32];
+          // 32 positions x 64 channels as 8 x 8 fragments (see gemm_2sm.cu): a thread's bias is 16 values for the whole launch
+          uint32_t v[4][16];  // [half of the channels][half of the positions]
           const uint32_t at = tmem + acc * COUT + ((uint32_t)(quarter * 32) << 16);
-          ptx::tmem_ld_32x32b_x32(at, v[0]);
-          ptx::tmem_ld_32x32b_x32(at + 32, v[1]);
+#pragma unroll
+          for (int q = 0; q < 4; q++) ptx::tmem_ld_16x256b_x4(at + (q >> 1) * 32 + ((uint32_t)((q & 1) * 16) << 16), v[q]);
           ptx::tmem_ld_wait();
           ptx::tc_fence_before();
           __syncwarp();
           if (lane == 0) ptx::mbar_arrive(&acc_empty[acc]);
 #pragma unroll
-          for (int q = 0; q < 8; q++) {  // 16-byte pieces of this lane's position
-            uint4 o;
-            __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&o);
+          for (int q = 0; q < 4; q++) {
+            uint32_t o[8];  // [channel group][position group of 8]
 #pragma unroll
-            for (int t = 0; t < 4; t++) {
-              const int ch = q * 8 + 2 * t;
-              float f0 = __uint_as_float(v[q >> 2][(q & 3) * 8 + 2 * t]) + s_bias[ch];
-              float f1 = __uint_as_float(v[q >> 2][(q & 3) * 8 + 2 * t + 1]) + s_bias[ch + 1];
-              if (p.relu) {
-                f0 = fmaxf(f0, 0.f);
-                f1 = fmaxf(f1, 0.f);
-              }
-              h[t] = __floats2bfloat162_rn(f0, f1);
+            for (int k = 0; k < 8; k++) {
+              float2 f = __fadd2_rn(make_float2(__uint_as_float(v[q][2 * k]), __uint_as_float(v[q][2 * k + 1])), bias[(q >> 1) * 4 + (k >> 1)]);
+              if (p.relu) f = make_float2(fmaxf(f.x, 0.f), fmaxf(f.y, 0.f));
+              const __nv_bfloat162 h = __floats2bfloat162_rn(f.x, f.y);
+              o[k] = *reinterpret_cast<const uint32_t*>(&h);
             }
-            *reinterpret_cast<uint4*>(stage + lane * 128 + ((q ^ (lane & 7)) << 4)) = o;
+            const int row = (q & 1) * 16 + (lane & 15);
+#pragma unroll
+            for (int g = 0; g < 4; g += 2)  // the two position groups of channel groups g, g + 1
+              ptx::stmatrix_x4(ptx::smem_u32(stage) + row * 128 + ((((q >> 1) * 4 + g + (lane >> 4)) ^ (row & 7)) << 4), o[2 * g], o[2 * g + 1],
+                               o[2 * g + 2], o[2 * g + 3]);
           }
           __syncwarp();
           const int pos0 = first + r * BM + quarter * 32 + (lane >> 3);
