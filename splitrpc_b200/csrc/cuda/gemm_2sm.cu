@@ -117,6 +117,10 @@ struct TileOrder {
   int clusters;  // clusters that compute tiles (the grid may hold copier clusters after them)
   int tiles_m2, tiles_n;
   int group_m;   // pair row blocks per group
+  // From the last tile to the first.  Products that read more than they write go this way: the rows that the kernel before wrote
+  // last are still in the L2 cache, and the rows read last are again when a later product takes them as its residual, in order
+  // (200704 x 64 x 256 behind the layer that writes its 103 MB 21.7 -> 18.5 us; ResNet-50, 64 images 936 -> 930).
+  int reverse;
   int m_rot2;    // rotation of the pair row blocks (tensor-parallel: which rank's rows come first)
   int late_trigger;  // the next kernel starts behind this CTA's last load only (pdl_launch.h)
   FastDiv fd_group, fd_gm;  // by group_m * tiles_n and group_m
@@ -126,8 +130,9 @@ struct TileOrder {
 // tiles, about a square.  8192^3 runs at the power limit, and what it does not read again from DRAM it has for the tensor
 // cores: 875 us with groups of four row blocks, 848 with eight, 880 with sixteen.
 __device__ __forceinline__ bool pair_tile(int j, const TileOrder& o, PairTile* out) {
-  const int tile = (int)(blockIdx.x >> 1) + j * o.clusters;
+  int tile = (int)(blockIdx.x >> 1) + j * o.clusters;
   if (tile >= o.tiles_m2 * o.tiles_n) return false;
+  if (o.reverse) tile = o.tiles_m2 * o.tiles_n - 1 - tile;
   const int g = (int)fdiv(o.fd_group, (uint32_t)tile), in_g = tile - g * o.group_m * o.tiles_n;
   const int m_first = g * o.group_m;
   int m2;
@@ -691,6 +696,7 @@ cudaError_t launch_2sm(const AInput& in, const void* B, int ldb, int M, int N, i
   TileOrder o;
   order_tiles(&o, M, N, 2 * RPC, BN, std::min(max_clusters, srpc_gemm_grid_sms() / 2), 8);
   o.m_rot2 = 0;
+  o.reverse = K > N;
   o.late_trigger = srpc_gemm_reserved_sms() > 0;
   return launch_pdl(gemm_2sm_kernel<BN, RPC, false>, dim3(2 * o.clusters), dim3(C::THREADS), C::SMEM_BYTES, stream, ta, tb, to, ta2, M,
                     N, K, o, src, ep, status, TpParams{});
@@ -740,6 +746,7 @@ cudaError_t launch_2sm_tp(const void* A, int lda, const void* B, int ldb, int M,
   TileOrder o;
   order_tiles(&o, M, N, 2 * BM, BN, max_clusters - copy_clusters, group_m);
   o.late_trigger = 0;
+  o.reverse = 0;
   // all-gather: own rows first (they are here already); reduce-scatter: own rows last (the peers' cross NVLink)
   o.m_rot2 = (tp.rs ? (tp.rank + 1) % tp.tp : tp.rank) * m2_per_rank;
   tp.tiles_per_owner = tp.mblocks_per_rank * o.tiles_n;
