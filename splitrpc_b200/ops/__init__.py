@@ -19,7 +19,8 @@ GEMM_IMPL = int(__import__("os").environ.get("SPLITRPC_GEMM_IMPL", "2"))
 
 
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    # The handle itself: a torch.cuda.Stream object around it costs 3 us of a call that otherwise takes 7.
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
 def _ptr(t: torch.Tensor | None) -> int:
