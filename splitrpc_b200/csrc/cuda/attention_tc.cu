@@ -5,6 +5,11 @@
 //   P = softmax(scores)   8 or 16 warps, 1/2 or 1/4 of a query row per thread, from TMEM,
 //                         written as bf16 into 128-byte-swizzled shared memory
 //   O = P . V             tcgen05.mma, M=128, N=64, K=SEQ, fp32 in TMEM
+// With several tiles the scores of tile t+1 are issued before the P.V of tile t, and the output of tile t-1 leaves while
+// they are computed (two output accumulators): what stays in series per tile of 384 keys is scores (0.8 us with the hand-over),
+// maxima and their exchange (0.6 us) and the exponentials (2.0 us; 1.6 us of the special-function unit).  16 x 384 tokens of
+// 16 heads, two rounds of CTAs: 32.2 us with each tile's steps in sequence, 31.2 with the scores first, 29.3 with the
+// output behind them; 1 x 384: 15.7 -> 14.4.
 // All operands arrive by TMA (no multicast) from this GPU's memory:
 //   Q and K from the [tokens, 2*hidden] output of the fused Q|K projection,
 //   V^T from the [hidden, tokens] output of the V projection computed with
@@ -49,7 +54,7 @@ struct AttSmem {
   static constexpr bool ALIAS = SEQ == QT;
   static constexpr int P_OFFSET = ALIAS ? 0 : Q_BYTES + K_BYTES + VT_BYTES;
   static constexpr int TOTAL = ALIAS ? Q_BYTES + K_BYTES + VT_BYTES : Q_BYTES + K_BYTES + VT_BYTES + P_BYTES;
-  static constexpr int TMEM_COLS = ALIAS ? 128 : ((SEQ + HD) <= 256 ? 256 : 512);
+  static constexpr int TMEM_COLS = ALIAS ? 128 : ((SEQ + 2 * HD) <= 256 ? 256 : 512);
   static_assert(!ALIAS || P_BYTES <= Q_BYTES + K_BYTES, "P must fit over Q and K");
 };
 
@@ -88,7 +93,7 @@ attention_tc(const __grid_constant__ CUtensorMap tmap_qk, const __grid_constant_
   __shared__ __align__(8) uint64_t bar_k, bar_v, bar_q, bar_s, bar_p, bar_o;
   __shared__ uint32_t tmem_base_smem;
   __shared__ uint32_t s_error;
-  __shared__ float s_max[SHARES][QT], s_sum[SHARES][QT];
+  __shared__ float s_max[SHARES][QT], s_sum[2][SHARES][QT];  // sums of alternating tiles
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int head = blockIdx.x, seq_idx = blockIdx.y;
@@ -117,7 +122,8 @@ attention_tc(const __grid_constant__ CUtensorMap tmap_qk, const __grid_constant_
   ptx::grid_dep_wait();
   ptx::tc_fence_after();
   const uint32_t tmem_s = tmem_base_smem;          // scores: columns [0, SEQ)
-  const uint32_t tmem_o = tmem_base_smem + (L::ALIAS ? 0 : SEQ);  // output: columns [SEQ, SEQ+64), or over the scores
+  // Outputs of alternating tiles: columns [SEQ, SEQ+64) and [SEQ+64, SEQ+128), or, with one tile, over the scores.
+  auto tmem_o = [&](int qt) { return tmem_base_smem + (L::ALIAS ? 0 : SEQ + (qt & 1) * HD); };
 
   if (warp == SOFT_THREADS / 32) {
     // The warp walks the tiles together, one elected lane issues: descriptors and addresses stay in uniform registers
@@ -168,20 +174,20 @@ attention_tc(const __grid_constant__ CUtensorMap tmap_qk, const __grid_constant_
       // P ready (written by the softmax warps, which have read all scores by then)
       if (!(ok = ptx::mbar_wait_warp(&bar_p, ph))) break;
       ptx::tc_fence_after();
+      // The next tile's scores go first: its maxima are looked for while P.V runs.
+      if (qt + 1 < NQT) {
+        if (!(ok = ptx::mbar_wait_warp(&bar_q, ph ^ 1u))) break;
+        scores();
+      }
       if (elected) {
 #pragma unroll
         for (int kk = 0; kk < SEQ / 16; kk++) {
           const uint32_t atom = (uint32_t)kk >> 2, sub = (uint32_t)kk & 3u;
           const uint32_t v_at = VMN ? (uint32_t)kk * (2048 / 16) : atom * (64 * 128 / 16) + sub * 2;
-          ptx::umma_bf16(tmem_o, ptx::umma_desc_join(p_lo + atom * (QT * 128 / 16) + sub * 2), ptx::umma_desc_join(v_lo + v_at),
+          ptx::umma_bf16(tmem_o(qt), ptx::umma_desc_join(p_lo + atom * (QT * 128 / 16) + sub * 2), ptx::umma_desc_join(v_lo + v_at),
                          idesc_o, kk != 0 ? 1u : 0u);
         }
         ptx::umma_commit(&bar_o);
-      }
-      // The next tile's scores run behind P.V, while the output is written.
-      if (qt + 1 < NQT) {
-        if (!(ok = ptx::mbar_wait_warp(&bar_q, ph ^ 1u))) break;
-        scores();
       }
     }
     if (!ok && elected) atomicCAS(&s_error, 0u, 1u);
@@ -191,10 +197,39 @@ attention_tc(const __grid_constant__ CUtensorMap tmap_qk, const __grid_constant_
     constexpr int COLS = SEQ / SHARES;
     const int c0 = share * COLS;
     const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
+    // Output of tile qt: every share writes its part of the head's 64 columns.
+    auto output = [&](int qt) {
+      constexpr int OC = HD / SHARES;
+      float total = s_sum[qt & 1][0][row];
+#pragma unroll
+      for (int k = 1; k < SHARES; k++) total += s_sum[qt & 1][k][row];
+      const float inv = 1.f / total;
+      __nv_bfloat16* orow = out + (size_t)(tok0 + qt * QT + row) * ld_out + head * HD;
+      const int c = share * OC;
+      uint32_t r[OC];
+      if constexpr (OC == 32) ptx::tmem_ld_32x32b_x32(tmem_o(qt) + lane_base + c, r);
+      else ptx::tmem_ld_32x32b_x16(tmem_o(qt) + lane_base + c, r);
+      ptx::tmem_ld_wait();
+#pragma unroll
+      for (int j = 0; j < OC / 8; j++) {
+        uint4 q;
+        __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&q);
+#pragma unroll
+        for (int t = 0; t < 4; t++) {
+          const int d = c + j * 8 + 2 * t;
+          const float b0 = v_bias ? *(v_bias + head * HD + d) : 0.f;
+          const float b1 = v_bias ? *(v_bias + head * HD + d + 1) : 0.f;
+          h[t] = __floats2bfloat162_rn(__uint_as_float(r[j * 8 + 2 * t]) * inv + b0,
+                                       __uint_as_float(r[j * 8 + 2 * t + 1]) * inv + b1);
+        }
+        *reinterpret_cast<uint4*>(orow + c + j * 8) = q;
+      }
+    };
+    bool ok = true;
     for (int qt = 0; qt < NQT; qt++) {
       const uint32_t ph = (uint32_t)qt & 1u;
-      const bool got = *(volatile uint32_t*)&s_error == 0 && ptx::mbar_wait(&bar_s, ph);
-      if (!soft_all<SOFT_THREADS>(got)) {
+      ok = *(volatile uint32_t*)&s_error == 0 && ptx::mbar_wait(&bar_s, ph);
+      if (!(ok = soft_all<SOFT_THREADS>(ok))) {
         if (lane == 0) atomicCAS(&s_error, 0u, 2u);
         break;
       }
@@ -206,17 +241,21 @@ attention_tc(const __grid_constant__ CUtensorMap tmap_qk, const __grid_constant_
         ptx::tmem_ld_32x32b_x32(tmem_s + lane_base + c0 + c, r);
         ptx::tmem_ld_wait();
 #pragma unroll
-        for (int j = 0; j < 32; j++) mx = fmaxf(mx, __uint_as_float(r[j]));
+        for (int j = 0; j < 32; j += 2) mx = ptx::max3(mx, __uint_as_float(r[j]), __uint_as_float(r[j + 1]));
       }
       s_max[share][row] = mx;
-      soft_sync<SOFT_THREADS>();
+      // behind the barrier the previous tile's P.V is through as well, and P may be written again
+      if (!(ok = soft_all<SOFT_THREADS>(qt == 0 || ptx::mbar_wait(&bar_o, ph ^ 1u)))) {
+        if (lane == 0) atomicCAS(&s_error, 0u, 3u);
+        break;
+      }
+      ptx::tc_fence_after();
 #pragma unroll
       for (int k = 0; k < SHARES; k++) mx = fmaxf(mx, s_max[k][row]);
       // pass 2: exponentials, row sum, P in bf16 to swizzled shared memory.  Packed differences and products; the fast exponential
       // flushes subnormal results, so 32 weights of which one may be subnormal (below 2^-126 of the row's largest) are made
-      // again with exp2f.  16 x 384 x 16 heads / 32 x 128 x 12 heads: 32.2 / 8.5 us; exp2f for every weight 35.1 / 8.7 us, subnormal
-      // weights lost 31.3 / 8.3 us.
-      float sum = 0.f;
+      // again with exp2f.
+      float2 sum = make_float2(0.f, 0.f);
       const float2 neg_mx = make_float2(-mx, -mx), scale2 = make_float2(scale_log2e, scale_log2e);
       for (int c = c0; c < c0 + COLS; c += 32) {
         uint32_t r[32];
@@ -224,7 +263,7 @@ attention_tc(const __grid_constant__ CUtensorMap tmap_qk, const __grid_constant_
         ptx::tmem_ld_wait();
         uint8_t* prow = sP + (size_t)(c >> 6) * QT * 128 + (size_t)row * 128;
         const int chunk0 = (c & 63) >> 3;
-        const float sum_before = sum;
+        const float2 sum_before = sum;
         float least = 0.f;  // smallest exponent
         auto weights = [&](auto exponential) {
 #pragma unroll
@@ -236,10 +275,8 @@ attention_tc(const __grid_constant__ CUtensorMap tmap_qk, const __grid_constant_
               const float2 x = make_float2(__uint_as_float(r[j * 8 + 2 * t]), __uint_as_float(r[j * 8 + 2 * t + 1]));
               const float2 y = __fmul2_rn(__fadd2_rn(x, neg_mx), scale2);
               h[t] = __floats2bfloat162_rn(exponential(y.x), exponential(y.y));
-              least = fminf(least, fminf(y.x, y.y));
-              // the row sum uses the rounded values that the second product will see
-              float2 back = __bfloat1622float2(h[t]);
-              sum += back.x + back.y;
+              least = ptx::min3(least, y.x, y.y);
+              sum = __fadd2_rn(sum, __bfloat1622float2(h[t]));  // of the rounded values that the second product will see
             }
             *reinterpret_cast<uint4*>(prow + (((chunk0 + j) ^ (row & 7)) << 4)) = q;
           }
@@ -254,41 +291,20 @@ attention_tc(const __grid_constant__ CUtensorMap tmap_qk, const __grid_constant_
           weights([](float y) { return exp2f(y); });
         }
       }
-      s_sum[share][row] = sum;
+      s_sum[qt & 1][share][row] = sum.x + sum.y;
       ptx::tc_fence_before();
       ptx::fence_proxy_async_smem();
       __syncwarp();
       if (lane == 0) ptx::mbar_arrive(&bar_p);
-      // output tile: the first two shares write 32 of the head's 64 columns each
-      if (!soft_all<SOFT_THREADS>(ptx::mbar_wait(&bar_o, ph))) {
-        if (lane == 0) atomicCAS(&s_error, 0u, 3u);
-        break;
-      }
+      // The previous tile's output leaves while the tensor core works on the next scores.
+      if (qt > 0) output(qt - 1);
+      ptx::tc_fence_before();
+    }
+    if (ok) {
+      ok = soft_all<SOFT_THREADS>(ptx::mbar_wait(&bar_o, (uint32_t)(NQT - 1) & 1u));
+      if (!ok && lane == 0) atomicCAS(&s_error, 0u, 3u);
       ptx::tc_fence_after();
-      if (share >= 2) continue;
-      float total = s_sum[0][row];
-#pragma unroll
-      for (int k = 1; k < SHARES; k++) total += s_sum[k][row];
-      const float inv = 1.f / total;
-      __nv_bfloat16* orow = out + (size_t)(tok0 + qt * QT + row) * ld_out + head * HD;
-      const int c = share * 32;
-      uint32_t r[32];
-      ptx::tmem_ld_32x32b_x32(tmem_o + lane_base + c, r);
-      ptx::tmem_ld_wait();
-#pragma unroll
-      for (int j = 0; j < 4; j++) {
-        uint4 q;
-        __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&q);
-#pragma unroll
-        for (int t = 0; t < 4; t++) {
-          const int d = c + j * 8 + 2 * t;
-          const float b0 = v_bias ? *(v_bias + head * HD + d) : 0.f;
-          const float b1 = v_bias ? *(v_bias + head * HD + d + 1) : 0.f;
-          h[t] = __floats2bfloat162_rn(__uint_as_float(r[j * 8 + 2 * t]) * inv + b0,
-                                       __uint_as_float(r[j * 8 + 2 * t + 1]) * inv + b1);
-        }
-        *reinterpret_cast<uint4*>(orow + c + j * 8) = q;
-      }
+      if (ok) output(NQT - 1);
       ptx::tc_fence_before();
     }
   }
