@@ -154,6 +154,26 @@ void bind_ops(py::module_& m) {
         py::arg("ring_slots") = 0, py::arg("slot_bytes") = 0, py::arg("in2") = 0, py::arg("h2") = 0, py::arg("w2") = 0,
         py::arg("cin2") = 0, py::arg("stride2") = 1);
 
+  m.def("conv_chain",
+        [](uintptr_t x, uintptr_t x2, uintptr_t w_wide, uintptr_t b_wide, uintptr_t residual, uintptr_t w_narrow, uintptr_t b_narrow,
+           uintptr_t wide, uintptr_t narrow, int pixels, int narrow_channels, uintptr_t status, uintptr_t stream) {
+          ConvChain c;
+          c.x = (const void*)x;
+          c.x2 = (const void*)x2;
+          c.w_wide = (const void*)w_wide;
+          c.b_wide = (const float*)b_wide;
+          c.residual = (const void*)residual;
+          c.w_narrow = (const void*)w_narrow;
+          c.b_narrow = (const float*)b_narrow;
+          c.wide = (void*)wide;
+          c.narrow = (void*)narrow;
+          c.pixels = pixels;
+          c.narrow_channels = narrow_channels;
+          check(srpc_conv_chain(c, (uint32_t*)status, (cudaStream_t)stream), "conv_chain");
+        },
+        py::arg("x"), py::arg("x2"), py::arg("w_wide"), py::arg("b_wide"), py::arg("residual"), py::arg("w_narrow"),
+        py::arg("b_narrow"), py::arg("wide"), py::arg("narrow"), py::arg("pixels"), py::arg("narrow_channels"), py::arg("status"),
+        py::arg("stream"));
   m.def("gemm_reserve_sms", [](int n) { srpc_gemm_reserve_sms(n); }, py::arg("n"));
   m.def("gemm_grid_sms", []() { return srpc_gemm_grid_sms(); });
   m.def("gemm_reserved_sms", []() { return srpc_gemm_reserved_sms(); });

@@ -76,6 +76,18 @@ bool srpc_conv_2sm_eligible(const ConvShape& cs, const GemmEpilogue& ep);
 cudaError_t srpc_conv_bf16_2sm(const void* input, const void* weight, const ConvShape& cs, int bn, int rows, const GemmEpilogue& ep,
                                uint32_t* status, cudaStream_t stream);
 
+// Expansion to 256 channels and the next block's reduction to 64 or 128 in one kernel (conv_chain.cu):
+//   wide = relu(w_wide . [x; x2] + b_wide + residual), narrow = relu(w_narrow . wide + b_narrow)
+// over `pixels` dense pixels of 64 channels.  Either a second input x2 (then 64 narrow channels) or a residual; pointers 16-byte
+// aligned.
+struct ConvChain {
+  const void *x = nullptr, *x2 = nullptr, *w_wide = nullptr, *w_narrow = nullptr, *residual = nullptr;
+  const float *b_wide = nullptr, *b_narrow = nullptr;
+  void *wide = nullptr, *narrow = nullptr;
+  int pixels = 0, narrow_channels = 0;
+};
+cudaError_t srpc_conv_chain(const ConvChain& c, uint32_t* status, cudaStream_t stream);
+
 // Leaves `n` SMs out of the grids of the persistent kernels (see num_sms in gemm_persistent.cu); takes effect for
 // launches (and graph captures) made afterwards.  srpc_gemm_grid_sms returns the SM count the grids are sized for.
 void srpc_gemm_reserve_sms(int n);

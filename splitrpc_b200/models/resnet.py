@@ -101,7 +101,8 @@ class ResNet50:
                 self.buf[name + ".ds"] = torch.empty((nb, ho, ho, width * 4), dtype=bf, device=dev)
             h = ho
         per_ds = 0 if self.fuse_shortcut else 1
-        self.kernels_per_forward = self._kernels_per_forward_base = 3 + sum(3 + (per_ds if b[4] else 0) for b in self.blocks) + 3
+        self.kernels_per_forward = self._kernels_per_forward_base = (
+            3 + sum(3 + (per_ds if b[4] else 0) - self._chained(i) for i, b in enumerate(self.blocks)) + 3)
         self.ingress_ring = None
 
     # ------------------------------------------------------------------ forward
@@ -113,6 +114,18 @@ class ResNet50:
         ops.gemm(x.view(n * h * w, cin), wt.view(cout, cin), bias=self.params[name + ".b"],
                  residual=None if residual is None else residual.view(n * h * w, cout), act=act,
                  out=out.view(n * h * w, cout))
+        return out
+
+    def _chained(self, i: int) -> bool:
+        """Whether block ``i``'s last convolution and the next block's first run as one kernel (both filters fit a CTA's memory)."""
+        return self.blocks[i][2] == 64
+
+    def _expand_reduce(self, i: int, t2, nb: int, residual=None, x2=None):
+        name, nxt, p, b = self.blocks[i][0], self.blocks[i + 1][0], self.params, self.buf
+        c3 = name + (".c3" if x2 is None else ".c3ds")
+        out = b[name + ".out"][:nb]
+        ops.conv1x1_chain(t2, p[c3 + ".w"], p[c3 + ".b"], p[nxt + ".c1.w"], p[nxt + ".c1.b"], out, b[nxt + ".t1"][:nb],
+                          residual=residual, x2=x2)
         return out
 
     def enable_fused_ingress(self, ring_base: int, ring_slots: int, slot_bytes: int) -> dict:
@@ -142,10 +155,15 @@ class ResNet50:
             ops.stem_s2d(b["s2d"], nb, x=x, d_stub=d_stub, mean=self.mean, inv_std=self.inv_std)
             ops.stem_conv(b["s2d"], p["stem.w_s2d"], nb, bias=p["stem.b"], act="relu", out=b["stem"][:nb])
         cur = ops.maxpool3x3s2(b["stem"][:nb], out=b["pool"][:nb])
-        for name, cin, width, s, ds in self.blocks:
-            t1 = self._conv1x1(cur, name + ".c1", b[name + ".t1"][:nb], "relu")
+        reduced = False  # this block's first convolution ran with the last one of the block before
+        for i, (name, cin, width, s, ds) in enumerate(self.blocks):
+            t1 = b[name + ".t1"][:nb] if reduced else self._conv1x1(cur, name + ".c1", b[name + ".t1"][:nb], "relu")
             t2 = ops.conv2d_nhwc(t1, p[name + ".c2.w"], bias=p[name + ".c2.b"], stride=s, pad=1, act="relu",
                                  out=b[name + ".t2"][:nb])
+            reduced = self._chained(i)
+            if ds and self.fuse_shortcut and reduced:
+                cur = self._expand_reduce(i, t2, nb, x2=cur)
+                continue
             if ds and self.fuse_shortcut:
                 cur = ops.conv1x1_dual(t2, cur, p[name + ".c3ds.w"], bias=p[name + ".c3ds.b"], stride2=s, act="relu",
                                        out=b[name + ".out"][:nb])
@@ -158,6 +176,9 @@ class ResNet50:
                                           out=b[name + ".ds"][:nb])
             else:
                 idn = cur
+            if reduced:
+                cur = self._expand_reduce(i, t2, nb, residual=idn)
+                continue
             cur = self._conv1x1(t2, name + ".c3", b[name + ".out"][:nb], "relu", residual=idn)
         avg = ops.global_avgpool(cur, out=b["avg"][:nb])
         if nb <= 64:

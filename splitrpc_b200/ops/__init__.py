@@ -123,6 +123,23 @@ def conv1x1_dual(x1: torch.Tensor, x2: torch.Tensor, w: torch.Tensor, bias: torc
     return out
 
 
+def conv1x1_chain(x: torch.Tensor, w_wide: torch.Tensor, b_wide: torch.Tensor, w_narrow: torch.Tensor, b_narrow: torch.Tensor,
+                  wide: torch.Tensor, narrow: torch.Tensor, residual: torch.Tensor | None = None,
+                  x2: torch.Tensor | None = None) -> None:
+    """``wide = relu(w_wide . [x; x2] + b_wide + residual)`` and ``narrow = relu(w_narrow . wide + b_narrow)`` in one kernel: a
+    bottleneck's expansion to 256 channels, with its residual or its projected shortcut ``x2``, and the next one's reduction to
+    64 or 128.  All NHWC over the same pixels, inputs of 64 channels."""
+    px, n2 = x.numel() // 64, w_narrow.shape[0]
+    for t in (x, w_wide, w_narrow, wide, narrow, residual, x2):
+        assert t is None or (t.is_cuda and t.dtype == torch.bfloat16 and t.is_contiguous())
+    assert (x2 is None) != (residual is None) and x.shape[-1] == 64 and (x2 is None or x2.shape == x.shape)
+    assert w_wide.numel() == 256 * 64 * (1 if x2 is None else 2) and w_narrow.numel() == n2 * 256 and n2 in ((64, 128) if x2 is None else (64,))
+    assert wide.numel() == px * 256 and narrow.numel() == px * n2 and (residual is None or residual.numel() == px * 256)
+    assert b_wide.dtype == b_narrow.dtype == torch.float32 and b_wide.numel() == 256 and b_narrow.numel() == n2
+    _C.conv_chain(x.data_ptr(), _ptr(x2), w_wide.data_ptr(), b_wide.data_ptr(), _ptr(residual), w_narrow.data_ptr(), b_narrow.data_ptr(),
+                  wide.data_ptr(), narrow.data_ptr(), px, n2, status_word().data_ptr(), _stream())
+
+
 def sg_copy(items, impl: int = 0, n_blocks: int = 0) -> None:
     """Runs a copy list ``[(src_addr, dst_addr, nbytes)]`` on the current stream and waits for it."""
     _C.sg_copy(list(items), impl, n_blocks, _stream())

@@ -49,6 +49,10 @@ def _work(name, args, kwargs, out):
         st = kwargs.get("stride2", 1)
         by = 2 * (x1.numel() + x2.numel() // (st * st) + w.numel() + out.numel())
         return 2.0 * out.numel() * w.shape[1], by, f"{tuple(x1.shape)}+{tuple(x2.shape)}/s{st}->{w.shape[0]}"
+    if name == "conv1x1_chain":
+        px, k, n2 = args[5].numel() // 256, args[1].numel() // 256, args[3].shape[0]
+        by = 2 * px * (k + 256 + n2 + (256 if kwargs.get("residual") is not None else 0))
+        return 2.0 * px * 256 * (k + n2), by, f"{px} px {k}->256->{n2}"
     if name == "stem_s2d":
         batch = args[1]
         return 0.0, batch * (3 * 224 * 224 * 4 + 115 * 115 * 16 * 2), f"b{batch}"
@@ -94,7 +98,7 @@ def main():
 
     records = []
     if not args.no_events:
-        for name in ("gemm", "fc_skinny", "conv2d_nhwc", "conv1x1_dual", "stem_im2col", "stem_s2d", "stem_conv", "maxpool3x3s2", "global_avgpool", "softmax_response", "layernorm",
+        for name in ("gemm", "fc_skinny", "conv2d_nhwc", "conv1x1_dual", "conv1x1_chain", "stem_im2col", "stem_s2d", "stem_conv", "maxpool3x3s2", "global_avgpool", "softmax_response", "layernorm",
                      "bert_embed_ln", "attention_d64"):
             fn = getattr(ops, name)
 

@@ -116,6 +116,29 @@ def test_two_input_pointwise_conv(env, n, oh, c1, h2, c2, cout, stride2):
     assert _rel_err(torch, out, torch.relu(ref)) < 1e-2
 
 
+@pytest.mark.parametrize("narrow,second", [(64, False), (128, False), (64, True)])
+@pytest.mark.parametrize("n,h,w", [(1, 1, 1), (1, 8, 16), (2, 13, 11), (7, 56, 56), (40, 31, 31)])
+def test_expansion_and_reduction_in_one_kernel(env, n, h, w, narrow, second):
+    """One pixel, one whole tile, a ragged last tile, more tiles than SMs: the bits of the two separate kernels, nothing behind them."""
+    torch, ops = env
+    px, k = n * h * w, 128 if second else 64
+    x, x2 = ((torch.randn(n, h, w, 64, device="cuda")).bfloat16() for _ in range(2))
+    residual = torch.randn(n, h, w, 256, device="cuda").bfloat16()
+    w3, w1 = (torch.randn(256, k, device="cuda") * 0.1).bfloat16(), (torch.randn(narrow, 256, device="cuda") * 0.1).bfloat16()
+    b3, b1 = torch.randn(256, device="cuda"), torch.randn(narrow, device="cuda")
+    wide, nar = (torch.full((px + 128, c), 7.0, device="cuda", dtype=torch.bfloat16) for c in (256, narrow))
+    ops.conv1x1_chain(x, w3, b3, w1, b1, wide[:px].view(n, h, w, 256), nar[:px].view(n, h, w, narrow),
+                      residual=None if second else residual, x2=x2 if second else None)
+    ops.check_status()
+    a = torch.cat([x, x2], dim=3).view(px, 128) if second else x.view(px, 64)
+    want = ops.gemm(a, w3, bias=b3, residual=None if second else residual.view(px, 256), act="relu")
+    assert torch.equal(wide[:px], want) and torch.equal(nar[:px], ops.gemm(want, w1, bias=b1, act="relu"))
+    assert (wide[px:] == 7.0).all() and (nar[px:] == 7.0).all()
+    ref = torch.relu(a.double() @ w3.double().t() + b3 + (0 if second else residual.view(px, 256).double()))
+    # half a unit of bf16 (2^-9 of the value), and the fp32 sums: K 2^-24 times the sum of |products| (about 0.064 K)
+    assert ((want.double() - ref).abs() <= ref.abs() * 2.0 ** -8 + k * k * 0.064 * 2.0 ** -24 + 1e-6).all()
+
+
 @pytest.mark.parametrize("n,h,w,cout,r,s", [(1, 20, 16, 128, 4, 1), (1, 11, 14, 72, 4, 1), (1, 20, 16, 128, 2, 1), (1, 20, 16, 200, 3, 1), (2, 20, 16, 64, 4, 1)])
 def test_conv_with_few_wide_load_groups(env, n, h, w, cout, r, s):
     """Short filters on small images: all row taps of a column travel in one load group, and the ring holds one to three."""
