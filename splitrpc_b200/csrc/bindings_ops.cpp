@@ -340,8 +340,9 @@ void bind_ops(py::module_& m) {
     check(nn_global_avgpool((const void*)in, (void*)out, n, hw, c, (cudaStream_t)stream), "global_avgpool");
   });
   m.def("fc_skinny", [](uintptr_t a, int lda, uintptr_t w, int ldw, uintptr_t bias, uintptr_t out, int ldo, int M, int N, int K,
-                        uintptr_t stream) {
-    check(nn_fc_skinny((const void*)a, lda, (const void*)w, ldw, (const float*)bias, (float*)out, ldo, M, N, K, (cudaStream_t)stream),
+                        uintptr_t status, uintptr_t stream) {
+    check(nn_fc_skinny((const void*)a, lda, (const void*)w, ldw, (const float*)bias, (float*)out, ldo, M, N, K, (uint32_t*)status,
+                       (cudaStream_t)stream),
           "fc_skinny");
   });
   m.def("softmax_response",

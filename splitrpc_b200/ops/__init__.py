@@ -82,7 +82,8 @@ def fc_skinny(a: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None = None
     assert out.dtype == torch.float32 and out.shape == (M, N) and out.stride(1) == 1
     if bias is not None:
         assert bias.dtype == torch.float32 and bias.numel() == N
-    _C.fc_skinny(a.data_ptr(), a.stride(0), w.data_ptr(), w.stride(0), _ptr(bias), out.data_ptr(), out.stride(0), M, N, K, _stream())
+    _C.fc_skinny(a.data_ptr(), a.stride(0), w.data_ptr(), w.stride(0), _ptr(bias), out.data_ptr(), out.stride(0), M, N, K,
+                  status_word().data_ptr(), _stream())
     return out
 
 

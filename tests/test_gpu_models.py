@@ -77,6 +77,31 @@ def test_fc_skinny_forms(torch_cuda, m_rows, n_cols, k):
     assert bool((out[m_rows] == 7).all()) and bool((out[:, n_cols:] == 7).all())
 
 
+@pytest.mark.parametrize("m_rows", [1, 31, 33, 64, 70])
+@pytest.mark.parametrize("n_cols,k", [(1, 1544), (127, 1600), (129, 1792), (1000, 2040), (300, 2048)])
+def test_fc_on_clusters(torch_cuda, m_rows, n_cols, k):
+    """K just above the dispatch line, with CTAs that get one or no k-block, ragged k-blocks, and one or two phases; ragged rows and columns."""
+    torch = torch_cuda
+    from splitrpc_b200 import ops
+
+    g = torch.Generator(device="cuda").manual_seed(m_rows * n_cols + k)
+    a = torch.randn(m_rows, k + 8, device="cuda", generator=g).bfloat16()[:, :k]
+    w = torch.randn(n_cols, k + 16, device="cuda", generator=g).bfloat16()[:, :k]
+    bias = torch.randn(n_cols, device="cuda", generator=g)
+    out = torch.full((m_rows + 1, n_cols + 3), 7.0, device="cuda")
+    ops.fc_skinny(a, w, bias=bias, out=out[:m_rows, :n_cols])
+    ops.check_status()
+    want = a.double() @ w.double().t() + bias.double()
+    # 16 products per accumulator, each cut to 2^-23 of the largest, then seven levels of fp32 additions and the bias
+    bound = (a.double().abs() @ w.double().abs().t() + bias.double().abs()) * (40 * 2.0 ** -24)
+    assert bool(((out[:m_rows, :n_cols].double() - want).abs() <= bound).all())
+    assert bool((out[m_rows] == 7).all()) and bool((out[:, n_cols:] == 7).all())
+    # a row's result does not depend on the rows beside it, and rows that share their memory are taken as before
+    assert torch.equal(ops.fc_skinny(a[-1:], w, bias=bias)[0], out[m_rows - 1, :n_cols])
+    same = ops.fc_skinny(a[:1].expand(3, k), w, bias=bias).double()
+    assert bool(((same - want[:1]).abs() <= bound[:1] * (k + 8) / 40).all())
+
+
 @pytest.mark.parametrize("seq", [128, 384])
 @pytest.mark.parametrize("exponent", [-120, -126.3, -128, -131])
 def test_attention_keeps_subnormal_weights(torch_cuda, seq, exponent):
