@@ -314,28 +314,28 @@ lstm_wavefront_kernel(const g_params* stub, const float* direct_in, float* direc
 
 // ------------------------------------------------------------------ LSTM, whole-GPU dataflow
 // The cluster kernel above gives a layer one SM, whose threads each walk one 1 KB weight row: a wave takes 74 us.  Here a
-// layer has LSTM_LAYER_BLOCKS SMs and a warp owns one hidden unit for the whole kernel: its eight gate rows of W and U (8 KB)
-// are loaded once and stay in its registers, so the weights cross the memory system once per launch instead of once per
+// layer has LSTM_LAYER_BLOCKS SMs and a warp owns two hidden units for the whole kernel: their eight gate rows of W and U each
+// (16 KB) are loaded once and stay in its registers, so the weights cross the memory system once per launch instead of once per
 // step.  What is left is the chain of 15 exchanges along the anti-diagonals (layer l, step t needs all 256 outputs of
 // (l-1, t) and of (l, t-1)).  Outputs travel as 8-byte {value, tag} words through L2, stored and read whole: a reader that
 // finds the launch's tag has the value with it, so an exchange is one store and one read, with no counter, no fence
 // and no grid-wide barrier, and layers run apart as far as their inputs allow.  The tag is a launch counter in device memory
 // (lstm_bump_kernel adds one before every launch; graph replays count too), so nothing has to be cleared in between.
-// A block stages the vectors of a step in shared memory for its warps; the 4 x NB gate sums of a warp are reduced together
-// (values are halved between lane pairs as they are added).  The kernel is launched cooperatively: all blocks are resident,
-// and every wait is bounded.  30.3 / 35.6 / 47.4 / 79.4 us for 1 / 2 / 4 / 8 requests back to back (61.8 / 84.0 / 128.9 / 216.7 us with a
-// grid barrier per wave); what is left is the exchange latency, 2 us per step for one request, and 0.4 us per further request.
+// A block stages the vectors of a step in shared memory for its warps; the 8 x NB gate sums of a warp are reduced together
+// (values are halved between lane pairs as they are added).  Two units per warp read every vector from shared memory half as often
+// as one (16 warps): 29.8 / 34.3 / 46.4 / 77.0 us for 1 / 2 / 4 / 8 requests then, 28.0 / 33.9 / 41.2 / 69.1 now; the sums are the same bits.  The kernel is launched cooperatively: all blocks are resident,
+// and every wait is bounded.  61.8 / 84.0 / 128.9 / 216.7 us with a grid barrier per wave.  What is left
+// is the exchange latency, 1.9 us per step for one request, and 0.3 - 0.4 us per further request.
 constexpr int LSTM_GROUP = 8;          // requests per launch
 constexpr int LSTM_LAYER_BLOCKS = 16;  // 8 x 16 = 128 of 148 SMs
-constexpr int LSTM_WARPS = (LH + LSTM_LAYER_BLOCKS - 1) / LSTM_LAYER_BLOCKS;  // hidden units per block
-constexpr int LSTM_THREADS = LSTM_WARPS * 32;
+constexpr int LSTM_UNITS = LH / LSTM_LAYER_BLOCKS;  // hidden units per block
+static_assert(LH % LSTM_LAYER_BLOCKS == 0, "every warp has its units");
 // A cooperative launch waits until all its blocks fit, and the blocks of resident copy engines (16 each) do not leave between
-// requests: with 128 registers a block of this kernel took all of its SM, and two engines left it 116 SMs.  512 threads x 112
-// registers leave room for one engine block on every SM (256 threads, held to 32 registers by its launch bounds, sg_kernels.cu);
-// the 20 SMs that no block needs may hold any number.  Two requests' sums at a time keep the warp within 112 registers.
-// 1 / 2 / 4 / 5 / 8 requests: 30.3 / 35.6 / 47.4 / 58.0 / 79.4 us; all sums at once with 128 registers 30.5 / 39.3 / 49.9 / 57.1 / 74.7 us; with 104
-// registers 30.5 / 41.3 / 55.1 / 65.5 / 82.8 us, with 96 it spills more.
-constexpr int LSTM_REGS = 112;
+// requests: a block that took all of its SM left two engines' LSTM 116 SMs.  256 threads x 216 registers leave room for one
+// engine block on every SM (256 threads, held to 32 registers by its launch bounds, sg_kernels.cu); the 20 SMs that no block
+// needs may hold any number.  128 of the registers hold weights; two requests' sums at a time keep a warp within the rest.
+constexpr int LSTM_PER_WARP = 2;       // hidden units per warp
+constexpr int LSTM_WARPS = LSTM_UNITS / LSTM_PER_WARP, LSTM_THREADS = LSTM_WARPS * 32, LSTM_REGS = 216;
 static_assert(LSTM_THREADS * LSTM_REGS + 256 * 32 <= 65536, "a block and a resident copy block share an SM's registers");
 
 struct LstmGridArgs {
@@ -376,43 +376,48 @@ __global__ void lstm_bump_kernel(unsigned* epoch) { *epoch += 1; }
 
 template <int NB>
 __global__ void __maxnreg__(LSTM_REGS) lstm_grid_kernel(const LstmGridArgs a) {
+  constexpr int PW = LSTM_PER_WARP;
   constexpr int P = NB == 1 ? 1 : 2, PASSES = NB / P;            // requests whose sums a warp forms together
-  constexpr int PV = 4 * P, REP = 32 / PV;                       // their gate sums, lanes per sum after the reduction
+  constexpr int PV = 4 * P * PW, REP = 32 / PV;                  // their gate sums, lanes per sum after the reduction
+  constexpr int SUMS = PASSES > REP ? PASSES / REP : 1, LPP = PASSES > REP ? 1 : REP / PASSES;  // sums per lane at the end, lanes per sum
   constexpr int ROWS = LSTM_THREADS / (LH / 2);                  // vectors that the block stages at once
   constexpr int MAXQ = (2 * NB + ROWS - 1) / ROWS;               // word pairs a thread stages per step
   static_assert(LSTM_THREADS % (LH / 2) == 0 && (NB % ROWS == 0 || MAXQ == 1), "constant distance between a thread's vectors");
   __shared__ __align__(16) float s_vec[2][2][NB][LH];            // [buffer][input, own layer's previous output][request][unit]
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int l = blockIdx.x / LSTM_LAYER_BLOCKS, part = blockIdx.x - l * LSTM_LAYER_BLOCKS;
-  const int j = part * LSTM_WARPS + warp;                        // this warp's hidden unit
-  const bool unit = j < LH;
+  const int j0 = part * LSTM_UNITS + warp * PW;                     // this warp's first hidden unit
   const unsigned tag = *a.epoch;
   const float* in_base = (a.direct_in ? a.direct_in : reinterpret_cast<const float*>(a.stub->req)) + (size_t)a.first * LSTEPS * LH;
   float* out_base = (a.direct_out ? a.direct_out : reinterpret_cast<float*>(a.stub->resp)) + (size_t)a.first * LH;
   const float* W = a.weights + (size_t)l * ((size_t)8 * LH * LH + 4 * LH);
   const float* U = W + (size_t)4 * LH * LH;
   const float* B = U + (size_t)4 * LH * LH;
-  float4 w[4][2], u[4][2];
+  float4 w[PW][4][2], u[PW][4][2];
 #pragma unroll
-  for (int g = 0; g < 4; g++) {
-    const float4* wr = reinterpret_cast<const float4*>(W + ((size_t)g * LH + (unit ? j : 0)) * LH);
-    const float4* ur = reinterpret_cast<const float4*>(U + ((size_t)g * LH + (unit ? j : 0)) * LH);
-    w[g][0] = __ldg(wr + lane);
-    w[g][1] = __ldg(wr + 32 + lane);
-    u[g][0] = __ldg(ur + lane);
-    u[g][1] = __ldg(ur + 32 + lane);
-  }
-  // After the reductions a lane has gate `gate` of request `req`; with the other gates it computes that request's cell.
+  for (int n = 0; n < PW; n++)
+#pragma unroll
+    for (int g = 0; g < 4; g++) {
+      const float4* wr = reinterpret_cast<const float4*>(W + ((size_t)g * LH + j0 + n) * LH);
+      const float4* ur = reinterpret_cast<const float4*>(U + ((size_t)g * LH + j0 + n) * LH);
+      w[n][g][0] = __ldg(wr + lane);
+      w[n][g][1] = __ldg(wr + 32 + lane);
+      u[n][g][0] = __ldg(ur + lane);
+      u[n][g][1] = __ldg(ur + 32 + lane);
+    }
+  // After the reductions a lane has gate `gate` of unit `j` for SUMS requests; with the other gates it computes their cells.
   const int lane_of_sum = lane & (REP - 1), gate = (lane / REP) & 3, src_lane = lane - gate * REP;
-  const int req = lane_of_sum / (REP / PASSES) * P + lane / (4 * REP);
-  const bool stores = unit && gate == 0 && lane_of_sum % (REP / PASSES) == 0 && req < a.batch;
-  const float bias = B[gate * LH + (unit ? j : 0)] + (gate == 2 ? a.forget_bias : 0.f);
+  const int item = lane / (4 * REP), req0 = lane_of_sum / LPP * SUMS * P + item % P, j = j0 + item / P;  // sum k: request req0 + k * P
+  const bool stores = gate == 0 && lane_of_sum % LPP == 0;
+  const float bias = B[gate * LH + j] + (gate == 2 ? a.forget_bias : 0.f);
   // Staging: a thread takes two units of every ROWS-th of the step's 2 x NB vectors.  Both sources lie on one line through
   // hbuf, so each further vector of a thread is the first one's address plus a constant.
   const int row0 = (int)threadIdx.x / (LH / 2), pr2 = 2 * ((int)threadIdx.x % (LH / 2));
   const int from0 = row0 / NB, b0 = row0 % NB;
   const int words0 = (((l - 1 + from0) * LSTEPS - from0) * LSTM_GROUP + b0) * LH + pr2;  // at step 0; + LSTM_GROUP * LH per step
-  float cell = 0.f;
+  float cell[SUMS];
+#pragma unroll
+  for (int k = 0; k < SUMS; k++) cell[k] = 0.f;
   for (int t = 0; t < LSTEPS; t++) {
     float(*vec)[NB][LH] = s_vec[t & 1];
     // ---- stage the step's vectors (source 0: the layer below or the request, 1: this layer's previous output)
@@ -457,8 +462,8 @@ __global__ void __maxnreg__(LSTM_REGS) lstm_grid_kernel(const LstmGridArgs a) {
       // Every block that waits for this one's words gives up in turn; the last layer's blocks leave no number of an earlier
       // batch behind in the rows that they do not compute.
       if (l == LLAYERS - 1)
-        for (int i = (int)threadIdx.x; i < a.batch * LSTM_WARPS; i += LSTM_THREADS)
-          out_base[(size_t)(i / LSTM_WARPS) * LH + part * LSTM_WARPS + i % LSTM_WARPS] = __int_as_float(0x7fffffff);
+        for (int i = (int)threadIdx.x; i < a.batch * LSTM_UNITS; i += LSTM_THREADS)
+          out_base[(size_t)(i / LSTM_UNITS) * LH + part * LSTM_UNITS + i % LSTM_UNITS] = __int_as_float(0x7fffffff);
       if (threadIdx.x == 0 && a.status) *a.status = 0x4C53u;  // 'LS': a wait of the LSTM ran out
       return;
     }
@@ -474,18 +479,24 @@ __global__ void __maxnreg__(LSTM_REGS) lstm_grid_kernel(const LstmGridArgs a) {
       for (int b = 0; b < P; b++) {
         if (p * P + b > NB / 2 && p * P + b >= a.batch) {  // (a launch has more than NB / 2 requests)
 #pragma unroll
-          for (int g = 0; g < 4; g++) v[b * 4 + g] = 0.f;
+          for (int n = 0; n < PW; n++)
+#pragma unroll
+            for (int g = 0; g < 4; g++) v[(n * P + b) * 4 + g] = 0.f;
           continue;
         }
         const float4* xv = reinterpret_cast<const float4*>(vec[0][p * P + b]);
         const float4 x0 = xv[lane], x1 = xv[32 + lane];
 #pragma unroll
-        for (int g = 0; g < 4; g++) v[b * 4 + g] = dot4(w[g][0], x0) + dot4(w[g][1], x1);
+        for (int n = 0; n < PW; n++)
+#pragma unroll
+          for (int g = 0; g < 4; g++) v[(n * P + b) * 4 + g] = dot4(w[n][g][0], x0) + dot4(w[n][g][1], x1);
         if (t > 0) {
           const float4* hv = reinterpret_cast<const float4*>(vec[1][p * P + b]);
           const float4 h0 = hv[lane], h1 = hv[32 + lane];
 #pragma unroll
-          for (int g = 0; g < 4; g++) v[b * 4 + g] += dot4(u[g][0], h0) + dot4(u[g][1], h1);
+          for (int n = 0; n < PW; n++)
+#pragma unroll
+            for (int g = 0; g < 4; g++) v[(n * P + b) * 4 + g] += dot4(u[n][g][0], h0) + dot4(u[n][g][1], h1);
         }
       }
 #pragma unroll
@@ -494,18 +505,22 @@ __global__ void __maxnreg__(LSTM_REGS) lstm_grid_kernel(const LstmGridArgs a) {
     }
 #pragma unroll
     for (int half = PASSES / 2, off = REP / 2; off > 0; half /= 2, off /= 2) keep_half(sum, half, off);
-    sum[0] += bias;
-    const float gi = __shfl_sync(0xffffffffu, sum[0], src_lane);
-    const float gg = __shfl_sync(0xffffffffu, sum[0], src_lane + REP);
-    const float gf = __shfl_sync(0xffffffffu, sum[0], src_lane + 2 * REP);
-    const float go = __shfl_sync(0xffffffffu, sum[0], src_lane + 3 * REP);
-    cell = sigmoidf_(gf) * cell + sigmoidf_(gi) * tanhf(gg);
-    const float h = tanhf(cell) * sigmoidf_(go);
-    if (stores) {
-      unsigned long long* dst = a.hbuf + (((size_t)l * LSTEPS + t) * LSTM_GROUP + req) * LH + j;
-      const unsigned long long word = ((unsigned long long)tag << 32) | __float_as_uint(h);
-      asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(dst), "l"(word) : "memory");
-      if (l == LLAYERS - 1 && t == LSTEPS - 1) out_base[(size_t)req * LH + j] = h;
+#pragma unroll
+    for (int k = 0; k < SUMS; k++) {
+      sum[k] += bias;
+      const float gi = __shfl_sync(0xffffffffu, sum[k], src_lane);
+      const float gg = __shfl_sync(0xffffffffu, sum[k], src_lane + REP);
+      const float gf = __shfl_sync(0xffffffffu, sum[k], src_lane + 2 * REP);
+      const float go = __shfl_sync(0xffffffffu, sum[k], src_lane + 3 * REP);
+      cell[k] = sigmoidf_(gf) * cell[k] + sigmoidf_(gi) * tanhf(gg);
+      const float h = tanhf(cell[k]) * sigmoidf_(go);
+      const int req = req0 + k * P;
+      if (stores && req < a.batch) {
+        unsigned long long* dst = a.hbuf + (((size_t)l * LSTEPS + t) * LSTM_GROUP + req) * LH + j;
+        const unsigned long long word = ((unsigned long long)tag << 32) | __float_as_uint(h);
+        asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(dst), "l"(word) : "memory");
+        if (l == LLAYERS - 1 && t == LSTEPS - 1) out_base[(size_t)req * LH + j] = h;
+      }
     }
   }
 }
