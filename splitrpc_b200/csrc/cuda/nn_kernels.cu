@@ -209,7 +209,8 @@ __global__ void __launch_bounds__(256) global_avgpool(const __nv_bfloat16* in, _
 // Us, before (weights staged whole, as fp32, before any arithmetic; 128 shuffles per thread) and now: 64 x 1000 x 2048 12.85 and
 // 11.75, 64 x 1192 x 512 9.9 and 7.4, 128 x 1000 x 512 10.1 and 7.6, 64 x 8192 x 768 38 and 31, 32 x 1192 x 512 6.4 and 5.2.  The loop
 // is bound by what it reads through the L1 / shared-memory path (9.5 of the first, the FMAs are 4.2): deeper prefetch, twice the
-// warps or scalar FMAs change nothing.  The order of every sum is the same in all forms.
+// warps or scalar FMAs change nothing.  The order of every sum is the same in all forms.  K from 1537 to 2048 goes to fc_cluster.cu,
+// see nn_fc_skinny.
 constexpr int FC_NB = 8, FC_PARTS = 4;
 template <int RPT, int PER_SM>
 __global__ void __launch_bounds__(256, PER_SM) fc_skinny(const __nv_bfloat16* a, int lda, const __nv_bfloat16* w,
