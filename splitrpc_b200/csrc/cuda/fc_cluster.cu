@@ -147,7 +147,8 @@ fc_cluster(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ C
     }
   }
   ptx::cluster_arrive_relaxed();  // nothing more goes to a peer
-  ok = ptx::mbar_wait_warp(&recv_full, 0) && ok;
+  // The peers' sums; every lane acquires for itself what it reads below.
+  ok = __all_sync(0xffffffffu, ptx::mbar_wait<ptx::mbar_try_wait_cluster>(&recv_full, 0)) && ok;
   if (!ok && lane == 0) atomicExch(&s_error, (uint32_t)GEMM_ERR_EPILOGUE_WAIT);
   if (threadIdx.x < COLS) {
     const int c = threadIdx.x, n = n0 + c, m = m0 + (int)rank * 4;

@@ -91,21 +91,35 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
+// For shared memory that other CTAs of the cluster fill with st.async: their completions are releases at cluster scope, and the
+// plain form above acquires at CTA scope only, which does not include the writers.
+__device__ __forceinline__ bool mbar_try_wait_cluster(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}\n"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
 // Bounded wait: gives up after SRPC_MBAR_WAIT_CYCLES SM clock cycles (about two seconds), far beyond any healthy
 // wait inside a kernel.  The bound uses the SM-local cycle counter, which costs a few cycles to read; the global
 // nanosecond timer is far slower to read and would sit on the critical path of every producer/consumer hand-off.
 #ifndef SRPC_MBAR_WAIT_CYCLES
 #define SRPC_MBAR_WAIT_CYCLES 4000000000ll
 #endif
+template <bool (*TRY)(uint64_t*, uint32_t) = mbar_try_wait>
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
 #pragma unroll 1
   for (int i = 0; i < 1024; i++)
-    if (mbar_try_wait(bar, parity)) return true;
+    if (TRY(bar, parity)) return true;
   const long long t0 = clock64();
   for (;;) {
 #pragma unroll 1
     for (int i = 0; i < 256; i++)
-      if (mbar_try_wait(bar, parity)) return true;
+      if (TRY(bar, parity)) return true;
     if (clock64() - t0 > SRPC_MBAR_WAIT_CYCLES) return false;
   }
 }

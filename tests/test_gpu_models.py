@@ -102,6 +102,30 @@ def test_fc_on_clusters(torch_cuda, m_rows, n_cols, k):
     assert bool(((same - want[:1]).abs() <= bound[:1] * (k + 8) / 40).all())
 
 
+def test_fc_on_clusters_repeats_itself(torch_cuda):
+    """Partial sums that cross between CTAs: launches behind one another on two streams give the bits of launches waited for."""
+    torch = torch_cuda
+    from splitrpc_b200 import ops
+
+    g = torch.Generator(device="cuda").manual_seed(5)
+    sets = [(torch.randn(64, 2048, device="cuda", generator=g).bfloat16(), torch.randn(1000, 2048, device="cuda", generator=g).bfloat16())
+            for _ in range(4)]
+    want = []
+    for a, w in sets:
+        want.append(ops.fc_skinny(a, w))
+        torch.cuda.synchronize()
+    outs = [[torch.empty_like(want[0]) for _ in range(40)] for _ in range(2)]
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    torch.cuda.synchronize()
+    for i in range(40):
+        for s, mine in zip(streams, outs):
+            with torch.cuda.stream(s):
+                ops.fc_skinny(*sets[i % 4], out=mine[i])
+    torch.cuda.synchronize()
+    ops.check_status()
+    assert all(torch.equal(mine[i], want[i % 4]) for mine in outs for i in range(40))
+
+
 @pytest.mark.parametrize("seq", [128, 384])
 @pytest.mark.parametrize("exponent", [-120, -126.3, -128, -131])
 def test_attention_keeps_subnormal_weights(torch_cuda, seq, exponent):
