@@ -158,6 +158,7 @@ struct ASource {
   int stride, pad, stride2;
   FastDiv fd_img, fd_ow;      // by output pixels per image and per row
   FastDiv fd_cblocks, fd_s;   // by channel blocks and filter columns
+  FastDiv fd_rows;            // by filter rows where they are innermost (srpc_conv_rows_innermost), by 1 otherwise
 };
 
 template <int BN, int RPC, bool TP>
@@ -285,11 +286,21 @@ gemm_2sm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
         for (int b = 0; b < KPS; b++) {
           if (b >= blocks) break;
           const int kb = st * KPS + b;
+          int kb_w = kb;  // its place in a row of weights
           if (!src.im2col && kb < src.kb_split) {
             if (elected) ptx::tma_load_2d_2sm(sa + b * KB_BYTES, &tmap_a, full_leader, kb * BK, row0);
           } else if (kb < src.kb_split) {
-            const int tap = (int)fdiv(src.fd_cblocks, (uint32_t)kb), cb = kb - tap * (int)src.fd_cblocks.d;
-            const int fr = (int)fdiv(src.fd_s, (uint32_t)tap), fs = tap - fr * (int)src.fd_s.d;
+            const int group = (int)fdiv(src.fd_rows, (uint32_t)kb), tap = (int)fdiv(src.fd_cblocks, (uint32_t)group);
+            const int cb = group - tap * (int)src.fd_cblocks.d;
+            int fr, fs;
+            if (src.fd_rows.d > 1) {
+              fr = kb - group * (int)src.fd_rows.d;
+              fs = tap;
+              kb_w = (fr * (int)src.fd_s.d + fs) * (int)src.fd_cblocks.d + cb;
+            } else {
+              fr = (int)fdiv(src.fd_s, (uint32_t)tap);
+              fs = tap - fr * (int)src.fd_s.d;
+            }
             if (elected)
               ptx::tma_load_im2col_2sm(sa + b * KB_BYTES, &tmap_a, full_leader, cb * BK, x * src.stride - src.pad, y * src.stride - src.pad,
                                        img, (uint16_t)fs, (uint16_t)fr);
@@ -300,7 +311,7 @@ gemm_2sm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
           } else if (elected) {
             ptx::tma_load_2d_2sm(sa + b * KB_BYTES, &tmap_a2, full_leader, (kb - src.kb_split) * BK, row0);
           }
-          if (elected) ptx::tma_load_2d_2sm(sa + b * KB_BYTES + A_BYTES, &tmap_b, full_leader, kb * BK, brow0);
+          if (elected) ptx::tma_load_2d_2sm(sa + b * KB_BYTES + A_BYTES, &tmap_b, full_leader, kb_w * BK, brow0);
         }
         if (j == 0 && st == 0 && lane == 0) GEMM2_TRACE(2);
         seq += PRODUCERS;
@@ -633,7 +644,7 @@ ASource matrix_source(int num_kb) {
   ASource src = {};
   src.kb_split = num_kb;
   src.stride = src.stride2 = 1;
-  src.fd_img = src.fd_ow = src.fd_cblocks = src.fd_s = make_fastdiv(1);
+  src.fd_img = src.fd_ow = src.fd_cblocks = src.fd_s = src.fd_rows = make_fastdiv(1);
   return src;
 }
 
@@ -668,6 +679,7 @@ cudaError_t a_maps(const AInput& in, int M, int K, int rows_per_cta, ASource* sr
   src->fd_ow = make_fastdiv((uint32_t)cs.ow);
   src->fd_cblocks = make_fastdiv((uint32_t)(cs.cin / BK));
   src->fd_s = make_fastdiv((uint32_t)cs.s);
+  src->fd_rows = make_fastdiv(srpc_conv_rows_innermost(cs) ? (uint32_t)cs.r : 1u);
   cudaError_t e = src->im2col ? srpc_tensor_map_im2col(ta, in.a, cs.n, cs.h, cs.w, cs.cin, cs.r, cs.s, cs.stride, cs.pad, rows_per_cta)
                               : srpc_tensor_map_2d(ta, in.a, (uint64_t)cs.cin, (uint64_t)M, (uint64_t)cs.cin * 2, BK, (uint32_t)rows_per_cta);
   *ta2 = *ta;

@@ -1058,7 +1058,7 @@ cudaError_t srpc_conv_bf16_tma(const void* in, const void* weight, const ConvSha
   // Row-tap reuse: 8-pixel-wide patches, so that a step of one image row inside the box is 1024 bytes (one swizzle
   // atom) and the shifted A descriptors stay aligned; the box (ph + r - 1 rows) must fit the 128-row A slot.
   static const int allow_reuse = [] { const char* e = getenv("SPLITRPC_CONV_REUSE"); return e ? atoi(e) : 1; }();
-  const bool reuse = allow_reuse && cs.stride == 1 && cs.r >= 2 && cs.r <= 4 && cs.ow >= 14 && cs.oh >= 8;
+  const bool reuse = allow_reuse && srpc_conv_rows_innermost(cs);
   int bn;
   if (reuse) {
     p.reuse = 1;

@@ -72,6 +72,12 @@ cudaError_t srpc_stem_conv(const void* in, const void* weight, const ConvShape& 
 bool srpc_gemm_2sm_eligible(int K, const GemmEpilogue& ep);
 cudaError_t srpc_gemm_bf16_2sm(const void* A, int lda, const void* B, int ldb, int M, int N, int K, int bn, int rows,
                                const GemmEpilogue& ep, uint32_t* status, cudaStream_t stream);
+// Order in which a convolution's products are summed: filter column, channel block, filter row where the one-SM form walks the
+// filter rows of one load (8-pixel-wide patches, a box of up to 16 rows), and row, column, channel block for every other shape.  Both
+// forms keep to it, so that a result has the same bits from either.
+inline bool srpc_conv_rows_innermost(const ConvShape& cs) {
+  return cs.stride == 1 && cs.r >= 2 && cs.r <= 4 && cs.ow >= 14 && cs.oh >= 8;
+}
 bool srpc_conv_2sm_eligible(const ConvShape& cs, const GemmEpilogue& ep);
 cudaError_t srpc_conv_bf16_2sm(const void* input, const void* weight, const ConvShape& cs, int bn, int rows, const GemmEpilogue& ep,
                                uint32_t* status, cudaStream_t stream);

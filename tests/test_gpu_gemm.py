@@ -215,3 +215,35 @@ def test_conv_linear_pixels(env, h, w, cin, cout, r, s, stride, pad):
         part = ops.conv2d_nhwc(x[:n].contiguous(), wt, bias=bias, residual=res[:n].contiguous(), stride=stride, pad=pad, act="relu")
         assert torch.equal(part, whole[:n])
     ops.check_status()
+
+
+def _one_sm_conv(torch, ops, x, w, bias=None, residual=None, stride=1, pad=0, act=None):
+    """The convolution by the one-SM kernel: inputs with strides of their own (here the dense ones) always take it."""
+    from splitrpc_b200 import _C
+
+    (n, h, wd, c), (cout, r, s, _) = x.shape, w.shape
+    out = torch.empty(n, (h + 2 * pad - r) // stride + 1, (wd + 2 * pad - s) // stride + 1, cout, device="cuda", dtype=torch.bfloat16)
+    _C.conv_bf16(x.data_ptr(), w.data_ptr(), n, h, wd, c, cout, r, s, stride, pad, out.data_ptr(), 0 if bias is None else bias.data_ptr(),
+                 0 if residual is None else residual.data_ptr(), ops.ACT[act], ops.status_word().data_ptr(),
+                 torch.cuda.current_stream().cuda_stream, 2, c, wd * c, h * wd * c)
+    return out
+
+
+@pytest.mark.parametrize("n,h,w,cin,cout,r,s,stride,pad", [(3, 56, 56, 64, 64, 3, 3, 1, 1), (5, 14, 14, 256, 136, 3, 3, 1, 1), (2, 8, 14, 128, 64, 2, 5, 1, 0),
+                                                           (2, 20, 16, 192, 72, 4, 2, 1, 2), (3, 8, 13, 64, 64, 3, 3, 1, 1), (9, 7, 7, 512, 264, 3, 3, 1, 1),
+                                                           (2, 20, 20, 64, 64, 5, 5, 1, 2), (2, 28, 28, 128, 128, 3, 3, 2, 1), (3, 9, 30, 64, 200, 1, 1, 1, 0)])
+def test_conv_forms_give_the_same_bits(env, n, h, w, cin, cout, r, s, stride, pad):
+    """Both sides of the rule for the order of the filter taps: the pair kernel and the one-SM kernel sum alike, residual included."""
+    torch, ops = env
+    x = torch.randn(n, h, w, cin, device="cuda").bfloat16()
+    f = (torch.randn(cout, r, s, cin, device="cuda") / (cin * r * s) ** 0.5).bfloat16()
+    bias = torch.randn(cout, device="cuda")
+    want = _one_sm_conv(torch, ops, x, f, bias, None, stride, pad, "relu")
+    res = torch.randn_like(want)
+    for q in (None, res):
+        got = ops.conv2d_nhwc(x, f, bias=bias, residual=q, stride=stride, pad=pad, act="relu")
+        assert torch.equal(got, want if q is None else _one_sm_conv(torch, ops, x, f, bias, res, stride, pad, "relu"))
+    ops.check_status()
+    ref = torch.nn.functional.conv2d(x.double().permute(0, 3, 1, 2), f.double().permute(0, 3, 1, 2), bias.double(), stride, pad)
+    ref = torch.relu(ref.permute(0, 2, 3, 1))
+    assert ((want.double() - ref).norm() / ref.norm()).item() < 2.0 ** -8  # one rounding to bf16
