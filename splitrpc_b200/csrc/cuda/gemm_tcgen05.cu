@@ -29,7 +29,6 @@ constexpr int UMMA_K = 16;
 constexpr int GEMM_THREADS = 192;  // warp 0 producer, warp 1 mma, warps 2-5 epilogue
 constexpr int CONV_THREADS = 320;  // warps 0-3 gather producers, warp 4 B-loader, warp 5 mma, warps 6-9 epilogue
 
-__device__ __forceinline__ float gelu_f(float x) { return ptx::gelu_erf_fast(x); }
 
 template <int BN>
 struct SmemLayout {
@@ -83,7 +82,11 @@ __device__ __forceinline__ void epilogue_store(const GemmEpilogue& ep, uint32_t 
       for (int j = 0; j < 32; j++) v[j] = fmaxf(v[j], 0.f);
     } else if (ep.act == GEMM_ACT_GELU) {
 #pragma unroll
-      for (int j = 0; j < 32; j++) v[j] = gelu_f(v[j]);
+      for (int j = 0; j < 32; j += 2) {
+        const float2 g = ptx::gelu_erf_fast2(make_float2(v[j], v[j + 1]));
+        v[j] = g.x;
+        v[j + 1] = g.y;
+      }
     } else if (ep.act == GEMM_ACT_TANH) {
 #pragma unroll
       for (int j = 0; j < 32; j++) v[j] = tanhf(v[j]);

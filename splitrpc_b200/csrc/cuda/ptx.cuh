@@ -143,25 +143,11 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity) {
 
 // ---------------------------------------------------------------- math
 // GELU with the exact (erf) definition, x * Phi(x), from the rational approximation of erfc by Abramowitz & Stegun
-// 7.1.26 (absolute error of erf below 1.5e-7, far under bf16 resolution): 7 FMA/MUL, one rcp.approx and one ex2.approx
-// per value, no branches.  erff() costs about three times as many instructions and made GELU epilogues the slowest
-// stage of the FFN GEMMs.
-__device__ __forceinline__ float gelu_erf_fast(float x) {
-  const float ax = fabsf(x) * 0.70710678118654752f;
-  float t, e;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(t) : "f"(fmaf(0.3275911f, ax, 1.0f)));
-  float p = fmaf(t, 1.061405429f, -1.453152027f);
-  p = fmaf(p, t, 1.421413741f);
-  p = fmaf(p, t, -0.284496736f);
-  p = fmaf(p, t, 0.254829592f);
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(-1.4426950408889634f * ax * ax));
-  const float h = 0.5f * p * t * e;  // 0.5 * erfc(|x| / sqrt 2)
-  return x * (x < 0.f ? h : 1.0f - h);
-}
-
-// The same approximation for two values, in the form x Phi(x) = max(x, 0) - |x| erfc(|x| / sqrt 2) / 2: no selection by the sign,
-// constants folded (2 MIN, 2 MAX, 11 packed operations, 4 MUFU for two values; the GELU epilogue of a 128 x 256 half tile
-// is bound by them).  |x| is capped where the second term has long been zero, so that infinities give infinity and 0; NaN stays.
+// 7.1.26 (absolute error of erf below 1.5e-7, far under bf16 resolution), in the form max(x, 0) - |x| erfc(|x| / sqrt 2) / 2: no
+// selection by the sign, constants folded (2 MIN, 2 MAX, 11 packed operations, 4 MUFU for two values; the GELU epilogue of a
+// 128 x 256 half tile is bound by them; erff() costs about three times as much).  |x| is capped where the second term has long been
+// zero, so that infinities give infinity and 0; NaN stays.  Every kernel uses this one form: which of them runs a product depends on
+// its number of rows, and a row must not.
 __device__ __forceinline__ float2 gelu_erf_fast2(float2 x) {
   float2 t, e, relu;
   const float2 a = make_float2(fminf(fabsf(x.x), 64.f), fminf(fabsf(x.y), 64.f));

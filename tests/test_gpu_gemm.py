@@ -99,6 +99,34 @@ def test_gelu_epilogue_matches_erf_definition(env):
     assert (out - ref).abs().max().item() < 2e-6
 
 
+def test_gelu_epilogue_at_the_ends(env):
+    """Infinities, NaN, large and tiny arguments through every kernel that has the epilogue: fp32 by the one-SM kernel, bf16 by CTA
+    pairs, both by the first-generation kernel."""
+    import math
+    torch, ops = env
+    x = [math.inf, -math.inf, math.nan, 3e38, -3e38, 70.0, -70.0, 14.0, -14.0, 0.0, -0.0, 1e-30, -1e-30, 1e-40, -1e-40, 5.5, -5.5, 1.0, -1.0]
+    bias = torch.tensor(x + [0.5] * (64 - len(x)), device="cuda")
+    a, b = torch.zeros(3, 64, device="cuda").bfloat16(), torch.zeros(64, 64, device="cuda").bfloat16()
+    ref = torch.nn.functional.gelu(bias.double())
+    ref[1] = 0.0  # the limit; the product of infinity and zero is not a number there
+    for impl in (1, 2):
+        for dtype in (torch.float32, torch.bfloat16):
+            ops.GEMM_IMPL, keep = impl, ops.GEMM_IMPL
+            try:
+                out = ops.gemm(a, b, bias=bias, act="gelu", out_dtype=dtype)
+            finally:
+                ops.GEMM_IMPL = keep
+            ops.check_status()
+            out, want = out.double(), ref.expand(3, 64)
+            assert torch.equal(out.isnan(), want.isnan())
+            assert torch.equal(out[want.isinf()], want[want.isinf()])
+            # 7.1.26's 1.5e-7 times |x| / 2 and fp32 rounding; bf16 rounds once more
+            tol = 2e-7 * bias.double().abs().clamp(max=6.0) + want.abs() * (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -22) + 1e-37
+            fin = want.isfinite()
+            assert ((out - want).abs() <= tol)[fin].all(), (impl, dtype)
+    ops.check_status()
+
+
 @pytest.mark.parametrize("n,oh,c1,h2,c2,cout,stride2", [(2, 56, 64, 56, 64, 256, 1), (3, 28, 128, 56, 256, 512, 2),
                                                         (2, 14, 256, 28, 512, 1024, 2), (5, 7, 512, 14, 1024, 2048, 2)])
 def test_two_input_pointwise_conv(env, n, oh, c1, h2, c2, cout, stride2):

@@ -52,6 +52,30 @@ def test_all_gather_gemm_emulated_ranks(env, T, K, N, tp):
         assert all(int(mblock[m]) == 5 for m in remote)
 
 
+@pytest.mark.parametrize("act", ["gelu", "relu", None])
+def test_rows_do_not_depend_on_the_kernel(env, act):
+    """The same rows with the tokens per rank on both sides of the line between the one-SM kernel (384) and CTA pairs (512)."""
+    torch, C, ops = env
+    K, N = 320, 384
+    x = torch.randn(1024, K, device="cuda").bfloat16()
+    w = (torch.randn(N, K, device="cuda") * 0.1).bfloat16()
+    bias = torch.randn(N, device="cuda")
+    outs = []
+    for T in (768, 1024):
+        gathered, out = x[:T].clone(), torch.zeros(T, N, dtype=torch.bfloat16, device="cuda")
+        ready = torch.full((8,), 5, dtype=torch.int32, device="cuda")
+        mblock = torch.zeros(T // 128, dtype=torch.int32, device="cuda")
+        shards = [x[r * (T // 2):(r + 1) * (T // 2)].clone() for r in range(2)]
+        C.gemm_tp(gathered.data_ptr(), K, w.data_ptr(), K, T, N, K, out.data_ptr(), N, bias.data_ptr(), ops.ACT[act], 2, 0, 5,
+                  mblock.data_ptr(), 6, [s.data_ptr() for s in shards], gathered.data_ptr(), ready.data_ptr(), 0, [], [], 0,
+                  ops.status_word().data_ptr(), torch.cuda.current_stream().cuda_stream, 0)
+        torch.cuda.synchronize()
+        ops.check_status()
+        outs.append(out)
+    assert torch.equal(outs[0], outs[1][:768])
+    assert torch.equal(outs[1], ops.gemm(x, w, bias=bias, act=act))
+
+
 @pytest.mark.parametrize("T,Kl,N,tp", [(512, 256, 384, 2), (1024, 512, 1024, 4), (2048, 2048, 1024, 2), (768, 256, 384, 2),
                                        (6144, 512, 1024, 2), (6144, 128, 1024, 8), (2048, 256, 640, 4)])
 def test_gemm_reduce_scatter_emulated_ranks(env, T, Kl, N, tp):
