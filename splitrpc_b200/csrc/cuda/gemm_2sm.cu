@@ -161,6 +161,26 @@ struct ASource {
   FastDiv fd_rows;            // by filter rows where they are innermost (srpc_conv_rows_innermost), by 1 otherwise
 };
 
+// Channels of A, filter tap and columns of the weights that k-block kb of a convolution multiplies (the second input's: columns only).
+struct KBlock {
+  int c, w;
+  uint16_t fs, fr;
+};
+__device__ __forceinline__ KBlock conv_kblock(const ASource& src, int kb) {
+  const int group = (int)fdiv(src.fd_rows, (uint32_t)kb), tap = (int)fdiv(src.fd_cblocks, (uint32_t)group);
+  const int cb = group - tap * (int)src.fd_cblocks.d;
+  int fr, fs;
+  if (src.fd_rows.d > 1) {
+    fr = kb - group * (int)src.fd_rows.d;
+    fs = tap;
+  } else {
+    fr = (int)fdiv(src.fd_s, (uint32_t)tap);
+    fs = tap - fr * (int)src.fd_s.d;
+  }
+  const int at = src.fd_rows.d > 1 ? (fr * (int)src.fd_s.d + fs) * (int)src.fd_cblocks.d + cb : kb;
+  return KBlock{cb * BK, at * BK, (uint16_t)fs, (uint16_t)fr};
+}
+
 template <int BN, int RPC, bool TP>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Cfg<BN, RPC, TP>::THREADS, 1)
 gemm_2sm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
@@ -266,6 +286,15 @@ gemm_2sm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
         }
       }
       for (; st < num_st; st += PRODUCERS) {
+        // Which weights and, in a convolution, which tap and channels the stage takes: worked out before the wait (behind it, 1 % of
+        // a 3x3 convolution).
+        KBlock at[KPS];
+#pragma unroll
+        for (int b = 0; b < KPS; b++) {
+          const int kb = st * KPS + b;
+          at[b].w = kb * BK;
+          if (src.im2col) at[b] = conv_kblock(src, kb);
+        }
         ok = ptx::mbar_wait_warp(&empty_bar[s], ph ^ 1u);
         if (!ok) {
           if (elected) atomicExch(&s_error, GEMM_ERR_PRODUCER_WAIT);
@@ -286,24 +315,12 @@ gemm_2sm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
         for (int b = 0; b < KPS; b++) {
           if (b >= blocks) break;
           const int kb = st * KPS + b;
-          int kb_w = kb;  // its place in a row of weights
           if (!src.im2col && kb < src.kb_split) {
             if (elected) ptx::tma_load_2d_2sm(sa + b * KB_BYTES, &tmap_a, full_leader, kb * BK, row0);
           } else if (kb < src.kb_split) {
-            const int group = (int)fdiv(src.fd_rows, (uint32_t)kb), tap = (int)fdiv(src.fd_cblocks, (uint32_t)group);
-            const int cb = group - tap * (int)src.fd_cblocks.d;
-            int fr, fs;
-            if (src.fd_rows.d > 1) {
-              fr = kb - group * (int)src.fd_rows.d;
-              fs = tap;
-              kb_w = (fr * (int)src.fd_s.d + fs) * (int)src.fd_cblocks.d + cb;
-            } else {
-              fr = (int)fdiv(src.fd_s, (uint32_t)tap);
-              fs = tap - fr * (int)src.fd_s.d;
-            }
             if (elected)
-              ptx::tma_load_im2col_2sm(sa + b * KB_BYTES, &tmap_a, full_leader, cb * BK, x * src.stride - src.pad, y * src.stride - src.pad,
-                                       img, (uint16_t)fs, (uint16_t)fr);
+              ptx::tma_load_im2col_2sm(sa + b * KB_BYTES, &tmap_a, full_leader, at[b].c, x * src.stride - src.pad, y * src.stride - src.pad,
+                                       img, at[b].fs, at[b].fr);
           } else if (src.im2col2) {
             if (elected)
               ptx::tma_load_im2col_2sm(sa + b * KB_BYTES, &tmap_a2, full_leader, (kb - src.kb_split) * BK, x * src.stride2, y * src.stride2, img,
@@ -311,7 +328,7 @@ gemm_2sm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
           } else if (elected) {
             ptx::tma_load_2d_2sm(sa + b * KB_BYTES, &tmap_a2, full_leader, (kb - src.kb_split) * BK, row0);
           }
-          if (elected) ptx::tma_load_2d_2sm(sa + b * KB_BYTES + A_BYTES, &tmap_b, full_leader, kb_w * BK, brow0);
+          if (elected) ptx::tma_load_2d_2sm(sa + b * KB_BYTES + A_BYTES, &tmap_b, full_leader, at[b].w, brow0);
         }
         if (j == 0 && st == 0 && lane == 0) GEMM2_TRACE(2);
         seq += PRODUCERS;
