@@ -126,9 +126,7 @@ struct TileOrder {
   FastDiv fd_group, fd_gm;  // by group_m * tiles_n and group_m
 };
 
-// j-th tile of this cluster, grouped so that tiles in flight share A and B blocks in L2: eight row blocks by nine or ten columns of
-// tiles, about a square.  8192^3 runs at the power limit, and what it does not read again from DRAM it has for the tensor
-// cores: 875 us with groups of four row blocks, 848 with eight, 880 with sixteen.
+// j-th tile of this cluster, grouped so that tiles in flight share A and B blocks in L2 (see row_blocks_per_group).
 __device__ __forceinline__ bool pair_tile(int j, const TileOrder& o, PairTile* out) {
   int tile = (int)(blockIdx.x >> 1) + j * o.clusters;
   if (tile >= o.tiles_m2 * o.tiles_n) return false;
@@ -674,6 +672,12 @@ void order_tiles(TileOrder* o, int M, int N, int rows, int bn, int max_clusters,
   o->fd_gm = make_fastdiv((uint32_t)group_m);
 }
 
+// Row blocks that walk the columns together.  B is read again for every group: while it stays in L2 four are best, and once it takes
+// more than half of the 126 MB eight save reads from DRAM, and with them power that the tensor cores have instead.  Us with four /
+// eight, sustained: 8192^3 911 / 858, 8192 x 8192 x 4096 445 / 415, 6000^3 368 / 354; 16384 x 4096 x 4096 401 / 414, 8192 x 1024 x
+// 8192 114.0 / 116.5, 8192 x 8192 x 1024 113.1 / 114.9; 5000^3 and 4096 x 4096 x 8192 (50 and 67 MB) alike.
+int row_blocks_per_group(int N, int K) { return (uint64_t)N * K * 2 > 63u * 1000 * 1000 ? 8 : 4; }
+
 // What a launch reads its A rows from: makes the tensor maps for tiles of `rows_per_cta` rows per CTA.
 struct AInput {
   const void* a = nullptr;
@@ -723,7 +727,7 @@ cudaError_t launch_2sm(const AInput& in, const void* B, int ldb, int M, int N, i
   e = srpc_tensor_map_2d(&to, ep.out, (uint64_t)N, (uint64_t)M, (uint64_t)ep.ldo * 2, 32, 32);
   if (e != cudaSuccess) return e;
   TileOrder o;
-  order_tiles(&o, M, N, 2 * RPC, BN, std::min(max_clusters, srpc_gemm_grid_sms() / 2), 8);
+  order_tiles(&o, M, N, 2 * RPC, BN, std::min(max_clusters, srpc_gemm_grid_sms() / 2), row_blocks_per_group(N, K));
   o.m_rot2 = 0;
   o.reverse = K > N;
   o.late_trigger = srpc_gemm_reserved_sms() > 0;
