@@ -894,7 +894,8 @@ int srpc_gemm_trace_read(unsigned long long* out, int n) {
 // 8 .. 8192 columns and K 64 .. 8192, each measured with every shape; the choice is within 0.5 % of the best one on average, 9 % at
 // worst.  Pairs win nearly everywhere (us, one-SM against pairs): 128 x 768 x 3072 14.2 against 8.1, 512 x 768 x 768 6.8 and 4.4,
 // 4096 x 768 x 768 10.8 and 7.6; the one-SM kernel is left with fp32 and unaligned outputs and with the shapes that stream a
-// residual (srpc_gemm_bf16_v2).  Every shape sums a result's products in the same order, so that a row does not depend on the
+// residual (srpc_gemm_bf16_v2).  The residual of a 256-wide pair tile hides only behind long k loops, except in the first round
+// (13144 x 1024 x 768 31.5 us, 192 wide 25.4; 9953 x 1024 x 2048 40.2, 192 wide 41.5).  Every shape sums a result's products in the same order, so that a row does not depend on the
 // batch that it is computed in.
 struct TileShape {
   int bn, rows;  // columns; rows of a CTA pair, 0: the one-SM kernel (128 rows)
@@ -923,7 +924,8 @@ static TileShape pick_tile(int M, int N, int num_kb, const GemmEpilogue& ep, boo
     const int rows = c.rows ? c.rows : BM, units = c.rows ? sms / 2 : sms;
     const long tiles = (long)((M + rows - 1) / rows) * ((N + c.bn - 1) / c.bn);
     const long rounds = (tiles + units - 1) / units;
-    const double cost = c.fixed + (double)rounds * (num_kb * c.kb + c.round + (ep.residual ? c.res : 0) + (ep.act == GEMM_ACT_GELU ? c.gelu : 0));
+    const double res = c.bn == 256 && c.rows && rounds > 1 ? std::max(c.res, 4.0 - 0.05 * num_kb) : c.res;
+    const double cost = c.fixed + (double)rounds * (num_kb * c.kb + c.round + (ep.residual ? res : 0) + (ep.act == GEMM_ACT_GELU ? c.gelu : 0));
     if (cost < best_cost) {
       best_cost = cost;
       best = {c.bn, c.rows};
@@ -940,12 +942,13 @@ cudaError_t srpc_gemm_bf16_v2(const void* A, int lda, const void* B, int ldb, in
   int use_tma_store = (!ep.out_fp32 && (ep.ldo % 8) == 0 && ((uintptr_t)ep.out & 15) == 0) ? 1 : 0;
   static const int allow_res_tma = [] { const char* e = getenv("SPLITRPC_GEMM_RES_TMA"); return e ? atoi(e) : 1; }();
   static const int res_tma_max_k = [] { const char* e = getenv("SPLITRPC_GEMM_RES_TMA_MAXK"); return e ? atoi(e) : 512; }();
-  // Short-K shapes of many tiles are bound by memory and gain from the residual that TMA prefetches tiles ahead (us, against the
-  // best pair tiles: 200704 x 256 x 64 42 and 63, 12544 x 1024 x 256 14.2 and 15.4; 62720 x 256 x 64 13.7 and 20).  Fewer than four
-  // rounds are bound by the launch and the first and last tile (3136 x 2048 x 512 12.7 and 10.4, 980 x 1024 x 256 5.8 and 4.2), and
-  // with a long K the plain residual loads of the epilogue hide behind the next tile's MMAs.
+  // Short-K shapes of many tiles are bound by memory and gain from the residual that TMA prefetches tiles ahead; few rounds of tiles
+  // are bound by the launch and the first and last tile, and with a long K the plain residual loads of the epilogue hide behind the
+  // next tile's MMAs.  The line, in rounds of full tiles, us by TMA and with the best pair tiles: K up to 256 from two rounds on
+  // (25088 x 256 x 64 7.8 and 10.2, 28331 x 256 x 256 9.3 and 10.9, 6326 x 1000 x 64 11.0 and 13.1; 1.7 rounds: 4154 x 1000 x 128
+  // 8.9 and 8.1, 200704 x 256 x 64 42 and 63), up to 512 from three (12544 x 1024 x 256 14.2 and 15.4; 5616 x 1000 x 512 14.0 and 10.6).
   const int rt_bn = N <= 64 ? 64 : 128;
-  const bool many_tiles = (long)((M + BM - 1) / BM) * ((N + rt_bn - 1) / rt_bn) > 3l * num_sms();
+  const bool many_tiles = (long)M * N > (K <= 256 ? 2l : 3l) * num_sms() * BM * rt_bn;
   const bool pairs = srpc_gemm_2sm_eligible(K, ep);
   const bool res_tma = allow_res_tma && use_tma_store == 1 && ep.residual && (ep.ldr % 8) == 0 &&
                        ((uintptr_t)ep.residual & 15) == 0 && K <= res_tma_max_k && (many_tiles || !pairs);

@@ -221,6 +221,28 @@ def test_gemm_few_rows(env, M, N, K):
         assert (buf[M] == 7.0).all() and (buf[:, N:] == 7.0).all()
 
 
+@pytest.mark.parametrize("N,K,act,residual", [(256, 64, "relu", True), (128, 256, "gelu", True), (256, 512, None, True), (1000, 832, "gelu", False),
+                                              (768, 3072, None, True), (64, 1024, "relu", False), (192, 40, None, True)])
+def test_gemm_rows_do_not_depend_on_their_number(env, N, K, act, residual):
+    """A row's bits through every kernel and tile that the number of rows selects: 128- and 256-row pairs of all widths, the one-SM
+    kernel, the residual by TMA on both sides of its lines."""
+    torch, ops = env
+    rows = [1, 64, 129, 700, 2100, 5000, 9000, 14000, 19000, 29000, 45000, 60000]
+    rows = [m for m in rows if m * (N + K) <= 6e7]
+    a = torch.randn(rows[-1], K, device="cuda").bfloat16()
+    b = (torch.randn(N, K, device="cuda") / K ** 0.5).bfloat16()
+    bias = torch.randn(N, device="cuda")
+    res = torch.randn(rows[-1], N, device="cuda").bfloat16() if residual else None
+    whole = ops.gemm(a, b, bias=bias, residual=res, act=act)
+    for m in rows[:-1]:
+        assert torch.equal(ops.gemm(a[:m], b, bias=bias, residual=res[:m] if residual else None, act=act), whole[:m]), m
+    ops.check_status()
+    ref = a[:700].double() @ b.double().t() + bias.double() + (res[:700].double() if residual else 0)
+    ref = torch.relu(ref) if act == "relu" else (torch.nn.functional.gelu(ref) if act == "gelu" else ref)
+    # half a unit of bf16 (2^-9 of the value), and the fp32 sums: K 2^-24 times the sum of |products| (about 0.64 sqrt(K))
+    assert ((whole[:700].double() - ref).abs() <= ref.abs() * 2.0 ** -8 + K ** 1.5 * 0.64 * 2.0 ** -24 + 1e-6).all()
+
+
 @pytest.mark.parametrize("h,w,cin,cout,r,s,stride,pad", [(14, 14, 64, 128, 3, 3, 1, 1), (19, 23, 64, 136, 2, 5, 1, 2), (19, 23, 128, 72, 5, 2, 2, 3),
                                                          (15, 15, 64, 64, 3, 1, 1, 0), (30, 30, 64, 64, 7, 7, 4, 3), (9, 9, 128, 64, 1, 1, 3, 0),
                                                          (7, 7, 512, 512, 3, 3, 1, 1), (5, 5, 64, 8, 3, 3, 2, 1)])
