@@ -1032,6 +1032,11 @@ cudaError_t srpc_conv_bf16_tma(const void* in, const void* weight, const ConvSha
       return cudaErrorInvalidValue;
     if ((cs.h2 - 1) / cs.stride2 + 1 != cs.oh || (cs.w2 - 1) / cs.stride2 + 1 != cs.ow) return cudaErrorInvalidValue;
   }
+  // A dense pointwise convolution is a matrix product and takes its routes, the residual by TMA among them (us as runs of pixels on
+  // pairs, 200704 x 256 x 256 with residual 94, 53 as a product; 64 x 28 x 28 pixels, 64 -> 256 18.6 and 12.2; the same bits).
+  const bool dense = !cs.in_stub && !cs.in_pix_stride && !cs.in_row_stride && !cs.in_img_stride;
+  if (dense && !cs.in2 && cs.r == 1 && cs.s == 1 && cs.stride == 1 && cs.pad == 0)
+    return srpc_gemm_bf16_v2(in, cs.cin, weight, cs.cin, cs.n * cs.h * cs.w, cs.cout, cs.cin, ep2, status, stream);
   if (srpc_conv_2sm_eligible(cs, ep2)) {
     const TileShape ts = pick_tile(cs.n * cs.oh * cs.ow, cs.cout, (cs.r * cs.s * cs.cin + (cs.in2 ? cs.cin2 : 0)) / BK, ep2, false, true);
     return srpc_conv_bf16_2sm(in, weight, cs, ts.bn, ts.rows, ep2, status, stream);
