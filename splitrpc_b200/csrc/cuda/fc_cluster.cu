@@ -3,10 +3,12 @@
 // The weights are the M operand of the tensor core: a cluster of eight CTAs makes 128 output columns of up to 32 rows, and each
 // CTA takes an eighth of K.  64 x 1000 x 2048 is 128 short loads side by side (two CTAs fit an SM) instead of 126 long loops.
 //
-// The tensor core cuts what it adds to an accumulator to fewer bits than an fp32 addition keeps: one accumulator over K =
-// 2048 is 25 times further from the exact sum than chains of fp32 FMAs.  So an accumulator gets one instruction only, 16 products per
-// output, and everything beyond is added in pairs in fp32.  Relative error against 64 bits, 64 x 1000 x 2048: 7.9e-8; chains of FMAs
-// (fc_skinny) 8.3e-8; accumulators of 32, 64, 128, 2048 products 8.1e-8, 9.2e-8, 1.3e-7, 2.1e-6.
+// The tensor core keeps fewer bits of a long sum than chains of fp32 additions do: one accumulator over K = 2048 is 25 times further
+// from the exact sum than chains of fp32 FMAs.  So an accumulator gets one instruction only, 16 products per output (a sum of 16 products
+// of one sign comes out 1.6e-8 low on average), and everything beyond is added in pairs in fp32.  The last four levels weigh most; there
+// the rounding errors are kept and added at the end.  Relative error against 64 bits, 64 x 1000 outputs, chains of FMAs (fc_skinny) / here /
+// here without the kept errors, K = 2048: operands of both signs 7.9e-8 / 6.3e-8 / 7.4e-8, one operand positive 7.9e-8 / 6.3e-8 / 7.5e-8, both
+// positive 3.2e-8 / 2.8e-8 / 3.5e-8; K = 1544: 7.5e-8 / 6.3e-8 / 7.4e-8, 7.5e-8 / 6.3e-8 / 7.4e-8, 3.5e-8 / 3.3e-8 / 4.7e-8.
 //
 // The CTAs' sums travel by st.async: CTA r finishes rows r*4 .. r*4+3 for all 128 columns, and its mbarrier counts the bytes.
 // 64 x 1000 x 2048: 11.8 (fc_skinny) -> 5.0 us, 32 rows 9.0 -> 4.3, 32 x 4096 x 2048 28.0 -> 5.5; most of it is the chain of load, product, exchange
@@ -39,6 +41,13 @@ __device__ __forceinline__ void st_async_v4(uint32_t addr, float4 v, uint32_t ba
   asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(addr), "f"(v.x),
                "f"(v.y), "f"(v.z), "f"(v.w), "r"(bar)
                : "memory");
+}
+
+// a + b, and what the rounding took away is added to err (Knuth's TwoSum).
+__device__ __forceinline__ float add_keep_error(float a, float b, float& err) {
+  const float s = a + b, t = s - a;
+  err += (a - (s - t)) + (b - t);
+  return s;
 }
 
 __global__ void __cluster_dims__(CLUSTER, 1, 1) __launch_bounds__(THREADS, 2)
@@ -152,22 +161,27 @@ fc_cluster(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ C
   if (!ok && lane == 0) atomicExch(&s_error, (uint32_t)GEMM_ERR_EPILOGUE_WAIT);
   if (threadIdx.x < COLS) {
     const int c = threadIdx.x, n = n0 + c, m = m0 + (int)rank * 4;
-    float4 v[CLUSTER];
+    float v[CLUSTER][4], err[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-    for (int s = 0; s < CLUSTER; s++) v[s] = recv[s * COLS + c];
+    for (int s = 0; s < CLUSTER; s++) {
+      const float4 q = recv[s * COLS + c];
+      v[s][0] = q.x, v[s][1] = q.y, v[s][2] = q.z, v[s][3] = q.w;
+    }
 #pragma unroll
     for (int d = 1; d < CLUSTER; d *= 2)
 #pragma unroll
-      for (int s = 0; s < CLUSTER; s += 2 * d) {
-        v[s].x += v[s + d].x;
-        v[s].y += v[s + d].y;
-        v[s].z += v[s + d].z;
-        v[s].w += v[s + d].w;
-      }
+      for (int s = 0; s < CLUSTER; s += 2 * d)
+#pragma unroll
+        for (int k = 0; k < 4; k++) v[s][k] = add_keep_error(v[s][k], v[s + d][k], err[k]);
     if (ok && n < N) {
       const float b = bias ? *(bias + n) : 0.f;
       float* o = out + (size_t)m * ldo + n;
-      const float r[4] = {v[0].x + b, v[0].y + b, v[0].z + b, v[0].w + b};
+      float r[4];
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        r[k] = add_keep_error(v[0][k], b, err[k]);
+        r[k] += err[k] == err[k] ? err[k] : 0.f;  // (not a number beside infinities; r is right then)
+      }
 #pragma unroll
       for (int k = 0; k < 4; k++)
         if (m + k < M) o[(size_t)k * ldo] = r[k];

@@ -730,10 +730,10 @@ cudaError_t nn_fc_skinny(const void* a, int lda, const void* w, int ldw, const f
                          uint32_t* status, cudaStream_t s) {
   const size_t smem = (size_t)FC_NB * K * sizeof(__nv_bfloat16);
   if (K % 8 || lda % 8 || ldw % 8 || (((uintptr_t)a | (uintptr_t)w) & 15) || smem > 100 * 1024 || M <= 0) return cudaErrorInvalidValue;
-  // Above 1536 the sums of 16 products that the tensor core makes are both faster and closer (us and relative error against 64 bits,
-  // here / there: 32 x 1000 x 2048 9.0 / 4.3, 64 x 1000 x 2048 11.8 / 5.0, 8.3e-8 / 7.9e-8; 64 x 1000 x 1544 7.90e-8 / 7.77e-8).  Below, the
-  // chains of FMAs per lane are short and the error there is up to 2 % larger than here (K = 512: 5.2e-8 / 5.3e-8), although it is
-  // faster too (64 x 1192 x 512 7.5 / 3.8).  Rows that overlap (broadcast ones, say) have no tensor map.
+  // Above 1536 the sums of 16 products that the tensor core makes are both faster and closer (us here / there: 32 x 1000 x 2048 9.0 / 4.3,
+  // 64 x 1000 x 2048 11.8 / 5.0; errors in fc_cluster.cu).  Below, they were faster too (64 x 1192 x 512 7.5 / 3.8), but up to 2 % further from
+  // the exact sums than the short chains of FMAs per lane (K = 512: 5.2e-8 / 5.3e-8) when the line was drawn, before rounding errors were
+  // kept there.  Rows that overlap (broadcast ones, say) have no tensor map.
   if (K > 1536 && K <= 2048 && lda >= K && ldw >= K && M <= (1 << 20) && nn_fc_cluster_fits())
     return nn_fc_cluster(a, lda, w, ldw, bias, out, ldo, M, N, K, status, s);
   static PerDeviceFlag attr_set;
