@@ -455,16 +455,24 @@ __global__ void __launch_bounds__(256) layernorm_rows(const __nv_bfloat16* x,
 // LayerNorm for hidden sizes of 256, 512, 768 and 1024: a thread has eight columns of R rows, so that a row's 8 bytes of
 // parameters per column are read once for R rows (a warp with a row of its own read twice as many bytes of parameters as of the
 // row); rows never leave registers, both reductions halve their list of rows at every step through the warp and meet in
-// shared memory.  Us, a warp per row against this: 6144 x 1024 6.6 and 5.35, 4096 x 768 3.95 and 3.55, 2048 x 1024 4.6 and 2.8,
-// 1024 x 768 2.9 and 2.2, 128 x 768 2.05 and 1.5 (1184 x 768, eight rows for every SM, 2.1 and 2.3).
-// v[r]: this thread's eight columns of rows row0 + r (values of rows behind the last one are not stored).  One warp per 256 columns.
+// shared memory.  Us with the product of hidden columns before it, a warp per row against this: 6144 x 1024 20.1 and 18.5, 4096 x 768
+// 11.6 and 11.0, 2368 x 1024 13.1 and 11.3, 1184 x 768 8.65 and 7.7, 128 x 768 6.0 and 5.6, 6144 x 512 10.65 and 9.8, 4096 x 256 7.1 and 6.85.
+// (Alone, one after the other, a warp per row wins where its blocks fill the SMs exactly: 1184 x 768 2.0 and 2.4, 1176 x 768 3.2 and 2.4.)
+// v[r]: this thread's eight columns of rows row0 + r (values of rows behind the last one are not stored).  One warp per 256 columns,
+// and for the narrow rows several groups of warps per block (row_groups), each with rows of its own: 12288 x 256 9.2 us with four
+// groups, 12.3 with one, 6144 x 512 9.8 and 10.6.
+constexpr int row_groups(int vpl) { return vpl == 1 ? 4 : vpl == 2 ? 2 : 1; }
+template <int VPL>
+__device__ __forceinline__ int row_group() {
+  return row_groups(VPL) == 1 ? 0 : threadIdx.x / (32 * VPL);
+}
 template <int VPL, int R>
 __device__ __forceinline__ void normalise_rows(float (&v)[R][8], float (&s)[R], const float* gamma, const float* beta, __nv_bfloat16* y,
                                                int row0, int rows, float eps) {
   static_assert(R == 2 || R == 4, "a power of two; the steps of the reduction below");
   constexpr int HIDDEN = VPL * 256;
-  __shared__ __align__(16) float sh[2][VPL][R];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, c0 = threadIdx.x * 8;
+  __shared__ __align__(16) float shared[2][row_groups(VPL)][VPL][R];
+  const int group = row_group<VPL>(), warp = (threadIdx.x >> 5) - group * VPL, lane = threadIdx.x & 31, c0 = (warp * 32 + lane) * 8;
   float4 g4[2], b4[2];
 #pragma unroll
   for (int i = 0; i < 2; i++) {
@@ -486,13 +494,14 @@ __device__ __forceinline__ void normalise_rows(float (&v)[R][8], float (&s)[R], 
         s[0] += __shfl_xor_sync(0xffffffffu, s[0], d);
       }
     }
-    if (lane < R) sh[buf][warp][lane] = s[0];
+    float(*sh)[R] = shared[buf][group];
+    if (lane < R) sh[warp][lane] = s[0];
     __syncthreads();
 #pragma unroll
     for (int r = 0; r < R; r++) {
-      s[r] = sh[buf][0][r];
+      s[r] = sh[0][r];
 #pragma unroll
-      for (int w = 1; w < VPL; w++) s[r] += sh[buf][w][r];
+      for (int w = 1; w < VPL; w++) s[r] += sh[w][r];
     }
   };
   block_sums(s, 0);
@@ -524,15 +533,15 @@ __device__ __forceinline__ void normalise_rows(float (&v)[R][8], float (&s)[R], 
 }
 
 template <int VPL, int R>  // hidden = VPL * 256
-__global__ void __launch_bounds__(32 * VPL) layernorm_rows_vec(const __nv_bfloat16* x, const __nv_bfloat16* residual, const float* gamma,
+__global__ void __launch_bounds__(32 * VPL * row_groups(VPL)) layernorm_rows_vec(const __nv_bfloat16* x, const __nv_bfloat16* residual, const float* gamma,
                                                                const float* beta, __nv_bfloat16* y, int rows, float eps) {
   ptx::grid_dep_launch();
   ptx::grid_dep_wait();
-  const int row0 = blockIdx.x * R;
+  const int group = row_group<VPL>(), row0 = (blockIdx.x * row_groups(VPL) + group) * R, c0 = (threadIdx.x - group * 32 * VPL) * 8;
   uint4 q[R], q2[R];
 #pragma unroll
   for (int r = 0; r < R; r++) {
-    const size_t at = (size_t)min(row0 + r, rows - 1) * (VPL * 256) + threadIdx.x * 8;
+    const size_t at = (size_t)min(row0 + r, rows - 1) * (VPL * 256) + c0;
     q[r] = *reinterpret_cast<const uint4*>(x + at);
     q2[r] = residual ? *reinterpret_cast<const uint4*>(residual + at) : make_uint4(0u, 0u, 0u, 0u);
   }
@@ -588,16 +597,16 @@ __global__ void __launch_bounds__(256) bert_embed_ln(const g_params* stub, const
 }
 
 // The same with eight columns of R tokens per thread (see layernorm_rows_vec).  Us, a block per token against this: 4096 tokens of
-// 768 12.6 and 4.5, 6144 of 1024 20.8 and 6.6, 128 of 768 3.0 and 1.9.
+// 768 12.6 and 4.5, 6144 of 1024 20.8 and 6.5, 128 of 768 3.1 and 1.9.
 template <int VPL, int R>
-__global__ void __launch_bounds__(32 * VPL) bert_embed_ln_vec(const g_params* stub, const int* direct_ids, size_t req_stride, int seq,
+__global__ void __launch_bounds__(32 * VPL * row_groups(VPL)) bert_embed_ln_vec(const g_params* stub, const int* direct_ids, size_t req_stride, int seq,
                                                               int tokens, const __nv_bfloat16* word, const __nv_bfloat16* pos,
                                                               const __nv_bfloat16* type, const float* gamma, const float* beta,
                                                               __nv_bfloat16* y, int vocab, float eps) {
   ptx::grid_dep_launch();
   ptx::grid_dep_wait();
   constexpr int HIDDEN = VPL * 256;
-  const int row0 = blockIdx.x * R, c0 = threadIdx.x * 8;
+  const int group = row_group<VPL>(), row0 = (blockIdx.x * row_groups(VPL) + group) * R, c0 = (threadIdx.x - group * 32 * VPL) * 8;
   uint4 q[R], q2[R];
 #pragma unroll
   for (int r = 0; r < R; r++) {
@@ -768,6 +777,13 @@ cudaError_t nn_softmax_response(const float* logits, int rows, int n, int ld, co
   return launch_pdl(softmax_response, dim3(rows), dim3(256), 0, s, logits, n, ld, (const g_params*)d_stub, (uint8_t*)direct_out,
                     resp_stride, write_argmax, counter, flag, flag_value, (const RespPushCtx*)d_push);
 }
+// Four rows per block instead of two once there is enough for every SM: about 4000 rows of 768, 3000 of 1024, 7500 of 512, never for 256 (us,
+// two against four, with the product of hidden columns before it: 3072 x 768 9.3 / 9.9, 4096 x 768 11.06 / 11.01, 4736 x 768 12.44 / 12.34, 2368 x
+// 1024 11.3 / 11.9, 4096 x 1024 14.3 / 13.8, 6144 x 512 9.8 / 10.4, 8192 x 512 11.7 / 11.5, 12288 x 256 9.2 / 9.6; embedding 2560 x 768 10.1 / 10.8,
+// 5120 x 768 13.75 / 13.4).  Eight: 5.8 for 6144 x 1024 alone against 5.35, 121 registers.
+static bool four_rows(int rows, int hidden) {
+  return hidden > 256 && (size_t)rows * hidden >= (hidden == 512 ? 26000u : 20480u) * (size_t)srpc_gemm_grid_sms();
+}
 cudaError_t nn_layernorm(const void* x, const void* residual, const float* gamma, const float* beta, void* y, int rows,
                          int hidden, float eps, cudaStream_t s) {
   if (hidden > 2048) return cudaErrorInvalidValue;
@@ -775,16 +791,15 @@ cudaError_t nn_layernorm(const void* x, const void* residual, const float* gamma
   const __nv_bfloat16 *xp = (const __nv_bfloat16*)x, *rp = (const __nv_bfloat16*)residual;
   __nv_bfloat16* yp = (__nv_bfloat16*)y;
   if (aligned && rows > 0 && hidden % 256 == 0 && hidden <= 1024) {
-    // Four rows per block once that gives every SM three of them, two for fewer rows (us, two against four: 6144 x 1024 5.8 / 5.35,
-    // 2048 x 1024 3.1 / 2.8, 1184 x 768 2.3 / 2.5); eight: 5.8 for the first, 121 registers.
-    const bool many = rows >= 12 * srpc_gemm_grid_sms();
-    auto go = [&](auto* kernel, int r) {
-      return launch_pdl(kernel, dim3((rows + r - 1) / r), dim3(hidden / 8), 0, s, xp, rp, gamma, beta, yp, rows, eps);
+    const bool many = four_rows(rows, hidden);
+    auto go = [&](auto* kernel, int vpl, int r) {
+      const int per_block = r * row_groups(vpl);
+      return launch_pdl(kernel, dim3((rows + per_block - 1) / per_block), dim3(32 * vpl * row_groups(vpl)), 0, s, xp, rp, gamma, beta, yp, rows, eps);
     };
-    if (hidden == 256) return many ? go(layernorm_rows_vec<1, 4>, 4) : go(layernorm_rows_vec<1, 2>, 2);
-    if (hidden == 512) return many ? go(layernorm_rows_vec<2, 4>, 4) : go(layernorm_rows_vec<2, 2>, 2);
-    if (hidden == 768) return many ? go(layernorm_rows_vec<3, 4>, 4) : go(layernorm_rows_vec<3, 2>, 2);
-    return many ? go(layernorm_rows_vec<4, 4>, 4) : go(layernorm_rows_vec<4, 2>, 2);
+    if (hidden == 256) return go(layernorm_rows_vec<1, 2>, 1, 2);
+    if (hidden == 512) return many ? go(layernorm_rows_vec<2, 4>, 2, 4) : go(layernorm_rows_vec<2, 2>, 2, 2);
+    if (hidden == 768) return many ? go(layernorm_rows_vec<3, 4>, 3, 4) : go(layernorm_rows_vec<3, 2>, 3, 2);
+    return many ? go(layernorm_rows_vec<4, 4>, 4, 4) : go(layernorm_rows_vec<4, 2>, 4, 2);
   }
   return launch_pdl(layernorm_rows, dim3(rows), dim3(256), 0, s, xp, rp, gamma, beta, yp, hidden, eps);
 }
@@ -795,14 +810,15 @@ cudaError_t nn_bert_embed_ln(const void* d_stub, const int* direct_ids, size_t r
   const int tokens = batch * seq;
   const uintptr_t all = (uintptr_t)word | (uintptr_t)pos | (uintptr_t)type | (uintptr_t)gamma | (uintptr_t)beta | (uintptr_t)y;
   if ((all & 15) == 0 && tokens > 0 && (hidden == 768 || hidden == 1024)) {
-    const bool many = tokens >= 12 * srpc_gemm_grid_sms();  // as in nn_layernorm
-    auto go = [&](auto* kernel, int r) {
-      return launch_pdl(kernel, dim3((tokens + r - 1) / r), dim3(hidden / 8), 0, s, (const g_params*)d_stub, direct_ids, req_stride, seq,
-                        tokens, (const __nv_bfloat16*)word, (const __nv_bfloat16*)pos, (const __nv_bfloat16*)type, gamma, beta,
-                        (__nv_bfloat16*)y, vocab, eps);
+    const bool many = four_rows(tokens, hidden);
+    auto go = [&](auto* kernel, int vpl, int r) {
+      const int per_block = r * row_groups(vpl);
+      return launch_pdl(kernel, dim3((tokens + per_block - 1) / per_block), dim3(32 * vpl * row_groups(vpl)), 0, s, (const g_params*)d_stub,
+                        direct_ids, req_stride, seq, tokens, (const __nv_bfloat16*)word, (const __nv_bfloat16*)pos,
+                        (const __nv_bfloat16*)type, gamma, beta, (__nv_bfloat16*)y, vocab, eps);
     };
-    if (hidden == 768) return many ? go(bert_embed_ln_vec<3, 4>, 4) : go(bert_embed_ln_vec<3, 2>, 2);
-    return many ? go(bert_embed_ln_vec<4, 4>, 4) : go(bert_embed_ln_vec<4, 2>, 2);
+    if (hidden == 768) return many ? go(bert_embed_ln_vec<3, 4>, 3, 4) : go(bert_embed_ln_vec<3, 2>, 3, 2);
+    return many ? go(bert_embed_ln_vec<4, 4>, 4, 4) : go(bert_embed_ln_vec<4, 2>, 4, 2);
   }
   return launch_pdl(bert_embed_ln, dim3(tokens), dim3(256), 0, s, (const g_params*)d_stub, direct_ids, req_stride, seq,
                     (const __nv_bfloat16*)word, (const __nv_bfloat16*)pos, (const __nv_bfloat16*)type, gamma, beta,

@@ -382,9 +382,9 @@ def test_model_server_end_to_end_resnet(torch_cuda, fused_ingress):
 
 
 @pytest.mark.parametrize("hidden", [256, 512, 768, 1024])
-@pytest.mark.parametrize("rows", [1, 2, 3, 127, 1775, 1777, 2051])
+@pytest.mark.parametrize("rows", [1, 2, 3, 7, 127, 1775, 1777, 2051, 2959, 3949, 7517])
 def test_layernorm_rows_per_block(torch_cuda, rows, hidden):
-    """Two and four rows per block, last blocks with rows missing, residual added or not, rows with a large offset."""
+    """Two and four rows per group, one to four groups per block, last blocks with rows or groups missing, residual added or not, rows with a large offset."""
     torch = torch_cuda
     from splitrpc_b200 import ops
 
@@ -401,9 +401,10 @@ def test_layernorm_rows_per_block(torch_cuda, rows, hidden):
         assert (buf[rows] == 7.0).all()
 
 
-@pytest.mark.parametrize("batch,seq,hidden", [(1, 1, 768), (1, 3, 1024), (5, 7, 768), (14, 127, 768), (14, 127, 1024)])
+@pytest.mark.parametrize("batch,seq,hidden", [(1, 1, 768), (1, 3, 1024), (5, 7, 768), (14, 127, 768), (14, 127, 1024), (32, 127, 768), (24, 127, 1024)])
 def test_embedding_layernorm_tokens_per_block(torch_cuda, batch, seq, hidden):
-    """Two and four tokens per block, last blocks with tokens missing, blocks across sequences, ids outside the vocabulary."""
+    """Two and four tokens per group, one to four groups per block, last blocks with tokens or groups missing, groups across sequences, ids
+    outside the vocabulary."""
     torch = torch_cuda
     from splitrpc_b200 import ops
 
