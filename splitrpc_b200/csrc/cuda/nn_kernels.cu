@@ -597,7 +597,7 @@ __global__ void __launch_bounds__(256) bert_embed_ln(const g_params* stub, const
 }
 
 // The same with eight columns of R tokens per thread (see layernorm_rows_vec).  Us, a block per token against this: 4096 tokens of
-// 768 12.6 and 4.5, 6144 of 1024 20.8 and 6.5, 128 of 768 3.1 and 1.9.
+// 768 12.6 and 4.5, 6144 of 1024 20.8 and 6.5, 128 of 768 3.1 and 1.9, 4096 of 512 10.6 and 3.9, 4096 of 256 8.6 and 3.3, 128 of 256 2.1 and 1.8.
 template <int VPL, int R>
 __global__ void __launch_bounds__(32 * VPL * row_groups(VPL)) bert_embed_ln_vec(const g_params* stub, const int* direct_ids, size_t req_stride, int seq,
                                                               int tokens, const __nv_bfloat16* word, const __nv_bfloat16* pos,
@@ -780,7 +780,7 @@ cudaError_t nn_softmax_response(const float* logits, int rows, int n, int ld, co
 // Four rows per block instead of two once there is enough for every SM: about 4000 rows of 768, 3000 of 1024, 7500 of 512, never for 256 (us,
 // two against four, with the product of hidden columns before it: 3072 x 768 9.3 / 9.9, 4096 x 768 11.06 / 11.01, 4736 x 768 12.44 / 12.34, 2368 x
 // 1024 11.3 / 11.9, 4096 x 1024 14.3 / 13.8, 6144 x 512 9.8 / 10.4, 8192 x 512 11.7 / 11.5, 12288 x 256 9.2 / 9.6; embedding 2560 x 768 10.1 / 10.8,
-// 5120 x 768 13.75 / 13.4).  Eight: 5.8 for 6144 x 1024 alone against 5.35, 121 registers.
+// 5120 x 768 13.75 / 13.4, 6144 x 512 10.7 / 11.2).  Eight: 5.8 for 6144 x 1024 alone against 5.35, 121 registers.
 static bool four_rows(int rows, int hidden) {
   return hidden > 256 && (size_t)rows * hidden >= (hidden == 512 ? 26000u : 20480u) * (size_t)srpc_gemm_grid_sms();
 }
@@ -809,7 +809,7 @@ cudaError_t nn_bert_embed_ln(const void* d_stub, const int* direct_ids, size_t r
   if (hidden > 2048) return cudaErrorInvalidValue;
   const int tokens = batch * seq;
   const uintptr_t all = (uintptr_t)word | (uintptr_t)pos | (uintptr_t)type | (uintptr_t)gamma | (uintptr_t)beta | (uintptr_t)y;
-  if ((all & 15) == 0 && tokens > 0 && (hidden == 768 || hidden == 1024)) {
+  if ((all & 15) == 0 && tokens > 0 && hidden % 256 == 0 && hidden <= 1024) {
     const bool many = four_rows(tokens, hidden);
     auto go = [&](auto* kernel, int vpl, int r) {
       const int per_block = r * row_groups(vpl);
@@ -817,6 +817,8 @@ cudaError_t nn_bert_embed_ln(const void* d_stub, const int* direct_ids, size_t r
                         direct_ids, req_stride, seq, tokens, (const __nv_bfloat16*)word, (const __nv_bfloat16*)pos,
                         (const __nv_bfloat16*)type, gamma, beta, (__nv_bfloat16*)y, vocab, eps);
     };
+    if (hidden == 256) return go(bert_embed_ln_vec<1, 2>, 1, 2);
+    if (hidden == 512) return many ? go(bert_embed_ln_vec<2, 4>, 2, 4) : go(bert_embed_ln_vec<2, 2>, 2, 2);
     if (hidden == 768) return many ? go(bert_embed_ln_vec<3, 4>, 3, 4) : go(bert_embed_ln_vec<3, 2>, 3, 2);
     return many ? go(bert_embed_ln_vec<4, 4>, 4, 4) : go(bert_embed_ln_vec<4, 2>, 4, 2);
   }

@@ -401,7 +401,8 @@ def test_layernorm_rows_per_block(torch_cuda, rows, hidden):
         assert (buf[rows] == 7.0).all()
 
 
-@pytest.mark.parametrize("batch,seq,hidden", [(1, 1, 768), (1, 3, 1024), (5, 7, 768), (14, 127, 768), (14, 127, 1024), (32, 127, 768), (24, 127, 1024)])
+@pytest.mark.parametrize("batch,seq,hidden", [(1, 1, 768), (1, 3, 1024), (5, 7, 768), (14, 127, 768), (14, 127, 1024), (32, 127, 768), (24, 127, 1024),
+                                              (1, 1, 256), (3, 3, 256), (7, 127, 256), (1, 3, 512), (5, 7, 512), (60, 127, 512)])
 def test_embedding_layernorm_tokens_per_block(torch_cuda, batch, seq, hidden):
     """Two and four tokens per group, one to four groups per block, last blocks with tokens or groups missing, groups across sequences, ids
     outside the vocabulary."""
