@@ -3,8 +3,18 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 
-_LAUNCHES = ("gemm", "fc_skinny", "conv2d_nhwc", "conv1x1_dual", "stem_s2d", "stem_conv", "maxpool3x3s2", "global_avgpool",
-             "softmax_response", "layernorm", "bert_embed_ln", "attention_tc_qkv")
+# what the models call at the least
+_CALLS = {"resnet": {"stem_s2d", "stem_conv", "maxpool3x3s2", "gemm", "conv2d_nhwc", "conv1x1_chain", "conv1x1_dual", "global_avgpool", "fc_skinny", "softmax_response"},
+          "bert": {"bert_embed_ln", "gemm", "attention_tc_qkv", "layernorm", "softmax_response"}}
+
+
+def _launches():
+    """Every function of ``ops`` that launches something, so that a kernel which joins a model is waited for as well."""
+    import inspect
+    from splitrpc_b200 import ops
+
+    return [n for n, f in vars(ops).items() if inspect.isfunction(f) and f.__module__ == ops.__name__ and not n.startswith("_")
+            and n not in ("status_word", "check_status")]
 
 
 def _model(name):
@@ -28,14 +38,17 @@ def _want(name, run, out, monkeypatch):
     import torch
     from splitrpc_b200 import ops
 
+    calls = set()
     with monkeypatch.context() as mp:
-        for f in _LAUNCHES:
-            def waited(*a, _f=getattr(ops, f), **k):
+        for f in _launches():
+            def waited(*a, _n=f, _f=getattr(ops, f), **k):
                 r = _f(*a, **k)
+                calls.add(_n)
                 torch.cuda.synchronize()
                 return r
             mp.setattr(ops, f, waited)
         run(out)
+    assert calls >= _CALLS[name.rstrip("0123456789")]
     return out.clone()
 
 
