@@ -1,12 +1,13 @@
-// Persistent tcgen05 GEMM / convolution kernel (the production path).
+// Persistent tcgen05 GEMM / convolution kernel on single SMs, and the choice between it and CTA pairs.
 //
 //   D[M,N] = act(A[M,K] . B[N,K]^T + bias + residual)          (GEMM mode)
 //   out = act(conv(in NHWC, filter [Cout][R][S][Cin]) + bias + residual)   (convolution mode)
 //
 // One CTA per SM loops over output tiles (128 x BN).  Warp roles:
-//   warp 0 and the last warp   one thread each issues the TMA loads of every second
-//            k-block of this CTA's tiles, running ahead through a STAGES-deep
-//            shared-memory ring that is not drained at tile boundaries;
+//   warp 0 and the last warp   walk the schedule as one; an elected lane of each
+//            issues the TMA loads of every second k-block of this CTA's tiles,
+//            running ahead through a STAGES-deep shared-memory ring that is not
+//            drained at tile boundaries;
 //   warp 1   walks the schedule as one and waits; one elected lane issues
 //            tcgen05.mma into one of ACC TMEM accumulators (BN columns each), so
 //            tile i+1 accumulates while tile i is being written out;
@@ -21,7 +22,10 @@
 // PW x PH x PN patch of output pixels, and the rows for filter tap (fr, fs) are
 // one 4-D TMA box over the NHWC input shifted by the tap offset, with element
 // strides equal to the convolution stride; out-of-image coordinates are
-// zero-filled by the TMA unit, which is exactly the padding.
+// zero-filled by the TMA unit, which is exactly the padding.  Dense inputs go
+// to CTA pairs (gemm_2sm.cu); this form has the inputs with pixel strides or in
+// a request ring that stem_conv.cu does not take, and every input when
+// SPLITRPC_GEMM_2SM=0 turns pairs off.
 // All operands live in this GPU's memory; no load uses multicast.  Every wait
 // is bounded; on a timeout the kernel records an error code, stops issuing work,
 // frees its tensor memory and returns.
@@ -384,7 +388,7 @@ gemm_conv_persistent(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
         if (p.reuse) {
           // r filter rows: A a patch row further into the box, B the next filter row of this (filter column, channel block).
           // One unrolled run of MMAs per load group: issuing them was what a 64-wide tile took its time for (56 ns per MMA, 27 now;
-          // 64 images of 56 x 56 x 64 29.5 -> 23.9 us, 28 x 28 x 128 22.2 -> 20.3, 14 x 14 x 256 21.6 -> 18.7).
+          // 64 images with pairs turned off: 28 x 28 x 128 22.2 -> 20.3 us, 14 x 14 x 256 21.6 -> 18.7; pairs 17.0 and 16.5).
           const uint32_t sb = p.b_stationary ? panel_lo + (uint32_t)kb * (B_BYTES / 16) : sa + A_BYTES / 16;
           if (elected) {
             if (p.r == 3) {

@@ -167,16 +167,46 @@ def test_expansion_and_reduction_in_one_kernel(env, n, h, w, narrow, second):
     assert ((want.double() - ref).abs() <= ref.abs() * 2.0 ** -8 + k * k * 0.064 * 2.0 ** -24 + 1e-6).all()
 
 
+def _one_sm_conv(torch, ops, x, w, bias=None, residual=None, stride=1, pad=0, act=None, x2=None, stride2=1):
+    """The convolution by the one-SM kernel: inputs with strides of their own (here the dense ones) always take it."""
+    from splitrpc_b200 import _C
+
+    (n, h, wd, c), (cout, r, s, _) = x.shape, w.shape
+    out = torch.empty(n, (h + 2 * pad - r) // stride + 1, (wd + 2 * pad - s) // stride + 1, cout, device="cuda", dtype=torch.bfloat16)
+    _C.conv_bf16(x.data_ptr(), w.data_ptr(), n, h, wd, c, cout, r, s, stride, pad, out.data_ptr(), 0 if bias is None else bias.data_ptr(),
+                 0 if residual is None else residual.data_ptr(), ops.ACT[act], ops.status_word().data_ptr(),
+                 torch.cuda.current_stream().cuda_stream, 2, c, wd * c, h * wd * c,
+                 **({} if x2 is None else dict(in2=x2.data_ptr(), h2=x2.shape[1], w2=x2.shape[2], cin2=x2.shape[3], stride2=stride2)))
+    return out
+
+
 @pytest.mark.parametrize("n,h,w,cout,r,s", [(1, 20, 16, 128, 4, 1), (1, 11, 14, 72, 4, 1), (1, 20, 16, 128, 2, 1), (1, 20, 16, 200, 3, 1), (2, 20, 16, 64, 4, 1)])
 def test_conv_with_few_wide_load_groups(env, n, h, w, cout, r, s):
-    """Short filters on small images: all row taps of a column travel in one load group, and the ring holds one to three."""
+    """Short filters on small images in the one-SM kernel: all row taps of a column travel in one load group, and the ring holds one to
+    three.  CTA pairs, which dense inputs take, give the same bits."""
     torch, ops = env
     x = torch.randn(n, h, w, 64, device="cuda").bfloat16()
     f = (torch.randn(cout, r, s, 64, device="cuda") / (64 * r * s) ** 0.5).bfloat16()
-    out = ops.conv2d_nhwc(x, f)
+    out = _one_sm_conv(torch, ops, x, f)
     ops.check_status()
     ref = torch.nn.functional.conv2d(x.double().permute(0, 3, 1, 2), f.double().permute(0, 3, 1, 2)).permute(0, 2, 3, 1)
     assert out.shape == ref.shape and ((out.double() - ref).norm() / ref.norm()).item() < 2.0 ** -8  # one rounding to bf16
+    assert torch.equal(ops.conv2d_nhwc(x, f), out)
+
+
+@pytest.mark.parametrize("n,oh,c1,h2,c2,cout,stride2", [(2, 14, 64, 14, 64, 256, 1), (3, 9, 128, 17, 64, 72, 2), (2, 7, 512, 14, 256, 512, 2), (1, 30, 64, 90, 64, 64, 3)])
+def test_two_inputs_in_the_one_sm_kernel(env, n, oh, c1, h2, c2, cout, stride2):
+    """The two-input form for inputs with strides of their own gives the bits of CTA pairs."""
+    torch, ops = env
+    x1, x2 = torch.randn(n, oh, oh, c1, device="cuda").bfloat16(), torch.randn(n, h2, h2, c2, device="cuda").bfloat16()
+    w = (torch.randn(cout, c1 + c2, device="cuda") / (c1 + c2) ** 0.5).bfloat16()
+    bias = torch.randn(cout, device="cuda")
+    out = _one_sm_conv(torch, ops, x1, w.view(cout, 1, 1, c1 + c2), bias, act="relu", x2=x2, stride2=stride2)
+    got = ops.conv1x1_dual(x1, x2, w, bias=bias, stride2=stride2, act="relu")
+    ops.check_status()
+    ref = torch.relu(x1.double() @ w[:, :c1].double().t() + x2[:, ::stride2, ::stride2].double() @ w[:, c1:].double().t() + bias.double())
+    assert ((out.double() - ref).norm() / ref.norm()).item() < 2.0 ** -8  # one rounding to bf16
+    assert torch.equal(got, out)
 
 
 @pytest.mark.parametrize("n,h,cin,cout,r,stride,pad", [(2, 56, 64, 64, 3, 1, 1), (4, 28, 128, 128, 3, 1, 1),
@@ -265,18 +295,6 @@ def test_conv_linear_pixels(env, h, w, cin, cout, r, s, stride, pad):
         part = ops.conv2d_nhwc(x[:n].contiguous(), wt, bias=bias, residual=res[:n].contiguous(), stride=stride, pad=pad, act="relu")
         assert torch.equal(part, whole[:n])
     ops.check_status()
-
-
-def _one_sm_conv(torch, ops, x, w, bias=None, residual=None, stride=1, pad=0, act=None):
-    """The convolution by the one-SM kernel: inputs with strides of their own (here the dense ones) always take it."""
-    from splitrpc_b200 import _C
-
-    (n, h, wd, c), (cout, r, s, _) = x.shape, w.shape
-    out = torch.empty(n, (h + 2 * pad - r) // stride + 1, (wd + 2 * pad - s) // stride + 1, cout, device="cuda", dtype=torch.bfloat16)
-    _C.conv_bf16(x.data_ptr(), w.data_ptr(), n, h, wd, c, cout, r, s, stride, pad, out.data_ptr(), 0 if bias is None else bias.data_ptr(),
-                 0 if residual is None else residual.data_ptr(), ops.ACT[act], ops.status_word().data_ptr(),
-                 torch.cuda.current_stream().cuda_stream, 2, c, wd * c, h * wd * c)
-    return out
 
 
 @pytest.mark.parametrize("n,h,w,cin,cout,r,s,stride,pad", [(3, 56, 56, 64, 64, 3, 3, 1, 1), (5, 14, 14, 256, 136, 3, 3, 1, 1), (2, 8, 14, 128, 64, 2, 5, 1, 0),
