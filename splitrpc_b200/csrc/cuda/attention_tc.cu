@@ -58,13 +58,7 @@ struct AttSmem {
   static_assert(!ALIAS || P_BYTES <= Q_BYTES + K_BYTES, "P must fit over Q and K");
 };
 
-// VMN = true: V is read in place from the fused Q|K|V projection ([tokens, 3*hidden], V in the last third).  A V tile
-// is then [keys, 64] with the head dimension contiguous, i.e. an MN-major B operand of the second product: same
-// 128-byte-swizzled shared-memory tile and descriptor, "B is MN-major" in the instruction descriptor, and a step of 16
-// keys along K is 2048 bytes (two 8-row groups) instead of 32.  No transposed copy of V and no separate V GEMM.
-template <int SOFT_THREADS>
-__device__ __forceinline__ void soft_sync() { asm volatile("bar.sync 1, %0;" ::"n"(SOFT_THREADS) : "memory"); }
-// The same barrier with the AND of the threads' predicates.
+// Barrier of the softmax warps with the AND of their threads' predicates.
 template <int SOFT_THREADS>
 __device__ __forceinline__ bool soft_all(bool pred) {
   uint32_t out;
@@ -77,6 +71,10 @@ __device__ __forceinline__ bool soft_all(bool pred) {
   return out != 0;
 }
 
+// VMN = true: V is read in place from the fused Q|K|V projection ([tokens, 3*hidden], V in the last third).  A V tile
+// is then [keys, 64] with the head dimension contiguous, i.e. an MN-major B operand of the second product: same
+// 128-byte-swizzled shared-memory tile and descriptor, "B is MN-major" in the instruction descriptor, and a step of 16
+// keys along K is 2048 bytes (two 8-row groups) instead of 32.  No transposed copy of V and no separate V GEMM.
 template <int SEQ, bool VMN>
 __global__ void __launch_bounds__(AttThreads<SEQ>::TOTAL, SEQ == QT ? 3 : 1)
 attention_tc(const __grid_constant__ CUtensorMap tmap_qk, const __grid_constant__ CUtensorMap tmap_vt,

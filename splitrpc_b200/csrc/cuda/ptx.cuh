@@ -323,9 +323,6 @@ __device__ __forceinline__ uint32_t mapa_shared(uint32_t addr, uint32_t rank) {
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
   return r;
 }
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 // The two halves of a cluster barrier without memory ordering: for set-up (mbarrier initialisation has its own fence) and
 // for leaving (nothing is read that the peer wrote).  The ordered form takes 0.85 us, each time.
 __device__ __forceinline__ void cluster_arrive_relaxed() {
