@@ -381,6 +381,37 @@ def test_model_server_end_to_end_resnet(torch_cuda, fused_ingress):
     torch.testing.assert_close(got, direct[0].cpu(), rtol=1e-3, atol=1e-5)
 
 
+@pytest.mark.parametrize("n", [1, 7, 255, 257, 2047, 2048, 2049, 5000])
+def test_softmax_response_lengths(torch_cuda, n):
+    """Rows shorter than a block, as long as its registers, longer; rows with -infinity, of one value, with no finite value or a NaN; the
+    largest logit in every part of the row."""
+    torch = torch_cuda
+    from splitrpc_b200 import ops
+
+    g = torch.Generator(device="cuda").manual_seed(n)
+    x = torch.randn(12, n + 3, device="cuda", generator=g)[:, :n] * 4
+    for r in range(6):
+        x[r, (r * (n - 1)) // 5] = 17.0 + r  # the first, the last, and between
+    x[6, ::2] = -float("inf")
+    x[6, n - 1] = 3.0
+    x[7] = -3e38
+    x[8] = -float("inf")
+    x[9, n // 2] = float("nan")
+    x[10] = 0.25
+    out = torch.full((13, n + 5), 7.0, device="cuda")
+    ops.softmax_response(x, 12, out=out, resp_stride=(n + 5) * 4, write_argmax=True)
+    torch.cuda.synchronize()
+    want = torch.softmax(x.double(), -1)
+    got = out[:12, :n]
+    assert torch.equal(got.isnan(), want.isnan())
+    # the fast exponential is off by up to 2 + 1.2 |x| units of 2^-23 for differences |x| up to about 40, twice (weight and sum)
+    ok = [0, 1, 2, 3, 4, 5, 6, 7, 10, 11]
+    assert bool(((got[ok].double() - want[ok]).abs() <= want[ok] * (2 * 50 * 2.0 ** -23) + 1e-37).all())
+    arg = out[:12, n].contiguous().view(torch.int32)
+    assert [int(a) for a in arg[:6]] == [(r * (n - 1)) // 5 for r in range(6)] and (n < 3 or int(arg[6]) == int(x[6].argmax()))
+    assert bool((out[12] == 7).all()) and bool((out[:, n + 1:] == 7).all())
+
+
 @pytest.mark.parametrize("hidden", [256, 512, 768, 1024])
 @pytest.mark.parametrize("rows", [1, 2, 3, 7, 127, 1775, 1777, 2051, 2959, 3949, 7517])
 def test_layernorm_rows_per_block(torch_cuda, rows, hidden):
