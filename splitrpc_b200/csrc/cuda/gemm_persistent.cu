@@ -1041,6 +1041,9 @@ cudaError_t srpc_conv_bf16_tma(const void* in, const void* weight, const ConvSha
   const bool dense = !cs.in_stub && !cs.in_pix_stride && !cs.in_row_stride && !cs.in_img_stride;
   if (dense && !cs.in2 && cs.r == 1 && cs.s == 1 && cs.stride == 1 && cs.pad == 0)
     return srpc_gemm_bf16_v2(in, cs.cin, weight, cs.cin, cs.n * cs.h * cs.w, cs.cout, cs.cin, ep2, status, stream);
+  // Every other dense convolution goes to pairs: of 745 (filters of 1 to 5 rows, steps of 1 and 2, 7 .. 224 pixels wide, 64 .. 512 channels, 1 .. 64 images)
+  // the one-SM form is 1.34 times slower on average; it is ahead by up to 11 % on a few of the largest (16 x 224 x 224 x 64, 3x3 90 and 83 us; 8 x
+  // 28 x 28 x 512, 5x5 66 and 58), where pairs still gain on what was there before them (105 and 79).
   if (srpc_conv_2sm_eligible(cs, ep2)) {
     const TileShape ts = pick_tile(cs.n * cs.oh * cs.ow, cs.cout, (cs.r * cs.s * cs.cin + (cs.in2 ? cs.cin2 : 0)) / BK, ep2, false, true);
     return srpc_conv_bf16_2sm(in, weight, cs, ts.bn, ts.rows, ep2, status, stream);
