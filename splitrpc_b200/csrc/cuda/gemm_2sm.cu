@@ -30,6 +30,7 @@
 //                come first, so that their transfer overlaps the rest of the GEMM.
 #include <algorithm>
 #include <cstdlib>
+#include <type_traits>
 
 #include "fast_div.h"
 #include "gemm_tcgen05.h"
@@ -152,6 +153,7 @@ __device__ __forceinline__ bool pair_tile(int j, const TileOrder& o, PairTile* o
 // Where the rows of A come from.  GEMM: a matrix.  Convolution: row i of the product is output pixel i (rows and images in
 // sequence), its A row for filter tap (fr, fs) the pixel that the tap meets, read through an im2col tensor map; k-blocks from
 // kb_split on come from a second input (two-input 1x1 convolution) by tmap_a2.
+enum { MATRIX, CONVOLUTION, TWO_INPUTS };
 struct ASource {
   int im2col, im2col2;  // of the first / second input
   int kb_split;
@@ -181,17 +183,22 @@ __device__ __forceinline__ KBlock conv_kblock(const ASource& src, int kb) {
   return KBlock{cb * BK, at * BK, (uint16_t)fs, (uint16_t)fr};
 }
 
+// The tensor-parallel part of the arguments; the plain kernel's launches do not carry its 288 bytes.
+struct NoTp {};
+template <bool TP>
+using TpArg = std::conditional_t<TP, TpParams, NoTp>;
+
 template <int BN, int RPC, bool TP>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Cfg<BN, RPC, TP>::THREADS, 1)
 gemm_2sm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                 const __grid_constant__ CUtensorMap tmap_out, const __grid_constant__ CUtensorMap tmap_a2, int M, int N, int K,
-                const TileOrder order, const ASource src, GemmEpilogue ep, uint32_t* status, const TpParams tp_in) {
+                const TileOrder order, const ASource src, GemmEpilogue ep, uint32_t* status, const TpArg<TP> tp_in) {
   using C = Cfg<BN, RPC, TP>;
   constexpr int A_BYTES = C::A_BYTES, KB_BYTES = C::KB_BYTES, KPS = C::KPS, STAGE_BYTES = C::STAGE_BYTES, STAGES = C::STAGES;
   constexpr int EPI_THREADS = C::EPI_THREADS, ACC_STRIDE = C::ACC_STRIDE, NCH = C::NCH;
   constexpr int PASSES = C::PASSES, PASS_COLS = C::PASS_COLS;
   extern __shared__ __align__(1024) uint8_t smem[];
-  TpParams tp = tp_in;
+  TpArg<TP> tp = tp_in;
   if constexpr (TP) {
     if (tp.epoch_base) tp.epoch += *tp.epoch_base;
     if ((int)(blockIdx.x >> 1) >= order.clusters) {
@@ -255,6 +262,63 @@ gemm_2sm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
     uint32_t ph = 0;
     PairTile t;
     bool ok = layout_ok, first = true;
+    // The rest of a tile's stages.  A matrix, a convolution and one with a second input have a loop each: with the choices inside one
+    // loop a stage took 50 ns more of the issuing warps' time (128 x 768 x 3072 8.1 us, now 6.8; 3x3 over 32 x 56 x 56 x 64 13.9 and 11.6,
+    // 64 x 28 x 28 x 128 16.9 and 14.7).
+    auto stages = [&](auto source, int row0, int brow0, int img, int y, int x, bool first_tile) {
+      constexpr int SOURCE = decltype(source)::value;
+      for (; st < num_st; st += PRODUCERS) {
+        // Which tap, channels and weights the stage takes: worked out before the wait (behind it, 1 % of a 3x3 convolution).
+        KBlock at[KPS];
+        if (SOURCE == CONVOLUTION || (SOURCE == TWO_INPUTS && src.im2col)) {
+#pragma unroll
+          for (int b = 0; b < KPS; b++) at[b] = conv_kblock(src, st * KPS + b);
+        }
+        ok = ptx::mbar_wait_warp(&empty_bar[s], ph ^ 1u);
+        if (!ok) {
+          if (elected) atomicExch(&s_error, GEMM_ERR_PRODUCER_WAIT);
+          break;
+        }
+        const uint32_t full_leader = ptx::mapa_shared(ptx::smem_u32(&full_bar[s]), 0);
+        uint8_t* sa = smem + (size_t)s * STAGE_BYTES;
+        if (first) {
+          // everything above overlaps the kernel before; its results are read below
+          ptx::cluster_wait();
+          if (lane == 0 && warp == 0) GEMM2_TRACE(1);
+          ptx::grid_dep_wait();
+          first = false;
+        }
+        const int blocks = KPS == 1 || st * KPS + 1 < num_kb ? KPS : 1;
+        if (elected && leader) ptx::mbar_expect_tx(&full_bar[s], 2u * KB_BYTES * blocks);
+#pragma unroll
+        for (int b = 0; b < KPS; b++) {
+          if (b >= blocks) break;
+          const int kb = st * KPS + b;
+          if (SOURCE == MATRIX || (SOURCE == TWO_INPUTS && !src.im2col && kb < src.kb_split)) {
+            if (elected) ptx::tma_load_2d_2sm(sa + b * KB_BYTES, &tmap_a, full_leader, kb * BK, row0);
+          } else if (SOURCE == CONVOLUTION || kb < src.kb_split) {
+            if (elected)
+              ptx::tma_load_im2col_2sm(sa + b * KB_BYTES, &tmap_a, full_leader, at[b].c, x * src.stride - src.pad, y * src.stride - src.pad,
+                                       img, at[b].fs, at[b].fr);
+          } else if (src.im2col2) {
+            if (elected)
+              ptx::tma_load_im2col_2sm(sa + b * KB_BYTES, &tmap_a2, full_leader, (kb - src.kb_split) * BK, x * src.stride2, y * src.stride2, img,
+                                       0, 0);
+          } else if (elected) {
+            ptx::tma_load_2d_2sm(sa + b * KB_BYTES, &tmap_a2, full_leader, (kb - src.kb_split) * BK, row0);
+          }
+          if (elected) ptx::tma_load_2d_2sm(sa + b * KB_BYTES + A_BYTES, &tmap_b, full_leader, SOURCE == CONVOLUTION || (SOURCE == TWO_INPUTS && src.im2col) ? at[b].w : kb * BK, brow0);
+        }
+        if (first_tile && st == 0 && lane == 0) GEMM2_TRACE(2);
+        seq += PRODUCERS;
+        s += PRODUCERS;
+        if (s >= STAGES) {
+          s -= STAGES;
+          ph ^= 1u;
+        }
+      }
+    };
+    const int source = src.kb_split < num_kb ? TWO_INPUTS : src.im2col ? CONVOLUTION : MATRIX;
     while (ok) {
       for (; st >= num_st; st -= num_st) j++;
       ok = __all_sync(0xffffffffu, *(volatile uint32_t*)&s_error == 0);
@@ -285,59 +349,9 @@ gemm_2sm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
           }
         }
       }
-      for (; st < num_st; st += PRODUCERS) {
-        // Which weights and, in a convolution, which tap and channels the stage takes: worked out before the wait (behind it, 1 % of
-        // a 3x3 convolution).
-        KBlock at[KPS];
-#pragma unroll
-        for (int b = 0; b < KPS; b++) {
-          const int kb = st * KPS + b;
-          at[b].w = kb * BK;
-          if (src.im2col) at[b] = conv_kblock(src, kb);
-        }
-        ok = ptx::mbar_wait_warp(&empty_bar[s], ph ^ 1u);
-        if (!ok) {
-          if (elected) atomicExch(&s_error, GEMM_ERR_PRODUCER_WAIT);
-          break;
-        }
-        const uint32_t full_leader = ptx::mapa_shared(ptx::smem_u32(&full_bar[s]), 0);
-        uint8_t* sa = smem + (size_t)s * STAGE_BYTES;
-        if (first) {
-          // everything above overlaps the kernel before; its results are read below
-          ptx::cluster_wait();
-          if (lane == 0 && warp == 0) GEMM2_TRACE(1);
-          ptx::grid_dep_wait();
-          first = false;
-        }
-        const int blocks = KPS == 1 || st * KPS + 1 < num_kb ? KPS : 1;
-        if (elected && leader) ptx::mbar_expect_tx(&full_bar[s], 2u * KB_BYTES * blocks);
-#pragma unroll
-        for (int b = 0; b < KPS; b++) {
-          if (b >= blocks) break;
-          const int kb = st * KPS + b;
-          if (!src.im2col && kb < src.kb_split) {
-            if (elected) ptx::tma_load_2d_2sm(sa + b * KB_BYTES, &tmap_a, full_leader, kb * BK, row0);
-          } else if (kb < src.kb_split) {
-            if (elected)
-              ptx::tma_load_im2col_2sm(sa + b * KB_BYTES, &tmap_a, full_leader, at[b].c, x * src.stride - src.pad, y * src.stride - src.pad,
-                                       img, at[b].fs, at[b].fr);
-          } else if (src.im2col2) {
-            if (elected)
-              ptx::tma_load_im2col_2sm(sa + b * KB_BYTES, &tmap_a2, full_leader, (kb - src.kb_split) * BK, x * src.stride2, y * src.stride2, img,
-                                       0, 0);
-          } else if (elected) {
-            ptx::tma_load_2d_2sm(sa + b * KB_BYTES, &tmap_a2, full_leader, (kb - src.kb_split) * BK, row0);
-          }
-          if (elected) ptx::tma_load_2d_2sm(sa + b * KB_BYTES + A_BYTES, &tmap_b, full_leader, at[b].w, brow0);
-        }
-        if (j == 0 && st == 0 && lane == 0) GEMM2_TRACE(2);
-        seq += PRODUCERS;
-        s += PRODUCERS;
-        if (s >= STAGES) {
-          s -= STAGES;
-          ph ^= 1u;
-        }
-      }
+      if (source == MATRIX) stages(std::integral_constant<int, MATRIX>{}, row0, brow0, img, y, x, j == 0);
+      else if (source == CONVOLUTION) stages(std::integral_constant<int, CONVOLUTION>{}, row0, brow0, img, y, x, j == 0);
+      else stages(std::integral_constant<int, TWO_INPUTS>{}, row0, brow0, img, y, x, j == 0);
     }
     if (order.late_trigger && warp == 0) {
       __syncwarp();
@@ -734,7 +748,7 @@ cudaError_t launch_2sm(const AInput& in, const void* B, int ldb, int M, int N, i
   o.reverse = K > N;
   o.late_trigger = srpc_gemm_reserved_sms() > 0;
   return launch_pdl(gemm_2sm_kernel<BN, RPC, false>, dim3(2 * o.clusters), dim3(C::THREADS), C::SMEM_BYTES, stream, ta, tb, to, ta2, M,
-                    N, K, o, src, ep, status, TpParams{});
+                    N, K, o, src, ep, status, TpArg<false>{});
 }
 
 cudaError_t launch_shape(int bn, int rows, const AInput& in, const void* B, int ldb, int M, int N, int K, const GemmEpilogue& ep,
