@@ -895,8 +895,10 @@ int srpc_gemm_trace_read(unsigned long long* out, int n) {
 
 // Tile shape: the one with the lowest estimated time, a launch plus rounds of tiles over the SMs (or SM pairs) x (k-blocks x time
 // per k-block + hand-over, more with a residual or GELU).  The figures are a fit to 200 products and convolutions of 49 .. 200704 rows,
-// 8 .. 8192 columns and K 64 .. 8192, each measured with every shape; the choice is within 0.5 % of the best one on average, 9 % at
-// worst.  Pairs win nearly everywhere (us, one-SM against pairs): 128 x 768 x 3072 14.2 against 8.1, 512 x 768 x 768 6.8 and 4.4,
+// 8 .. 8192 columns and K 64 .. 8192, each measured with every shape.  On 1050 others the choice is within 1.2 % of the best one on average, and
+// 15 - 30 % behind where a few rows meet thousands of columns (10 x 4696 x 4720 15.6 us, 128 x 128 tiles 11.7); a fit to those with the
+// producers' present loops (128 x 128 tiles 0.095 us per k-block instead of 0.123) makes that 1.0 %, but ResNet-50 888 -> 899 us.
+// Pairs win nearly everywhere (us, one-SM against pairs): 128 x 768 x 3072 14.2 against 6.8, 512 x 768 x 768 6.8 and 4.4,
 // 4096 x 768 x 768 10.8 and 7.6; the one-SM kernel is left with fp32 and unaligned outputs and with the shapes that stream a
 // residual (srpc_gemm_bf16_v2).  The residual of a 256-wide pair tile hides only behind long k loops, except in the first round
 // (13144 x 1024 x 768 31.5 us, 192 wide 25.4; 9953 x 1024 x 2048 40.2, 192 wide 41.5).  Every shape sums a result's products in the same order, so that a row does not depend on the
