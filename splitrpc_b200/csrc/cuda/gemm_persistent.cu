@@ -388,7 +388,7 @@ gemm_conv_persistent(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
         if (p.reuse) {
           // r filter rows: A a patch row further into the box, B the next filter row of this (filter column, channel block).
           // One unrolled run of MMAs per load group: issuing them was what a 64-wide tile took its time for (56 ns per MMA, 27 now;
-          // 64 images with pairs turned off: 28 x 28 x 128 22.2 -> 20.3 us, 14 x 14 x 256 21.6 -> 18.7; pairs 17.0 and 16.5).
+          // 64 images with pairs turned off: 28 x 28 x 128 22.2 -> 20.3 us, 14 x 14 x 256 21.6 -> 18.7; pairs 13.9 and 15.6).
           const uint32_t sb = p.b_stationary ? panel_lo + (uint32_t)kb * (B_BYTES / 16) : sa + A_BYTES / 16;
           if (elected) {
             if (p.r == 3) {
@@ -1043,9 +1043,9 @@ cudaError_t srpc_conv_bf16_tma(const void* in, const void* weight, const ConvSha
   const bool dense = !cs.in_stub && !cs.in_pix_stride && !cs.in_row_stride && !cs.in_img_stride;
   if (dense && !cs.in2 && cs.r == 1 && cs.s == 1 && cs.stride == 1 && cs.pad == 0)
     return srpc_gemm_bf16_v2(in, cs.cin, weight, cs.cin, cs.n * cs.h * cs.w, cs.cout, cs.cin, ep2, status, stream);
-  // Every other dense convolution goes to pairs: of 745 (filters of 1 to 5 rows, steps of 1 and 2, 7 .. 224 pixels wide, 64 .. 512 channels, 1 .. 64 images)
-  // the one-SM form is 1.34 times slower on average; it is ahead by up to 11 % on a few of the largest (16 x 224 x 224 x 64, 3x3 90 and 83 us; 8 x
-  // 28 x 28 x 512, 5x5 66 and 58), where pairs still gain on what was there before them (105 and 79).
+  // Every other dense convolution goes to pairs: on 745 (filters of 1 to 5 rows, steps of 1 and 2, 7 .. 224 pixels wide, 64 .. 512 channels, 1 .. 64
+  // images) the one-SM form takes 1.5 times as long on average; it is ahead by up to 10 % on a few of the largest (8 x 28 x 28 x 512, 5x5 65 and 60 us;
+  // 32 x 56 x 56, 64 -> 128, 3x3 20.9 and 19.9).
   if (srpc_conv_2sm_eligible(cs, ep2)) {
     const TileShape ts = pick_tile(cs.n * cs.oh * cs.ow, cs.cout, (cs.r * cs.s * cs.cin + (cs.in2 ? cs.cin2 : 0)) / BK, ep2, false, true);
     return srpc_conv_bf16_2sm(in, weight, cs, ts.bn, ts.rows, ep2, status, stream);
